@@ -75,6 +75,72 @@ __device__ __forceinline__ V3 scale_m(M& mm, double s, V3 a) {
   return mk(mm.mul(s, a.x), mm.mul(s, a.y), mm.mul(s, a.z));
 }
 
+__device__ __forceinline__ bool zero3(V3 v) {
+  return ((emu_bits(v.x) | emu_bits(v.y) | emu_bits(v.z)) << 1) == 0;
+}
+
+// The moment update mom += (kr (w_j - w_i)) dt and its rolling clip, decided on
+// the integer pipe for a zero history (signed zeros; a new pair, and every pair
+// after its clip).  Returns false where the arithmetic has to run.
+//   d = w_j - w_i, p = (kr d) dt, m = mom + p.
+// kr = +0: p is the zero of d's sign, m the zero that is negative only when both
+//   are, and the clip leaves it: mom^2 > 0 is false.
+// kr > 0, a spin w_i that is not zero and the operands in the range of the clip's
+//   first case: the clip gives m * (+0), the zero of m's sign.  m = p where d_c
+//   is not zero, and the sum of two zeros where it is; mom^2 > 0 holds when some
+//   d_c is not zero: spin components are zero or at least 2^-200, so d_c is a
+//   multiple of 2^-252, and kr, dt >= 2^-60 keep p^2 above the subnormals; with
+//   every d_c zero the clip changes nothing.
+// The sign of d_c is that of the comparison of its operands; equal operands give
+// +0, except (-0) - (+0) = -0.
+__device__ __forceinline__ bool moment_zero(V3 branch, V3 vrot_i, V3 vrot_j, V3 fn, double kr, double dt, V3& mom) {
+  auto window = [](double x) {
+    const uint32_t e = (uint32_t)(emu_bits(x) >> 52) & 0x7ffu;
+    return e - (1023u - 200u) < 400u || emu_is_zero(x);
+  };
+  auto scale = [](double x) { return (uint32_t)(emu_bits(x) >> 52) - (1023u - 60u) < 120u; };  // positive
+  if (!zero3(mom) || !window(vrot_i.x) || !window(vrot_i.y) || !window(vrot_i.z) || !window(vrot_j.x) ||
+      !window(vrot_j.y) || !window(vrot_j.z) || !scale(dt))
+    return false;
+  const bool rolls = emu_bits(kr) != 0;
+  if (rolls && (!scale(kr) || zero3(vrot_i) || !exp_below(branch.x, 200) || !exp_below(branch.y, 200) ||
+                !exp_below(branch.z, 200) || !exp_below(fn.x, 500) || !exp_below(fn.y, 500) || !exp_below(fn.z, 500)))
+    return false;
+  auto out = [rolls](double wj, double wi, double mo) {
+    const uint64_t uj = emu_bits(wj), ui = emu_bits(wi);
+    const bool eq = uj == ui || ((uj | ui) << 1) == 0;
+    const uint64_t neg = eq ? (uj & ~ui) >> 63 : (emu_key(wj) < emu_key(wi) ? 1ull : 0ull);
+    return emu_double((rolls && !eq ? neg : (neg & emu_sign(mo))) << 63);
+  };
+  mom = mk(out(vrot_j.x, vrot_i.x, mom.x), out(vrot_j.y, vrot_i.y, mom.y), out(vrot_j.z, vrot_i.z, mom.z));
+  return true;
+}
+
+// t + mo; the sums with a zero moment on the integer pipe
+template <class M>
+__device__ __forceinline__ V3 add_moment(M& mm, V3 t, V3 mo) {
+  if (zero3(mo)) {
+    bool a, b, c;
+    const V3 r = mk(emu_add_zero(t.x, emu_sign(mo.x), a), emu_add_zero(t.y, emu_sign(mo.y), b),
+                    emu_add_zero(t.z, emu_sign(mo.z), c));
+    if (a && b && c) return r;
+  }
+  return add_m(mm, t, mo);
+}
+
+// Velocity of a body's point: vel - cross(cpos - pos, vrot).  Without spin the
+// cross product of a finite arm is a zero vector and vel - (+-0) is vel itself,
+// unless a component of vel is -0.
+template <class M>
+__device__ __forceinline__ V3 point_velocity(M& mm, V3 vel, V3 cpos, V3 pos, V3 vrot) {
+  auto plain = [](double x) { return exp_below(x, 1000) && emu_bits(x) != 0x8000000000000000ull; };
+  if (zero3(vrot) && exp_below(cpos.x, 1000) && exp_below(cpos.y, 1000) && exp_below(cpos.z, 1000) &&
+      exp_below(pos.x, 1000) && exp_below(pos.y, 1000) && exp_below(pos.z, 1000) && plain(vel.x) && plain(vel.y) &&
+      plain(vel.z))
+    return vel;
+  return sub_m(mm, vel, cross_m(mm, sub_m(mm, cpos, pos), vrot));
+}
+
 // contact_force_core below with its multiplies through mm, in the same
 // operation order, and the rolling clip through rolling_clip_mur0 (same
 // result); the clip's arithmetic keeps the FP64 pipe.
@@ -95,13 +161,14 @@ __device__ __forceinline__ void contact_force_core_m(M& mm, bool cohesive, doubl
     }
   }
   const double damp = Damp ? meff : mm.mul(mm.twice(hkp.damp_rate), sqrt(mm.mul(hkp.kn, meff)));
-  const V3 contribution_i = sub_m(mm, vel_i, cross_m(mm, sub_m(mm, cpos, pos_i), vrot_i));
-  const V3 contribution_j = sub_m(mm, vel_j, cross_m(mm, sub_m(mm, cpos, pos_j), vrot_j));
+  const V3 contribution_i = point_velocity(mm, vel_i, cpos, pos_i, vrot_i);
+  const V3 contribution_j = point_velocity(mm, vel_j, cpos, pos_j, vrot_j);
   const V3 vel = sub_m(mm, contribution_j, contribution_i);
   const double vn = dot_m(mm, vel, n);
+  const double kd = mm.mul(hkp.kn, dn);
   V3 fn;
   {
-    const double fne = mm.mul(-hkp.kn, dn);
+    const double fne = -kd;  // (-kn) dn: the product with the sign flipped
     const double fnv = mm.mul(damp, vn);
     const double s = mm.add(fnv, fne);
     double nf = emu_gt0(s) ? s : 0;
@@ -118,8 +185,7 @@ __device__ __forceinline__ void contact_force_core_m(M& mm, bool cohesive, doubl
   }
   double threshold_ft;
   if (!cohesive) {
-    const double fne = mm.mul(hkp.kn, dn);
-    threshold_ft = fabs(mm.mul(hkp.mu, fne));
+    threshold_ft = fabs(mm.mul(hkp.mu, kd));
   } else {
     threshold_ft = fabs(mm.mul(hkp.mu, mm.add(dot_m(mm, fn, n), hkp.fc)));
   }
@@ -135,12 +201,13 @@ __device__ __forceinline__ void contact_force_core_m(M& mm, bool cohesive, doubl
     const double F = mm.mul(mm.mul(2.0 * 3.14159265358979323846, reff), hkp.gamma);
     f_i = sub_m(mm, f_i, scale_m(mm, F, n));
   }
-  {
+  const V3 branch = sub_m(mm, cpos, pos_i);
+  if (!moment_zero(branch, vrot_i, vrot_j, fn, hkp.kr, dt, mom_i)) {
     const V3 d = sub_m(mm, vrot_j, vrot_i);
     mom_i = add_m(mm, mom_i, mk(mm.mul(mm.mul(hkp.kr, d.x), dt), mm.mul(mm.mul(hkp.kr, d.y), dt),
                                 mm.mul(mm.mul(hkp.kr, d.z), dt)));
+    rolling_clip_mur0_m(mm, branch, vrot_i, fn, mom_i);
   }
-  rolling_clip_mur0_m(mm, sub_m(mm, cpos, pos_i), vrot_i, fn, mom_i);
 }
 
 // apply_dmt_force (contact_force.hpp:115-127): in contact (dn < 0) and for

@@ -164,13 +164,14 @@ EMU_HD double emu_mulnhalf_nb(double x, bool& bad) {
   return emu_double((z ? u : u - (1ull << 52)) ^ 0x8000000000000000ull);
 }
 
-// x * 2 and x * 0.5 for normal x whose result stays normal: exponent +-1.
-// Both are exact, so the result equals the IEEE product; other inputs take
-// the hardware multiply.
+// x * 2, x * 0.5 and x * -0.5 exactly as the multiply gives them, on the integer
+// pipe: an exponent step for a normal x whose result stays normal, a zero itself
+// (sign adjusted); other inputs take the hardware multiply.
 EMU_HD double emu_mul2(double x) {
   const uint64_t u = emu_bits(x);
   const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
   if (e - 1u < 2045u) return emu_double(u + (1ull << 52));
+  if ((u << 1) == 0) return x;
   return emu_native_mul(x, 2.0);
 }
 
@@ -178,15 +179,16 @@ EMU_HD double emu_mulhalf(double x) {
   const uint64_t u = emu_bits(x);
   const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
   if (e - 2u < 2045u) return emu_double(u - (1ull << 52));
+  if ((u << 1) == 0) return x;
   return emu_native_mul(x, 0.5);
 }
 
-// x * -0.5: the exact halving with the sign flipped, otherwise the hardware
-// multiply by -0.5 (so NaN operands keep the hardware's bits).
+// (NaN operands keep the hardware's bits)
 EMU_HD double emu_mulnhalf(double x) {
   const uint64_t u = emu_bits(x);
   const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
   if (e - 2u < 2045u) return emu_double((u - (1ull << 52)) ^ 0x8000000000000000ull);
+  if ((u << 1) == 0) return emu_double(u ^ 0x8000000000000000ull);
   return emu_native_mul(x, -0.5);
 }
 

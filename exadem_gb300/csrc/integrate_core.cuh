@@ -330,6 +330,25 @@ __device__ __forceinline__ EpiOut epilog_math(R& rm, L& lm, Q4 Q, V3 vrot, V3 I,
   return o;
 }
 
+// Equal principal inertias (every sphere; cubes, regular tetrahedra and
+// octahedra): the Euler terms ((I.z - I.y) omega.y) omega.z are zeros for a
+// finite omega, and M - (+-0) is M itself unless a component of M is -0, so the
+// spin need not be rotated into the body frame.  omega is finite when the
+// quaternion and the spin are moderate (|Q_c| < 2^100, |w_c| < 2^400).
+__device__ __forceinline__ bool moderate(Q4 Q, V3 w) {
+  auto below = [](double x, uint32_t e2) { return ((uint32_t)(emu_bits(x) >> 52) & 0x7ffu) < 1023u + e2; };
+  return below(Q.w, 100) && below(Q.x, 100) && below(Q.y, 100) && below(Q.z, 100) && below(w.x, 400) &&
+         below(w.y, 400) && below(w.z, 400);
+}
+__device__ __forceinline__ bool isotropic(V3 I) {
+  const uint64_t b = emu_bits(I.x);
+  return b == emu_bits(I.y) && b == emu_bits(I.z) && (b >> 52) < 0x7ffu;  // positive, finite
+}
+__device__ __forceinline__ bool no_negative_zero(V3 v) {
+  constexpr uint64_t nz = 0x8000000000000000ull;
+  return emu_bits(v.x) != nz && emu_bits(v.y) != nz && emu_bits(v.z) != nz;
+}
+
 // A particle whose spin and torque are all +0.0 keeps arot = +0 and w = +0
 // bit for bit, provided the quaternion is finite and the inertia and its
 // reciprocal are positive and finite: every product of a quaternion or inertia
@@ -340,10 +359,12 @@ __device__ __forceinline__ EpiOut epilog_math(R& rm, L& lm, Q4 Q, V3 vrot, V3 I,
 // = +0 and w = +0 + (+0 * dt/2) = +0.
 __device__ __forceinline__ bool finite_bits(double x) { return ((emu_bits(x) >> 52) & 0x7ffu) != 0x7ffu; }
 __device__ __forceinline__ bool positive_finite_bits(double x) { return (emu_bits(x) >> 52) < 0x7ffu; }
+// With equal inertias the same holds for any moderate spin: the Euler terms are
+// zeros whatever omega is, arot = +0 and w + (+0) is w (a -0 becomes +0).
 __device__ __forceinline__ bool rotation_idle(Q4 Q, V3 vrot, V3 mom, V3 I, V3 II) {
-  const uint64_t z = emu_bits(vrot.x) | emu_bits(vrot.y) | emu_bits(vrot.z) | emu_bits(mom.x) | emu_bits(mom.y) |
-                     emu_bits(mom.z);
-  return z == 0 && finite_bits(Q.w) && finite_bits(Q.x) && finite_bits(Q.y) && finite_bits(Q.z) &&
+  const uint64_t z = emu_bits(mom.x) | emu_bits(mom.y) | emu_bits(mom.z);
+  const uint64_t zw = emu_bits(vrot.x) | emu_bits(vrot.y) | emu_bits(vrot.z);
+  return z == 0 && (zw == 0 || (isotropic(I) && moderate(Q, vrot))) && finite_bits(Q.w) && finite_bits(Q.x) && finite_bits(Q.y) && finite_bits(Q.z) &&
          positive_finite_bits(I.x) && positive_finite_bits(I.y) && positive_finite_bits(I.z) &&
          positive_finite_bits(II.x) && positive_finite_bits(II.y) && positive_finite_bits(II.z);
 }
@@ -380,12 +401,13 @@ __device__ __forceinline__ void epilog_rotation(const PArrays& P, uint64_t s, do
     const V3 I = mk(P.f[IX][s], P.f[IY][s], P.f[IZ][s]);
     const V3 II = mk(P.f[IIX][s], P.f[IIY][s], P.f[IIZ][s]);
     const Q4 Qinv = {Q.w, -Q.x, -Q.y, -Q.z};
-    const V3 omega = qrotate_m(rm, Qinv, vrot);
-    const V3 M = qrotate_m(rm, Qinv, tq);
-    const double nx = M.x - rm.mul(rm.mul(I.z - I.y, omega.y), omega.z);
-    const double ny = M.y - rm.mul(rm.mul(I.x - I.z, omega.z), omega.x);
-    const double nz = M.z - rm.mul(rm.mul(I.y - I.x, omega.x), omega.y);
-    const V3 domega = mk(div_rn_m(lm, nx, I.x, II.x), div_rn_m(lm, ny, I.y, II.y), div_rn_m(lm, nz, I.z, II.z));
+    V3 N = qrotate_m(rm, Qinv, tq);
+    if (!(isotropic(I) && moderate(Q, vrot) && no_negative_zero(N))) {
+      const V3 omega = qrotate_m(rm, Qinv, vrot);
+      N = mk(N.x - rm.mul(rm.mul(I.z - I.y, omega.y), omega.z), N.y - rm.mul(rm.mul(I.x - I.z, omega.z), omega.x),
+             N.z - rm.mul(rm.mul(I.y - I.x, omega.x), omega.y));
+    }
+    const V3 domega = mk(div_rn_m(lm, N.x, I.x, II.x), div_rn_m(lm, N.y, I.y, II.y), div_rn_m(lm, N.z, I.z, II.z));
     arot = qrotate_m(rm, Q, domega);
     w = mk(vrot.x + lm.mul(arot.x, half_delta_t), vrot.y + lm.mul(arot.y, half_delta_t),
            vrot.z + lm.mul(arot.z, half_delta_t));

@@ -169,7 +169,7 @@ __device__ __forceinline__ int detect_pair(const CArgs& a, uint32_t k, double& d
     if (contact || (a.cohesive && emu_le(dn, dncut)) || a.cs.dn) {  // n and cpos are used only then
       const double inv_dist_norm = 1.0 / dist_norm;
       n = dist * inv_dist_norm;
-      cpos = ri - n * (rad_i + 0.5 * dn);
+      cpos = ri - n * (rad_i + emu_mulhalf(dn));
     }
   } else {
     const DriverDev& d = a.drv[j];
@@ -188,7 +188,7 @@ __device__ __forceinline__ int detect_pair(const CArgs& a, uint32_t k, double& d
       contact = !emu_gt0(dn);
       if (contact) {
         n = s2p / dd;
-        cpos = ri - n * (rad_i + 0.5 * dn);
+        cpos = ri - n * (rad_i + emu_mulhalf(dn));
       }
     } else {
       const V3 proj = ri * mk(d.axis[0], d.axis[1], d.axis[2]);
@@ -198,7 +198,7 @@ __device__ __forceinline__ int detect_pair(const CArgs& a, uint32_t k, double& d
       contact = !emu_gt0(dn);
       if (contact) {
         n = dir / dd;
-        cpos = ri - n * (rad_i + 0.5 * dn);
+        cpos = ri - n * (rad_i + emu_mulhalf(dn));
       }
     }
     dncut = a.pt.drv(a.cpd, a.P.group[i], j).dncut;
@@ -230,9 +230,10 @@ __device__ __forceinline__ void attract_pair(const CArgs& a, uint32_t k, double 
       is_vv ? a.pt.pair(a.cp, a.P.group[i], a.P.group[j]) : a.pt.drv(a.cpd, a.P.group[i], j);
   const double fn_value = (hkp.fc / hkp.dncut) * dn - hkp.fc;
   const V3 f = mk(0, 0, 0) + fn_value * n;
-  const V3 ti = cross(cpos - ri, f) + mo;
+  MulFP64 mm;
+  const V3 ti = add_moment(mm, cross(cpos - ri, f), mo);
   V3 tj = mk(0, 0, 0);
-  if (is_vv) tj = cross(cpos - partner_pos(a, meta, i, j), -f) + (-mo);
+  if (is_vv) tj = add_moment(mm, cross(cpos - partner_pos(a, meta, i, j), -f), -mo);
   write_result(a, k, mk(0, 0, 0), mo, f, ti, tj);
   a.R.live[k] = 1;
   a.cs.write(k, dn, cpos, f - mk(0, 0, 0), mk(0, 0, 0));  // ft = 0 before contact
@@ -297,8 +298,8 @@ __device__ __forceinline__ void hooke_run(M& mm, const CArgs& a, uint32_t k, dou
     const dem_contact_params& cp = a.pt.pair(a.cp, a.P.group[i], a.P.group[j]);
     contact_force_core_m<M, true>(mm, a.cohesive, dn, n, a.dt, cp, a.I.damp[k], ft, cpos, ri, vi, f, mo, wi, rj,
                                   vj, wj, a.dmt, reff);
-    ti = add_m(mm, cross_m(mm, sub_m(mm, cpos, ri), f), mo);
-    tj = add_m(mm, cross_m(mm, sub_m(mm, cpos, rj), -f), -mo);
+    ti = add_moment(mm, cross_m(mm, sub_m(mm, cpos, ri), f), mo);
+    tj = add_moment(mm, cross_m(mm, sub_m(mm, cpos, rj), -f), -mo);
   } else {
     const DriverDev& d = a.drv[j];
     const V3 dpos = mk(d.center[0], d.center[1], d.center[2]);
@@ -307,7 +308,7 @@ __device__ __forceinline__ void hooke_run(M& mm, const CArgs& a, uint32_t k, dou
     const dem_contact_params& cpd = a.pt.drv(a.cpd, a.P.group[i], j);
     contact_force_core_m<M, true>(mm, a.cohesive, dn, n, a.dt, cpd, a.I.damp[k], ft, cpos, ri, vi, f, mo, wi, dpos,
                                   dvel, dvrot, a.dmt, a.P.f[RAD][i]);
-    ti = add_m(mm, cross_m(mm, sub_m(mm, cpos, ri), f), mo);
+    ti = add_moment(mm, cross_m(mm, sub_m(mm, cpos, ri), f), mo);
   }
 }
 
@@ -378,6 +379,10 @@ __device__ __forceinline__ void run_queued(const CArgs& a, int q, uint32_t idx, 
 // pair is computed exactly as by k_cdetect + k_chooke and writes only its own
 // records: the same bits.  The overlapping pairs are counted into *n_active
 // (zeroed by the launcher).
+// Bound by the FP64 pipe (about 190 instructions per overlapping pair before, 160
+// with the moment update and its clip, the sums with a zero moment and the spin
+// of a resting partner decided on the integer pipe): with the same decisions in
+// the epilog and the trigger a step of the 2 M bed went from 3.62 to 3.23 ms.
 // IntTiles: the instance with the integer-pipe tiles (int_share > 0); it needs
 // more registers, so the FP64-only instance stays the lean one.
 template <int Mode, bool IntTiles>
@@ -450,6 +455,34 @@ __global__ void __launch_bounds__(FT, (Mode ? 4 : (IntTiles ? 3 : 1))) k_cfused(
   if (t == 0 && q_tot) atomicAdd(a.n_active, (unsigned long long)q_tot);
 }
 
+// |r - b|^2 >= thr2.  Where the coordinates of r and b have the same sign and
+// exponent their difference is the exact difference of the significands: three
+// FP32 roundings of relative 2^-24 each give the sum of squares to 2^-21, and
+// outside the band of 2^-16 the comparison is the FP64 one, whose own sum is
+// good to 2^-51.  Inside it, and across a power of two, the FP64 pipe decides.
+__device__ __forceinline__ bool displ_over(V3 r, V3 b, double thr2) {
+  float s = 0.f;
+  bool ok = true;
+  auto part = [&](double x, double y) {
+    const uint64_t ux = emu_bits(x), uy = emu_bits(y);
+    const uint32_t e = (uint32_t)(ux >> 52) & 0x7ffu;
+    ok = ok && ((ux ^ uy) >> 52) == 0 && e - (1075u - 100u) < 160u;  // |x| in [2^-48, 2^112)
+    const float d = (float)(int64_t)(ux - uy) * __uint_as_float((e - 1075u + 127u) << 23);
+    s = s + d * d;
+  };
+  part(r.x, b.x);
+  part(r.y, b.y);
+  part(r.z, b.z);
+  const uint32_t et = (uint32_t)(emu_bits(thr2) >> 52);  // positive, far from the FP32 limits
+  if (ok && et - (1023u - 60u) < 120u) {
+    const float t = __double2float_rn(thr2);
+    if (s < t * 0.99998f) return false;
+    if (s > t * 1.00002f) return true;
+  }
+  const double dx = r.x - b.x, dy = r.y - b.y, dz = r.z - b.z;
+  return emu_ge_nonneg(dx * dx + dy * dy + dz * dz, thr2);  // >= on the integer pipe
+}
+
 // prolog + displacement trigger.  Every particle gets its translation and, when
 // it does not spin, its (exact, integer sign logic) quaternion step here; the
 // spinning particles run the full quaternion update in place when most of their
@@ -466,8 +499,7 @@ __global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_fused_prolog(PArrays P,
   bool over = false, need = false;
   if (s < n) {
     need = prolog_cheap<Mode>(P, s, delta_t, half_delta_t, delta_t2_2);
-    const double dx = P.f[RX][s] - P.f[BX][s], dy = P.f[RY][s] - P.f[BY][s], dz = P.f[RZ][s] - P.f[BZ][s];
-    over = emu_ge_nonneg(dx * dx + dy * dy + dz * dz, thr2);  // >= on the integer pipe
+    over = displ_over(mk(P.f[RX][s], P.f[RY][s], P.f[RZ][s]), mk(P.f[BX][s], P.f[BY][s], P.f[BZ][s]), thr2);
     if (over && sv.nsys > 1) atomicOr(&sv.trig[sv.of(s)], 1u);  // this system's own trigger
   }
   if (__any_sync(0xffffffffu, over) && (threadIdx.x & 31) == 0) atomicOr(flag, 1ull);
@@ -573,16 +605,19 @@ __global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_fused_epilog(PArrays P,
     P.f[VZ][s] = v.z;
     const V3 vrot = mk(P.f[WX][s], P.f[WY][s], P.f[WZ][s]);
     need = true;
-    if (((emu_bits(vrot.x) | emu_bits(vrot.y) | emu_bits(vrot.z) | emu_bits(mom.x) | emu_bits(mom.y) |
-          emu_bits(mom.z))) == 0) {
+    if ((emu_bits(mom.x) | emu_bits(mom.y) | emu_bits(mom.z)) == 0) {
       const Q4 Q = {P.f[QW][s], P.f[QX][s], P.f[QY][s], P.f[QZ][s]};
       const V3 I = mk(P.f[IX][s], P.f[IY][s], P.f[IZ][s]);
       const V3 II = mk(P.f[IIX][s], P.f[IIY][s], P.f[IIZ][s]);
       if (rotation_idle(Q, vrot, mom, I, II)) {
         need = false;
-        P.f[AX][s] = 0.0;  // w stays +0
+        P.f[AX][s] = 0.0;
         P.f[AY][s] = 0.0;
         P.f[AZ][s] = 0.0;
+        // w + (+0): w itself, +0 for a -0
+        if (emu_bits(vrot.x) == 0x8000000000000000ull) P.f[WX][s] = 0.0;
+        if (emu_bits(vrot.y) == 0x8000000000000000ull) P.f[WY][s] = 0.0;
+        if (emu_bits(vrot.z) == 0x8000000000000000ull) P.f[WZ][s] = 0.0;
       }
     }
   }

@@ -18,9 +18,10 @@ struct MulFP64 {
   __device__ __forceinline__ double mul(double a, double b) const { return __dmul_rn(a, b); }
   __device__ __forceinline__ double add(double a, double b) const { return __dadd_rn(a, b); }
   __device__ __forceinline__ double sub(double a, double b) const { return __dsub_rn(a, b); }
-  __device__ __forceinline__ double twice(double a) const { return __dmul_rn(a, 2.0); }
-  __device__ __forceinline__ double half(double a) const { return __dmul_rn(a, 0.5); }
-  __device__ __forceinline__ double neghalf(double a) const { return __dmul_rn(a, -0.5); }
+  // powers of two: an exponent step on the integer pipe, the multiply's bits
+  __device__ __forceinline__ double twice(double a) const { return emu_mul2(a); }
+  __device__ __forceinline__ double half(double a) const { return emu_mulhalf(a); }
+  __device__ __forceinline__ double neghalf(double a) const { return emu_mulnhalf(a); }
   __device__ __forceinline__ bool failed() const { return false; }
 };
 struct MulInt {
