@@ -18,6 +18,8 @@
 //    are one kernel, prolog + displacement trigger another.
 // Order of summation, operation order and rounding are those of the operator
 // kernels (contact_core.cuh, integrate_core.cuh).
+#include <algorithm>
+
 #include "contact_core.cuh"
 #include "integrate_core.cuh"
 #include "mesh_core.cuh"
@@ -56,6 +58,7 @@ struct CArgs {
   ParamTable pt;  // multi-material parameters (pt.pp == nullptr: cp / cpd)
   ContactStateArrays cs;  // analysis (cs.dn == nullptr: off)
   int screen;
+  float dncut_f;  // config.dncut in FP32 (not below 0)
   uint32_t* L1;
   uint32_t* L2;
   double* D[7];  // dn, n(3), cp(3) of the L2 entries
@@ -103,6 +106,35 @@ __device__ __forceinline__ V3 partner_pos(const CArgs& a, uint32_t meta, uint32_
   return rj;
 }
 
+// |a - b| for finite a, b in FP32 without the FP64 pipe: the significands aligned to
+// the larger exponent (bits of the smaller operand below the larger one's last are
+// dropped: an error of at most 2^-52 of the larger operand) and subtracted as
+// integers, the magnitude rounded to FP32 in two halves (relative 2^-22) and scaled
+// by the power of two.  ok is cleared outside [2^-48, 2^112) (zeros aside); top
+// becomes the largest biased exponent met.
+__device__ __forceinline__ float diff_f32(double a, double b, bool& ok, uint32_t& top) {
+  const uint64_t ua = emu_bits(a), ub = emu_bits(b);
+  const uint32_t ea = (uint32_t)(ua >> 52) & 0x7ffu, eb = (uint32_t)(ub >> 52) & 0x7ffu;
+  const uint32_t e = ea > eb ? ea : eb;
+  const uint64_t frac = 0xfffffffffffffull;
+  const uint32_t sa = e - ea, sb = e - eb;
+  const int64_t ma = sa < 64u ? (int64_t)(((ua & frac) | (1ull << 52)) >> sa) : 0;
+  const int64_t mb = sb < 64u ? (int64_t)(((ub & frac) | (1ull << 52)) >> sb) : 0;
+  const int64_t d = ((int64_t)(ua ^ ub) < 0) ? ma + mb : ma - mb;
+  const uint64_t m = (uint64_t)(d < 0 ? -d : d);
+  ok = ok && e - (1075u - 100u) < 160u;
+  top = top > e ? top : e;
+  const float f = (float)(uint32_t)(m >> 32) * 4294967296.f + (float)(uint32_t)m;
+  return f * __uint_as_float((e - 1075u + 127u) << 23);
+}
+// x > 0 cut to FP32 on the integer pipe (relative error below 2^-23, downwards)
+__device__ __forceinline__ float trunc_f32(double x, bool& ok) {
+  const uint64_t u = emu_bits(x);
+  const uint32_t e = (uint32_t)(u >> 52);
+  ok = ok && e - (1023u - 100u) < 200u;
+  return __uint_as_float(((e - 1023u + 127u) << 23) | ((uint32_t)(u >> 29) & 0x7fffffu));
+}
+
 __global__ void __launch_bounds__(FT) k_cscreen(CArgs a) {
   const uint64_t ni = a.ni_dev ? *a.ni_dev : a.ni;
   const uint64_t stride = (uint64_t)gridDim.x * FT;
@@ -117,14 +149,22 @@ __global__ void __launch_bounds__(FT) k_cscreen(CArgs a) {
       const uint32_t i = a.I.owner[k], j = a.I.partner[k];
       const V3 ri = ldv(a.P, RX, i);
       const V3 rj = partner_pos(a, meta, i, j);
-      const double rad_i = a.P.f[RAD][i], rad_j = a.P.f[RAD][j];
-      // same proof of separation as the one-pass kernel (k_contact_sphere.cu)
-      const float ex = (float)(ri.x - rj.x), ey = (float)(ri.y - rj.y), ez = (float)(ri.z - rj.z);
+      // the proof of separation of the one-pass kernel (k_contact_sphere.cu) without
+      // its FP64 instructions (six conversions and six additions a pair, 870 of a
+      // warp's cycles): differences from the significands, good to 2^-22, and radii
+      // rounded on the integer pipe, good to 2^-23, within the margin of 2^-17.
+      bool ok = true;
+      uint32_t top = 0;
+      const float ex = diff_f32(ri.x, rj.x, ok, top), ey = diff_f32(ri.y, rj.y, ok, top),
+                  ez = diff_f32(ri.z, rj.z, ok, top);
       const float d2f = ex * ex + ey * ey + ez * ez;
-      const double lim =
-          rad_i + rad_j + (a.cohesive ? fmax(a.pt.pair(a.cp, a.P.group[i], a.P.group[j]).dncut, 0.0) : 0.0);
-      const float limf = (float)lim;
-      if (lim > 1e-15 && lim < 1e15 && d2f > limf * limf * 1.0000039f) {
+      const float dncut = a.cohesive ? (a.pt.pp ? fmaxf((float)a.pt.pair(a.cp, a.P.group[i], a.P.group[j]).dncut, 0.f)
+                                                : a.dncut_f)
+                                     : 0.f;
+      const float limf = trunc_f32(a.P.f[RAD][i], ok) + trunc_f32(a.P.f[RAD][j], ok) + dncut;
+      // 2^28 lim above the coordinates: what diff_f32 drops is below 2^-24 of lim
+      ok = ok && top < (__float_as_uint(limf) >> 23) - 127u + 1023u + 28u;
+      if (ok && limf > 1e-15f && limf < 1e15f && d2f > limf * limf * 1.0000077f) {
         want = false;
         if (a.R.live[k]) {  // not yet zero: reset history and record once
           const V3 z = mk(0, 0, 0);
@@ -455,29 +495,20 @@ __global__ void __launch_bounds__(FT, (Mode ? 4 : (IntTiles ? 3 : 1))) k_cfused(
   if (t == 0 && q_tot) atomicAdd(a.n_active, (unsigned long long)q_tot);
 }
 
-// |r - b|^2 >= thr2.  Where the coordinates of r and b have the same sign and
-// exponent their difference is the exact difference of the significands: three
-// FP32 roundings of relative 2^-24 each give the sum of squares to 2^-21, and
-// outside the band of 2^-16 the comparison is the FP64 one, whose own sum is
-// good to 2^-51.  Inside it, and across a power of two, the FP64 pipe decides.
-__device__ __forceinline__ bool displ_over(V3 r, V3 b, double thr2) {
-  float s = 0.f;
-  bool ok = true;
-  auto part = [&](double x, double y) {
-    const uint64_t ux = emu_bits(x), uy = emu_bits(y);
-    const uint32_t e = (uint32_t)(ux >> 52) & 0x7ffu;
-    ok = ok && ((ux ^ uy) >> 52) == 0 && e - (1075u - 100u) < 160u;  // |x| in [2^-48, 2^112)
-    const float d = (float)(int64_t)(ux - uy) * __uint_as_float((e - 1075u + 127u) << 23);
-    s = s + d * d;
-  };
-  part(r.x, b.x);
-  part(r.y, b.y);
-  part(r.z, b.z);
-  const uint32_t et = (uint32_t)(emu_bits(thr2) >> 52);  // positive, far from the FP32 limits
-  if (ok && et - (1023u - 60u) < 120u) {
-    const float t = __double2float_rn(thr2);
-    if (s < t * 0.99998f) return false;
-    if (s > t * 1.00002f) return true;
+// |r - b|^2 >= thr2, decided from FP32 differences (diff_f32) outside a band of
+// 2^-15 about the threshold: their error is 2^-23 of the difference and 2^-52 of the
+// coordinate, which the lower bound on the threshold keeps below 2^-20 of it.
+// Inside the band, or for a skin below 2^-30 of a coordinate, the FP64 pipe decides.
+__device__ __forceinline__ bool displ_over(V3 r, V3 b, double thr2, float thr2f) {
+  bool ok = thr2f > 1e-30f && thr2f < 1e30f;
+  uint32_t top = 0;
+  const float ex = diff_f32(r.x, b.x, ok, top), ey = diff_f32(r.y, b.y, ok, top), ez = diff_f32(r.z, b.z, ok, top);
+  const float s = ex * ex + ey * ey + ez * ez;
+  // 2^(top - 1022) bounds the coordinates; sqrt(thr2) >= 2^-30 of it
+  const int et = (int)(__float_as_uint(thr2f) >> 23) - 127;
+  if (ok && et >= 2 * ((int)top - 1022 - 30)) {
+    if (s < thr2f * 0.99997f) return false;
+    if (s > thr2f * 1.00003f) return true;
   }
   const double dx = r.x - b.x, dy = r.y - b.y, dz = r.z - b.z;
   return emu_ge_nonneg(dx * dx + dy * dy + dz * dz, thr2);  // >= on the integer pipe
@@ -492,19 +523,20 @@ __device__ __forceinline__ bool displ_over(V3 r, V3 b, double thr2) {
 template <int Mode>
 __global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_fused_prolog(PArrays P, uint64_t n, double delta_t,
                                                                      double half_delta_t, double delta_t2_2,
-                                                                     double thr2, unsigned long long* flag,
+                                                                     double thr2, float thr2f, unsigned long long* flag,
                                                                      SysView sv, uint32_t* prl_list,
-                                                                     unsigned long long* prl_cnt) {
+                                                                     unsigned long long* prl_cnt, int dense) {
   const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   bool over = false, need = false;
   if (s < n) {
     need = prolog_cheap<Mode>(P, s, delta_t, half_delta_t, delta_t2_2);
-    over = displ_over(mk(P.f[RX][s], P.f[RY][s], P.f[RZ][s]), mk(P.f[BX][s], P.f[BY][s], P.f[BZ][s]), thr2);
+    over = displ_over(mk(P.f[RX][s], P.f[RY][s], P.f[RZ][s]), mk(P.f[BX][s], P.f[BY][s], P.f[BZ][s]), thr2,
+                       thr2f);
     if (over && sv.nsys > 1) atomicOr(&sv.trig[sv.of(s)], 1u);  // this system's own trigger
   }
   if (__any_sync(0xffffffffu, over) && (threadIdx.x & 31) == 0) atomicOr(flag, 1ull);
   const unsigned busy = __ballot_sync(0xffffffffu, need);
-  if (__popc(busy) > 24) {
+  if (__popc(busy) > dense) {
     if (need) prolog_rotation<Mode>(P, s, delta_t, half_delta_t);
   } else {
     const uint32_t pos = warp_append(need, prl_cnt);
@@ -538,7 +570,7 @@ __global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_fused_epilog(PArrays P,
                                                                      const uint32_t* __restrict__ rev_idx,
                                                                      double gx, double gy, double gz,
                                                                      double half_delta_t, uint32_t* rot_list,
-                                                                     unsigned long long* rot_cnt) {
+                                                                     unsigned long long* rot_cnt, int dense) {
   const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   bool need = false;
   V3 mom = mk(0.0, 0.0, 0.0);
@@ -622,7 +654,7 @@ __global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_fused_epilog(PArrays P,
     }
   }
   const unsigned busy = __ballot_sync(0xffffffffu, need);
-  if (__popc(busy) > 24) {
+  if (__popc(busy) > dense) {
     if (need) epilog_rotation<Mode>(P, s, half_delta_t, mom);
   } else {
     const uint32_t pos = warp_append(need, rot_cnt);
@@ -661,6 +693,7 @@ CArgs make_cargs(dem_ctx* c) {
   a.pt = c->ptable();
   a.cs = c->cs;
   a.screen = c->prm.fp32_contact_screen && !c->analysis;  // analysis: every pair's state
+  a.dncut_f = (float)std::max(c->prm.config.dncut, 0.0);
   a.L1 = c->L1;
   a.L2 = c->L2;
   for (int q = 0; q < 7; q++) a.D[q] = c->Dscr[q];
@@ -672,24 +705,40 @@ CArgs make_cargs(dem_ctx* c) {
 }
 }  // namespace
 
+// Lanes of a warp above which the rotations run in place.  While the particles give
+// every scheduler at most one warp (32 lanes a scheduler, four schedulers an SM) the
+// FP64 pipes wait for that warp alone, so a list only adds a second pass over it:
+// every rotation in place and no list kernel (9 + 5 us of the 10 k box's 90 us
+// step).  With more warps a sparse one keeps its pipe from the next, and more than 24
+// lanes pay for the pass.
+static int rotation_dense(const dem_ctx* c) { return c->n <= (uint64_t)c->num_sms * 128u ? 0 : 24; }
+// Threads per block of the prolog and the epilog: the tuned size, halved while the
+// grid leaves SMs without a block (at 10 k particles 256 threads reach 40 SMs).
+static unsigned particle_block(const dem_ctx* c) {
+  unsigned b = (unsigned)c->tune_block;
+  while (b > 32u && c->n < (uint64_t)b * (uint64_t)c->num_sms) b >>= 1;
+  return b;
+}
+
 int launch_fused_prolog(dem_ctx* c) {
   const double delta_t = c->prm.dt;
   const double half_delta_t = delta_t * 0.5;
   const double delta_t2_2 = delta_t * delta_t * 0.5;
   const double max_displ = c->prm.rcut_inc * 0.5;
+  const int dense = rotation_dense(c);
+  const unsigned block = particle_block(c);
   DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars, 0, sizeof(unsigned long long), c->stream));
   unsigned long long* prl_cnt = c->d_scalars + SC_ROT_CNT;  // the rotation list is free until the epilog
-  DEM_CUDA_TRY(c, cudaMemsetAsync(prl_cnt, 0, sizeof(unsigned long long), c->stream));
-  ProfScope ps(c, K_PROLOG, c->n ? 2 : 0);
+  if (dense) DEM_CUDA_TRY(c, cudaMemsetAsync(prl_cnt, 0, sizeof(unsigned long long), c->stream));
+  ProfScope ps(c, K_PROLOG, c->n ? (dense ? 2 : 1) : 0);
   const auto kern = by_mode(c->mul_mode, k_fused_prolog<0>, k_fused_prolog<1>, k_fused_prolog<2>, k_fused_prolog<3>);
   const auto krot = by_mode(c->mul_mode, k_prolog_rotation<0>, k_prolog_rotation<1>, k_prolog_rotation<2>,
                             k_prolog_rotation<3>);
   if (c->n) {
-    kern<<<grid_for(c->n, c->tune_block), c->tune_block, 0, c->stream>>>(c->P[c->pcur], c->n, delta_t, half_delta_t,
-                                                                         delta_t2_2, max_displ * max_displ,
-                                                                         c->d_scalars, c->sysview(), c->rot_list,
-                                                                         prl_cnt);
-    krot<<<(unsigned)c->num_sms * 3, 256, 0, c->stream>>>(c->P[c->pcur], c->rot_list, prl_cnt, delta_t,
+    kern<<<grid_for(c->n, block), block, 0, c->stream>>>(c->P[c->pcur], c->n, delta_t, half_delta_t, delta_t2_2,
+                                                         max_displ * max_displ, (float)(max_displ * max_displ), c->d_scalars, c->sysview(),
+                                                         c->rot_list, prl_cnt, dense);
+    if (dense) krot<<<(unsigned)c->num_sms * 3, 256, 0, c->stream>>>(c->P[c->pcur], c->rot_list, prl_cnt, delta_t,
                                                             half_delta_t);
   }
   DEM_CUDA_TRY(c, cudaGetLastError());
@@ -729,17 +778,19 @@ int launch_contact_compact(dem_ctx* c) {
 }
 
 int launch_fused_epilog(dem_ctx* c) {
-  ProfScope ps(c, K_EPILOG, c->n ? 2 : 0);
+  const int dense = rotation_dense(c);
+  const unsigned block = particle_block(c);
+  ProfScope ps(c, K_EPILOG, c->n ? (dense ? 2 : 1) : 0);
   const auto kern = by_mode(c->mul_mode, k_fused_epilog<0>, k_fused_epilog<1>, k_fused_epilog<2>, k_fused_epilog<3>);
   const auto krot = by_mode(c->mul_mode, k_epilog_rotation<0>, k_epilog_rotation<1>, k_epilog_rotation<2>,
                             k_epilog_rotation<3>);
   unsigned long long* rot_cnt = c->d_scalars + SC_ROT_CNT;
-  DEM_CUDA_TRY(c, cudaMemsetAsync(rot_cnt, 0, sizeof(unsigned long long), c->stream));
+  if (dense) DEM_CUDA_TRY(c, cudaMemsetAsync(rot_cnt, 0, sizeof(unsigned long long), c->stream));
   if (c->n) {
-    kern<<<grid_for(c->n, c->tune_block), c->tune_block, 0, c->stream>>>(
+    kern<<<grid_for(c->n, block), block, 0, c->stream>>>(
         c->P[c->pcur], c->R, c->n, c->own_off[c->icur], c->rev_off, c->rev_idx, c->prm.gravity[0],
-        c->prm.gravity[1], c->prm.gravity[2], c->prm.dt * 0.5, c->rot_list, rot_cnt);
-    krot<<<(unsigned)c->num_sms * 3, 256, 0, c->stream>>>(c->P[c->pcur], c->rot_list, rot_cnt, c->prm.dt * 0.5);
+        c->prm.gravity[1], c->prm.gravity[2], c->prm.dt * 0.5, c->rot_list, rot_cnt, dense);
+    if (dense) krot<<<(unsigned)c->num_sms * 3, 256, 0, c->stream>>>(c->P[c->pcur], c->rot_list, rot_cnt, c->prm.dt * 0.5);
   }
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;
