@@ -79,23 +79,19 @@ int alloc_particles(dem_ctx* c, uint64_t n) {
   cudaFree(c->srec);
   cudaFree(c->rev_off);
   cudaFree(c->rev_cnt);
-  cudaFree(c->rev_nlong);
   cudaFree(c->own_off[0]);
   cudaFree(c->own_off[1]);
   DEM_CUDA_TRY(c, cudaMalloc(&c->cell_of, cap * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->cell_tmp, cap * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->perm, cap * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->pcnt, (cap + 1) * 4));
-  DEM_CUDA_TRY(c, cudaMalloc(&c->srec, cap * 16 * 4));
+  DEM_CUDA_TRY(c, cudaMalloc(&c->srec, cap * 16 * sizeof(uint4)));
   DEM_CUDA_TRY(c, cudaMalloc(&c->rev_off, (cap + 1) * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->rev_cnt, (cap + 1) * 4));
-  DEM_CUDA_TRY(c, cudaMalloc(&c->rev_nlong, sizeof(unsigned int)));
   DEM_CUDA_TRY(c, cudaMalloc(&c->own_off[0], (cap + 1) * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->own_off[1], (cap + 1) * 4));
-  for (int q = 0; q < 4; q++) {
-    cudaFree(c->crel[q]);
-    DEM_CUDA_TRY(c, cudaMalloc(&c->crel[q], cap * sizeof(float)));
-  }
+  cudaFree(c->crel);
+  DEM_CUDA_TRY(c, cudaMalloc(&c->crel, cap * sizeof(float4)));
   cudaFree(c->rot_list);
   DEM_CUDA_TRY(c, cudaMalloc(&c->rot_list, cap * 4));
   c->pcap = cap;
@@ -234,6 +230,16 @@ static int make_grid(dem_ctx* c, const double* lo, const double* hi, const int32
     } else {
       g.dims[d] = std::max(1, (int)std::ceil(g.L[d] / cs));
       g.csz[d] = cs;
+    }
+    g.lof[d] = (float)g.lo[d];
+    g.csf[d] = (float)g.csz[d];
+    g.icsz[d] = (float)(1.0 / g.csz[d]);
+    g.cmaxf = std::max(g.cmaxf, g.csf[d]);
+    if (d < 2 && g.dims[d] > 1) {
+      uint32_t l = 0;
+      while ((1ull << l) < (uint64_t)g.dims[d]) l++;
+      g.dmul[d] = (uint32_t)(((1ull << (31 + l)) + (uint64_t)g.dims[d] - 1) / (uint64_t)g.dims[d]);
+      g.dshift[d] = l - 1;
     }
     nc *= (uint64_t)g.dims[d];
   }
@@ -500,7 +506,7 @@ int update_neighbors(dem_ctx* c) {
   c->ni = total;
   c->have_list = true;
   c->hist_valid = true;
-  if ((rc = launch_reverse_lists(c))) return rc;
+  if ((rc = launch_reverse_lists(c, fill_counts_partners(c)))) return rc;
   if ((rc = mark_records_live(c))) return rc;  // new list indices: every record is stale
   DEM_CUDA_TRY(c, cudaMemsetAsync(c->trig_dev, 0, c->nsys * sizeof(uint32_t), c->stream));
   c->rebuilds++;
@@ -662,7 +668,6 @@ int dem_ctx_destroy(dem_ctx* c) {
   free_bonds(c);
   cudaFree(c->shapes_dev);
   cudaFree(c->rev_off);
-  cudaFree(c->rev_nlong);
   cudaFree(c->rev_cnt);
   cudaFree(c->cell_cnt);
   cudaFree(c->cell_start);
@@ -671,7 +676,7 @@ int dem_ctx_destroy(dem_ctx* c) {
   cudaFree(c->perm);
   cudaFree(c->srec);
   cudaFree(c->pcnt);
-  for (int q = 0; q < 4; q++) cudaFree(c->crel[q]);
+  cudaFree(c->crel);
   cudaFree(c->rot_list);
   cudaFree(c->scan_blk);
   cudaFree(c->d_scalars);
@@ -856,6 +861,20 @@ static int add_driver(dem_ctx* c, const DriverDev& d) {
   if (c->ndrv >= DEM_MAX_DRIVERS) return c->fail(DEM_ERR_INVALID_ARG, "too many drivers");
   c->gen++;
   c->drv_host[c->ndrv] = d;
+  {
+    DriverDev& h = c->drv_host[c->ndrv];
+    auto sum = [](const double* v) { return (float)(std::fabs(v[0]) + std::fabs(v[1]) + std::fabs(v[2])); };
+    for (int k = 0; k < 3; k++) {
+      h.nf[k] = (float)d.normal[k];
+      h.cpf[k] = (float)d.center_proj[k];
+      h.af[k] = (float)d.axis[k];
+      h.cf[k] = (float)d.center[k];
+    }
+    h.rf = (float)d.radius;
+    h.n1 = sum(d.normal);
+    h.cp1 = sum(d.center_proj);
+    h.c1 = sum(d.center);
+  }
   DEM_CUDA_TRY(c, cudaMemcpyAsync(c->drv_dev + c->ndrv, &c->drv_host[c->ndrv], sizeof(DriverDev),
                                   cudaMemcpyHostToDevice, c->stream));
   DEM_CUDA_TRY(c, cudaStreamSynchronize(c->stream));

@@ -116,8 +116,8 @@ struct dem_ctx {
   uint32_t* cell_tmp = nullptr;    // n, cell of each particle in the old order
   uint32_t* perm = nullptr;        // n, new slot -> old slot
   uint32_t* pcnt = nullptr;        // n+1 candidate counts (then offsets)
-  uint32_t* srec = nullptr;        // spheres: 8 (partner, meta) candidates per particle from the count pass
-  float* crel[4] = {};             // n each: cell-relative x, y, z and radius in FP32 (broad phase)
+  uint32_t* srec = nullptr;        // spheres: 16 (partner, meta, partner id) candidates per particle from the count pass
+  float4* crel = nullptr;          // n: cell-relative x, y, z and radius in FP32 (broad phase)
 
   // interactions (double-buffered for the history carry-over)
   uint64_t ni = 0;
@@ -131,7 +131,6 @@ struct dem_ctx {
   dem::Records R{};
   uint32_t* rev_off = nullptr;  // n+1
   uint32_t* rev_cnt = nullptr;  // n+1
-  unsigned int* rev_nlong = nullptr;  // reverse lists too long for a thread (k_rev_short -> k_rev_rank)
   uint32_t* rev_idx = nullptr;  // rcap
   // compacted contact passes (rcap each): work lists and detection results
   uint32_t* L1 = nullptr;
@@ -292,7 +291,8 @@ int refresh_pair_damp(dem_ctx* c);  // k_neigh_sphere.cu
 int mark_records_live(dem_ctx* c);  // dem_api.cu
 int ext_ensure_contact_state(dem_ctx* c);  // dem_api.cu: analysis arrays of the records' capacity
 int launch_fill_sphere(dem_ctx* c, uint32_t* new_off, uint64_t total);
-int launch_reverse_lists(dem_ctx* c);
+int launch_reverse_lists(dem_ctx* c, bool counted = false);
+bool fill_counts_partners(const dem_ctx* c);
 // k_mesh.cu: bins of the mesh drivers for the current radius bound and skin
 int ensure_mesh_bins(dem_ctx* c);
 void free_meshes(dem_ctx* c);

@@ -26,7 +26,7 @@ int launch_bin_particles(dem_ctx* c);
 int launch_reorder_particles(dem_ctx* c);
 int launch_count_sphere(dem_ctx* c);
 int launch_fill_sphere(dem_ctx* c, uint32_t* new_off, uint64_t total);
-int launch_reverse_lists(dem_ctx* c);
+
 int launch_fused_prolog(dem_ctx* c);
 int launch_contact_compact(dem_ctx* c);
 int launch_fused_epilog(dem_ctx* c);
@@ -129,7 +129,7 @@ int rebuild_body(dem_ctx* c) {
   k_graph_copy_list<<<(unsigned)c->num_sms * 4u, 256, 0, c->stream>>>(c->I[0], c->I[1], c->own_off[1], c->own_off[0],
                                                                        n, c->d_gs);
   DEM_CUDA_TRY(c, cudaGetLastError());
-  if ((rc = launch_reverse_lists(c))) return rc;
+  if ((rc = launch_reverse_lists(c, fill_counts_partners(c)))) return rc;
   if ((rc = mark_records_live(c))) return rc;  // new list indices: every record is stale
   DEM_CUDA_TRY(c, cudaMemsetAsync(c->trig_dev, 0, c->nsys * sizeof(uint32_t), c->stream));
   return DEM_OK;

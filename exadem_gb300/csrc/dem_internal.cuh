@@ -131,6 +131,8 @@ struct DriverDev {
   int mesh;  // kind 2: index into the context's mesh table
   double offset, radius;
   double normal[3], center[3], center_proj[3], axis[3], vel[3], vrot[3];
+  // FP32 roundings and magnitude sums for the sphere list's first test (driver_far)
+  float nf[3], cpf[3], af[3], cf[3], rf, n1, cp1, c1;
 };
 
 // Mesh driver (RShapeDriver, rshape.hpp:104-420) on the device.  World vertices
@@ -165,7 +167,25 @@ struct GridDev {
   double csz[3];
   int periodic[3];
   double L[3];
+  // FP32 roundings of lo, csz, 1 / csz and the largest csz, and the multipliers and
+  // shifts that divide a cell index by dims[0] and dims[1] (cell_coords)
+  float lof[3], csf[3], icsz[3], cmaxf;
+  uint32_t dmul[2], dshift[2];
 };
+// x, y, z of cell c < 2^31 of the grid: exact quotients by a multiplication
+// (Granlund and Montgomery, "Division by invariant integers using multiplication",
+// PLDI 1994: for c < 2^31 and m = ceil(2^(31 + l) / d), l = ceil(log2 d),
+// floor(c / d) is the high part of c m shifted by l - 1).
+__host__ __device__ inline uint32_t div_by(uint32_t c, uint32_t mul, uint32_t shift) {
+  return mul ? (uint32_t)(((uint64_t)c * mul) >> 32) >> shift : c;
+}
+__host__ __device__ inline void cell_coords(const GridDev& g, uint32_t c, int& x, int& y, int& z) {
+  const uint32_t r = div_by(c, g.dmul[0], g.dshift[0]);
+  const uint32_t p = div_by(r, g.dmul[1], g.dshift[1]);
+  x = (int)(c - r * (uint32_t)g.dims[0]);
+  y = (int)(r - p * (uint32_t)g.dims[1]);
+  z = (int)p;
+}
 
 // Systems of a batched context (one system when not batched).  System k owns
 // particles [pfirst[k], pfirst[k+1]) (the cell sort keeps particles inside

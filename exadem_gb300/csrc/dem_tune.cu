@@ -26,7 +26,7 @@
 namespace dem {
 int ext_update_neighbors(dem_ctx* c);
 int ext_setup_grid(dem_ctx* c);
-int launch_reverse_lists(dem_ctx* c);
+
 
 namespace {
 // max |v| over the particles: non-negative floats order like their bit patterns

@@ -14,7 +14,9 @@
 //     (interaction_manager.hpp:89-112, placeholder_interaction.hpp:398-408).
 // Plain FP64 path (k_count / k_fill): one thread per owner particle; particles
 // are in cell order so the stencil reads of neighbouring threads hit the same
-// cells (L1/L2 reuse).  FP32 broad phase (k_cell_count / k_cell_fill): one warp
+// cells (L1/L2 reuse).  FP32 broad phase (k_count_pairs / k_fill_entries): each pair
+// met once, appended to its owner's record, the records ordered by rank; or, as an
+// option, (k_cell_count / k_cell_fill): one warp
 // per cell, its 27-cell neighbourhood staged in shared memory, candidates
 // compacted with ballots, each owner's list ordered by a warp rank sort; the
 // drivers per particle (k_pre_count / k_pre_fill).  In a batched context the particle's system gives the grid, its cell block and
@@ -40,15 +42,14 @@ struct BPArgs {
   double skin;
   double rcut2;
   // FP32 broad phase: cell-relative coordinates and radii, cell sizes, skin
-  const float* xr;
-  const float* yr;
-  const float* zr;
-  const float* rf;
+  const float4* crel;
   float skin_f;
   uint64_t cap;  // interaction buffer capacity (graph step): a fill beyond it writes nothing
   // FP32 path: the count pass's candidates of each particle (SREC per particle:
-  // partner, meta), read by the fill when they fit
+  // partner, meta, partner id), read by the fill when they fit
   uint32_t* srec;
+  uint32_t* rev_cnt;  // FP32 path: the fill's count of each particle's partner list
+  uint32_t* rev_pos;  // and the place of each entry in it (a scratch of the records' capacity)
   // per-pair damping damp_rate 2 sqrt(kn meff), in the operation order of the
   // contact law: (damp_rate * 2) * sqrt(kn * meff), meff = (m_i m_j)/(m_i + m_j)
   // for particle pairs, m_i for drivers; the pair's parameter set
@@ -101,6 +102,25 @@ __device__ inline bool driver_filter(const DriverDev& d, double rcut, V3 p) {
   return dn <= 0;
 }
 
+// FP32 proof that driver_filter fails: the distance is evaluated in FP32, where the
+// coordinates (a sum of three FP32 terms) and every operation carry at most 2^-21 of
+// the magnitudes that enter, and the margin is 2^-18 of their sum.  Away from the walls it spares the FP64 filter (26 FP64
+// instructions with a square root per particle and driver; a box has six).
+__device__ __forceinline__ bool driver_far(const DriverDev& d, float rc, float px, float py, float pz) {
+  if (d.kind == 0) {
+    const float h = px * d.nf[0] + py * d.nf[1] + pz * d.nf[2];
+    const float ex = h * d.nf[0] - d.cpf[0], ey = h * d.nf[1] - d.cpf[1], ez = h * d.nf[2] - d.cpf[2];
+    const float pp = fabsf(px) + fabsf(py) + fabsf(pz);
+    const float lim = rc + (pp * d.n1 * d.n1 + d.cp1 + rc) * 3.8146973e-06f;
+    return lim > 1e-15f && lim < 1e15f && ex * ex + ey * ey + ez * ez > lim * lim;
+  }
+  const float qx = px * d.af[0], qy = py * d.af[1], qz = pz * d.af[2];
+  const float ex = qx - d.cf[0], ey = qy - d.cf[1], ez = qz - d.cf[2];
+  const float mag = fabsf(qx) + fabsf(qy) + fabsf(qz) + d.c1 + d.rf + rc;
+  const float lim = d.rf - rc - mag * 3.8146973e-06f;
+  return lim > 1e-15f && mag < 1e15f && ex * ex + ey * ey + ez * ez < lim * lim;
+}
+
 // the stationary drivers (surfaces, cylinders) of particle s's system that pass the filter
 template <class Emit>
 __device__ inline void for_each_driver(const BPArgs& a, uint32_t s, int sys, Emit&& emit) {
@@ -132,10 +152,11 @@ __device__ inline void for_each_particle(const BPArgs& a, uint32_t s, int sys, E
   float xri = 0.f, yri = 0.f, zri = 0.f, rfi = 0.f, si = 0.f, cmax = 0.f;
   const float csx = (float)g.csz[0], csy = (float)g.csz[1], csz = (float)g.csz[2];
   if (F32) {
-    xri = a.xr[s];
-    yri = a.yr[s];
-    zri = a.zr[s];
-    rfi = a.rf[s];
+    const float4 me = a.crel[s];
+    xri = me.x;
+    yri = me.y;
+    zri = me.z;
+    rfi = me.w;
     si = fmaxf(fabsf(xri), fmaxf(fabsf(yri), fabsf(zri)));
     cmax = fmaxf(csx, fmaxf(csy, csz));
   }
@@ -197,10 +218,11 @@ __device__ inline void for_each_particle(const BPArgs& a, uint32_t s, int sys, E
           if (!ghost && idi >= idj) continue;  // owner rule (kept: the suffix already satisfies it)
           int keep = -1;
           if (F32) {
-            const float xj = a.xr[q], yj = a.yr[q], zj = a.zr[q];
+            const float4 cq = a.crel[q];
+            const float xj = cq.x, yj = cq.y, zj = cq.z;
             const float sj = fmaxf(fabsf(xj), fmaxf(fabsf(yj), fabsf(zj)));
             keep = f32_decide((xj - xri) + oxf, (yj - yri) + oyf, (zj - zri) + ozf, si, sj, cmax,
-                              rfi + a.rf[q] + a.skin_f);
+                              rfi + cq.w + a.skin_f);
           }
           if (keep < 0) {
             V3 rj = mk(rx[q], ry[q], rz[q]);
@@ -290,13 +312,16 @@ __device__ uint32_t mesh_phase(const BPArgs& a, uint64_t s, bool want, uint32_t 
 // features gets a warp of its own.  Kept out of k_count / k_fill so the
 // particle-pair passes keep their register budget.
 template <bool F32>
-__global__ void k_mesh_count(BPArgs a, uint32_t* __restrict__ mcnt) {
+__global__ void k_mesh_count(BPArgs a, uint32_t* __restrict__ mcnt, uint32_t* __restrict__ cnt) {
   const uint64_t s = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (s >= a.n) return;  // the whole warp
   const bool lead = (threadIdx.x & 31) == 0;
   const bool trig = a.sv.triggered(a.sv.of(s));
   const uint32_t m = mesh_phase<F32, false>(a, s, lead && trig, 0u, 0u, IArrays{});
-  if (lead) mcnt[s] = trig ? m : 0u;
+  if (lead) {
+    mcnt[s] = trig ? m : 0u;
+    cnt[s] = trig ? m : 0u;  // the particle candidates are added to it
+  }
 }
 template <bool F32>
 __global__ void k_mesh_fill(BPArgs a, const uint32_t* __restrict__ off, IArrays dst) {
@@ -307,33 +332,207 @@ __global__ void k_mesh_fill(BPArgs a, const uint32_t* __restrict__ off, IArrays 
   mesh_phase<F32, true>(a, s, (threadIdx.x & 31) == 0 && trig, b, e, dst);
 }
 
-constexpr uint32_t SREC = 8;
+constexpr uint32_t SREC = 16;
 
-template <bool F32>
 __global__ void k_count(BPArgs a, uint32_t* __restrict__ cnt, const uint32_t* __restrict__ old_off) {
   const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= a.n) return;
-  if (!a.sv.triggered(a.sv.of(s))) {  // slot kept (k_perm_keep): the previous list is copied
+  if (!a.sv.triggered(a.sv.of(s))) {  // slot kept (k_reorder): the previous list is copied
     cnt[s] = old_off[s + 1] - old_off[s];
     return;
   }
-  const uint32_t m0 = a.has_mesh ? a.mcnt[s] : 0u;
-  uint32_t m = m0;
-  uint32_t* rec = F32 ? a.srec + s * (2 * SREC) : nullptr;
-  for_each_candidate<F32>(a, (uint32_t)s, [&](uint32_t q, uint64_t, uint32_t meta, uint32_t) {
-    if (F32 && m - m0 < SREC) {
-      rec[2 * (m - m0)] = q;
-      rec[2 * (m - m0) + 1] = meta;
-    }
-    m++;
-  });
+  uint32_t m = a.has_mesh ? a.mcnt[s] : 0u;
+  for_each_candidate<false>(a, (uint32_t)s, [&](uint32_t, uint64_t, uint32_t, uint32_t) { m++; });
   cnt[s] = m;
+}
+
+// FP32 broad phase, count pass.  Each unordered pair is met once, from the
+// particle whose cell comes first: the rest of its own cell and the 13 forward
+// cells of the stencil, five rows of cells along x whose particles follow each
+// other in memory (cells that wrap around a periodic x one by one).  A kept pair
+// goes to the record of its owner (the smaller id; a pair across a periodic face to
+// both), in any order: the fill orders it.  So a pair costs one FP32 test instead
+// of two, no bisection of the cells by id, and ids are read for kept pairs only.
+// Recording a pair waits for ids and for an atomic's value, so a lane first collects
+// its kept pairs in shared memory (PAIR_HITS; the rare further ones are recorded at
+// once) and records them together at the end, their loads and atomics in flight at
+// the same time: a warp that recorded at every step with a kept pair took 45 us at
+// 125 k particles.
+// PAIR_LANES lanes share a particle, a row's candidates two at a time.  Measured with
+// one, two and four lanes: 10 k box 18.8, 14.8, 14.4 us; 125 k bed 32, 28, 33 us; 2 M
+// bed 332, 323, 473 us (a thread per owner over its whole stencil: 37, 48, 468 us).
+// cnt starts at the mesh candidates (k_mesh_count) or zero (k_reorder).
+constexpr int PAIR_BLOCK = 128;
+constexpr int PAIR_HITS = 8;
+constexpr int PAIR_LANES = 2;
+__global__ void __launch_bounds__(PAIR_BLOCK) k_count_pairs(BPArgs a, uint32_t* __restrict__ cnt,
+                                                            const uint32_t* __restrict__ old_off) {
+  __shared__ uint32_t hit_q[PAIR_HITS][PAIR_BLOCK];
+  __shared__ uint8_t hit_c[PAIR_HITS][PAIR_BLOCK];  // image shift (two bits an axis) and undecided bit (64)
+  constexpr uint32_t HOME = 1u | 1u << 2 | 1u << 4;   // no shift, decided
+  const uint32_t gl = threadIdx.x % PAIR_LANES;
+  const uint64_t s = ((uint64_t)blockIdx.x * PAIR_BLOCK + threadIdx.x) / PAIR_LANES;
+  if (s >= a.n) return;
+  if (gl == 0) a.rev_cnt[s] = 0u;  // the fill counts the partner lists
+  const int sys = a.sv.of(s);
+  if (!a.sv.triggered(sys)) {  // slot kept (k_reorder): the previous list is copied
+    if (gl == 0) cnt[s] = old_off[s + 1] - old_off[s];
+    return;
+  }
+  const GridDev& g = a.sv.g[sys];
+  const uint32_t coff = a.sv.coff[sys];
+  const float csx = g.csf[0], csy = g.csf[1], csz = g.csf[2], cmax = g.cmaxf;
+  const int d0 = g.dims[0], d1 = g.dims[1], d2n = g.dims[2];
+  const float4 me = a.crel[s];
+  int cx, cy, cz;
+  cell_coords(g, a.cell_of[s] - coff, cx, cy, cz);
+  uint4* const rec = reinterpret_cast<uint4*>(a.srec);
+  auto store = [&](uint32_t o, uint32_t at, uint32_t q, uint32_t meta, uint64_t pid) {
+    const uint32_t m = at - (a.has_mesh ? a.mcnt[o] : 0u);
+    if (m < SREC) rec[(uint64_t)o * SREC + m] = make_uint4(q, meta, (uint32_t)pid, (uint32_t)(pid >> 32));
+  };
+  auto append = [&](uint32_t o, uint32_t q, uint32_t meta, uint64_t pid) {
+    store(o, atomicAdd(&cnt[o], 1u), q, meta, pid);
+  };
+  // the FP64 filter from particle p to the image of q shifted by the system's lengths
+  auto exact = [&](uint32_t p, uint32_t q, int sx, int sy, int sz) {
+    V3 rj = mk(a.P.f[RX][q], a.P.f[RY][q], a.P.f[RZ][q]);
+    if (sx) rj.x = rj.x + (double)sx * g.L[0];
+    if (sy) rj.y = rj.y + (double)sy * g.L[1];
+    if (sz) rj.z = rj.z + (double)sz * g.L[2];
+    const double dx = rj.x - a.P.f[RX][p], dy = rj.y - a.P.f[RY][p], dz = rj.z - a.P.f[RZ][p];
+    const double d2 = dx * dx + dy * dy + dz * dz;
+    const double rmax = a.P.f[RAD][p] + a.P.f[RAD][q] + a.skin;
+    return d2 > 0.0 && d2 < rmax * rmax && d2 < a.rcut2;
+  };
+  // a pair across a periodic face, or one that FP32 left undecided
+  auto record_any = [&](uint32_t q, uint32_t code) {
+    const int sx = (int)(code & 3u) - 1, sy = (int)((code >> 2) & 3u) - 1, sz = (int)((code >> 4) & 3u) - 1;
+    const bool sure = (code & 64u) == 0;
+    const uint32_t p = (uint32_t)s;
+    const uint64_t idp = a.P.id[p], idq = a.P.id[q];
+    if (sx | sy | sz) {  // both own it
+      if (sure || exact(p, q, sx, sy, sz)) append(p, q, make_meta(DEM_ITYPE_VERTEX_VERTEX, sx, sy, sz, true), idq);
+      if (sure || exact(q, p, -sx, -sy, -sz))
+        append(q, p, make_meta(DEM_ITYPE_VERTEX_VERTEX, -sx, -sy, -sz, true), idp);
+    } else if (idp != idq) {
+      const bool mine = idp < idq;
+      const uint32_t o = mine ? p : q, r = mine ? q : p;
+      if (sure || exact(o, r, 0, 0, 0))
+        append(o, r, make_meta(DEM_ITYPE_VERTEX_VERTEX, 0, 0, 0, false), mine ? idq : idp);
+    }
+  };
+  if (gl == 0) {
+    const int2 dr = a.sv.drange[sys];
+    const float px = g.lof[0] + (float)cx * csx + me.x, py = g.lof[1] + (float)cy * csy + me.y,
+                pz = g.lof[2] + (float)cz * csz + me.z;
+    for (int k = dr.x; k < dr.x + dr.y; k++) {
+      const DriverDev& d = a.drv[k];
+      if (d.kind == 2 || driver_far(d, me.w + a.skin_f, px, py, pz)) continue;  // mesh drivers: mesh_phase
+      if (driver_filter(d, a.P.f[RAD][s] + a.skin, mk(a.P.f[RX][s], a.P.f[RY][s], a.P.f[RZ][s])))
+        append((uint32_t)s, (uint32_t)k,
+               make_meta(d.kind == 0 ? DEM_ITYPE_VERTEX_SURFACE : DEM_ITYPE_VERTEX_CYLINDER, 0, 0, 0, false),
+               (uint64_t)k);
+    }
+  }
+  const float si = fmaxf(fabsf(me.x), fmaxf(fabsf(me.y), fabsf(me.z)));
+  const float reach = me.w + a.skin_f;
+  uint32_t nh = 0;
+  auto scan = [&](uint32_t q, uint32_t q1, uint32_t u0, uint32_t u1, float oy, float oz, uint32_t shift) {
+    for (q += gl; q < q1; q += PAIR_LANES) {
+      const float4 cq = a.crel[q];
+      const float sj = fmaxf(fabsf(cq.x), fmaxf(fabsf(cq.y), fabsf(cq.z)));
+      const float ox = q < u0 ? -csx : (q < u1 ? 0.f : csx);
+      const int keep = f32_decide((cq.x - me.x) + ox, (cq.y - me.y) + oy, (cq.z - me.z) + oz, si, sj, cmax,
+                                  reach + cq.w);
+      if (keep) {
+        const uint32_t code = shift | (keep < 0 ? 64u : 0u);
+        if (nh < PAIR_HITS) {
+          hit_q[nh][threadIdx.x] = q;
+          hit_c[nh][threadIdx.x] = (uint8_t)code;
+          nh++;
+        } else {
+          record_any(q, code);
+        }
+      }
+    }
+  };
+#pragma unroll 1
+  for (int r = 0; r < 5; r++) {  // rows (dy, dz): (0, 0), (1, 0), (-1, 1), (0, 1), (1, 1)
+    const int dy = r == 0 || r == 3 ? 0 : (r == 2 ? -1 : 1), dz = r < 2 ? 0 : 1;
+    int y = cy + dy, z = cz + dz, sy = 0, sz = 0;
+    if (y < 0 || y >= d1) {
+      if (!g.periodic[1]) continue;
+      sy = y < 0 ? -1 : 1;
+      y -= sy * d1;
+    }
+    if (z >= d2n) {
+      if (!g.periodic[2]) continue;
+      sz = 1;
+      z -= d2n;
+    }
+    const float oy = (float)dy * csy, oz = (float)dz * csz;
+    const uint32_t rb = coff + (uint32_t)d0 * ((uint32_t)y + (uint32_t)d1 * (uint32_t)z);
+    const uint32_t shift = (uint32_t)(sy + 1) << 2 | (uint32_t)(sz + 1) << 4;
+    const uint32_t* const st = a.cell_start + rb + (uint32_t)cx;
+    const uint32_t u0 = st[0], u1 = st[1];
+    const uint32_t q0 = r == 0 ? (uint32_t)s + 1u : (cx > 0 ? st[-1] : u0);
+    const uint32_t q1 = cx < d0 - 1 ? st[2] : u1;
+    scan(q0, q1, u0, u1, oy, oz, shift | 1u);
+    if (g.periodic[0] && (cx == d0 - 1 || (r && cx == 0))) {  // the cell that x wraps to (at least three along x)
+      const bool left = cx == 0;
+      const uint32_t cc = rb + (left ? (uint32_t)d0 - 1u : 0u);
+      scan(a.cell_start[cc], a.cell_start[cc + 1], left ? ~0u : 0u, left ? ~0u : 0u, oy, oz, shift | (left ? 0u : 2u));
+    }
+  }
+  const uint32_t p = (uint32_t)s;
+  const uint64_t idp = a.P.id[p];
+  uint64_t idq[PAIR_HITS];
+  uint32_t at[PAIR_HITS];
+#pragma unroll
+  for (int k = 0; k < PAIR_HITS; k++)
+    if (k < (int)nh && hit_c[k][threadIdx.x] == HOME) idq[k] = a.P.id[hit_q[k][threadIdx.x]];
+#pragma unroll
+  for (int k = 0; k < PAIR_HITS; k++)
+    if (k < (int)nh && hit_c[k][threadIdx.x] == HOME && idq[k] != idp)
+      at[k] = atomicAdd(&cnt[idp < idq[k] ? p : hit_q[k][threadIdx.x]], 1u);
+#pragma unroll
+  for (int k = 0; k < PAIR_HITS; k++) {
+    if (k >= (int)nh) continue;
+    const uint32_t q = hit_q[k][threadIdx.x], code = hit_c[k][threadIdx.x];
+    if (code != HOME) {
+      record_any(q, code);
+    } else if (idq[k] != idp) {
+      const bool mine = idp < idq[k];
+      store(mine ? p : q, at[k], mine ? q : p, make_meta(DEM_ITYPE_VERTEX_VERTEX, 0, 0, 0, false), mine ? idq[k] : idp);
+    }
+  }
 }
 
 // InteractionPair order inside the owner: (partner id, type, partner sub); swap
 // and the owner sub are 0 for spheres
 __device__ inline bool key_less(uint64_t pa, uint32_t ta, uint32_t sa, uint64_t pb, uint32_t tb, uint32_t sb) {
   return pa < pb || (pa == pb && (ta < tb || (ta == tb && sa < sb)));
+}
+
+// entry y of the previous list as entry x of the new one, owned by slot s
+__device__ __forceinline__ void copy_entry(const IArrays& dst, uint32_t x, const IArrays& old, uint32_t y, uint32_t s) {
+  const uint32_t partner = old.partner[y], meta = old.meta[y], sub = old.sub[y];
+  const uint64_t pid = old.pid[y];
+  const double f0 = old.ft[0][y], f1 = old.ft[1][y], f2 = old.ft[2][y];
+  const double m0 = old.mo[0][y], m1 = old.mo[1][y], m2 = old.mo[2][y], damp = old.damp[y];
+  dst.owner[x] = s;
+  dst.partner[x] = partner;
+  dst.pid[x] = pid;
+  dst.meta[x] = meta;
+  dst.sub[x] = sub;
+  dst.ft[0][x] = f0;
+  dst.ft[1][x] = f1;
+  dst.ft[2][x] = f2;
+  dst.mo[0][x] = m0;
+  dst.mo[1][x] = m1;
+  dst.mo[2][x] = m2;
+  dst.damp[x] = damp;
 }
 
 // orders owner s's segment [b, e) by InteractionPair order and carries the
@@ -404,7 +603,6 @@ __device__ inline void finish_owner(const BPArgs& a, uint32_t s, uint32_t b, uin
 // reuse_damp: the previous list's damping was computed with the current contact
 // parameters (no dem_set_params / dem_set_multimat since, not a list installed by
 // dem_set_interactions), so a pair found in it keeps its damping bits.
-template <bool F32>
 __global__ void k_fill(BPArgs a, const uint32_t* __restrict__ off, IArrays dst, IArrays old,
                        const uint32_t* __restrict__ old_off, const uint32_t* __restrict__ perm, int have_old,
                        int reuse_damp) {
@@ -414,44 +612,133 @@ __global__ void k_fill(BPArgs a, const uint32_t* __restrict__ off, IArrays dst, 
   if (e > a.cap) return;
   if (!a.sv.triggered(a.sv.of(s))) {  // slot kept, partners of the same system kept: copy
     const uint32_t ob = old_off[s];
-    for (uint32_t x = b; x < e; x++) {
-      const uint32_t y = ob + (x - b);
-      dst.owner[x] = (uint32_t)s;
-      dst.partner[x] = old.partner[y];
-      dst.pid[x] = old.pid[y];
-      dst.meta[x] = old.meta[y];
-      dst.sub[x] = old.sub[y];
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        dst.ft[d][x] = old.ft[d][y];
-        dst.mo[d][x] = old.mo[d][y];
-      }
-      dst.damp[x] = old.damp[y];
-    }
+    for (uint32_t x = b; x < e; x++) copy_entry(dst, x, old, ob + (x - b), (uint32_t)s);
     return;
   }
   uint32_t w = b + (a.has_mesh ? a.mcnt[s] : 0u);  // mesh items first (k_mesh_fill)
-  if (F32 && e - w <= SREC) {  // the count pass recorded the drivers and particles
-    const uint32_t* rec = a.srec + s * (2 * SREC);
-    for (uint32_t x = w; x < e; x++) {
-      const uint32_t q = rec[2 * (x - w)], meta = rec[2 * (x - w) + 1];
-      dst.partner[x] = q;
-      dst.pid[x] = meta_type(meta) == DEM_ITYPE_VERTEX_VERTEX ? a.P.id[q] : (uint64_t)q;
-      dst.meta[x] = meta;
-      dst.sub[x] = 0u;
+  for_each_candidate<false>(a, (uint32_t)s, [&](uint32_t q, uint64_t pid, uint32_t meta, uint32_t sub) {
+    if (w < e) {
+      dst.partner[w] = q;
+      dst.pid[w] = pid;
+      dst.meta[w] = meta;
+      dst.sub[w] = sub;
     }
-  } else {
-    for_each_candidate<F32>(a, (uint32_t)s, [&](uint32_t q, uint64_t pid, uint32_t meta, uint32_t sub) {
-      if (w < e) {
-        dst.partner[w] = q;
-        dst.pid[w] = pid;
-        dst.meta[w] = meta;
-        dst.sub[w] = sub;
-      }
-      w++;
-    });
-  }
+    w++;
+  });
   finish_owner(a, (uint32_t)s, b, e, dst, old, old_off, perm, have_old, reuse_damp);
+}
+
+// owner slot of every entry of the new list (nothing beyond the capacity)
+__global__ void k_expand_owner(BPArgs a, const uint32_t* __restrict__ off, uint32_t* __restrict__ owner) {
+  const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= a.n || off[a.n] > a.cap) return;
+  const uint32_t b = off[s], e = off[s + 1];
+  for (uint32_t x = b; x < e; x++) owner[x] = (uint32_t)s;
+}
+
+// FP32 broad phase, fill: a thread per entry of the new list.  Entry x of
+// particle s takes the particle's record x, ranks its key among the particle's
+// records and goes to that place, so each list is in InteractionPair order; the
+// history is the entry of the same key in the particle's previous list.  The
+// lanes of a warp share the records, ids and previous lists of a dozen particles
+// in L1, every lane works and the writes are consecutive but for the order inside
+// a list.  Bound by the latency of about six dependent loads below 100 k particles,
+// above by its traffic (300 bytes an entry).  Measured: 10 k box 9 us, 2 M bed 297 us;
+// a thread per particle sorting its list in global memory, a chain of loads for
+// every comparison and move: 57 and 421 us; eight lanes per particle with shuffles:
+// 9 and 538 us, with two of three lanes idle.
+// The partner lists are counted on the way: the atomic's value is the entry's
+// place in its partner's list (rev_pos).  Particles with mesh candidates or more
+// than SREC others are filled and sorted by the thread of their first entry.
+__global__ void __launch_bounds__(128) k_fill_entries(BPArgs a, const uint32_t* __restrict__ off,
+                                                      IArrays dst, IArrays old, const uint32_t* __restrict__ old_off,
+                                                      const uint32_t* __restrict__ perm, int have_old,
+                                                      int reuse_damp) {
+  const uint64_t total = off[a.n];
+  if (total > a.cap) return;  // nothing, and empty partner lists
+  auto partner_list = [&](uint64_t x, uint32_t q, uint32_t meta) {
+    if (meta_type(meta) == DEM_ITYPE_VERTEX_VERTEX && !meta_owner_only(meta)) a.rev_pos[x] = atomicAdd(&a.rev_cnt[q], 1u);
+  };
+  const uint4* const recs = reinterpret_cast<const uint4*>(a.srec);
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += stride) {
+    const uint32_t s = dst.owner[k];
+    const uint32_t b = off[s], m = off[s + 1] - b, x = (uint32_t)k - b;
+    if (!a.sv.triggered(a.sv.of(s))) {  // slot kept, partners of the same system kept: copy
+      const uint32_t y = old_off[s] + x;
+      copy_entry(dst, (uint32_t)k, old, y, s);
+      partner_list(k, old.partner[y], old.meta[y]);
+      continue;
+    }
+    const uint32_t mm = a.has_mesh ? a.mcnt[s] : 0u;
+    const uint4* const rec = recs + (uint64_t)s * SREC;
+    auto pid_of = [](uint4 v) { return (uint64_t)v.z | (uint64_t)v.w << 32; };
+    if (mm || m > SREC) {
+      if (x) continue;
+      const uint32_t e = b + m;
+      uint32_t w = b + mm;  // mesh items first (k_mesh_fill)
+      if (m - mm <= SREC) {
+        for (uint32_t y = 0; y < m - mm; y++) {
+          const uint4 v = rec[y];
+          dst.partner[w + y] = v.x;
+          dst.pid[w + y] = pid_of(v);
+          dst.meta[w + y] = v.y;
+          dst.sub[w + y] = 0u;
+        }
+      } else {
+        for_each_candidate<true>(a, s, [&](uint32_t q, uint64_t pid, uint32_t meta, uint32_t sub) {
+          if (w < e) {
+            dst.partner[w] = q;
+            dst.pid[w] = pid;
+            dst.meta[w] = meta;
+            dst.sub[w] = sub;
+          }
+          w++;
+        });
+      }
+      finish_owner(a, s, b, e, dst, old, old_off, perm, have_old, reuse_damp);
+      for (uint32_t y = b; y < e; y++) partner_list(y, dst.partner[y], dst.meta[y]);
+      continue;
+    }
+    const uint4 v = rec[x];
+    const uint64_t pid = pid_of(v);
+    const uint32_t type = meta_type(v.y);
+    uint32_t rank = 0;
+    for (uint32_t y = 0; y < m; y++) {
+      const uint4 u = rec[y];
+      rank += key_less(pid_of(u), meta_type(u.y), 0u, pid, type, 0u) ? 1u : 0u;
+    }
+    uint32_t hit = ~0u;
+    if (have_old) {
+      const uint32_t os = perm[s];
+      const uint32_t oe = old_off[os + 1];
+      for (uint32_t y = old_off[os]; y < oe; y++)
+        if (old.pid[y] == pid && meta_type(old.meta[y]) == type && old.sub[y] == 0u) hit = y;
+    }
+    double h[6] = {0, 0, 0, 0, 0, 0};
+    double damp = 0.0;
+    if (hit != ~0u) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        h[d] = old.ft[d][hit];
+        h[3 + d] = old.mo[d][hit];
+      }
+      damp = old.damp[hit];
+    }
+    if (hit == ~0u || !reuse_damp) damp = pair_damp(a, s, v.x, v.y);
+    const uint64_t w = b + rank;
+    dst.partner[w] = v.x;
+    dst.pid[w] = pid;
+    dst.meta[w] = v.y;
+    dst.sub[w] = 0u;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      dst.ft[d][w] = h[d];
+      dst.mo[d][w] = h[3 + d];
+    }
+    dst.damp[w] = damp;
+    partner_list(w, v.x, v.y);
+  }
 }
 
 // ---- warp-per-cell broad phase (FP32 decisions)
@@ -529,10 +816,11 @@ __device__ inline uint32_t stage_cell(const BPArgs& a, const GridDev& g, uint32_
           hi = mid - 1;
       }
       const uint32_t q = st.q0[lo] + (i - st.pre[lo]);
-      st.x[i] = a.xr[q];
-      st.y[i] = a.yr[q];
-      st.z[i] = a.zr[q];
-      st.r[i] = a.rf[q];
+      const float4 cq = a.crel[q];
+      st.x[i] = cq.x;
+      st.y[i] = cq.y;
+      st.z[i] = cq.z;
+      st.r[i] = cq.w;
       st.id[i] = a.P.id[q];
       st.q[i] = q;
       st.l[i] = (uint8_t)lo;
@@ -612,7 +900,8 @@ __device__ inline void cell_particles(const BPArgs& a, uint32_t C, uint32_t o0, 
       if (e > a.cap) continue;
       w = off[s] + (a.has_mesh ? a.mcnt[s] : 0u);
     }
-    const float xri = a.xr[s], yri = a.yr[s], zri = a.zr[s], rfi = a.rf[s];
+    const float4 me = a.crel[s];
+    const float xri = me.x, yri = me.y, zri = me.z, rfi = me.w;
     const float si = fmaxf(fabsf(xri), fmaxf(fabsf(yri), fabsf(zri)));
     const uint64_t idi = a.P.id[s];
     const V3 ri = mk(a.P.f[RX][s], a.P.f[RY][s], a.P.f[RZ][s]);
@@ -664,20 +953,7 @@ __global__ void k_pre_fill(BPArgs a, const uint32_t* __restrict__ off, IArrays d
   const int sys = a.sv.of(s);
   if (!a.sv.triggered(sys)) {
     const uint32_t ob = old_off[s];
-    for (uint32_t x = b; x < e; x++) {
-      const uint32_t y = ob + (x - b);
-      dst.owner[x] = (uint32_t)s;
-      dst.partner[x] = old.partner[y];
-      dst.pid[x] = old.pid[y];
-      dst.meta[x] = old.meta[y];
-      dst.sub[x] = old.sub[y];
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        dst.ft[d][x] = old.ft[d][y];
-        dst.mo[d][x] = old.mo[d][y];
-      }
-      dst.damp[x] = old.damp[y];
-    }
+    for (uint32_t x = b; x < e; x++) copy_entry(dst, x, old, ob + (x - b), (uint32_t)s);
     return;
   }
   uint32_t nd = 0;
@@ -740,11 +1016,6 @@ __global__ void k_pair_damp(BPArgs a, IArrays I, uint64_t ni) {
     I.damp[k] = pair_damp(a, I.owner[k], I.partner[k], I.meta[k]);
 }
 
-__global__ void k_zero_u32(uint32_t* p, uint64_t n) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = 0u;
-}
-
 // partner-side lists: interactions whose partner is a real particle that receives -f
 // ni_dev != nullptr: the interaction count is read on the device (graph step)
 __global__ void k_rev_count(IArrays I, uint64_t ni, const unsigned long long* ni_dev, uint32_t* __restrict__ cnt) {
@@ -755,82 +1026,55 @@ __global__ void k_rev_count(IArrays I, uint64_t ni, const unsigned long long* ni
   }
 }
 __global__ void k_rev_fill(IArrays I, uint64_t ni, const unsigned long long* ni_dev, const uint32_t* __restrict__ off,
-                           uint32_t* __restrict__ cursor, uint32_t* __restrict__ idx) {
+                           uint32_t* __restrict__ cursor, const uint64_t* __restrict__ id, uint32_t* __restrict__ idx,
+                           uint64_t* __restrict__ oid) {
   const uint64_t nn = ni_dev ? *ni_dev : ni;
   for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t m = I.meta[k];
     if (meta_type(m) <= DEM_ITYPE_EDGE_EDGE && !meta_owner_only(m)) {
       const uint32_t j = I.partner[k];
-      idx[off[j] + atomicAdd(&cursor[j], 1u)] = (uint32_t)k;
+      const uint32_t w = off[j] + atomicAdd(&cursor[j], 1u);
+      idx[w] = (uint32_t)k;
+      oid[w] = id[I.owner[k]];
     }
   }
 }
-// order of the partner-side contributions: InteractionPair order = (owner id, index).
-// A list of at most REV_SHORT entries (spheres: a few) is copied from `unsorted`
-// and insertion-sorted by its particle's thread; a longer one (polyhedra: tens)
-// is queued in `longs` for k_rev_rank.
-constexpr uint32_t REV_SHORT = 12;
-__global__ void k_rev_short(uint64_t n, const uint32_t* __restrict__ off, const uint32_t* __restrict__ owner,
-                            const uint64_t* __restrict__ id, const uint32_t* __restrict__ unsorted,
-                            uint32_t* __restrict__ idx, uint32_t* __restrict__ longs, unsigned int* __restrict__ nlong) {
-  const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  const uint32_t b = off[s], e = off[s + 1];
-  if (e - b > REV_SHORT) {
-    longs[atomicAdd(nlong, 1u)] = (uint32_t)s;
-    return;
-  }
-  for (uint32_t x = b; x < e; x++) {
-    const uint32_t k = unsorted[x];
-    const uint64_t ok = id[owner[k]];
-    uint32_t y = x;
-    while (y > b) {
-      const uint32_t kp = idx[y - 1];
-      const uint64_t op = id[owner[kp]];
-      if (op < ok || (op == ok && kp < k)) break;
-      idx[y] = kp;
-      y--;
+// the entries at their counted places (k_fill_entries), and their owners' ids
+__global__ void k_rev_place(IArrays I, uint64_t ni, const unsigned long long* ni_dev, const uint32_t* __restrict__ off,
+                            const uint32_t* __restrict__ pos, const uint64_t* __restrict__ id,
+                            uint32_t* __restrict__ idx, uint64_t* __restrict__ oid) {
+  const uint64_t nn = ni_dev ? *ni_dev : ni;
+  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t m = I.meta[k];
+    if (meta_type(m) <= DEM_ITYPE_EDGE_EDGE && !meta_owner_only(m)) {
+      const uint32_t w = off[I.partner[k]] + pos[k];
+      idx[w] = (uint32_t)k;
+      oid[w] = id[I.owner[k]];
     }
-    idx[y] = k;
   }
 }
-// One warp per queued particle: the entries of its reverse list go to idx at
-// their rank, the number of entries of the list with a smaller (owner id,
-// index) key (keys are distinct: the index is).  Lanes hold 32 entries at a time
-// and count against every chunk of 32 of the list broadcast by shuffles.
-__global__ void __launch_bounds__(256) k_rev_rank(const unsigned int* __restrict__ nlong,
-                                                  const uint32_t* __restrict__ longs, const uint32_t* __restrict__ off,
-                                                  const uint32_t* __restrict__ owner,
-                                                  const uint64_t* __restrict__ id,
-                                                  const uint32_t* __restrict__ unsorted, uint32_t* __restrict__ idx) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  const uint64_t nl = *nlong;
-  for (uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nl; t += nw) {
-    const uint32_t s = longs[t];
-    const uint32_t b = off[s], m = off[s + 1] - b;
-    for (uint32_t i0 = 0; i0 < m; i0 += 32) {
-      const bool have = i0 + lane < m;
-      const uint32_t k = have ? unsorted[b + i0 + lane] : 0u;
-      const uint64_t o = have ? id[owner[k]] : 0ull;
-      uint32_t rank = 0;
-      for (uint32_t j0 = 0; j0 < m; j0 += 32) {
-        uint32_t kj = k;
-        uint64_t oj = o;
-        if (j0 != i0) {
-          const bool hj = j0 + lane < m;
-          kj = hj ? unsorted[b + j0 + lane] : 0u;
-          oj = hj ? id[owner[kj]] : 0ull;
-        }
-        const uint32_t nj = m - j0 < 32u ? m - j0 : 32u;
-        for (uint32_t q = 0; q < nj; q++) {
-          const uint32_t kq = __shfl_sync(0xffffffffu, kj, (int)q);
-          const uint64_t oq = __shfl_sync(0xffffffffu, oj, (int)q);
-          rank += (oq < o || (oq == o && kq < k)) ? 1u : 0u;
-        }
-      }
-      if (have) idx[b + rank] = k;
+// order of the partner-side contributions: InteractionPair order = (owner id,
+// index).  A thread per entry: its rank is the number of entries of its partner's
+// list with a smaller key (keys are distinct: the index is); the lanes of a warp
+// share their lists in L1.  No lane idles whatever the lists' lengths are (about
+// three for spheres, 34 for the fragmentation bed's cubes).
+__global__ void __launch_bounds__(256) k_rev_rank(uint64_t n, const uint32_t* __restrict__ off,
+                                                  const uint32_t* __restrict__ partner,
+                                                  const uint32_t* __restrict__ unsorted,
+                                                  const uint64_t* __restrict__ oid, uint32_t* __restrict__ idx) {
+  const uint64_t total = off[n];
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += stride) {
+    const uint32_t k = unsorted[w];
+    const uint64_t o = oid[w];
+    const uint32_t j = partner[k];
+    const uint32_t b = off[j], e = off[j + 1];
+    uint32_t rank = 0;
+    for (uint32_t y = b; y < e; y++) {
+      const uint64_t oy = oid[y];
+      if (oy < o || (oy == o && unsorted[y] < k)) rank++;
     }
+    idx[b + rank] = k;
   }
 }
 
@@ -849,13 +1093,12 @@ BPArgs make_args(dem_ctx* c) {
   a.skin = c->prm.rcut_inc;
   const double nd = 2 * c->rad_max + c->prm.rcut_inc;
   a.rcut2 = nd * nd;
-  a.xr = c->crel[0];
-  a.yr = c->crel[1];
-  a.zr = c->crel[2];
-  a.rf = c->crel[3];
+  a.crel = c->crel;
   a.skin_f = (float)c->prm.rcut_inc;
   a.cap = c->capturing ? c->gcap : ~0ull;
   a.srec = c->srec;
+  a.rev_cnt = c->rev_cnt;
+  a.rev_pos = c->L2;
   a.cp = c->prm.config;
   a.cpd = c->prm.config_driver;
   a.pt = c->ptable();
@@ -886,9 +1129,9 @@ int launch_count_sphere(dem_ctx* c) {
   if (c->n && mesh) {
     if (!c->mesh_cnt) return c->fail(DEM_ERR_STATE, "mesh count buffer missing");
     if (c->prm.fp32_broad_phase)
-      k_mesh_count<true><<<grid_for(c->n * 32, 128), 128, 0, c->stream>>>(make_args(c), c->mesh_cnt);
+      k_mesh_count<true><<<grid_for(c->n * 32, 128), 128, 0, c->stream>>>(make_args(c), c->mesh_cnt, c->pcnt);
     else
-      k_mesh_count<false><<<grid_for(c->n * 32, 128), 128, 0, c->stream>>>(make_args(c), c->mesh_cnt);
+      k_mesh_count<false><<<grid_for(c->n * 32, 128), 128, 0, c->stream>>>(make_args(c), c->mesh_cnt, c->pcnt);
   }
   if (c->n) {
     if (c->prm.fp32_broad_phase && c->cell_broad_phase) {
@@ -896,9 +1139,10 @@ int launch_count_sphere(dem_ctx* c) {
       k_pre_count<<<grid_for(c->n, 128), 128, 0, c->stream>>>(a, c->pcnt, c->own_off[c->icur]);
       k_cell_count<<<cell_grid(c), CELL_WARPS * 32, 0, c->stream>>>(a, c->pcnt, c->ncell);
     } else if (c->prm.fp32_broad_phase) {
-      k_count<true><<<grid_for(c->n, 128), 128, 0, c->stream>>>(make_args(c), c->pcnt, c->own_off[c->icur]);
+      k_count_pairs<<<grid_for(c->n * PAIR_LANES, PAIR_BLOCK), PAIR_BLOCK, 0, c->stream>>>(make_args(c), c->pcnt,
+                                                                                           c->own_off[c->icur]);
     } else {
-      k_count<false><<<grid_for(c->n, 128), 128, 0, c->stream>>>(make_args(c), c->pcnt, c->own_off[c->icur]);
+      k_count<<<grid_for(c->n, 128), 128, 0, c->stream>>>(make_args(c), c->pcnt, c->own_off[c->icur]);
     }
   }
   DEM_CUDA_TRY(c, cudaGetLastError());
@@ -906,10 +1150,10 @@ int launch_count_sphere(dem_ctx* c) {
 }
 
 int launch_fill_sphere(dem_ctx* c, uint32_t* new_off, uint64_t total) {
-  (void)total;
   const int nw = 1 - c->icur;
   const bool mesh = !c->meshes.empty();
-  ProfScope ps(c, K_BROAD_FILL, c->n ? (mesh ? 2 : 1) : 0);
+  const bool cells = c->prm.fp32_broad_phase && c->cell_broad_phase;
+  ProfScope ps(c, K_BROAD_FILL, c->n ? (mesh ? 1 : 0) + (cells ? 3 : c->prm.fp32_broad_phase ? 2 : 1) : 0);
   if (c->n && mesh) {
     if (c->prm.fp32_broad_phase)
       k_mesh_fill<true><<<grid_for(c->n * 32, 128), 128, 0, c->stream>>>(make_args(c), new_off, c->I[nw]);
@@ -925,18 +1169,26 @@ int launch_fill_sphere(dem_ctx* c, uint32_t* new_off, uint64_t total) {
       k_cell_fill<<<cell_grid(c), CELL_WARPS * 32, 0, c->stream>>>(a, new_off, c->I[nw], c->ncell);
       k_fill_finish<<<grid_for(c->n, 128), 128, 0, c->stream>>>(a, new_off, c->I[nw], c->I[c->icur],
                                                                 c->own_off[c->icur], c->perm, have_old, reuse);
-    } else if (c->prm.fp32_broad_phase)
-      k_fill<true><<<grid_for(c->n, 128), 128, 0, c->stream>>>(make_args(c), new_off, c->I[nw], c->I[c->icur],
-                                                               c->own_off[c->icur], c->perm, have_old, reuse);
-    else
-      k_fill<false><<<grid_for(c->n, 128), 128, 0, c->stream>>>(make_args(c), new_off, c->I[nw], c->I[c->icur],
-                                                                c->own_off[c->icur], c->perm, have_old, reuse);
+    } else if (c->prm.fp32_broad_phase) {
+      const BPArgs a = make_args(c);
+      k_expand_owner<<<grid_for(c->n, 128), 128, 0, c->stream>>>(a, new_off, c->I[nw].owner);
+      // the total is on the device in a graph: a grid of about two entries a particle strides over it
+      const uint64_t want = c->capturing ? 2 * c->n : total;
+      if (want)
+        k_fill_entries<<<(unsigned)std::min<uint64_t>(grid_for(want, 128), (uint64_t)c->num_sms * 64), 128, 0,
+                         c->stream>>>(a, new_off, c->I[nw], c->I[c->icur], c->own_off[c->icur], c->perm,
+                                      have_old, reuse);
+    } else {
+      k_fill<<<grid_for(c->n, 128), 128, 0, c->stream>>>(make_args(c), new_off, c->I[nw], c->I[c->icur],
+                                                         c->own_off[c->icur], c->perm, have_old, reuse);
+    }
   }
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;
 }
 
-int launch_reverse_lists(dem_ctx* c) {
+// counted: the fill counted the partner lists (rev_cnt, L2: k_fill_entries)
+int launch_reverse_lists(dem_ctx* c, bool counted) {
   const uint64_t n = c->n, ni = c->ni;
   cudaStream_t st = c->stream;
   const IArrays& I = c->I[c->icur];
@@ -944,28 +1196,31 @@ int launch_reverse_lists(dem_ctx* c) {
   const unsigned long long* nd = c->capturing ? c->d_ni : nullptr;
   const bool go = c->capturing || ni;
   const unsigned gi = c->capturing ? (unsigned)c->num_sms * 8u : grid_for(ni, 256);
-  {
-  ProfScope ps(c, K_REVERSE, go ? 2 : 1);
-  k_zero_u32<<<grid_for(n + 1, 256), 256, 0, st>>>(c->rev_cnt, n + 1);
-  if (go) k_rev_count<<<gi, 256, 0, st>>>(I, ni, nd, c->rev_cnt);
-  }
-  int rc = scan_exclusive_u32(c, c->rev_cnt, c->rev_off, n);
-  if (rc) return rc;
-  ProfScope ps(c, K_REVERSE, 1 + (go ? 1 : 0) + (n ? 2 : 0));
   // the contact work list L1 (capacity rcap, like rev_idx) holds the unsorted
   // lists: the step's contact phase, after the rebuild, refills it
   uint32_t* unsorted = c->L1;
-  k_zero_u32<<<grid_for(n + 1, 256), 256, 0, st>>>(c->rev_cnt, n + 1);
-  if (go) k_rev_fill<<<gi, 256, 0, st>>>(I, ni, nd, c->rev_off, c->rev_cnt, unsorted);
-  if (n) {
-    // rev_cnt (the fill's cursors) is free again: the queue of long lists
-    DEM_CUDA_TRY(c, cudaMemsetAsync(c->rev_nlong, 0, sizeof(unsigned int), st));
-    k_rev_short<<<grid_for(n, 256), 256, 0, st>>>(n, c->rev_off, I.owner, c->P[c->pcur].id, unsorted, c->rev_idx,
-                                                  c->rev_cnt, c->rev_nlong);
-    k_rev_rank<<<(unsigned)c->num_sms * 16u, 256, 0, st>>>(c->rev_nlong, c->rev_cnt, c->rev_off, I.owner,
-                                                           c->P[c->pcur].id, unsorted, c->rev_idx);
+  if (!counted) {
+    ProfScope ps(c, K_REVERSE, go ? 1 : 0);
+    DEM_CUDA_TRY(c, cudaMemsetAsync(c->rev_cnt, 0, (n + 1) * 4, st));
+    if (go) k_rev_count<<<gi, 256, 0, st>>>(I, ni, nd, c->rev_cnt);
+  }
+  int rc = scan_exclusive_u32(c, c->rev_cnt, c->rev_off, n);
+  if (rc) return rc;
+  ProfScope ps(c, K_REVERSE, go ? 2 : 0);
+  const uint64_t* id = c->P[c->pcur].id;
+  uint64_t* oid = reinterpret_cast<uint64_t*>(c->Dscr[0]);  // a scratch of the contact pass (rcap), free here
+  if (!counted) DEM_CUDA_TRY(c, cudaMemsetAsync(c->rev_cnt, 0, (n + 1) * 4, st));
+  if (go) {
+    if (counted)
+      k_rev_place<<<gi, 256, 0, st>>>(I, ni, nd, c->rev_off, c->L2, id, unsorted, oid);
+    else
+      k_rev_fill<<<gi, 256, 0, st>>>(I, ni, nd, c->rev_off, c->rev_cnt, id, unsorted, oid);
+    k_rev_rank<<<gi, 256, 0, st>>>(n, c->rev_off, I.partner, unsorted, oid, c->rev_idx);
   }
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;
 }
+
+// whether launch_fill_sphere counts the partner lists itself
+bool fill_counts_partners(const dem_ctx* c) { return c->prm.fp32_broad_phase && !c->cell_broad_phase; }
 }  // namespace dem

@@ -249,10 +249,7 @@ struct UnitArgs {
   const ShapeDev* shapes;
   double rV;
   double rcut2;
-  const float* xr;
-  const float* yr;
-  const float* zr;
-  const float* rf;
+  const float4* crel;
   float csz[3];
   float skin_f;
   int f32;
@@ -329,10 +326,11 @@ __device__ inline void for_each_unit(const UnitArgs& a, uint32_t s, Emit&& emit)
   }
   float xri = 0.f, yri = 0.f, zri = 0.f, rfi = 0.f, si = 0.f, cmax = 0.f;
   if (a.f32) {
-    xri = a.xr[s];
-    yri = a.yr[s];
-    zri = a.zr[s];
-    rfi = a.rf[s];
+    const float4 me = a.crel[s];
+    xri = me.x;
+    yri = me.y;
+    zri = me.z;
+    rfi = me.w;
     si = fmaxf(fabsf(xri), fmaxf(fabsf(yri), fabsf(zri)));
     cmax = fmaxf(a.csz[0], fmaxf(a.csz[1], a.csz[2]));
   }
@@ -353,7 +351,7 @@ __device__ inline void for_each_unit(const UnitArgs& a, uint32_t s, Emit&& emit)
         if (x < 0 || x >= d0) continue;
         const uint32_t cc = (uint32_t)x + (uint32_t)d0 * ((uint32_t)y + (uint32_t)d1 * (uint32_t)z);
         const float oxf = (float)dx * a.csz[0], oyf = (float)dy * a.csz[1], ozf = (float)dz * a.csz[2];
-        // a cell's particles are in id order (k_cell_sort): the owner rule keeps
+        // a cell's particles are in id order (k_reorder): the owner rule keeps
         // the suffix of ids above idi, found by bisection
         uint32_t q0 = a.cell_start[cc], q1 = a.cell_start[cc + 1];
         while (q0 < q1) {
@@ -367,10 +365,11 @@ __device__ inline void for_each_unit(const UnitArgs& a, uint32_t s, Emit&& emit)
           const uint64_t idj = a.P.id[q];
           int keep = -1;
           if (a.f32) {
-            const float xj = a.xr[q], yj = a.yr[q], zj = a.zr[q];
+            const float4 cq = a.crel[q];
+            const float xj = cq.x, yj = cq.y, zj = cq.z;
             const float sj = fmaxf(fabsf(xj), fmaxf(fabsf(yj), fabsf(zj)));
             keep = f32_pair((xj - xri) + oxf, (yj - yri) + oyf, (zj - zri) + ozf, si, sj, cmax,
-                            rfi + a.rf[q] + a.skin_f);
+                            rfi + cq.w + a.skin_f);
           }
           if (keep < 0) {
             const double ddx = a.P.f[RX][q] - ri.x, ddy = a.P.f[RY][q] - ri.y, ddz = a.P.f[RZ][q] - ri.z;
@@ -2148,10 +2147,7 @@ int launch_poly_units(dem_ctx* c, uint64_t* nu_out, int (*grow_units)(dem_ctx*, 
   a.rV = c->prm.rcut_inc;
   const double nd = 2 * c->rad_max + c->prm.rcut_inc;
   a.rcut2 = nd * nd;
-  a.xr = c->crel[0];
-  a.yr = c->crel[1];
-  a.zr = c->crel[2];
-  a.rf = c->crel[3];
+  a.crel = c->crel;
   for (int d = 0; d < 3; d++) a.csz[d] = (float)c->grid.csz[d];
   a.skin_f = (float)c->prm.rcut_inc;
   a.f32 = c->prm.fp32_broad_phase;

@@ -1,8 +1,12 @@
 // k_scan.cu -- device-wide exclusive prefix sum of uint32 counts (n -> n+1 offsets).
 //
-// Three launches: per-tile totals, one-block scan of the tile totals, per-tile
-// scan plus tile offset.  A tile is 2048 counts (512 threads x 4); the counts
-// are read twice and the offsets written once.
+// Two launches up to SCAN_DIRECT tiles: per-tile totals, then per-tile scan, each
+// block summing the totals of the tiles before its own (at most 4 KB, from L2).
+// More tiles: a one-block scan of the tile totals between the two, since the
+// blocks' own sums grow with the square of the tiles (at 1024 tiles, 2 M counts,
+// they read 2 MB in all).  A tile is 2048 counts (512 threads x 4); the counts are
+// read twice and the offsets written once.  Below that size a scan is launch
+// latency: 9.6 us in three launches, 6.4 us in two (ncu, 10 k counts).
 // Integer addition is associative, so the result is deterministic.
 #include "dem_ctx.cuh"
 
@@ -11,6 +15,7 @@ namespace {
 constexpr int SCAN_THREADS = 512;
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+constexpr uint64_t SCAN_DIRECT = 1024;
 
 __device__ inline uint32_t warp_incl_scan(uint32_t v) {
   const int lane = threadIdx.x & 31;
@@ -71,6 +76,8 @@ __global__ void k_scan_tiles(uint32_t* __restrict__ tile_sum, uint64_t ntiles, u
   if (threadIdx.x == 0) *out_total = carry;
 }
 
+// Direct: tile_off holds the tiles' totals, and the last block writes out[n]
+template <bool Direct>
 __global__ void k_scan_apply(const uint32_t* __restrict__ in, uint64_t n, const uint32_t* __restrict__ tile_off,
                              uint32_t* __restrict__ out) {
   const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (uint64_t)threadIdx.x * SCAN_ITEMS;
@@ -81,7 +88,17 @@ __global__ void k_scan_apply(const uint32_t* __restrict__ in, uint64_t n, const 
     v[k] = base + k < n ? in[base + k] : 0u;
     s += v[k];
   }
-  uint32_t ex = block_excl_scan(s, nullptr) + tile_off[blockIdx.x];
+  uint32_t before = 0;
+  if (Direct) {
+    uint32_t mine = 0;
+    for (uint32_t t = threadIdx.x; t < blockIdx.x; t += SCAN_THREADS) mine += tile_off[t];
+    block_excl_scan(mine, &before);
+  } else {
+    before = tile_off[blockIdx.x];
+  }
+  uint32_t tot;
+  uint32_t ex = block_excl_scan(s, &tot) + before;
+  if (Direct && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = before + tot;
 #pragma unroll
   for (int k = 0; k < SCAN_ITEMS; k++) {
     if (base + k < n) out[base + k] = ex;
@@ -112,10 +129,15 @@ int scan_exclusive_u32(dem_ctx* c, const uint32_t* in, uint32_t* out, uint64_t n
     DEM_CUDA_TRY(c, cudaMalloc(&c->scan_blk, ntiles * sizeof(uint32_t)));
     c->scan_cap = ntiles;
   }
-  ProfScope ps(c, K_SCAN, 3);
+  const bool direct = ntiles <= SCAN_DIRECT;
+  ProfScope ps(c, K_SCAN, direct ? 2 : 3);
   k_tile_sums<<<(unsigned)ntiles, SCAN_THREADS, 0, c->stream>>>(in, n, c->scan_blk);
-  k_scan_tiles<<<1, SCAN_THREADS, 0, c->stream>>>(c->scan_blk, ntiles, out + n);
-  k_scan_apply<<<(unsigned)ntiles, SCAN_THREADS, 0, c->stream>>>(in, n, c->scan_blk, out);
+  if (direct) {
+    k_scan_apply<true><<<(unsigned)ntiles, SCAN_THREADS, 0, c->stream>>>(in, n, c->scan_blk, out);
+  } else {
+    k_scan_tiles<<<1, SCAN_THREADS, 0, c->stream>>>(c->scan_blk, ntiles, out + n);
+    k_scan_apply<false><<<(unsigned)ntiles, SCAN_THREADS, 0, c->stream>>>(in, n, c->scan_blk, out);
+  }
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;
 }
