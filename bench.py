@@ -55,7 +55,7 @@ PARTICLE_BYTES_PER_STEP = 344
 PREROLL = {"spheres": 3000, "polyhedra": 0, "polyhedra_dense": 0, "drums": 0, "mixer": 300, "polyhedra_mesh": 0,
            "fragments": 0}
 # DRAM bytes (read + write) per launch of k_cfused per listed pair and of
-# k_fused_epilog per particle, from the ncu capture of the pre-rolled 250k-sphere
+# the integration (epilog) per particle, from the ncu capture of the pre-rolled 250k-sphere
 # bed (the same workload at 1/8 of its size); they scale with the listed pairs and
 # the particles.  Both kernels run their FP64 pipe at the fraction recorded here
 # (sm__pipe_fp64_cycles_active of peak sustained).
@@ -676,7 +676,7 @@ def run_native(args, rank, world, local, dist):
     achieved_i = PARTICLE_BYTES_PER_STEP * w.n / t_integ / 1e9 if t_integ > 0 else 0.0
     t_e = TRAFFIC["epilog_bytes_per_particle"]
     roofline_integration = {
-        "bound": "hbm", "kernel": "integration (k_fused_prolog + k_fused_epilog + rotation kernels)",
+        "bound": "hbm", "kernel": "integration (k_integrate + k_rotations)",
         "achieved": achieved_i, "peak": peak, "unit": "GB/s", "frac": achieved_i / peak, "peak_kind": peak_kind,
         "epilog_traffic": (t_e * w.n if fused_contact else None),
         "algorithmic_bytes_per_launch": PARTICLE_BYTES_PER_STEP * w.n,

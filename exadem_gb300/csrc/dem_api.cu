@@ -1099,7 +1099,8 @@ int dem_step(dem_ctx* c, int nsteps) {
   if ((rc = refresh_pair_damp(c))) return rc;  // contact parameters changed since the list was built
   if ((rc = ensure_mesh_bins(c))) return rc;    // before a graph capture of the rebuild
   // graph replay unless per-kernel timing is on (events cannot be recorded inside a graph)
-  if (c->prm.graph_step && c->prm.fused_step && !c->poly && nsteps > 0 && !c->prof_on) return step_graph(c, nsteps);
+  if (c->prm.graph_step && c->prm.fused_step && !c->poly && c->n && nsteps > 0 && !c->prof_on)
+    return step_graph(c, nsteps);
   for (int s = 0; s < nsteps; s++) {
     if (c->poly && c->prm.fused_step) {
       // prolog + vertex_displ_over decided in FP32; interface criterion (raises the

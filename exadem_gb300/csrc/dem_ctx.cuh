@@ -94,7 +94,7 @@ struct dem_ctx {
 
   // graph step (dem_graph.cu)
   bool capturing = false;                  // kernels launched now go into a graph
-  unsigned long long* d_gs = nullptr;      // [0] ni, [1] overflow, [2] rebuilds, [3] capacity
+  unsigned long long* d_gs = nullptr;      // counters of the graph step (GS_*)
   unsigned long long* d_ni = nullptr;      // = d_gs
   uint64_t gcap = 0;                       // interaction capacity the graph was captured with
   cudaGraph_t graph = nullptr;
@@ -135,7 +135,7 @@ struct dem_ctx {
   // compacted contact passes (rcap each): work lists and detection results
   uint32_t* L1 = nullptr;
   uint32_t* L2 = nullptr;
-  uint32_t* rot_list = nullptr;  // pcap: particles whose epilog rotation runs in k_epilog_rotation
+  uint32_t* rot_list = nullptr;  // pcap: particles whose rotations run in k_rotations
   bool damp_stale = false;       // contact parameters changed since the list's per-pair damping was set
   // analysis (dem_set_analysis): per-interaction contact state, rcap entries
   bool analysis = false;
@@ -346,6 +346,10 @@ void clear_bonds(dem_ctx* c);
 int launch_fused_prolog(dem_ctx* c);
 int launch_contact_compact(dem_ctx* c);
 int launch_fused_epilog(dem_ctx* c);
+int launch_graph_integrate(dem_ctx* c, cudaGraphConditionalHandle cond);  // inside a capture
+// counters of the graph step (dem_ctx::d_gs): interactions, overflow, rebuilds, capacity, steps begun in
+// this call, blocks of the integration that are done
+enum : int { GS_NI = 0, GS_OVERFLOW = 1, GS_REBUILDS = 2, GS_CAP = 3, GS_STEP = 4, GS_DONE = 5, GS_COUNT = 6 };
 }  // namespace dem
 
 inline unsigned grid_for(uint64_t n, unsigned block) { return (unsigned)((n + block - 1) / block); }

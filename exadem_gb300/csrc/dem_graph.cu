@@ -1,14 +1,19 @@
 // dem_graph.cu -- the fused sphere step replayed as one CUDA graph.
 //
 // One graph replay is one Verlet iteration of the reference deck
-// (data/config/main-config.msp compute_loop, numerical_scheme_verlet):
-//   memset(trigger); k_fused_prolog (prolog + particle_displ_over)
-//   k_set_cond: the trigger enables the conditional node
+// (data/config/main-config.msp compute_loop, numerical_scheme_verlet), its epilog
+// run by the next replay, or after the last one by a launch of its own:
+//   k_integrate: the previous step's epilog (not in a call's first replay), then
+//               prolog + particle_displ_over; its last block enables the
+//               conditional node and zeroes the contact pass's counters
 //   IF trigger: the neighbour rebuild (bin, sort, reorder, count, scan, fill
 //               with history carry-over, reverse lists)
-//   compacted contact law (screen, detect, Hooke); k_fused_epilog
+//   compacted contact law (screen, detection and law)
 // so a step needs no host synchronisation: dem_step replays the graph nsteps
-// times and reads the device counters once at the end.
+// times and reads the device counters once at the end.  A step without a rebuild
+// is three kernels (four with a rotation list) and the conditional node, where it
+// was seven kernels and five memsets: 23 of the 66 us of a 1 k box's step were the
+// gaps between them.
 //
 // A graph fixes its buffers, so inside it the particle and interaction double
 // buffers do not alternate: the rebuild writes the new order and the new list
@@ -32,44 +37,45 @@ int launch_contact_compact(dem_ctx* c);
 int launch_fused_epilog(dem_ctx* c);
 
 namespace {
-enum : int { GS_NI = 0, GS_OVERFLOW = 1, GS_REBUILDS = 2, GS_CAP = 3 };
-
-__global__ void k_set_cond(cudaGraphConditionalHandle h, const unsigned long long* flag) {
-  cudaGraphSetConditional(h, *flag ? 1u : 0u);
-}
-
-// size of the new list (exclusive scan total) against the capacity
-__global__ void k_graph_total(const uint32_t* __restrict__ off_new, uint64_t n, unsigned long long* gs) {
-  const unsigned long long total = off_new[n];
-  if (total > gs[GS_CAP]) {
-    gs[GS_OVERFLOW] = 1ull;
-    gs[GS_NI] = 0ull;
-  } else {
-    gs[GS_NI] = total;
-  }
-  gs[GS_REBUILDS] += 1ull;
-}
-
-// the new list (buffer 1) onto the current one (buffer 0); empty after an overflow
+// The new list (buffer 1) onto the current one (buffer 0), its size (the exclusive
+// scan's total) into the counters; empty when it exceeds the capacity.  Every record
+// is live again (new list indices).
 __global__ void k_graph_copy_list(IArrays dst, IArrays src, const uint32_t* __restrict__ off_src,
-                                  uint32_t* __restrict__ off_dst, uint64_t n, const unsigned long long* gs) {
-  const bool ovf = gs[GS_OVERFLOW] != 0ull;
-  const uint64_t ni = gs[GS_NI];
+                                  uint32_t* __restrict__ off_dst, uint64_t n, uint64_t cap,
+                                  uint8_t* __restrict__ live, unsigned long long* gs) {
+  const uint64_t total = off_src[n];
+  const bool ovf = total > cap;
+  const uint64_t ni = ovf ? 0 : total;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t0 == 0) {
+    if (ovf) gs[GS_OVERFLOW] = 1ull;
+    gs[GS_NI] = ni;
+    gs[GS_REBUILDS] += 1ull;
+  }
   for (uint64_t s = t0; s <= n; s += stride) off_dst[s] = ovf ? 0u : off_src[s];
-  for (uint64_t k = t0; k < ni; k += stride) {
-    dst.owner[k] = src.owner[k];
-    dst.partner[k] = src.partner[k];
-    dst.pid[k] = src.pid[k];
-    dst.meta[k] = src.meta[k];
-    dst.sub[k] = src.sub[k];
+  for (uint64_t k = t0; k < ni; k += stride) {  // loads first: they may not pass the stores
+    const uint32_t owner = src.owner[k], partner = src.partner[k], meta = src.meta[k], sub = src.sub[k];
+    const uint64_t pid = src.pid[k];
+    double h[7];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-      dst.ft[d][k] = src.ft[d][k];
-      dst.mo[d][k] = src.mo[d][k];
+      h[d] = src.ft[d][k];
+      h[3 + d] = src.mo[d][k];
     }
-    dst.damp[k] = src.damp[k];
+    h[6] = src.damp[k];
+    dst.owner[k] = owner;
+    dst.partner[k] = partner;
+    dst.pid[k] = pid;
+    dst.meta[k] = meta;
+    dst.sub[k] = sub;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      dst.ft[d][k] = h[d];
+      dst.mo[d][k] = h[3 + d];
+    }
+    dst.damp[k] = h[6];
+    live[k] = 1;
   }
 }
 
@@ -124,14 +130,12 @@ int rebuild_body(dem_ctx* c) {
   }
   if ((rc = launch_count_sphere(c))) return rc;
   if ((rc = scan_exclusive_u32(c, c->pcnt, c->own_off[1], n))) return rc;
-  k_graph_total<<<1, 1, 0, c->stream>>>(c->own_off[1], n, c->d_gs);
   if ((rc = launch_fill_sphere(c, c->own_off[1], 0))) return rc;  // into I[1], history from I[0]
   k_graph_copy_list<<<(unsigned)c->num_sms * 4u, 256, 0, c->stream>>>(c->I[0], c->I[1], c->own_off[1], c->own_off[0],
-                                                                       n, c->d_gs);
+                                                                       n, c->gcap, c->R.live, c->d_gs);
   DEM_CUDA_TRY(c, cudaGetLastError());
   if ((rc = launch_reverse_lists(c, fill_counts_partners(c)))) return rc;
-  if ((rc = mark_records_live(c))) return rc;  // new list indices: every record is stale
-  DEM_CUDA_TRY(c, cudaMemsetAsync(c->trig_dev, 0, c->nsys * sizeof(uint32_t), c->stream));
+  if (c->nsys > 1) DEM_CUDA_TRY(c, cudaMemsetAsync(c->trig_dev, 0, c->nsys * sizeof(uint32_t), c->stream));
   return DEM_OK;
 }
 
@@ -165,10 +169,8 @@ int build_graph(dem_ctx* c) {
   c->gcap = std::min(std::min(c->icap[0], c->icap[1]), c->rcap);
   // scan scratch for the largest scan of the step (no allocation inside a capture)
   if ((rc = scan_reserve(c, std::max<uint64_t>(c->ncell, c->n)))) return rc;
-  if (!c->d_gs) DEM_CUDA_TRY(c, cudaMalloc(&c->d_gs, 4 * sizeof(unsigned long long)));
+  if (!c->d_gs) DEM_CUDA_TRY(c, cudaMalloc(&c->d_gs, GS_COUNT * sizeof(unsigned long long)));
   c->d_ni = c->d_gs;
-  const unsigned long long gs0[4] = {c->ni, 0ull, 0ull, c->gcap};
-  DEM_CUDA_TRY(c, cudaMemcpyAsync(c->d_gs, gs0, sizeof(gs0), cudaMemcpyHostToDevice, st));
   DEM_CUDA_TRY(c, cudaStreamSynchronize(st));
 
   std::memset(c->graph_launches_per_step, 0, sizeof(c->graph_launches_per_step));
@@ -179,15 +181,11 @@ int build_graph(dem_ctx* c) {
   cudaGraphConditionalHandle h;
   DEM_CUDA_TRY(c, cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
   c->capturing = true;
-  // part 1: prolog + trigger + condition
+  // part 1: the previous step's epilog, this step's prolog, trigger and condition
   cudaGraphNode_t last = nullptr;
   {
     DEM_CUDA_TRY(c, cudaStreamBeginCaptureToGraph(st, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    rc = launch_fused_prolog(c);
-    if (!rc) {
-      k_set_cond<<<1, 1, 0, st>>>(h, c->d_scalars);
-      c->graph_launches_per_step[K_PROLOG] += 1;
-    }
+    rc = launch_graph_integrate(c, h);
     cudaStreamCaptureStatus status;
     const cudaGraphNode_t* deps = nullptr;
     size_t ndeps = 0;
@@ -225,11 +223,10 @@ int build_graph(dem_ctx* c) {
       return rc ? rc : c->fail(DEM_ERR_CUDA, "graph capture of the rebuild failed");
     }
   }
-  // part 3: contact + epilog after the conditional node
+  // part 3: contact after the conditional node
   {
     DEM_CUDA_TRY(c, cudaStreamBeginCaptureToGraph(st, g, &cn, nullptr, 1, cudaStreamCaptureModeThreadLocal));
     rc = launch_contact_compact(c);
-    if (!rc) rc = launch_fused_epilog(c);
     cudaGraph_t out = nullptr;
     const cudaError_t e = cudaStreamEndCapture(st, &out);
     c->capturing = false;
@@ -298,9 +295,11 @@ int step_graph(dem_ctx* c, int nsteps) {
     }
     const uint64_t ni0 = c->ni;
     if ((rc = snapshot(c, true))) return rc;
-    unsigned long long gs[4] = {c->ni, 0ull, 0ull, c->gcap};
+    unsigned long long gs[GS_COUNT] = {c->ni, 0ull, 0ull, c->gcap, 0ull, 0ull};
     DEM_CUDA_TRY(c, cudaMemcpyAsync(c->d_gs, gs, sizeof(gs), cudaMemcpyHostToDevice, c->stream));
+    DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars, 0, (SC_ROT_CNT + 1) * sizeof(unsigned long long), c->stream));
     for (int s = 0; s < nsteps; s++) DEM_CUDA_TRY(c, cudaGraphLaunch(c->gexec, c->stream));
+    if ((rc = launch_fused_epilog(c))) return rc;  // of the last step
     DEM_CUDA_TRY(c, cudaMemcpyAsync(gs, c->d_gs, sizeof(gs), cudaMemcpyDeviceToHost, c->stream));
     DEM_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     if (!gs[GS_OVERFLOW]) {

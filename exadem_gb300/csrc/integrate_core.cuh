@@ -185,53 +185,39 @@ __device__ __forceinline__ ProlState prolog_math(R& rm, L& lm, const ProlState& 
   return o;
 }
 
-// Split form of the fused sphere prolog.  prolog_cheap: the translation and,
-// for a spin-free particle, its rotational half; returns true when the
-// particle spins (its rotational half is left to prolog_rotation).  The two
-// halves read disjoint inputs and write disjoint outputs, so running them in
-// separate launches gives the same bits as prolog_math.
+// Rotational half of the prolog of a spin-free particle (spin_free_step); returns
+// false, with nothing done, for any other: its half is left to prolog_rotation.  The
+// translational and rotational halves read disjoint inputs and write disjoint
+// outputs, so running them apart gives the same bits as prolog_math.
 template <int Mode>
-__device__ __forceinline__ bool prolog_cheap(const PArrays& P, uint64_t s, double delta_t, double half_delta_t,
-                                             double delta_t2_2) {
+__device__ __forceinline__ bool prolog_spin_free(const PArrays& P, uint64_t s, double delta_t, double half_delta_t) {
   const Q4 q0 = {P.f[QW][s], P.f[QX][s], P.f[QY][s], P.f[QZ][s]};
   const V3 w0 = mk(P.f[WX][s], P.f[WY][s], P.f[WZ][s]);
-  const bool spin_free = spin_free_step(q0, w0, delta_t);
-  auto run = [&](auto& rm, auto& lm, V3& r, V3& v, Q4& q, V3& w) {
-    r = mk(P.f[RX][s], P.f[RY][s], P.f[RZ][s]);
-    v = mk(P.f[VX][s], P.f[VY][s], P.f[VZ][s]);
-    transl_math_z(lm, r, v, mk(P.f[FX][s], P.f[FY][s], P.f[FZ][s]), delta_t, half_delta_t, delta_t2_2);
+  if (!spin_free_step(q0, w0, delta_t)) return false;
+  auto run = [&](auto& rm, auto& lm, Q4& q, V3& w) {
     q = {P.f[QW][s], P.f[QX][s], P.f[QY][s], P.f[QZ][s]};
     w = mk(P.f[WX][s], P.f[WY][s], P.f[WZ][s]);
-    if (spin_free)
-      quat_math<std::remove_reference_t<decltype(rm)>, std::remove_reference_t<decltype(lm)>, true>(
-          rm, lm, q, w, mk(P.f[AX][s], P.f[AY][s], P.f[AZ][s]), true, delta_t, half_delta_t);
+    quat_math<std::remove_reference_t<decltype(rm)>, std::remove_reference_t<decltype(lm)>, true>(
+        rm, lm, q, w, mk(P.f[AX][s], P.f[AY][s], P.f[AZ][s]), true, delta_t, half_delta_t);
   };
   RotMul<Mode> rm;
   LinMul<Mode> lm;
-  V3 r, v, w;
   Q4 q;
-  run(rm, lm, r, v, q, w);
+  V3 w;
+  run(rm, lm, q, w);
   if (rm.failed() || lm.failed()) {
     asm volatile("" ::: "memory");  // nothing is stored yet: reload
     MulFP64 n;
-    run(n, n, r, v, q, w);
+    run(n, n, q, w);
   }
-  P.f[RX][s] = r.x;
-  P.f[RY][s] = r.y;
-  P.f[RZ][s] = r.z;
-  P.f[VX][s] = v.x;
-  P.f[VY][s] = v.y;
-  P.f[VZ][s] = v.z;
-  if (spin_free) {
-    P.f[QW][s] = q.w;
-    P.f[QX][s] = q.x;
-    P.f[QY][s] = q.y;
-    P.f[QZ][s] = q.z;
-    P.f[WX][s] = w.x;
-    P.f[WY][s] = w.y;
-    P.f[WZ][s] = w.z;
-  }
-  return !spin_free;
+  P.f[QW][s] = q.w;
+  P.f[QX][s] = q.x;
+  P.f[QY][s] = q.y;
+  P.f[QZ][s] = q.z;
+  P.f[WX][s] = w.x;
+  P.f[WY][s] = w.y;
+  P.f[WZ][s] = w.z;
+  return true;
 }
 
 template <int Mode>

@@ -14,8 +14,8 @@
 //                 overlapping pairs append (k, dn, n, cp) to list L2;
 //      k_chooke   dense over L2: the full Hooke law with friction and rolling.
 //  * the divisions by mass and inertia use exact reciprocal-based division
-//    (math_exact.cuh) and reset + gravity + gather + force_to_accel + epilog
-//    are one kernel, prolog + displacement trigger another.
+//    (math_exact.cuh) and reset + gravity + gather + force_to_accel + epilog,
+//    with the next step's prolog + displacement trigger, are one kernel.
 // Order of summation, operation order and rounding are those of the operator
 // kernels (contact_core.cuh, integrate_core.cuh).
 #include <algorithm>
@@ -66,6 +66,7 @@ struct CArgs {
   uint64_t l1cap;           // L1 entries: particle pairs from the front, driver pairs from the back
   int int_share;            // k_cfused: Hooke tiles out of 8 run with AllInt (the integer pipe)
   unsigned long long* n_active;
+  unsigned long long* rot_cnt;  // graph step: the rotation list, run before this pass, is emptied by the screen
 };
 
 // L1 as one list: the particle pairs (front, n1 of them), then the driver pairs
@@ -137,6 +138,7 @@ __device__ __forceinline__ float trunc_f32(double x, bool& ok) {
 
 __global__ void __launch_bounds__(FT) k_cscreen(CArgs a) {
   const uint64_t ni = a.ni_dev ? *a.ni_dev : a.ni;
+  if (a.rot_cnt && blockIdx.x == 0 && threadIdx.x == 0) *a.rot_cnt = 0ull;
   const uint64_t stride = (uint64_t)gridDim.x * FT;
   for (uint64_t base = (uint64_t)blockIdx.x * FT; base < ni; base += stride) {
   const uint64_t k = base + threadIdx.x;
@@ -514,164 +516,200 @@ __device__ __forceinline__ bool displ_over(V3 r, V3 b, double thr2, float thr2f)
   return emu_ge_nonneg(dx * dx + dy * dy + dz * dz, thr2);  // >= on the integer pipe
 }
 
-// prolog + displacement trigger.  Every particle gets its translation and, when
-// it does not spin, its (exact, integer sign logic) quaternion step here; the
-// spinning particles run the full quaternion update in place when most of their
-// warp spins, otherwise through prl_list in k_prolog_rotation, so sparse
-// spinning particles do not hold whole warps on the FP64 pipe.  The trigger
-// depends on positions only.
-template <int Mode>
-__global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_fused_prolog(PArrays P, uint64_t n, double delta_t,
-                                                                     double half_delta_t, double delta_t2_2,
-                                                                     double thr2, float thr2f, unsigned long long* flag,
-                                                                     SysView sv, uint32_t* prl_list,
-                                                                     unsigned long long* prl_cnt, int dense) {
-  const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  bool over = false, need = false;
-  if (s < n) {
-    need = prolog_cheap<Mode>(P, s, delta_t, half_delta_t, delta_t2_2);
-    over = displ_over(mk(P.f[RX][s], P.f[RY][s], P.f[RZ][s]), mk(P.f[BX][s], P.f[BY][s], P.f[BZ][s]), thr2,
-                       thr2f);
-    if (over && sv.nsys > 1) atomicOr(&sv.trig[sv.of(s)], 1u);  // this system's own trigger
-  }
-  if (__any_sync(0xffffffffu, over) && (threadIdx.x & 31) == 0) atomicOr(flag, 1ull);
-  const unsigned busy = __ballot_sync(0xffffffffu, need);
-  if (__popc(busy) > dense) {
-    if (need) prolog_rotation<Mode>(P, s, delta_t, half_delta_t);
-  } else {
-    const uint32_t pos = warp_append(need, prl_cnt);
-    if (need) prl_list[pos] = (uint32_t)s;
-  }
-}
+struct IntegArgs {
+  PArrays P;
+  Records R;
+  uint64_t n;
+  const uint32_t* own_off;
+  const uint32_t* rev_off;
+  const uint32_t* rev_idx;
+  double g[3];
+  double dt, hdt, dt2_2;  // dt, dt/2, dt^2/2
+  double thr2;
+  float thr2f;
+  SysView sv;
+  uint32_t* list;             // particles whose rotations run in k_rotations
+  unsigned long long* scal;   // device scalars (flag, active contacts, work list and rotation list counts)
+  int dense;
+  int epilog, prolog;
+  unsigned long long* gs;     // graph step: its counters; epilog is then "not the call's first step"
+  cudaGraphConditionalHandle cond;
+};
+constexpr uint32_t ROT_EPILOG = 0x80000000u;  // list entry whose epilog rotation is due too
 
-// the rotational half of the prolog for the particles listed by k_fused_prolog
-template <int Mode>
-__global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_prolog_rotation(PArrays P, const uint32_t* __restrict__ list,
-                                                                        const unsigned long long* cnt, double delta_t,
-                                                                        double half_delta_t) {
-  const uint64_t m = *cnt;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < m; w += stride)
-    prolog_rotation<Mode>(P, list[w], delta_t, half_delta_t);
-}
-
-// reset_force_moment + gravity_force + contact gather + force_to_accel + epilog.
-// The velocity half of the epilog runs here for every particle.  The
-// rotational half is exactly zero for a particle without spin and torque
-// (rotation_idle); the others run it here when most of their warp needs it,
-// otherwise they are appended to rot_list for k_epilog_rotation, so sparse
-// rotating particles do not hold whole warps on the FP64 pipe.
+// The integration: reset_force_moment + gravity_force + contact gather +
+// force_to_accel + epilog of a step (epilog), then the prolog and the displacement
+// trigger of the next (prolog).  In the graph step one launch does both, so a
+// particle's velocity and acceleration stay in registers and a step has one launch
+// fewer; the host-launched step and the ends of a call run the halves apart.
+//
+// The rotational halves are exactly idle or integer logic for many particles
+// (rotation_idle, spin_free_step); the others run them here when more than `dense`
+// lanes of their warp need it, otherwise they are appended to a list for
+// k_rotations, so sparse rotating particles do not hold whole warps on the FP64 pipe.
+// The trigger depends on positions only.
+//
+// In the graph the last block to finish does what four memsets and a kernel of one
+// thread did: it hands the flag to the conditional rebuild and zeroes the counters
+// of the coming contact pass.
 // Mode != 0: the integer-pipe multiplies raise register use; at most 80
 // registers keep 3 blocks of 256 per SM (measured faster than 2 blocks)
 template <int Mode>
-__global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_fused_epilog(PArrays P, Records R, uint64_t n,
-                                                                     const uint32_t* __restrict__ own_off,
-                                                                     const uint32_t* __restrict__ rev_off,
-                                                                     const uint32_t* __restrict__ rev_idx,
-                                                                     double gx, double gy, double gz,
-                                                                     double half_delta_t, uint32_t* rot_list,
-                                                                     unsigned long long* rot_cnt, int dense) {
+__global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_integrate(IntegArgs a) {
+  const PArrays& P = a.P;
+  const Records& R = a.R;
   const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  bool need = false;
-  V3 mom = mk(0.0, 0.0, 0.0);
-  if (s < n) {
-    const double m = P.f[MASS][s];
-    // 0.0 + g_c m is +0 for g_c = +-0 and a finite m (+0 + +-0 = +0): no FP64 work
-    const bool mfin = ((emu_bits(m) >> 52) & 0x7ffu) != 0x7ffu;
-    V3 f = mk(emu_is_zero(gx) && mfin ? 0.0 : 0.0 + gx * m, emu_is_zero(gy) && mfin ? 0.0 : 0.0 + gy * m,
-              emu_is_zero(gz) && mfin ? 0.0 : 0.0 + gz * m);
-    // f and mom start at +0 or a nonzero value and, in round to nearest, never
-    // become -0 (x + (-x) = +0; -0 needs two -0 operands), so a record whose six
-    // components are all +-0 (a listed pair that does not touch) leaves them
-    // unchanged bit for bit and its additions are skipped.
-    // (a record whose live flag is 0 is zero and is not read)
-    // The owned records, then the partner records, in one loop: a particle's
-    // owned and partner counts vary a lot (by id order), their sum (its
-    // neighbour count) much less, so one loop keeps the warp's FP64 adds on
-    // most lanes.  The order of the additions is that of two loops.
-    const uint32_t o0 = own_off[s], no = own_off[s + 1] - o0;
-    const uint32_t r0 = rev_off[s], nt = no + (rev_off[s + 1] - r0);
-    for (uint32_t m = 0; m < nt; m++) {
-      const bool own = m < no;
-      const uint32_t k = own ? o0 + m : rev_idx[r0 + (m - no)];
-      if (!R.live[k]) continue;
-      const double* t0 = own ? R.ti[0] : R.tj[0];
-      const double* t1 = own ? R.ti[1] : R.tj[1];
-      const double* t2 = own ? R.ti[2] : R.tj[2];
-      const V3 rf = mk(R.f[0][k], R.f[1][k], R.f[2][k]), rt = mk(t0[k], t1[k], t2[k]);
-      if (((emu_bits(rf.x) | emu_bits(rf.y) | emu_bits(rf.z) | emu_bits(rt.x) | emu_bits(rt.y) | emu_bits(rt.z))
-           << 1) != 0) {
-        const uint64_t flip = own ? 0ull : 0x8000000000000000ull;  // -rf for a partner record (exact)
-        f = f + mk(emu_double(emu_bits(rf.x) ^ flip), emu_double(emu_bits(rf.y) ^ flip),
-                   emu_double(emu_bits(rf.z) ^ flip));
-        mom = mom + rt;
+  const bool epi = a.gs ? a.gs[GS_STEP] != 0ull : a.epilog != 0;
+  const bool pro = a.prolog != 0;
+  const bool mine = s < a.n;
+  V3 v = mk(0.0, 0.0, 0.0), acc = v;
+  bool late = false;  // the epilog's rotation is due in k_rotations
+  if (epi) {
+    bool need = false;
+    V3 mom = mk(0.0, 0.0, 0.0);
+    if (mine) {
+      const double m = P.f[MASS][s];
+      // 0.0 + g_c m is +0 for g_c = +-0 and a finite m (+0 + +-0 = +0): no FP64 work
+      const bool mfin = ((emu_bits(m) >> 52) & 0x7ffu) != 0x7ffu;
+      V3 f = mk(emu_is_zero(a.g[0]) && mfin ? 0.0 : 0.0 + a.g[0] * m, emu_is_zero(a.g[1]) && mfin ? 0.0 : 0.0 + a.g[1] * m,
+                emu_is_zero(a.g[2]) && mfin ? 0.0 : 0.0 + a.g[2] * m);
+      // f and mom start at +0 or a nonzero value and, in round to nearest, never
+      // become -0 (x + (-x) = +0; -0 needs two -0 operands), so a record whose six
+      // components are all +-0 (a listed pair that does not touch) leaves them
+      // unchanged bit for bit and its additions are skipped.
+      // (a record whose live flag is 0 is zero and is not read)
+      // The owned records, then the partner records, in one loop: a particle's
+      // owned and partner counts vary a lot (by id order), their sum (its
+      // neighbour count) much less, so one loop keeps the warp's FP64 adds on
+      // most lanes.  The order of the additions is that of two loops.
+      const uint32_t o0 = a.own_off[s], no = a.own_off[s + 1] - o0;
+      const uint32_t r0 = a.rev_off[s], nt = no + (a.rev_off[s + 1] - r0);
+      for (uint32_t q = 0; q < nt; q++) {
+        const bool own = q < no;
+        const uint32_t k = own ? o0 + q : a.rev_idx[r0 + (q - no)];
+        if (!R.live[k]) continue;
+        const double* t0 = own ? R.ti[0] : R.tj[0];
+        const double* t1 = own ? R.ti[1] : R.tj[1];
+        const double* t2 = own ? R.ti[2] : R.tj[2];
+        const V3 rf = mk(R.f[0][k], R.f[1][k], R.f[2][k]), rt = mk(t0[k], t1[k], t2[k]);
+        if (((emu_bits(rf.x) | emu_bits(rf.y) | emu_bits(rf.z) | emu_bits(rt.x) | emu_bits(rt.y) | emu_bits(rt.z))
+             << 1) != 0) {
+          const uint64_t flip = own ? 0ull : 0x8000000000000000ull;  // -rf for a partner record (exact)
+          f = f + mk(emu_double(emu_bits(rf.x) ^ flip), emu_double(emu_bits(rf.y) ^ flip),
+                     emu_double(emu_bits(rf.z) ^ flip));
+          mom = mom + rt;
+        }
+      }
+      const double im = P.f[IMASS][s];
+      LinMul<Mode> lm;
+      acc = mk(div_rn_m(lm, f.x, m, im), div_rn_m(lm, f.y, m, im), div_rn_m(lm, f.z, m, im));
+      const V3 vel = mk(P.f[VX][s], P.f[VY][s], P.f[VZ][s]);
+      // v + a dt/2: a zero a gives the zero addend of emu_add_zero (integer pipe)
+      const bool hok = emu_nonneg_finite(a.hdt);
+      auto vstep = [&](double vc, double ac) {
+        if (hok && emu_is_zero(ac)) {
+          bool ok;
+          const double r = emu_add_zero(vc, emu_sign(ac), ok);
+          if (ok) return r;
+        }
+        return vc + lm.mul(ac, a.hdt);
+      };
+      v = mk(vstep(vel.x, acc.x), vstep(vel.y, acc.y), vstep(vel.z, acc.z));
+      if (lm.failed()) {
+        acc = mk(div_rn(f.x, m, im), div_rn(f.y, m, im), div_rn(f.z, m, im));
+        v = mk(vel.x + acc.x * a.hdt, vel.y + acc.y * a.hdt, vel.z + acc.z * a.hdt);
+      }
+      P.f[FX][s] = acc.x;
+      P.f[FY][s] = acc.y;
+      P.f[FZ][s] = acc.z;
+      P.f[MX][s] = mom.x;
+      P.f[MY][s] = mom.y;
+      P.f[MZ][s] = mom.z;
+      if (!pro) {
+        P.f[VX][s] = v.x;
+        P.f[VY][s] = v.y;
+        P.f[VZ][s] = v.z;
+      }
+      const V3 vrot = mk(P.f[WX][s], P.f[WY][s], P.f[WZ][s]);
+      need = true;
+      if ((emu_bits(mom.x) | emu_bits(mom.y) | emu_bits(mom.z)) == 0) {
+        const Q4 Q = {P.f[QW][s], P.f[QX][s], P.f[QY][s], P.f[QZ][s]};
+        const V3 I = mk(P.f[IX][s], P.f[IY][s], P.f[IZ][s]);
+        const V3 II = mk(P.f[IIX][s], P.f[IIY][s], P.f[IIZ][s]);
+        if (rotation_idle(Q, vrot, mom, I, II)) {
+          need = false;
+          P.f[AX][s] = 0.0;
+          P.f[AY][s] = 0.0;
+          P.f[AZ][s] = 0.0;
+          // w + (+0): w itself, +0 for a -0
+          if (emu_bits(vrot.x) == 0x8000000000000000ull) P.f[WX][s] = 0.0;
+          if (emu_bits(vrot.y) == 0x8000000000000000ull) P.f[WY][s] = 0.0;
+          if (emu_bits(vrot.z) == 0x8000000000000000ull) P.f[WZ][s] = 0.0;
+        }
       }
     }
-    const double im = P.f[IMASS][s];
-    LinMul<Mode> lm;
-    V3 acc = mk(div_rn_m(lm, f.x, m, im), div_rn_m(lm, f.y, m, im), div_rn_m(lm, f.z, m, im));
-    const V3 vel = mk(P.f[VX][s], P.f[VY][s], P.f[VZ][s]);
-    // v + a dt/2: a zero a gives the zero addend of emu_add_zero (integer pipe)
-    const bool hok = emu_nonneg_finite(half_delta_t);
-    auto vstep = [&](double vc, double ac) {
-      if (hok && emu_is_zero(ac)) {
-        bool ok;
-        const double r = emu_add_zero(vc, emu_sign(ac), ok);
-        if (ok) return r;
-      }
-      return vc + lm.mul(ac, half_delta_t);
-    };
-    V3 v = mk(vstep(vel.x, acc.x), vstep(vel.y, acc.y), vstep(vel.z, acc.z));
-    if (lm.failed()) {
-      acc = mk(div_rn(f.x, m, im), div_rn(f.y, m, im), div_rn(f.z, m, im));
-      v = mk(vel.x + acc.x * half_delta_t, vel.y + acc.y * half_delta_t, vel.z + acc.z * half_delta_t);
-    }
-    P.f[FX][s] = acc.x;
-    P.f[FY][s] = acc.y;
-    P.f[FZ][s] = acc.z;
-    P.f[MX][s] = mom.x;
-    P.f[MY][s] = mom.y;
-    P.f[MZ][s] = mom.z;
-    P.f[VX][s] = v.x;
-    P.f[VY][s] = v.y;
-    P.f[VZ][s] = v.z;
-    const V3 vrot = mk(P.f[WX][s], P.f[WY][s], P.f[WZ][s]);
-    need = true;
-    if ((emu_bits(mom.x) | emu_bits(mom.y) | emu_bits(mom.z)) == 0) {
-      const Q4 Q = {P.f[QW][s], P.f[QX][s], P.f[QY][s], P.f[QZ][s]};
-      const V3 I = mk(P.f[IX][s], P.f[IY][s], P.f[IZ][s]);
-      const V3 II = mk(P.f[IIX][s], P.f[IIY][s], P.f[IIZ][s]);
-      if (rotation_idle(Q, vrot, mom, I, II)) {
-        need = false;
-        P.f[AX][s] = 0.0;
-        P.f[AY][s] = 0.0;
-        P.f[AZ][s] = 0.0;
-        // w + (+0): w itself, +0 for a -0
-        if (emu_bits(vrot.x) == 0x8000000000000000ull) P.f[WX][s] = 0.0;
-        if (emu_bits(vrot.y) == 0x8000000000000000ull) P.f[WY][s] = 0.0;
-        if (emu_bits(vrot.z) == 0x8000000000000000ull) P.f[WZ][s] = 0.0;
-      }
-    }
+    late = __popc(__ballot_sync(0xffffffffu, need)) <= a.dense && need;
+    if (need && !late) epilog_rotation<Mode>(P, s, a.hdt, mom);
   }
-  const unsigned busy = __ballot_sync(0xffffffffu, need);
-  if (__popc(busy) > dense) {
-    if (need) epilog_rotation<Mode>(P, s, half_delta_t, mom);
-  } else {
-    const uint32_t pos = warp_append(need, rot_cnt);
-    if (need) rot_list[pos] = (uint32_t)s;
+  bool over = false, turn = false;
+  if (pro && mine) {
+    if (!epi) {
+      v = mk(P.f[VX][s], P.f[VY][s], P.f[VZ][s]);
+      acc = mk(P.f[FX][s], P.f[FY][s], P.f[FZ][s]);
+    }
+    const V3 r0 = mk(P.f[RX][s], P.f[RY][s], P.f[RZ][s]);
+    LinMul<Mode> lm;
+    V3 r = r0, u = v;
+    transl_math_z(lm, r, u, acc, a.dt, a.hdt, a.dt2_2);
+    if (lm.failed()) {
+      MulFP64 nm;
+      r = r0;
+      u = v;
+      transl_math_z(nm, r, u, acc, a.dt, a.hdt, a.dt2_2);
+    }
+    P.f[RX][s] = r.x;
+    P.f[RY][s] = r.y;
+    P.f[RZ][s] = r.z;
+    P.f[VX][s] = u.x;
+    P.f[VY][s] = u.y;
+    P.f[VZ][s] = u.z;
+    if (!late) turn = !prolog_spin_free<Mode>(P, s, a.dt, a.hdt);
+    over = displ_over(r, mk(P.f[BX][s], P.f[BY][s], P.f[BZ][s]), a.thr2, a.thr2f);
+    if (over && a.sv.nsys > 1) atomicOr(&a.sv.trig[a.sv.of(s)], 1u);  // this system's own trigger
+  }
+  if (__any_sync(0xffffffffu, over) && (threadIdx.x & 31) == 0) atomicOr(a.scal, 1ull);
+  if (__popc(__ballot_sync(0xffffffffu, turn)) > a.dense && turn) {
+    prolog_rotation<Mode>(P, s, a.dt, a.hdt);
+    turn = false;
+  }
+  if (a.dense) {
+    const uint32_t pos = warp_append(late || turn, a.scal + SC_ROT_CNT);
+    if (late || turn) a.list[pos] = (uint32_t)s | (late ? ROT_EPILOG : 0u);
+  }
+  if (a.gs) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      if (atomicAdd(a.gs + GS_DONE, 1ull) == gridDim.x - 1) {  // every block's flag is in
+        const unsigned long long flag = atomicExch(a.scal, 0ull);
+        cudaGraphSetConditional(a.cond, flag ? 1u : 0u);
+        a.scal[1] = a.scal[3] = a.scal[4] = a.scal[5] = 0ull;  // active contacts, work list counts
+        a.gs[GS_DONE] = 0ull;
+        a.gs[GS_STEP] += 1ull;
+      }
+    }
   }
 }
 
-// the rotational half of the epilog for the particles listed by k_fused_epilog
+// the rotations listed by k_integrate: the epilog's where it is due, and the prolog's
 template <int Mode>
-__global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_epilog_rotation(PArrays P, const uint32_t* __restrict__ rot_list,
-                                                                        const unsigned long long* rot_cnt,
-                                                                        double half_delta_t) {
-  const uint64_t cnt = *rot_cnt;
+__global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_rotations(IntegArgs a) {
+  const uint64_t cnt = a.scal[SC_ROT_CNT];
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < cnt; w += stride) {
-    const uint32_t s = rot_list[w];
-    epilog_rotation<Mode>(P, s, half_delta_t, mk(P.f[MX][s], P.f[MY][s], P.f[MZ][s]));
+    const uint32_t e = a.list[w], s = e & ~ROT_EPILOG;
+    if (e & ROT_EPILOG) epilog_rotation<Mode>(a.P, s, a.hdt, mk(a.P.f[MX][s], a.P.f[MY][s], a.P.f[MZ][s]));
+    if (a.prolog && !prolog_spin_free<Mode>(a.P, s, a.dt, a.hdt)) prolog_rotation<Mode>(a.P, s, a.dt, a.hdt);
   }
 }
 
@@ -701,6 +739,7 @@ CArgs make_cargs(dem_ctx* c) {
   a.l1cap = c->rcap;
   a.int_share = c->tune_int_share;
   a.n_active = c->d_scalars + 1;
+  a.rot_cnt = c->capturing ? c->d_scalars + SC_ROT_CNT : nullptr;
   return a;
 }
 }  // namespace
@@ -720,33 +759,57 @@ static unsigned particle_block(const dem_ctx* c) {
   return b;
 }
 
-int launch_fused_prolog(dem_ctx* c) {
-  const double delta_t = c->prm.dt;
-  const double half_delta_t = delta_t * 0.5;
-  const double delta_t2_2 = delta_t * delta_t * 0.5;
+// cond: inside a capture, the handle of the conditional rebuild (both halves; the
+// first step of a call has no epilog)
+static int launch_integrate(dem_ctx* c, int epilog, int prolog, cudaGraphConditionalHandle cond) {
+  IntegArgs a;
+  a.P = c->P[c->pcur];
+  a.R = c->R;
+  a.n = c->n;
+  a.own_off = c->own_off[c->icur];
+  a.rev_off = c->rev_off;
+  a.rev_idx = c->rev_idx;
+  for (int d = 0; d < 3; d++) a.g[d] = c->prm.gravity[d];
+  a.dt = c->prm.dt;
+  a.hdt = a.dt * 0.5;
+  a.dt2_2 = a.dt * a.dt * 0.5;
   const double max_displ = c->prm.rcut_inc * 0.5;
-  const int dense = rotation_dense(c);
+  a.thr2 = max_displ * max_displ;
+  a.thr2f = (float)a.thr2;
+  a.sv = c->sysview();
+  a.list = c->rot_list;
+  a.scal = c->d_scalars;
+  a.dense = rotation_dense(c);
+  a.epilog = epilog;
+  a.prolog = prolog;
+  a.gs = c->capturing ? c->d_gs : nullptr;
+  a.cond = cond;
   const unsigned block = particle_block(c);
-  DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars, 0, sizeof(unsigned long long), c->stream));
-  unsigned long long* prl_cnt = c->d_scalars + SC_ROT_CNT;  // the rotation list is free until the epilog
-  if (dense) DEM_CUDA_TRY(c, cudaMemsetAsync(prl_cnt, 0, sizeof(unsigned long long), c->stream));
-  ProfScope ps(c, K_PROLOG, c->n ? (dense ? 2 : 1) : 0);
-  const auto kern = by_mode(c->mul_mode, k_fused_prolog<0>, k_fused_prolog<1>, k_fused_prolog<2>, k_fused_prolog<3>);
-  const auto krot = by_mode(c->mul_mode, k_prolog_rotation<0>, k_prolog_rotation<1>, k_prolog_rotation<2>,
-                            k_prolog_rotation<3>);
+  ProfScope ps(c, epilog ? K_EPILOG : K_PROLOG, c->n ? (a.dense ? 2 : 1) : 0);
+  if (!c->capturing && a.dense)
+    DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars + SC_ROT_CNT, 0, sizeof(unsigned long long), c->stream));
   if (c->n) {
-    kern<<<grid_for(c->n, block), block, 0, c->stream>>>(c->P[c->pcur], c->n, delta_t, half_delta_t, delta_t2_2,
-                                                         max_displ * max_displ, (float)(max_displ * max_displ), c->d_scalars, c->sysview(),
-                                                         c->rot_list, prl_cnt, dense);
-    if (dense) krot<<<(unsigned)c->num_sms * 3, 256, 0, c->stream>>>(c->P[c->pcur], c->rot_list, prl_cnt, delta_t,
-                                                            half_delta_t);
+    const auto kern = by_mode(c->mul_mode, k_integrate<0>, k_integrate<1>, k_integrate<2>, k_integrate<3>);
+    kern<<<grid_for(c->n, block), block, 0, c->stream>>>(a);
+    if (a.dense) {
+      const auto krot = by_mode(c->mul_mode, k_rotations<0>, k_rotations<1>, k_rotations<2>, k_rotations<3>);
+      krot<<<(unsigned)c->num_sms * 3, 256, 0, c->stream>>>(a);
+    }
   }
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;
 }
+int launch_fused_prolog(dem_ctx* c) {
+  DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars, 0, sizeof(unsigned long long), c->stream));
+  return launch_integrate(c, 0, 1, 0);
+}
+int launch_fused_epilog(dem_ctx* c) { return launch_integrate(c, 1, 0, 0); }
+int launch_graph_integrate(dem_ctx* c, cudaGraphConditionalHandle cond) { return launch_integrate(c, 1, 1, cond); }
 
 int launch_contact_compact(dem_ctx* c) {
-  DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars + 3, 0, 3 * sizeof(unsigned long long), c->stream));
+  // (in a graph the integration's last block zeroes these counts)
+  if (!c->capturing)
+    DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars + 3, 0, 3 * sizeof(unsigned long long), c->stream));
   const CArgs a = make_cargs(c);
   const unsigned persistent = (unsigned)c->num_sms * (unsigned)c->tune_contact_bps;
   {
@@ -757,7 +820,7 @@ int launch_contact_compact(dem_ctx* c) {
       k_cscreen<<<grid_for(c->ni, FT), FT, 0, c->stream>>>(a);
   }
   if (c->fuse_contact) {  // detection and law in one kernel (k_cfused)
-    DEM_CUDA_TRY(c, cudaMemsetAsync(a.n_active, 0, sizeof(unsigned long long), c->stream));
+    if (!c->capturing) DEM_CUDA_TRY(c, cudaMemsetAsync(a.n_active, 0, sizeof(unsigned long long), c->stream));
     ProfScope ps(c, K_CONTACT, 1);
     // mode bit 2: the contact law's multiplies on the integer pipe; int_share: a
     // share of its tiles with multiplies and additions there
@@ -777,22 +840,4 @@ int launch_contact_compact(dem_ctx* c) {
   return DEM_OK;
 }
 
-int launch_fused_epilog(dem_ctx* c) {
-  const int dense = rotation_dense(c);
-  const unsigned block = particle_block(c);
-  ProfScope ps(c, K_EPILOG, c->n ? (dense ? 2 : 1) : 0);
-  const auto kern = by_mode(c->mul_mode, k_fused_epilog<0>, k_fused_epilog<1>, k_fused_epilog<2>, k_fused_epilog<3>);
-  const auto krot = by_mode(c->mul_mode, k_epilog_rotation<0>, k_epilog_rotation<1>, k_epilog_rotation<2>,
-                            k_epilog_rotation<3>);
-  unsigned long long* rot_cnt = c->d_scalars + SC_ROT_CNT;
-  if (dense) DEM_CUDA_TRY(c, cudaMemsetAsync(rot_cnt, 0, sizeof(unsigned long long), c->stream));
-  if (c->n) {
-    kern<<<grid_for(c->n, block), block, 0, c->stream>>>(
-        c->P[c->pcur], c->R, c->n, c->own_off[c->icur], c->rev_off, c->rev_idx, c->prm.gravity[0],
-        c->prm.gravity[1], c->prm.gravity[2], c->prm.dt * 0.5, c->rot_list, rot_cnt, dense);
-    if (dense) krot<<<(unsigned)c->num_sms * 3, 256, 0, c->stream>>>(c->P[c->pcur], c->rot_list, rot_cnt, c->prm.dt * 0.5);
-  }
-  DEM_CUDA_TRY(c, cudaGetLastError());
-  return DEM_OK;
-}
 }  // namespace dem
