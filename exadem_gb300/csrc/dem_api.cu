@@ -513,11 +513,18 @@ int update_neighbors(dem_ctx* c) {
   return DEM_OK;
 }
 
+// The contact law of the operators: with fused_step the compacted kernels of the fused
+// step (same bits; the FP64 law on dense warps: 53 k bed 95 -> 45 us), which a
+// context without it keeps to the plain kernel.
+int sphere_contacts(dem_ctx* c) {
+  return c->prm.fused_step && c->n && c->ni ? launch_contact_compact(c, true) : launch_contact_sphere(c);
+}
+
 // gravity, contact laws, gather; then the inner bonds (config_fragmentation.msp compute_force)
 int compute_force(dem_ctx* c) {
   int rc;
   if ((rc = launch_gravity(c))) return rc;
-  if ((rc = c->poly ? launch_contact_poly(c) : launch_contact_sphere(c))) return rc;
+  if ((rc = c->poly ? launch_contact_poly(c) : sphere_contacts(c))) return rc;
   if ((rc = launch_gather_forces(c))) return rc;
   return c->poly ? launch_bond_force(c) : DEM_OK;
 }
@@ -532,12 +539,6 @@ int read_flag(dem_ctx* c, int idx) {
   DEM_CUDA_TRY(c, cudaMemcpyAsync(c->h_scalars + idx, c->d_scalars + idx, sizeof(unsigned long long),
                                   cudaMemcpyDeviceToHost, c->stream));
   DEM_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-  return DEM_OK;
-}
-
-int copy_field(dem_ctx* c, double* dst, const double* src, uint64_t n, cudaMemcpyKind k) {
-  if (!dst || !src || !n) return DEM_OK;
-  DEM_CUDA_TRY(c, cudaMemcpyAsync(dst, src, n * sizeof(double), k, c->stream));
   return DEM_OK;
 }
 
@@ -743,45 +744,53 @@ int dem_set_particles(dem_ctx* c, const dem_particles* p, int on_device) {
                             p->vrotz, p->arotx, p->aroty, p->arotz, p->momx, p->momy, p->momz, p->qw, p->qx,
                             p->qy, p->qz, p->inertiax, p->inertiay, p->inertiaz, p->mass, p->radius, p->homothety,
                             nullptr, nullptr, nullptr, nullptr, p->rx, p->ry, p->rz};
-  // defaults for absent fields: 0, except orientation w, inertia, mass and homothety = 1
-  std::vector<double> ones(n ? n : 1, 1.0);
+  // Arrays on the context's device go through one launch, others (host arrays, another
+  // device's, managed memory) through copies of their own.  Defaults for absent fields:
+  // 0, except orientation w, inertia, mass and homothety = 1.
+  CopyTab tab;
+  auto take = [&](void* dst, const void* from, size_t bytes) -> int {
+    if (!n) return DEM_OK;
+    if (on_device && device_memory(c, from)) {
+      tab.add(dst, from, bytes);
+    } else {
+      DEM_CUDA_TRY(c, cudaMemcpyAsync(dst, from, bytes, k, c->stream));
+    }
+    return DEM_OK;
+  };
+  constexpr uint64_t one = 0x3ff0000000000000ull;  // 1.0
   for (int f = 0; f < NPF; f++) {
     if (f >= IMASS && f <= IIZ) continue;  // derived below
     if (src[f]) {
-      if ((rc = copy_field(c, P.f[f], src[f], n, k))) return rc;
-    } else if (f == QW || f == IX || f == IY || f == IZ || f == MASS || f == HOM) {
-      if ((rc = copy_field(c, P.f[f], ones.data(), n, cudaMemcpyHostToDevice))) return rc;
-    } else if (n) {
-      DEM_CUDA_TRY(c, cudaMemsetAsync(P.f[f], 0, n * sizeof(double), c->stream));
+      if ((rc = take(P.f[f], src[f], n * sizeof(double)))) return rc;
+    } else {
+      tab.add(P.f[f], nullptr, n * sizeof(double),
+              f == QW || f == IX || f == IY || f == IZ || f == MASS || f == HOM ? one : 0ull);
     }
   }
   std::vector<uint64_t> ids;
   if (p->id) {
-    DEM_CUDA_TRY(c, cudaMemcpyAsync(P.id, p->id, n * 8, k, c->stream));
+    if ((rc = take(P.id, p->id, n * 8))) return rc;
   } else if (n) {
     ids.resize(n);
     std::iota(ids.begin(), ids.end(), 0ull);
     DEM_CUDA_TRY(c, cudaMemcpyAsync(P.id, ids.data(), n * 8, cudaMemcpyHostToDevice, c->stream));
   }
   if (p->type) {
-    DEM_CUDA_TRY(c, cudaMemcpyAsync(P.type, p->type, n * 4, k, c->stream));
+    if ((rc = take(P.type, p->type, n * 4))) return rc;
   } else if (n) {
     DEM_CUDA_TRY(c, cudaMemsetAsync(P.type, 0, n * 4, c->stream));
   }
   if (p->group) {
-    DEM_CUDA_TRY(c, cudaMemcpyAsync(P.group, p->group, n * 4, k, c->stream));
+    if ((rc = take(P.group, p->group, n * 4))) return rc;
   } else if (n) {
     DEM_CUDA_TRY(c, cudaMemsetAsync(P.group, 0, n * 4, c->stream));
   }
+  if ((rc = launch_copies(c, tab))) return rc;
   if ((rc = launch_reciprocals(c, n))) return rc;
   // r_max for nbh_dist (dem_rcut_max.cpp:49-66)
-  std::vector<double> rad(n);
-  if (n) {
-    DEM_CUDA_TRY(c, cudaMemcpyAsync(rad.data(), P.f[RAD], n * 8, cudaMemcpyDeviceToHost, c->stream));
-  }
-  DEM_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   double rmax = 0.0;
-  for (double r : rad) rmax = std::max(rmax, r);
+  if ((rc = launch_radius_max(c, P.f[RAD], n, &rmax))) return rc;
+  DEM_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   c->rad_max = rmax;
   c->n = n;
   c->systems.clear();
@@ -846,12 +855,23 @@ int dem_get_particles(dem_ctx* c, dem_particles* out, int on_device) {
                      out->vrotx, out->vroty, out->vrotz, out->arotx, out->aroty, out->arotz, out->momx,
                      out->momy, out->momz, out->qw, out->qx, out->qy, out->qz, out->inertiax, out->inertiay,
                      out->inertiaz, out->mass, out->radius, out->homothety};
+  CopyTab tab;  // as in dem_set_particles: arrays on the context's device in one launch
+  auto give = [&](void* to, const void* from, size_t bytes) -> int {
+    if (!to || !n) return DEM_OK;
+    if (on_device && device_memory(c, to)) {
+      tab.add(to, from, bytes);
+    } else {
+      DEM_CUDA_TRY(c, cudaMemcpyAsync(to, from, bytes, k, c->stream));
+    }
+    return DEM_OK;
+  };
   int rc;
   for (int f = 0; f < NUSER; f++)
-    if ((rc = copy_field(c, dst[f], P.f[f], n, k))) return rc;
-  if (out->id && n) DEM_CUDA_TRY(c, cudaMemcpyAsync(out->id, P.id, n * 8, k, c->stream));
-  if (out->type && n) DEM_CUDA_TRY(c, cudaMemcpyAsync(out->type, P.type, n * 4, k, c->stream));
-  if (out->group && n) DEM_CUDA_TRY(c, cudaMemcpyAsync(out->group, P.group, n * 4, k, c->stream));
+    if ((rc = give(dst[f], P.f[f], n * sizeof(double)))) return rc;
+  if ((rc = give(out->id, P.id, n * 8))) return rc;
+  if ((rc = give(out->type, P.type, n * 4))) return rc;
+  if ((rc = give(out->group, P.group, n * 4))) return rc;
+  if ((rc = launch_copies(c, tab))) return rc;
   DEM_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   out->n = n;
   return DEM_OK;
@@ -962,7 +982,7 @@ int dem_contact_sphere(dem_ctx* c) {
                    "(contact_force_sphere.cu.in:225-233)");
   int rc = need_list(c);
   if (rc) return rc;
-  if ((rc = launch_contact_sphere(c))) return rc;
+  if ((rc = sphere_contacts(c))) return rc;
   return launch_gather_forces(c);
 }
 

@@ -24,7 +24,7 @@ struct MlpState;  // k_mlp.cu
 // [3..4] compaction list counts, [8] learned-record overflows, [12] interfaces broken,
 // [16..23] learned bin counters and cursors (14 u32)
 constexpr int DEM_NSCALARS = 32;
-constexpr int SC_ROT_CNT = 6, SC_LEARNED_OVF = 8, SC_BROKEN = 12, SC_LEARNED_BINS = 16;
+constexpr int SC_ROT_CNT = 6, SC_RADMAX = 7, SC_LEARNED_OVF = 8, SC_BROKEN = 12, SC_LEARNED_BINS = 16;
 
 // features recorded per polyhedron unit by the count pass of the FP32-decided
 // enumeration; the fill pass copies them instead of deciding again
@@ -280,6 +280,26 @@ struct dem_ctx {
 };
 
 namespace dem {
+// k_copy.cu: several device-to-device copies (or fills) in one launch on the ctx stream
+struct CopyTab {
+  static constexpr int MAX = 48;
+  const void* src[MAX];  // nullptr: dst is filled with the 8-byte pattern fill
+  void* dst[MAX];
+  uint64_t bytes[MAX];
+  uint64_t fill[MAX];
+  int n = 0;
+  void add(void* d, const void* s, uint64_t b, uint64_t f = 0) {
+    if (!d || !b) return;
+    src[n] = s;
+    dst[n] = d;
+    bytes[n] = b;
+    fill[n] = f;
+    n++;
+  }
+};
+int launch_copies(dem_ctx* c, const CopyTab& t);
+int launch_radius_max(dem_ctx* c, const double* radius, uint64_t n, double* out);  // max(0, radii); waits
+bool device_memory(const dem_ctx* c, const void* p);  // memory of the ctx's device
 // k_scan.cu
 int scan_exclusive_u32(dem_ctx* c, const uint32_t* in, uint32_t* out, uint64_t n);
 // k_grid.cu
@@ -344,7 +364,8 @@ void free_bonds(dem_ctx* c);
 void clear_bonds(dem_ctx* c);
 // k_step_fused.cu
 int launch_fused_prolog(dem_ctx* c);
-int launch_contact_compact(dem_ctx* c);
+// overlap_only: a pair counts as active at dn < 0, as in the plain kernel, not at a driver's dn = 0
+int launch_contact_compact(dem_ctx* c, bool overlap_only = false);
 int launch_fused_epilog(dem_ctx* c);
 int launch_graph_integrate(dem_ctx* c, cudaGraphConditionalHandle cond);  // inside a capture
 // counters of the graph step (dem_ctx::d_gs): interactions, overflow, rebuilds, capacity, steps begun in
@@ -353,6 +374,13 @@ enum : int { GS_NI = 0, GS_OVERFLOW = 1, GS_REBUILDS = 2, GS_CAP = 3, GS_STEP = 
 }  // namespace dem
 
 inline unsigned grid_for(uint64_t n, unsigned block) { return (unsigned)((n + block - 1) / block); }
+// Threads per block for n threads: `block`, halved (to a warp at least) while the grid
+// leaves SMs without a block.  An SM's FP64 unit serves its warps in turn, so four warps
+// on each of 40 SMs take four times as long as one on each of 152.
+inline unsigned spread_block(const dem_ctx* c, uint64_t n, unsigned block) {
+  while (block > 32u && n < (uint64_t)block * (uint64_t)c->num_sms) block >>= 1;
+  return block;
+}
 
 // RAII scope around the launches of one kernel class on the ctx stream.
 struct ProfScope {

@@ -32,9 +32,6 @@ int launch_reorder_particles(dem_ctx* c);
 int launch_count_sphere(dem_ctx* c);
 int launch_fill_sphere(dem_ctx* c, uint32_t* new_off, uint64_t total);
 
-int launch_fused_prolog(dem_ctx* c);
-int launch_contact_compact(dem_ctx* c);
-int launch_fused_epilog(dem_ctx* c);
 
 namespace {
 // The new list (buffer 1) onto the current one (buffer 0), its size (the exclusive
@@ -77,6 +74,14 @@ __global__ void k_graph_copy_list(IArrays dst, IArrays src, const uint32_t* __re
     dst.damp[k] = h[6];
     live[k] = 1;
   }
+}
+
+// the counters of a call, and the scalars its first replay expects at zero
+__global__ void k_graph_begin(unsigned long long* gs, unsigned long long ni, unsigned long long cap,
+                              unsigned long long* scal) {
+  const int t = threadIdx.x;
+  if (t < GS_COUNT) gs[t] = t == GS_NI ? ni : (t == GS_CAP ? cap : 0ull);
+  if (t <= SC_ROT_CNT) scal[t] = 0ull;
 }
 
 size_t particle_block_bytes(const dem_ctx* c) {
@@ -250,29 +255,30 @@ int snapshot(dem_ctx* c, bool save) {
     c->snap_bytes = need + need / 4;
   }
   char* p = static_cast<char*>(c->snap);
-  const cudaMemcpyKind k = cudaMemcpyDeviceToDevice;
-  cudaStream_t st = c->stream;
-  auto mv = [&](void* dev, size_t bytes) -> cudaError_t {
-    const cudaError_t e = save ? cudaMemcpyAsync(p, dev, bytes, k, st) : cudaMemcpyAsync(dev, p, bytes, k, st);
+  CopyTab tab;  // one launch: 15 copies took 35 us of a call, whatever its size
+  auto mv = [&](void* dev, size_t bytes) {
+    if (save)
+      tab.add(p, dev, bytes);
+    else
+      tab.add(dev, p, bytes);
     p += (bytes + 15) & ~size_t(15);
-    return e;
   };
   IArrays& I = c->I[0];
-  DEM_CUDA_TRY(c, mv(c->pblock[0], pb));
-  DEM_CUDA_TRY(c, mv(c->own_off[0], (n + 1) * 4));
+  mv(c->pblock[0], pb);
+  mv(c->own_off[0], (n + 1) * 4);
   if (ni) {
-    DEM_CUDA_TRY(c, mv(I.owner, ni * 4));
-    DEM_CUDA_TRY(c, mv(I.partner, ni * 4));
-    DEM_CUDA_TRY(c, mv(I.pid, ni * 8));
-    DEM_CUDA_TRY(c, mv(I.meta, ni * 4));
-    DEM_CUDA_TRY(c, mv(I.sub, ni * 4));
+    mv(I.owner, ni * 4);
+    mv(I.partner, ni * 4);
+    mv(I.pid, ni * 8);
+    mv(I.meta, ni * 4);
+    mv(I.sub, ni * 4);
     for (int d = 0; d < 3; d++) {
-      DEM_CUDA_TRY(c, mv(I.ft[d], ni * 8));
-      DEM_CUDA_TRY(c, mv(I.mo[d], ni * 8));
+      mv(I.ft[d], ni * 8);
+      mv(I.mo[d], ni * 8);
     }
-    DEM_CUDA_TRY(c, mv(I.damp, ni * 8));
+    mv(I.damp, ni * 8);
   }
-  return DEM_OK;
+  return launch_copies(c, tab);
 }
 }  // namespace
 
@@ -295,12 +301,13 @@ int step_graph(dem_ctx* c, int nsteps) {
     }
     const uint64_t ni0 = c->ni;
     if ((rc = snapshot(c, true))) return rc;
-    unsigned long long gs[GS_COUNT] = {c->ni, 0ull, 0ull, c->gcap, 0ull, 0ull};
-    DEM_CUDA_TRY(c, cudaMemcpyAsync(c->d_gs, gs, sizeof(gs), cudaMemcpyHostToDevice, c->stream));
-    DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars, 0, (SC_ROT_CNT + 1) * sizeof(unsigned long long), c->stream));
+    k_graph_begin<<<1, 32, 0, c->stream>>>(c->d_gs, c->ni, c->gcap, c->d_scalars);
+    DEM_CUDA_TRY(c, cudaGetLastError());
     for (int s = 0; s < nsteps; s++) DEM_CUDA_TRY(c, cudaGraphLaunch(c->gexec, c->stream));
     if ((rc = launch_fused_epilog(c))) return rc;  // of the last step
-    DEM_CUDA_TRY(c, cudaMemcpyAsync(gs, c->d_gs, sizeof(gs), cudaMemcpyDeviceToHost, c->stream));
+    unsigned long long* const gs = c->h_scalars;  // pinned
+    static_assert(GS_COUNT <= 8, "h_scalars holds eight");
+    DEM_CUDA_TRY(c, cudaMemcpyAsync(gs, c->d_gs, GS_COUNT * sizeof(*gs), cudaMemcpyDeviceToHost, c->stream));
     DEM_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     if (!gs[GS_OVERFLOW]) {
       c->ni = gs[GS_NI];

@@ -1814,7 +1814,7 @@ __device__ __forceinline__ VView pview(const PCArgs& a, uint32_t s) {
 }
 
 __global__ void __launch_bounds__(PT) k_pdetect(PCArgs a) {
-  const uint64_t k = (uint64_t)blockIdx.x * PT + threadIdx.x;
+  const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   bool heavy = false;
   DetD d = det_none();
   if (k < a.ni) {
@@ -1973,8 +1973,8 @@ template <bool Fast>
 __global__ void __launch_bounds__(PT) k_phooke(PCArgs a) {
   const uint64_t n2 = a.cnt[1];
   if (blockIdx.x == 0 && threadIdx.x == 0) *a.n_active = n2 - a.cnt[2];
-  const uint64_t stride = (uint64_t)gridDim.x * PT;
-  for (uint64_t w = (uint64_t)blockIdx.x * PT + threadIdx.x; w < n2; w += stride) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < n2; w += stride) {
     const uint32_t k = a.L2[w];
     const double dn = a.D[0][w];
     const V3 n = mk(a.D[1][w], a.D[2][w], a.D[3][w]);
@@ -2080,7 +2080,8 @@ int launch_poly_fused_prolog(dem_ctx* c) {
   const double md = c->prm.rcut_inc * 0.5;
   const auto kern = by_mode(c->mul_mode, k_poly_fused_prolog<0>, k_poly_fused_prolog<1>, k_poly_fused_prolog<2>,
                             k_poly_fused_prolog<3>);
-  kern<<<grid_for(c->n, PT), PT, 0, c->stream>>>(a, dt, dt * 0.5, dt * dt * 0.5, md * md, (float)md, c->d_scalars);
+  const unsigned block = spread_block(c, c->n, PT);
+  kern<<<grid_for(c->n, block), block, 0, c->stream>>>(a, dt, dt * 0.5, dt * dt * 0.5, md * md, (float)md, c->d_scalars);
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;
 }
@@ -2109,7 +2110,8 @@ int launch_poly_vertices_listed(dem_ctx* c) {
   const PolyArgs a = make_pargs(c);
   const auto kern = by_mode(c->mul_mode, k_poly_vertices_listed<0>, k_poly_vertices_listed<1>,
                             k_poly_vertices_listed<2>, k_poly_vertices_listed<3>);
-  kern<<<grid_for(c->nvlist * (uint64_t)c->MV, PT), PT, 0, c->stream>>>(a, c->vlist, c->nvlist);
+  const unsigned block = spread_block(c, c->nvlist * (uint64_t)c->MV, PT);
+  kern<<<grid_for(c->nvlist * (uint64_t)c->MV, block), block, 0, c->stream>>>(a, c->vlist, c->nvlist);
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;
 }
@@ -2120,13 +2122,14 @@ int launch_poly_vertices(dem_ctx* c, int mode) {
   ProfScope ps(c, K_PROLOG, 1);
   const PolyArgs a = make_pargs(c);
   const double md = c->prm.rcut_inc * 0.5;
+  const unsigned block = spread_block(c, c->n, PT);
   if (mode == 1) {
     DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars, 0, sizeof(unsigned long long), c->stream));
-    k_poly_vertices<true, false><<<grid_for(c->n, PT), PT, 0, c->stream>>>(a, md * md, c->d_scalars);
+    k_poly_vertices<true, false><<<grid_for(c->n, block), block, 0, c->stream>>>(a, md * md, c->d_scalars);
   } else if (mode == 2) {
-    k_poly_vertices<false, true><<<grid_for(c->n, PT), PT, 0, c->stream>>>(a, 0.0, nullptr);
+    k_poly_vertices<false, true><<<grid_for(c->n, block), block, 0, c->stream>>>(a, 0.0, nullptr);
   } else {
-    k_poly_vertices<false, false><<<grid_for(c->n, PT), PT, 0, c->stream>>>(a, 0.0, nullptr);
+    k_poly_vertices<false, false><<<grid_for(c->n, block), block, 0, c->stream>>>(a, 0.0, nullptr);
   }
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;
@@ -2403,11 +2406,13 @@ int launch_contact_poly(dem_ctx* c) {
   for (int q = 0; q < 7; q++) a.D[q] = c->Dscr[q];
   a.cnt = c->d_scalars + 3;
   a.n_active = c->d_scalars + 1;
-  if (c->ni) k_pdetect<<<grid_for(c->ni, PT), PT, 0, c->stream>>>(a);
+  const unsigned block = spread_block(c, c->ni, PT);
+  if (c->ni) k_pdetect<<<grid_for(c->ni, block), block, 0, c->stream>>>(a);
+  const unsigned hb = (unsigned)std::min<uint64_t>(std::max<uint64_t>(grid_for(c->ni, block), 1), (uint64_t)c->num_sms * 8u * (PT / block));
   if (c->prm.fused_step)
-    k_phooke<true><<<(unsigned)c->num_sms * 8u, PT, 0, c->stream>>>(a);
+    k_phooke<true><<<hb, block, 0, c->stream>>>(a);
   else
-    k_phooke<false><<<(unsigned)c->num_sms * 8u, PT, 0, c->stream>>>(a);
+    k_phooke<false><<<hb, block, 0, c->stream>>>(a);
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;
 }

@@ -27,7 +27,7 @@
 namespace dem {
 namespace {
 
-constexpr int FT = 128;  // threads per block
+constexpr int FT = 128;  // threads per block of k_cdetect and k_chooke
 
 // All 32 lanes must call it.  Returns the slot of this lane when want is set.
 __device__ __forceinline__ uint32_t warp_append(bool want, unsigned long long* counter) {
@@ -66,6 +66,7 @@ struct CArgs {
   uint64_t l1cap;           // L1 entries: particle pairs from the front, driver pairs from the back
   int int_share;            // k_cfused: Hooke tiles out of 8 run with AllInt (the integer pipe)
   unsigned long long* n_active;
+  int overlap_only;             // a pair counts as active at dn < 0 only
   unsigned long long* rot_cnt;  // graph step: the rotation list, run before this pass, is emptied by the screen
 };
 
@@ -136,11 +137,11 @@ __device__ __forceinline__ float trunc_f32(double x, bool& ok) {
   return __uint_as_float(((e - 1023u + 127u) << 23) | ((uint32_t)(u >> 29) & 0x7fffffu));
 }
 
-__global__ void __launch_bounds__(FT) k_cscreen(CArgs a) {
+__global__ void __launch_bounds__(128) k_cscreen(CArgs a) {
   const uint64_t ni = a.ni_dev ? *a.ni_dev : a.ni;
   if (a.rot_cnt && blockIdx.x == 0 && threadIdx.x == 0) *a.rot_cnt = 0ull;
-  const uint64_t stride = (uint64_t)gridDim.x * FT;
-  for (uint64_t base = (uint64_t)blockIdx.x * FT; base < ni; base += stride) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < ni; base += stride) {
   const uint64_t k = base + threadIdx.x;
   bool want = false, drv = false;
   if (k < ni) {
@@ -395,9 +396,9 @@ __global__ void __launch_bounds__(FT, (Mode ? 4 : 1)) k_chooke(CArgs a) {
 
 // The law of queued pair idx of queue q (0: Hooke, 1: attraction); a share of
 // the Hooke tiles runs on the integer pipe, so both pipes work at once.
-template <int Mode, bool IntTiles>
+template <int Mode, bool IntTiles, int T>
 __device__ __forceinline__ void run_queued(const CArgs& a, int q, uint32_t idx, const uint32_t* qk,
-                                           const double (*qd)[2 * FT], uint32_t& tiles) {
+                                           const double (*qd)[2 * T], uint32_t& tiles) {
   const V3 n = mk(qd[1][idx], qd[2][idx], qd[3][idx]);
   const V3 cpos = mk(qd[4][idx], qd[5][idx], qd[6][idx]);
   if (q == 0) {
@@ -427,10 +428,12 @@ __device__ __forceinline__ void run_queued(const CArgs& a, int q, uint32_t idx, 
 // the epilog and the trigger a step of the 2 M bed went from 3.62 to 3.23 ms.
 // IntTiles: the instance with the integer-pipe tiles (int_share > 0); it needs
 // more registers, so the FP64-only instance stays the lean one.
-template <int Mode, bool IntTiles>
-__global__ void __launch_bounds__(FT, (Mode ? 4 : (IntTiles ? 3 : 1))) k_cfused(CArgs a) {
-  __shared__ uint32_t q_k[2][2 * FT];
-  __shared__ double q_d[2][7][2 * FT];
+// T: threads per block and pairs per tile, 128; or 32 for a small system, whose tiles
+// then reach every SM (launch_contact_compact).
+template <int Mode, bool IntTiles, int T>
+__global__ void __launch_bounds__(T, (T < 128 ? 1 : (Mode ? 4 : (IntTiles ? 3 : 1)))) k_cfused(CArgs a) {
+  __shared__ uint32_t q_k[2][2 * T];
+  __shared__ double q_d[2][7][2 * T];
   __shared__ uint32_t q_n[2], q_tot;
   if (threadIdx.x == 0) {
     q_n[0] = q_n[1] = 0;
@@ -438,11 +441,11 @@ __global__ void __launch_bounds__(FT, (Mode ? 4 : (IntTiles ? 3 : 1))) k_cfused(
   }
   __syncthreads();
   const uint64_t n1 = a.cnt[0], nl = n1 + a.cnt[2];
-  const uint64_t stride = (uint64_t)gridDim.x * FT;
+  const uint64_t stride = (uint64_t)gridDim.x * T;
   const int lane = threadIdx.x & 31;
   const uint32_t t = threadIdx.x;
   uint32_t tiles = 0;  // Hooke tiles run by this block (the same count in every thread)
-  for (uint64_t base = (uint64_t)blockIdx.x * FT; base < nl; base += stride) {  // the same trips for the block
+  for (uint64_t base = (uint64_t)blockIdx.x * T; base < nl; base += stride) {  // the same trips for the block
     const uint64_t w = base + threadIdx.x;
     int kind = PAIR_DONE;
     uint32_t k = 0;
@@ -457,13 +460,14 @@ __global__ void __launch_bounds__(FT, (Mode ? 4 : (IntTiles ? 3 : 1))) k_cfused(
       const bool mine = kind == (q == 0 ? PAIR_HOOKE : PAIR_ATTRACT);
       const unsigned mask = __ballot_sync(0xffffffffu, mine);
       uint32_t wb = 0;
+      const unsigned act = q == 0 ? __ballot_sync(0xffffffffu, mine && (!a.overlap_only || emu_lt0(dn))) : 0u;
+      if (lane == 0 && act) atomicAdd(&q_tot, (uint32_t)__popc(act));
       if (lane == 0 && mask) {
         wb = atomicAdd(&q_n[q], (uint32_t)__popc(mask));
-        if (q == 0) atomicAdd(&q_tot, (uint32_t)__popc(mask));
       }
       wb = __shfl_sync(0xffffffffu, wb, 0);
       if (mine) {
-        const uint32_t pos = wb + (uint32_t)__popc(mask & ((1u << lane) - 1u));  // < 2 FT: at most FT - 1 wait
+        const uint32_t pos = wb + (uint32_t)__popc(mask & ((1u << lane) - 1u));  // < 2 T: at most T - 1 wait
         q_k[q][pos] = k;
         q_d[q][0][pos] = dn;
         q_d[q][1][pos] = n.x;
@@ -478,22 +482,22 @@ __global__ void __launch_bounds__(FT, (Mode ? 4 : (IntTiles ? 3 : 1))) k_cfused(
 #pragma unroll
     for (int q = 0; q < 2; q++) {
       const uint32_t have = q_n[q];
-      if (have >= FT) {  // a full tile: one pair per thread
-        run_queued<Mode, IntTiles>(a, q, t, q_k[q], q_d[q], tiles);
+      if (have >= T) {  // a full tile: one pair per thread
+        run_queued<Mode, IntTiles, T>(a, q, t, q_k[q], q_d[q], tiles);
         __syncthreads();
-        const uint32_t rest = have - FT;  // < FT: the waiting pairs move to the front
+        const uint32_t rest = have - T;  // < T: the waiting pairs move to the front
         if (t < rest) {
-          q_k[q][t] = q_k[q][FT + t];
+          q_k[q][t] = q_k[q][T + t];
 #pragma unroll
-          for (int c = 0; c < 7; c++) q_d[q][c][t] = q_d[q][c][FT + t];
+          for (int c = 0; c < 7; c++) q_d[q][c][t] = q_d[q][c][T + t];
         }
         if (t == 0) q_n[q] = rest;
         __syncthreads();
       }
     }
   }
-  if (t < q_n[0]) run_queued<Mode, IntTiles>(a, 0, t, q_k[0], q_d[0], tiles);
-  if (t < q_n[1]) run_queued<Mode, IntTiles>(a, 1, t, q_k[1], q_d[1], tiles);
+  if (t < q_n[0]) run_queued<Mode, IntTiles, T>(a, 0, t, q_k[0], q_d[0], tiles);
+  if (t < q_n[1]) run_queued<Mode, IntTiles, T>(a, 1, t, q_k[1], q_d[1], tiles);
   if (t == 0 && q_tot) atomicAdd(a.n_active, (unsigned long long)q_tot);
 }
 
@@ -753,11 +757,7 @@ CArgs make_cargs(dem_ctx* c) {
 static int rotation_dense(const dem_ctx* c) { return c->n <= (uint64_t)c->num_sms * 128u ? 0 : 24; }
 // Threads per block of the prolog and the epilog: the tuned size, halved while the
 // grid leaves SMs without a block (at 10 k particles 256 threads reach 40 SMs).
-static unsigned particle_block(const dem_ctx* c) {
-  unsigned b = (unsigned)c->tune_block;
-  while (b > 32u && c->n < (uint64_t)b * (uint64_t)c->num_sms) b >>= 1;
-  return b;
-}
+static unsigned particle_block(const dem_ctx* c) { return spread_block(c, c->n, (unsigned)c->tune_block); }
 
 // cond: inside a capture, the handle of the conditional rebuild (both halves; the
 // first step of a call has no epilog)
@@ -806,27 +806,39 @@ int launch_fused_prolog(dem_ctx* c) {
 int launch_fused_epilog(dem_ctx* c) { return launch_integrate(c, 1, 0, 0); }
 int launch_graph_integrate(dem_ctx* c, cudaGraphConditionalHandle cond) { return launch_integrate(c, 1, 1, cond); }
 
-int launch_contact_compact(dem_ctx* c) {
+int launch_contact_compact(dem_ctx* c, bool overlap_only) {
   // (in a graph the integration's last block zeroes these counts)
   if (!c->capturing)
     DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars + 3, 0, 3 * sizeof(unsigned long long), c->stream));
-  const CArgs a = make_cargs(c);
+  CArgs a = make_cargs(c);
+  a.overlap_only = overlap_only ? 1 : 0;
   const unsigned persistent = (unsigned)c->num_sms * (unsigned)c->tune_contact_bps;
+  // Up to a particle for every lane of four warps an SM (20 k particles, some 60 k
+  // pairs) tiles of one warp spread over all SMs and its FP64 units; above, a block
+  // of four warps shares a queue, so fewer partly filled tiles run at its end.
+  const bool small = c->n <= (uint64_t)c->num_sms * 128u;
+  const unsigned warps = persistent * (FT / 32);
   {
     ProfScope ps(c, K_CSCREEN, c->capturing || c->ni ? 1 : 0);
+    const unsigned block = small ? 32u : 128u;
     if (c->capturing)
-      k_cscreen<<<persistent, FT, 0, c->stream>>>(a);
+      k_cscreen<<<small ? warps : persistent, block, 0, c->stream>>>(a);
     else if (c->ni)
-      k_cscreen<<<grid_for(c->ni, FT), FT, 0, c->stream>>>(a);
+      k_cscreen<<<grid_for(c->ni, block), block, 0, c->stream>>>(a);
   }
-  if (c->fuse_contact) {  // detection and law in one kernel (k_cfused)
+  if (c->fuse_contact || overlap_only) {  // detection and law in one kernel (k_cfused)
     if (!c->capturing) DEM_CUDA_TRY(c, cudaMemsetAsync(a.n_active, 0, sizeof(unsigned long long), c->stream));
     ProfScope ps(c, K_CONTACT, 1);
     // mode bit 2: the contact law's multiplies on the integer pipe; int_share: a
     // share of its tiles with multiplies and additions there
-    const auto kf = (c->mul_mode & 4) ? k_cfused<1, false>
-                                      : (c->tune_int_share > 0 ? k_cfused<0, true> : k_cfused<0, false>);
-    kf<<<persistent, FT, 0, c->stream>>>(a);
+    if (c->mul_mode & 4)
+      k_cfused<1, false, 128><<<persistent, 128, 0, c->stream>>>(a);
+    else if (c->tune_int_share > 0)
+      k_cfused<0, true, 128><<<persistent, 128, 0, c->stream>>>(a);
+    else if (small)
+      k_cfused<0, false, 32><<<warps, 32, 0, c->stream>>>(a);
+    else
+      k_cfused<0, false, 128><<<persistent, 128, 0, c->stream>>>(a);
   } else {
     {
       ProfScope ps(c, K_CDETECT, 1);
