@@ -333,6 +333,9 @@ void free_poly(dem_ctx* c) {
   cudaFree(c->pobb);
   cudaFree(c->pfbox);
   cudaFree(c->pqb);
+  cudaFree(c->pstamp);
+  c->pstamp = nullptr;
+  c->live_pass = 0;
   cudaFree(c->vneed);
   cudaFree(c->vneed_off);
   cudaFree(c->vlist);
@@ -363,6 +366,9 @@ int alloc_poly(dem_ctx* c) {
   DEM_CUDA_TRY(c, cudaMalloc(&c->urec, std::max<uint64_t>(c->pcap, 1) * 16 * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->pfbox, std::max<uint64_t>(c->pcap, 1) * 32 * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->pqb, std::max<uint64_t>(c->pcap, 1) * sizeof(float4)));
+  DEM_CUDA_TRY(c, cudaMalloc(&c->pstamp, std::max<uint64_t>(c->pcap, 1) * 4));
+  DEM_CUDA_TRY(c, cudaMemsetAsync(c->pstamp, 0, std::max<uint64_t>(c->pcap, 1) * 4, c->stream));
+  c->pass_count = 0;
   DEM_CUDA_TRY(c, cudaMalloc(&c->vneed, (std::max<uint64_t>(c->pcap, 1) + 1) * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->vneed_off, (std::max<uint64_t>(c->pcap, 1) + 1) * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->vlist, std::max<uint64_t>(c->pcap, 1) * 4));
@@ -551,6 +557,7 @@ int ext_ensure_contact_state(dem_ctx* c) { return ensure_contact_state(c); }
 // every record may be nonzero again (list rebuilt, state restored, or written by
 // a kernel that does not keep the flags)
 int mark_records_live(dem_ctx* c) {
+  c->live_pass = 0;
   if (c->R.live && c->rcap) DEM_CUDA_TRY(c, cudaMemsetAsync(c->R.live, 1, c->rcap, c->stream));
   return DEM_OK;
 }

@@ -22,9 +22,9 @@ struct MlpState;  // k_mlp.cu
 
 // device scalars (d_scalars, u64): [0] rebuild trigger, [1] active contacts,
 // [3..4] compaction list counts, [8] learned-record overflows, [12] interfaces broken,
-// [16..23] learned bin counters and cursors (14 u32)
+// [16..23] learned bin counters and cursors (14 u32), [24..28] work list counts of the polyhedron contact pass
 constexpr int DEM_NSCALARS = 32;
-constexpr int SC_ROT_CNT = 6, SC_RADMAX = 7, SC_LEARNED_OVF = 8, SC_BROKEN = 12, SC_LEARNED_BINS = 16;
+constexpr int SC_ROT_CNT = 6, SC_RADMAX = 7, SC_LEARNED_OVF = 8, SC_BROKEN = 12, SC_LEARNED_BINS = 16, SC_PLIST = 24;
 
 // features recorded per polyhedron unit by the count pass of the FP32-decided
 // enumeration; the fill pass copies them instead of deciding again
@@ -214,6 +214,11 @@ struct dem_ctx {
   uint32_t* f_cnt = nullptr;          // features per unit (ucap+1)
   uint32_t* f_off = nullptr;          // feature offsets (ucap+1)
   uint64_t ucap = 0;
+
+  // polyhedra, fused step: pass number of the last contact pass that wrote a live record
+  // of a particle, and the pass the current records belong to (0: not stamped)
+  uint32_t* pstamp = nullptr;         // pcap
+  uint32_t pass_count = 0, live_pass = 0;
 
   // inner bonds (k_bond.cu), double-buffered for the compaction at a rebuild
   uint64_t nb = 0, bcap = 0, nif = 0;

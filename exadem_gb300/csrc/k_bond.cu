@@ -31,7 +31,7 @@
 #include <unordered_map>
 #include <vector>
 
-#include "dem_ctx.cuh"
+#include "contact_core.cuh"
 #include "poly_core.cuh"
 
 namespace dem {
@@ -64,8 +64,9 @@ __device__ __forceinline__ void bond_law(double dn, V3 n, double dn0, double wei
                                          double& Et, V3& ft, V3 cp, V3 pos_i, V3 vel_i, V3& f_i, V3 vrot_i,
                                          V3 pos_j, V3 vel_j, V3 vrot_j) {
   const double damp = p.damp_rate * 2.0 * sqrt(p.kn * meff);
-  const V3 contribution_i = vel_i - cross(cp - pos_i, vrot_i);
-  const V3 contribution_j = vel_j - cross(cp - pos_j, vrot_j);
+  MulFP64 mm;
+  const V3 contribution_i = point_velocity(mm, vel_i, cp, pos_i, vrot_i);
+  const V3 contribution_j = point_velocity(mm, vel_j, cp, pos_j, vrot_j);
   const V3 vel = contribution_j - contribution_i;
   const double vn = dot(vel, n);
   const double delta = dn - dn0;
@@ -102,9 +103,10 @@ __global__ void __launch_bounds__(BT) k_bond_force(BondArgs a) {
   bond_law(d.dn, d.n, B.dn0[b], B.weight[b], a.dt, bond_params(a.ibp, a.ng, P.group[i], P.group[j]), meff, En, tds,
            Et, ft, d.cp, pos_i, mk(P.f[VX][i], P.f[VY][i], P.f[VZ][i]), f, mk(P.f[WX][i], P.f[WY][i], P.f[WZ][i]),
            pos_j, mk(P.f[VX][j], P.f[VY][j], P.f[VZ][j]), mk(P.f[WX][j], P.f[WY][j], P.f[WZ][j]));
+  MulFP64 mm;
   const V3 z = mk(0.0, 0.0, 0.0);
-  const V3 ti = cross(d.cp - pos_i, f) + z;  // compute_moments with a zero moment
-  const V3 tj = cross(d.cp - pos_j, -f) + z;
+  const V3 ti = add_moment(mm, cross(d.cp - pos_i, f), z);  // compute_moments with a zero moment
+  const V3 tj = add_moment(mm, cross(d.cp - pos_j, -f), z);
   const V3 fnv = f - ft;
   const double* src[15] = {&tds.x, &tds.y, &tds.z, &ft.x, &ft.y, &ft.z, &f.x, &f.y, &f.z,
                            &ti.x,  &ti.y,  &ti.z,  &tj.x, &tj.y, &tj.z};

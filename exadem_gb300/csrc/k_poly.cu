@@ -1760,11 +1760,16 @@ struct PCArgs {
   ParamTable pt;  // multi-material parameters (pt.pp == nullptr: cp / cpd)
   ContactStateArrays cs;  // analysis, in the contact law's frame (cs.dn == nullptr: off)
   const MeshDev* mesh;
-  uint32_t* L2;
-  double* D[7];
-  unsigned long long* cnt;  // [1] = L2 count, [2] = L2 entries with dn >= 0 (cohesive mesh items)
+  // work lists of the contact pass, one per kind of detection: vertex-vertex,
+  // vertex-edge, vertex-face, edge-edge, drivers
+  uint32_t* list[5];
+  unsigned long long* cnt;  // their counts
   unsigned long long* n_active;
+  // stamp[s] = pass: particle s has a live record of this pass (nullptr: not kept)
+  uint32_t* stamp;
+  uint32_t pass;
 };
+constexpr int PK = 5;
 
 __device__ __forceinline__ void pwrite(const PCArgs& a, uint64_t k, V3 ft, V3 mo, V3 f, V3 ti, V3 tj) {
   a.I.ft[0][k] = ft.x;
@@ -1813,143 +1818,98 @@ __device__ __forceinline__ VView pview(const PCArgs& a, uint32_t s) {
   return VView{a.vx + o, a.vy + o, a.vz + o};
 }
 
-__global__ void __launch_bounds__(PT) k_pdetect(PCArgs a) {
+// The FP32 screen of the listed features (particle pairs; a pair provably apart is
+// zeroed once and skipped), and the others sorted by kind of detection: a warp of the
+// contact pass then runs one kind, where the list's order, pair by pair, put all four
+// into most warps, one after the other.
+__global__ void k_pscreen(PCArgs a) {
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  bool heavy = false;
-  DetD d = det_none();
+  if (k == 0) *a.n_active = 0ull;
+  int kind = -1;
   if (k < a.ni) {
-    const uint32_t meta = a.I.meta[k];
-    const uint32_t type = meta_type(meta);
-    const V3 mo = mk(a.I.mo[0][k], a.I.mo[1][k], a.I.mo[2][k]);
-    bool contact;
-    V3 ri, rj = mk(0, 0, 0);
-    bool is_pp = type <= DEM_ITYPE_EDGE_EDGE;
-    bool is_mesh = false;  // mesh items go to the Hooke pass (types 11, 12 swap the law's roles)
-    double dncut;
-    const dem_contact_params* hp = &a.cp;
-    uint32_t swap = (meta >> 15) & 1u;
-    if (!is_pp) {
-      const uint32_t p = a.I.owner[k];
-      const ShapeDev& sh = a.shapes[a.P.type[p]];
-      const double rm = sh.r * a.P.f[HOM][p];
-      const V3 vert = pview(a, p)[a.I.sub[k] & 0xffffu];
-      const DriverDev& dv = a.drv[a.I.partner[k]];
-      d = det_none();
-      if (dv.kind == 2) {  // ContactLawRShapeDriverFunc (polyhedron/contact.hpp:305-432)
-        is_mesh = true;
-        d = poly_mesh_detect(a.mesh[dv.mesh], type, a.I.sub[k] & 0xffffu, a.I.sub[k] >> 16, pview(a, p), sh, rm);
-      } else if (dv.kind == 0) {
-        const V3 nrm = mk(dv.normal[0], dv.normal[1], dv.normal[2]);
-        const V3 proj = dot(vert, nrm) * nrm;
-        const V3 s2p = -(mk(dv.center_proj[0], dv.center_proj[1], dv.center_proj[2]) - proj);
-        const double dd = vnorm(s2p);
-        d.dn = dd - rm;
-        if (!(d.dn > 0)) {
-          d.c = true;
-          d.n = s2p / dd;
-          d.cp = vert - d.n * (rm + 0.5 * d.dn);
-        }
-      } else {
-        const V3 proj = vert * mk(dv.axis[0], dv.axis[1], dv.axis[2]);
-        const V3 dir = mk(dv.center[0], dv.center[1], dv.center[2]) - proj;
-        const double dd = vnorm(dir);
-        d.dn = dv.radius - (rm + dd);
-        if (!(d.dn > 0)) {
-          d.c = true;
-          d.n = dir / dd;
-          d.cp = vert - d.n * (rm + 0.5 * d.dn);
-        }
-      }
-      ri = mk(a.P.f[RX][p], a.P.f[RY][p], a.P.f[RZ][p]);
-      hp = &a.pt.drv(a.cpd, a.P.group[p], a.I.partner[k]);  // the pair's parameters (multimat)
-      dncut = hp->dncut;
-    } else {
+    const uint32_t type = meta_type(a.I.meta[k]);
+    kind = type > DEM_ITYPE_EDGE_EDGE ? 4 : (int)type;
+    if (a.screen && kind < 4) {
       const Roles R = roles(a, k);
       const ShapeDev& si = a.shapes[a.P.type[R.ip]];
       const ShapeDev& sj = a.shapes[a.P.type[R.jp]];
       const double rim = si.r * a.P.f[HOM][R.ip], rjm = sj.r * a.P.f[HOM][R.jp];
-      const VView vi = pview(a, R.ip), vj = pview(a, R.jp);
-      bool apart = false;
-      if (a.screen) {  // FP32 screen: a pair provably apart skips the FP64 detection
-        const uint64_t oi = (uint64_t)R.ip * a.MV, oj = (uint64_t)R.jp * a.MV;
-        auto wi = [&](int q) { return f3(a.wx[oi + q], a.wy[oi + q], a.wz[oi + q]); };
-        auto wj = [&](int q) { return f3(a.wx[oj + q], a.wy[oj + q], a.wz[oj + q]); };
-        const float Rf = (float)(rim + rjm) * 1.000001f;
-        if (type == DEM_ITYPE_VERTEX_VERTEX) {
-          apart = apart_vv(wi(R.sub_i), wj(R.sub_j), Rf);
-        } else if (type == DEM_ITYPE_VERTEX_EDGE) {
-          apart = apart_ve(wi(R.sub_i), wj(sj.e[2 * R.sub_j]), wj(sj.e[2 * R.sub_j + 1]), Rf);
-        } else if (type == DEM_ITYPE_VERTEX_FACE) {
-          const int b = sj.fo[R.sub_j], e = sj.fo[R.sub_j + 1];
-          apart = apart_vf(wi(R.sub_i), wj(sj.fv[b]), wj(sj.fv[b + 1]), wj(sj.fv[e - 1]), Rf);
-        } else {
-          apart = apart_ee(wi(si.e[2 * R.sub_i]), wi(si.e[2 * R.sub_i + 1]), wj(sj.e[2 * R.sub_j]),
-                           wj(sj.e[2 * R.sub_j + 1]), Rf);
+      const uint64_t oi = (uint64_t)R.ip * a.MV, oj = (uint64_t)R.jp * a.MV;
+      auto wi = [&](int q) { return f3(a.wx[oi + q], a.wy[oi + q], a.wz[oi + q]); };
+      auto wj = [&](int q) { return f3(a.wx[oj + q], a.wy[oj + q], a.wz[oj + q]); };
+      const float Rf = (float)(rim + rjm) * 1.000001f;
+      bool apart;
+      if (type == DEM_ITYPE_VERTEX_VERTEX) {
+        apart = apart_vv(wi(R.sub_i), wj(R.sub_j), Rf);
+      } else if (type == DEM_ITYPE_VERTEX_EDGE) {
+        apart = apart_ve(wi(R.sub_i), wj(sj.e[2 * R.sub_j]), wj(sj.e[2 * R.sub_j + 1]), Rf);
+      } else if (type == DEM_ITYPE_VERTEX_FACE) {
+        const int b = sj.fo[R.sub_j], e = sj.fo[R.sub_j + 1];
+        apart = apart_vf(wi(R.sub_i), wj(sj.fv[b]), wj(sj.fv[b + 1]), wj(sj.fv[e - 1]), Rf);
+      } else {
+        apart = apart_ee(wi(si.e[2 * R.sub_i]), wi(si.e[2 * R.sub_i + 1]), wj(sj.e[2 * R.sub_j]),
+                         wj(sj.e[2 * R.sub_j + 1]), Rf);
+      }
+      if (apart) {
+        kind = -1;
+        if (a.R.live[k]) {  // item.reset(): history and record zeroed once, then skipped by the gathers
+          const V3 z = mk(0, 0, 0);
+          pwrite(a, k, z, z, z, z, z);
+          a.R.live[k] = 0;
         }
       }
-      switch (apart ? ~0u : type) {
-        case ~0u:  // no contact: det_none
-          break;
-        case DEM_ITYPE_VERTEX_VERTEX:
-          d = detect_vv(vi[R.sub_i], rim, vj[R.sub_j], rjm);
-          break;
-        case DEM_ITYPE_VERTEX_EDGE:
-          d = detect_ve(vi[R.sub_i], rim, vj[sj.e[2 * R.sub_j]], vj[sj.e[2 * R.sub_j + 1]], rjm);
-          break;
-        case DEM_ITYPE_VERTEX_FACE:
-          d = detect_vf(vi[R.sub_i], rim, vj, sj, R.sub_j, rjm);
-          break;
-        default:
-          d = detect_ee(vi[si.e[2 * R.sub_i]], vi[si.e[2 * R.sub_i + 1]], rim, vj[sj.e[2 * R.sub_j]],
-                        vj[sj.e[2 * R.sub_j + 1]], rjm);
-      }
-      ri = mk(a.P.f[RX][R.ip], a.P.f[RY][R.ip], a.P.f[RZ][R.ip]);
-      rj = mk(a.P.f[RX][R.jp], a.P.f[RY][R.jp], a.P.f[RZ][R.jp]);
-      hp = &a.pt.pair(a.cp, a.P.group[R.ip], a.P.group[R.jp]);
-      dncut = hp->dncut;
     }
-    contact = d.c;
-    if (a.cohesive) contact = (contact || d.dn <= dncut);
-    if (!contact) {
-      const V3 z = mk(0, 0, 0);
-      if (a.R.live[k]) {  // item.reset(): history and record zeroed once, then skipped by the gathers
-        pwrite(a, k, z, z, z, z, z);
-        a.R.live[k] = 0;
-      }
-      a.cs.write(k, 0.0, d.cp, z, z);  // dn = 0, the detector's contact point
-    } else if (a.cohesive && d.dn >= 0 && !is_mesh) {
-      a.R.live[k] = 1;
-      const dem_contact_params& hkp = *hp;
-      const double fn_value = (hkp.fc / hkp.dncut) * d.dn - hkp.fc;
-      const V3 f = mk(0, 0, 0) + fn_value * d.n;
-      const V3 ti = cross(d.cp - ri, f) + mo;
-      a.cs.write(k, d.dn, d.cp, f - mk(0, 0, 0), mk(0, 0, 0));  // fn = f - friction, friction reset
-      if (!is_pp) {
-        pwrite(a, k, mk(0, 0, 0), mo, f, ti, mk(0, 0, 0));
-      } else {
-        const V3 tj = cross(d.cp - rj, -f) + (-mo);
-        if (swap) pwrite(a, k, mk(0, 0, 0), mo, -f, tj, ti);
-        else pwrite(a, k, mk(0, 0, 0), mo, f, ti, tj);
-      }
+  }
+#pragma unroll
+  for (int q = 0; q < PK; q++) {
+    const uint32_t pos = warp_append2(kind == q, a.cnt + q);
+    if (kind == q) a.list[q][pos] = (uint32_t)k;
+  }
+}
+
+// FP64 detection of interaction k by its kind; det_none where the detector rejects it
+__device__ __forceinline__ DetD pair_detect(const PCArgs& a, int kind, uint32_t k) {
+  const uint32_t type = meta_type(a.I.meta[k]);
+  if (kind == 4) {
+    const uint32_t p = a.I.owner[k];
+    const ShapeDev& sh = a.shapes[a.P.type[p]];
+    const double rm = sh.r * a.P.f[HOM][p];
+    const DriverDev& dv = a.drv[a.I.partner[k]];
+    if (dv.kind == 2)  // ContactLawRShapeDriverFunc (polyhedron/contact.hpp:305-432)
+      return poly_mesh_detect(a.mesh[dv.mesh], type, a.I.sub[k] & 0xffffu, a.I.sub[k] >> 16, pview(a, p), sh, rm);
+    const V3 vert = pview(a, p)[a.I.sub[k] & 0xffffu];
+    DetD d = det_none();
+    V3 to;
+    double dd;
+    if (dv.kind == 0) {
+      const V3 nrm = mk(dv.normal[0], dv.normal[1], dv.normal[2]);
+      const V3 proj = dot(vert, nrm) * nrm;
+      to = -(mk(dv.center_proj[0], dv.center_proj[1], dv.center_proj[2]) - proj);
+      dd = vnorm(to);
+      d.dn = dd - rm;
     } else {
-      heavy = true;
-      a.R.live[k] = 1;  // k_phooke writes the record
+      const V3 proj = vert * mk(dv.axis[0], dv.axis[1], dv.axis[2]);
+      to = mk(dv.center[0], dv.center[1], dv.center[2]) - proj;
+      dd = vnorm(to);
+      d.dn = dv.radius - (rm + dd);
     }
+    if (!emu_gt0(d.dn)) {
+      d.c = true;
+      d.n = div3(to, dd);
+      d.cp = vert - d.n * (rm + emu_mulhalf(d.dn));
+    }
+    return d;
   }
-  const uint32_t pos = warp_append2(heavy, a.cnt + 1);
-  const bool idle = heavy && !(d.dn < 0);  // in the Hooke pass without overlap
-  const unsigned im = __ballot_sync(0xffffffffu, idle);
-  if (im && (threadIdx.x & 31) == __ffs(im) - 1) atomicAdd(a.cnt + 2, (unsigned long long)__popc(im));
-  if (heavy) {
-    a.L2[pos] = (uint32_t)k;
-    a.D[0][pos] = d.dn;
-    a.D[1][pos] = d.n.x;
-    a.D[2][pos] = d.n.y;
-    a.D[3][pos] = d.n.z;
-    a.D[4][pos] = d.cp.x;
-    a.D[5][pos] = d.cp.y;
-    a.D[6][pos] = d.cp.z;
-  }
+  const Roles R = roles(a, k);
+  const ShapeDev& si = a.shapes[a.P.type[R.ip]];
+  const ShapeDev& sj = a.shapes[a.P.type[R.jp]];
+  const double rim = si.r * a.P.f[HOM][R.ip], rjm = sj.r * a.P.f[HOM][R.jp];
+  const VView vi = pview(a, R.ip), vj = pview(a, R.jp);
+  if (kind == 0) return detect_vv(vi[R.sub_i], rim, vj[R.sub_j], rjm);
+  if (kind == 1) return detect_ve(vi[R.sub_i], rim, vj[sj.e[2 * R.sub_j]], vj[sj.e[2 * R.sub_j + 1]], rjm);
+  if (kind == 2) return detect_vf(vi[R.sub_i], rim, vj, sj, R.sub_j, rjm);
+  return detect_ee(vi[si.e[2 * R.sub_i]], vi[si.e[2 * R.sub_i + 1]], rim, vj[sj.e[2 * R.sub_j]],
+                   vj[sj.e[2 * R.sub_j + 1]], rjm);
 }
 
 // Fast (the fused step): the contact law with the exact rolling-clip shortcut
@@ -1969,79 +1929,146 @@ __device__ __forceinline__ void hooke(bool cohesive, double dn, V3 n, double dt,
   }
 }
 
+// The contact law of interaction k with its detection d
 template <bool Fast>
-__global__ void __launch_bounds__(PT) k_phooke(PCArgs a) {
-  const uint64_t n2 = a.cnt[1];
-  if (blockIdx.x == 0 && threadIdx.x == 0) *a.n_active = n2 - a.cnt[2];
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < n2; w += stride) {
-    const uint32_t k = a.L2[w];
-    const double dn = a.D[0][w];
-    const V3 n = mk(a.D[1][w], a.D[2][w], a.D[3][w]);
-    const V3 cpos = mk(a.D[4][w], a.D[5][w], a.D[6][w]);
-    const uint32_t meta = a.I.meta[k];
-    V3 ft = mk(a.I.ft[0][k], a.I.ft[1][k], a.I.ft[2][k]);
-    V3 mo = mk(a.I.mo[0][k], a.I.mo[1][k], a.I.mo[2][k]);
-    V3 f = mk(0, 0, 0);
-    if (meta_type(meta) > DEM_ITYPE_EDGE_EDGE) {
-      const uint32_t p = a.I.owner[k];
-      const DriverDev& d = a.drv[a.I.partner[k]];
-      const V3 r = ldv(a.P, RX, p), v = ldv(a.P, VX, p), w_ = ldv(a.P, WX, p);
-      const double meff = a.P.f[MASS][p];
-      if (d.kind == 2) {
-        // ContactLawRShapeDriverFunc (polyhedron/contact.hpp:305-432): reff =
-        // compute_effective_radius of the two Minkowski radii; types 7-10 apply the
-        // law with the particle as i, 11-12 with the mesh as i: the particle takes
-        // -f and -moment, and the friction is stored negated
-        const double ra = a.P.f[HOM][p] * a.shapes[a.P.type[p]].r, mr = a.mesh[d.mesh].r;
-        const double reff = a.dmt ? (ra * mr) / (ra + mr) : 0.0;
-        const dem_contact_params& hp = a.pt.drv(a.cpd, a.P.group[p], a.I.partner[k]);
-        const V3 dpos = mk(d.center[0], d.center[1], d.center[2]);
-        const V3 dvel = mk(d.vel[0], d.vel[1], d.vel[2]), dvrot = mk(d.vrot[0], d.vrot[1], d.vrot[2]);
-        if (meta_type(meta) <= DEM_ITYPE_EDGE_MESH_EDGE) {
-          hooke<Fast>(a.cohesive, dn, n, a.dt, hp, meff, ft, cpos, r, v, f, mo, w_, dpos, dvel, dvrot, a.dmt, reff);
-          pwrite(a, k, ft, mo, f, cross(cpos - r, f) + mo, mk(0, 0, 0));
-          a.cs.write(k, dn, cpos, f - ft, ft);
-        } else {
-          hooke<Fast>(a.cohesive, dn, n, a.dt, hp, meff, ft, cpos, dpos, dvel, f, mo, dvrot, r, v, w_, a.dmt, reff);
-          const V3 fp = -f;
-          pwrite(a, k, -ft, mo, fp, cross(cpos - r, fp) + (-mo), mk(0, 0, 0));
-          a.cs.write(k, dn, cpos, ft - f, -ft);
-        }
-        continue;
+__device__ __forceinline__ void pair_law(const PCArgs& a, uint32_t k, const DetD& d0) {
+  const double dn = d0.dn;
+  const V3 n = d0.n, cpos = d0.cp;
+  const uint32_t meta = a.I.meta[k];
+  V3 ft = mk(a.I.ft[0][k], a.I.ft[1][k], a.I.ft[2][k]);
+  V3 mo = mk(a.I.mo[0][k], a.I.mo[1][k], a.I.mo[2][k]);
+  V3 f = mk(0, 0, 0);
+  MulFP64 mm;
+  if (meta_type(meta) > DEM_ITYPE_EDGE_EDGE) {
+    const uint32_t p = a.I.owner[k];
+    const DriverDev& d = a.drv[a.I.partner[k]];
+    const V3 r = ldv(a.P, RX, p), v = ldv(a.P, VX, p), w_ = ldv(a.P, WX, p);
+    const double meff = a.P.f[MASS][p];
+    if (d.kind == 2) {
+      // ContactLawRShapeDriverFunc (polyhedron/contact.hpp:305-432): reff =
+      // compute_effective_radius of the two Minkowski radii; types 7-10 apply the
+      // law with the particle as i, 11-12 with the mesh as i: the particle takes
+      // -f and -moment, and the friction is stored negated
+      const double ra = a.P.f[HOM][p] * a.shapes[a.P.type[p]].r, mr = a.mesh[d.mesh].r;
+      const double reff = a.dmt ? (ra * mr) / (ra + mr) : 0.0;
+      const dem_contact_params& hp = a.pt.drv(a.cpd, a.P.group[p], a.I.partner[k]);
+      const V3 dpos = mk(d.center[0], d.center[1], d.center[2]);
+      const V3 dvel = mk(d.vel[0], d.vel[1], d.vel[2]), dvrot = mk(d.vrot[0], d.vrot[1], d.vrot[2]);
+      if (meta_type(meta) <= DEM_ITYPE_EDGE_MESH_EDGE) {
+        hooke<Fast>(a.cohesive, dn, n, a.dt, hp, meff, ft, cpos, r, v, f, mo, w_, dpos, dvel, dvrot, a.dmt, reff);
+        pwrite(a, k, ft, mo, f, add_moment(mm, cross(cpos - r, f), mo), mk(0, 0, 0));
+        a.cs.write(k, dn, cpos, f - ft, ft);
+      } else {
+        hooke<Fast>(a.cohesive, dn, n, a.dt, hp, meff, ft, cpos, dpos, dvel, f, mo, dvrot, r, v, w_, a.dmt, reff);
+        const V3 fp = -f;
+        pwrite(a, k, -ft, mo, fp, add_moment(mm, cross(cpos - r, fp), -mo), mk(0, 0, 0));
+        a.cs.write(k, dn, cpos, ft - f, -ft);
       }
-      // DMT: reff = shp.minkowski(h) (polyhedron/contact.hpp:281)
-      const double reff = a.dmt ? a.P.f[HOM][p] * a.shapes[a.P.type[p]].r : 0.0;
-      hooke<Fast>(a.cohesive, dn, n, a.dt, a.pt.drv(a.cpd, a.P.group[p], a.I.partner[k]), meff, ft, cpos, r, v, f,
-                  mo, w_,
-                  mk(d.center[0], d.center[1], d.center[2]), mk(d.vel[0], d.vel[1], d.vel[2]),
-                  mk(d.vrot[0], d.vrot[1], d.vrot[2]), a.dmt, reff);
-      pwrite(a, k, ft, mo, f, cross(cpos - r, f) + mo, mk(0, 0, 0));
-      a.cs.write(k, dn, cpos, f - ft, ft);
-      continue;
+      return;
     }
-    const Roles R = roles(a, k);
-    const V3 r_i = ldv(a.P, RX, R.ip), r_j = ldv(a.P, RX, R.jp);
-    const V3 v_i = ldv(a.P, VX, R.ip), v_j = ldv(a.P, VX, R.jp);
-    const V3 w_i = ldv(a.P, WX, R.ip), w_j = ldv(a.P, WX, R.jp);
-    const double m_i = a.P.f[MASS][R.ip], m_j = a.P.f[MASS][R.jp];
-    const double meff = (m_i * m_j) / (m_i + m_j);
-    // DMT: reff = compute_effective_mass(rad_i, rad_j) of the Minkowski radii h r (polyhedron/contact.hpp:179-183)
-    double reff = 0.0;
-    if (a.dmt) {
-      const double rad_i = a.P.f[HOM][R.ip] * a.shapes[a.P.type[R.ip]].r;
-      const double rad_j = a.P.f[HOM][R.jp] * a.shapes[a.P.type[R.jp]].r;
-      reff = (rad_i * rad_j) / (rad_i + rad_j);
+    // DMT: reff = shp.minkowski(h) (polyhedron/contact.hpp:281)
+    const double reff = a.dmt ? a.P.f[HOM][p] * a.shapes[a.P.type[p]].r : 0.0;
+    hooke<Fast>(a.cohesive, dn, n, a.dt, a.pt.drv(a.cpd, a.P.group[p], a.I.partner[k]), meff, ft, cpos, r, v, f,
+                mo, w_,
+                mk(d.center[0], d.center[1], d.center[2]), mk(d.vel[0], d.vel[1], d.vel[2]),
+                mk(d.vrot[0], d.vrot[1], d.vrot[2]), a.dmt, reff);
+    pwrite(a, k, ft, mo, f, add_moment(mm, cross(cpos - r, f), mo), mk(0, 0, 0));
+    a.cs.write(k, dn, cpos, f - ft, ft);
+    return;
+  }
+  const Roles R = roles(a, k);
+  const V3 r_i = ldv(a.P, RX, R.ip), r_j = ldv(a.P, RX, R.jp);
+  const V3 v_i = ldv(a.P, VX, R.ip), v_j = ldv(a.P, VX, R.jp);
+  const V3 w_i = ldv(a.P, WX, R.ip), w_j = ldv(a.P, WX, R.jp);
+  const double m_i = a.P.f[MASS][R.ip], m_j = a.P.f[MASS][R.jp];
+  const double meff = (m_i * m_j) / (m_i + m_j);
+  // DMT: reff = compute_effective_mass(rad_i, rad_j) of the Minkowski radii h r (polyhedron/contact.hpp:179-183)
+  double reff = 0.0;
+  if (a.dmt) {
+    const double rad_i = a.P.f[HOM][R.ip] * a.shapes[a.P.type[R.ip]].r;
+    const double rad_j = a.P.f[HOM][R.jp] * a.shapes[a.P.type[R.jp]].r;
+    reff = (rad_i * rad_j) / (rad_i + rad_j);
+  }
+  hooke<Fast>(a.cohesive, dn, n, a.dt, a.pt.pair(a.cp, a.P.group[R.ip], a.P.group[R.jp]), meff, ft, cpos, r_i, v_i,
+              f, mo, w_i, r_j, v_j, w_j, a.dmt, reff);
+  const V3 t_i = add_moment(mm, cross(cpos - r_i, f), mo);
+  const V3 t_j = add_moment(mm, cross(cpos - r_j, -f), -mo);
+  a.cs.write(k, dn, cpos, f - ft, ft);  // the law's particle i (polyhedron/contact.hpp:191-210)
+  if ((meta >> 15) & 1u)
+    pwrite(a, k, ft, mo, -f, t_j, t_i);
+  else
+    pwrite(a, k, ft, mo, f, t_i, t_j);
+}
+
+// Detection and law of the screen's survivors, a warp of one kind at a time: the lists
+// are cut into chunks of 32 and dealt to the warps.  The screen leaves mostly pairs
+// that touch, so the law follows in the same thread; no detection goes through memory.
+// Bound by the latency of one kind's FP64 chain below some 10 k survivors.  Measured:
+// pile of 1452 polyhedra (2685 listed) 27 + 14 us in two kernels by list order.
+template <bool Fast>
+__global__ void __launch_bounds__(64) k_pcontact(PCArgs a) {
+  uint64_t first[PK + 1];  // chunks before each list
+  uint64_t cnt[PK];
+  first[0] = 0;
+#pragma unroll
+  for (int q = 0; q < PK; q++) {
+    cnt[q] = a.cnt[q];
+    first[q + 1] = first[q] + (cnt[q] + 31) / 32;
+  }
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < first[PK]; w += nw) {
+    int kind = 0;
+#pragma unroll
+    for (int q = 1; q < PK; q++) kind += w >= first[q] ? 1 : 0;
+    const uint64_t at = (w - first[kind]) * 32 + lane;
+    bool touch = false;
+    if (at < cnt[kind]) {
+      const uint32_t k = a.list[kind][at];
+      const uint32_t owner = a.I.owner[k], partner = a.I.partner[k];
+      const bool is_pp = kind < 4;
+      const bool is_mesh = !is_pp && a.drv[partner].kind == 2;
+      const DetD d = pair_detect(a, kind, k);
+      const dem_contact_params& hp = is_pp ? a.pt.pair(a.cp, a.P.group[owner], a.P.group[partner])
+                                           : a.pt.drv(a.cpd, a.P.group[owner], partner);
+      bool contact = d.c;
+      if (a.cohesive) contact = contact || emu_le(d.dn, hp.dncut);
+      if (!contact) {
+        const V3 z = mk(0, 0, 0);
+        if (a.R.live[k]) {  // item.reset(): history and record zeroed once, then skipped by the gathers
+          pwrite(a, k, z, z, z, z, z);
+          a.R.live[k] = 0;
+        }
+        a.cs.write(k, 0.0, d.cp, z, z);  // dn = 0, the detector's contact point
+      } else {
+        a.R.live[k] = 1;
+        if (a.stamp) {
+          a.stamp[owner] = a.pass;
+          if (is_pp) a.stamp[partner] = a.pass;
+        }
+        if (a.cohesive && emu_ge0(d.dn) && !is_mesh) {  // attraction before contact
+          const uint32_t swap = (a.I.meta[k] >> 15) & 1u;
+          const uint32_t ip = swap ? partner : owner, jp = swap ? owner : partner;
+          const V3 mo = mk(a.I.mo[0][k], a.I.mo[1][k], a.I.mo[2][k]);
+          const double fn_value = (hp.fc / hp.dncut) * d.dn - hp.fc;
+          const V3 f = mk(0, 0, 0) + fn_value * d.n;
+          const V3 ti = cross(d.cp - ldv(a.P, RX, ip), f) + mo;
+          a.cs.write(k, d.dn, d.cp, f - mk(0, 0, 0), mk(0, 0, 0));  // fn = f - friction, friction reset
+          if (!is_pp) {
+            pwrite(a, k, mk(0, 0, 0), mo, f, ti, mk(0, 0, 0));
+          } else {
+            const V3 tj = cross(d.cp - ldv(a.P, RX, jp), -f) + (-mo);
+            if (swap) pwrite(a, k, mk(0, 0, 0), mo, -f, tj, ti);
+            else pwrite(a, k, mk(0, 0, 0), mo, f, ti, tj);
+          }
+        } else {
+          touch = emu_lt0(d.dn);
+          pair_law<Fast>(a, k, d);
+        }
+      }
     }
-    hooke<Fast>(a.cohesive, dn, n, a.dt, a.pt.pair(a.cp, a.P.group[R.ip], a.P.group[R.jp]), meff, ft, cpos, r_i, v_i,
-                f, mo, w_i, r_j, v_j, w_j, a.dmt, reff);
-    const V3 t_i = cross(cpos - r_i, f) + mo;
-    const V3 t_j = cross(cpos - r_j, -f) + (-mo);
-    a.cs.write(k, dn, cpos, f - ft, ft);  // the law's particle i (polyhedron/contact.hpp:191-210)
-    if ((meta >> 15) & 1u)
-      pwrite(a, k, ft, mo, -f, t_j, t_i);
-    else
-      pwrite(a, k, ft, mo, f, t_i, t_j);
+    const unsigned tm = __ballot_sync(0xffffffffu, touch);
+    if (tm && lane == 0) atomicAdd(a.n_active, (unsigned long long)__popc(tm));
   }
 }
 
@@ -2377,7 +2404,7 @@ int launch_harvest(dem_ctx* c, float* x, uint8_t* y, uint64_t capacity, uint64_t
 }
 
 int launch_contact_poly(dem_ctx* c) {
-  DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars + 3, 0, 3 * sizeof(unsigned long long), c->stream));
+  DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars + SC_PLIST, 0, PK * sizeof(unsigned long long), c->stream));
   ProfScope ps(c, K_CONTACT, 2);
   PCArgs a;
   a.P = c->P[c->pcur];
@@ -2402,17 +2429,34 @@ int launch_contact_poly(dem_ctx* c) {
   a.pt = c->ptable();
   a.cs = c->cs;
   a.mesh = c->mesh_dev;
-  a.L2 = c->L2;
-  for (int q = 0; q < 7; q++) a.D[q] = c->Dscr[q];
-  a.cnt = c->d_scalars + 3;
+  // scratch of the records' capacity for the five lists
+  uint32_t* const scratch[PK] = {c->L1, c->L2, reinterpret_cast<uint32_t*>(c->Dscr[0]),
+                                 reinterpret_cast<uint32_t*>(c->Dscr[1]), reinterpret_cast<uint32_t*>(c->Dscr[2])};
+  for (int q = 0; q < PK; q++) a.list[q] = scratch[q];
+  a.cnt = c->d_scalars + SC_PLIST;
   a.n_active = c->d_scalars + 1;
+  c->live_pass = 0;
+  a.stamp = nullptr;
+  if (c->prm.fused_step && c->pstamp) {  // the gathers skip particles without a live record
+    if (++c->pass_count == 0) {
+      DEM_CUDA_TRY(c, cudaMemsetAsync(c->pstamp, 0, c->pcap * 4, c->stream));
+      c->pass_count = 1;
+    }
+    a.stamp = c->pstamp;
+    c->live_pass = c->pass_count;
+  }
+  a.pass = c->pass_count;
   const unsigned block = spread_block(c, c->ni, PT);
-  if (c->ni) k_pdetect<<<grid_for(c->ni, block), block, 0, c->stream>>>(a);
-  const unsigned hb = (unsigned)std::min<uint64_t>(std::max<uint64_t>(grid_for(c->ni, block), 1), (uint64_t)c->num_sms * 8u * (PT / block));
-  if (c->prm.fused_step)
-    k_phooke<true><<<hb, block, 0, c->stream>>>(a);
-  else
-    k_phooke<false><<<hb, block, 0, c->stream>>>(a);
+  k_pscreen<<<std::max(1u, grid_for(c->ni, block)), block, 0, c->stream>>>(a);
+  if (c->ni) {
+    // a warp per chunk and five part-filled ones; the survivors of the screen are not known here
+    const unsigned cb = c->ni < (uint64_t)c->num_sms * 64u ? 32u : 64u;
+    const unsigned grid = (unsigned)std::min<uint64_t>(grid_for(c->ni + 160, cb), (uint64_t)c->num_sms * 16u);
+    if (c->prm.fused_step)
+      k_pcontact<true><<<grid, cb, 0, c->stream>>>(a);
+    else
+      k_pcontact<false><<<grid, cb, 0, c->stream>>>(a);
+  }
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;
 }

@@ -527,6 +527,8 @@ struct IntegArgs {
   const uint32_t* own_off;
   const uint32_t* rev_off;
   const uint32_t* rev_idx;
+  const uint32_t* stamp;  // polyhedra: a particle without a live record of this pass gathers none
+  uint32_t pass;
   double g[3];
   double dt, hdt, dt2_2;  // dt, dt/2, dt^2/2
   double thr2;
@@ -587,7 +589,8 @@ __global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_integrate(IntegArgs a) 
       // neighbour count) much less, so one loop keeps the warp's FP64 adds on
       // most lanes.  The order of the additions is that of two loops.
       const uint32_t o0 = a.own_off[s], no = a.own_off[s + 1] - o0;
-      const uint32_t r0 = a.rev_off[s], nt = no + (a.rev_off[s + 1] - r0);
+      const uint32_t r0 = a.rev_off[s];
+      const uint32_t nt = a.pass && a.stamp[s] != a.pass ? 0u : no + (a.rev_off[s + 1] - r0);
       for (uint32_t q = 0; q < nt; q++) {
         const bool own = q < no;
         const uint32_t k = own ? o0 + q : a.rev_idx[r0 + (q - no)];
@@ -769,6 +772,8 @@ static int launch_integrate(dem_ctx* c, int epilog, int prolog, cudaGraphConditi
   a.own_off = c->own_off[c->icur];
   a.rev_off = c->rev_off;
   a.rev_idx = c->rev_idx;
+  a.stamp = c->pstamp;
+  a.pass = c->poly ? c->live_pass : 0u;
   for (int d = 0; d < 3; d++) a.g[d] = c->prm.gravity[d];
   a.dt = c->prm.dt;
   a.hdt = a.dt * 0.5;
