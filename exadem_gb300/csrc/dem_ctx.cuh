@@ -25,6 +25,7 @@ struct MlpState;  // k_mlp.cu
 // [16..23] learned bin counters and cursors (14 u32), [24..28] work list counts of the polyhedron contact pass
 constexpr int DEM_NSCALARS = 32;
 constexpr int SC_ROT_CNT = 6, SC_RADMAX = 7, SC_LEARNED_OVF = 8, SC_BROKEN = 12, SC_LEARNED_BINS = 16, SC_PLIST = 24;
+constexpr int PLISTS = 5;  // work lists of the polyhedron contact pass
 
 // features recorded per polyhedron unit by the count pass of the FP32-decided
 // enumeration; the fill pass copies them instead of deciding again
@@ -89,6 +90,7 @@ struct dem_ctx {
   int tune_contact_bps = 8;  // persistent blocks per SM of the compacted contact law
   bool fuse_contact = true;  // compacted contact: detection and law in one kernel (k_cfused), else two
   int mul_mode = 2;          // multiply placement of the fused integration kernels (integrate_core.cuh)
+  bool mul_auto = true;      // mul_mode is the default, not the caller's or the autotuner's choice
   int tune_int_share = 0;    // k_cfused: Hooke tiles out of 8 whose arithmetic runs on the integer pipe
   int cell_broad_phase = 0;  // spheres, FP32 broad phase: warp per cell with staged neighbourhoods
 
@@ -219,6 +221,7 @@ struct dem_ctx {
   // of a particle, and the pass the current records belong to (0: not stamped)
   uint32_t* pstamp = nullptr;         // pcap
   uint32_t pass_count = 0, live_pass = 0;
+  unsigned poly_gap = 8, poly_since = 0;  // steps between the last two rebuilds, and since the last one
 
   // inner bonds (k_bond.cu), double-buffered for the compaction at a rebuild
   uint64_t nb = 0, bcap = 0, nif = 0;
@@ -340,7 +343,9 @@ int launch_poly_vertices(dem_ctx* c, int mode);  // 0 plain, 1 + displacement fl
 int launch_poly_units(dem_ctx* c, uint64_t* nu_out, int (*grow_units)(dem_ctx*, uint64_t));
 int launch_poly_feature_count(dem_ctx* c, uint64_t nu, uint32_t* total);
 int launch_poly_feature_fill(dem_ctx* c, uint64_t nu);
-int launch_contact_poly(dem_ctx* c);
+// step: the step in a batch that runs ahead of the host (its kernels do nothing once a
+// trigger was raised), or 0
+int launch_contact_poly(dem_ctx* c, unsigned step = 0);
 int launch_state_systems(dem_ctx* c, dem_state* out);  // one state per system
 void mlp_free(dem_ctx* c);
 int mlp_rates(dem_ctx* c, const float* dev_x, uint64_t n, float* dev_rates);
@@ -356,17 +361,21 @@ void free_graph(dem_ctx* c);
 int ext_alloc_iarrays(dem_ctx* c, int b, uint64_t need);
 int ext_alloc_records(dem_ctx* c, uint64_t need);
 void ext_free_iarrays(IArrays& I);
-int launch_poly_fused_prolog(dem_ctx* c);     // prolog + FP32-decided vertex_displ_over flag
+// epilog of step `step`, then prolog + FP32-decided vertex_displ_over flag of the next
+int launch_poly_integrate(dem_ctx* c, int epilog, int prolog, unsigned step);
 int launch_vertex_list(dem_ctx* c);           // particles whose vertices the list uses (host sync)
-int launch_poly_vertices_listed(dem_ctx* c);  // FP64 vertices of those particles
+int launch_poly_vertices_listed(dem_ctx* c, unsigned step = 0);  // FP64 vertices of those particles
 // k_bond.cu
 int bonds_before_reorder(dem_ctx* c);  // rebuild: broken bonds -> history; interfaces
 int bonds_after_reorder(dem_ctx* c);   // rebuild: new slots, per-slot bond lists
-int launch_bond_criterion(dem_ctx* c); // ORs the rebuild flag when an interface breaks
-int launch_bond_force(dem_ctx* c);     // bond pass + bond gather (after the contact gather)
+int launch_bond_criterion(dem_ctx* c, unsigned step = 0); // ORs the rebuild flag when an interface breaks
+// the bond pass; step = 0: and the bond gather (after the contact gather), else left to the integration
+int launch_bond_force(dem_ctx* c, unsigned step = 0);
 int launch_bond_needs(dem_ctx* c, uint32_t* need);
 void free_bonds(dem_ctx* c);
 void clear_bonds(dem_ctx* c);
+struct IntegArgs;
+void bond_integ_args(const dem_ctx* c, IntegArgs& g);  // the bond records for the integration's gather
 // k_step_fused.cu
 int launch_fused_prolog(dem_ctx* c);
 // overlap_only: a pair counts as active at dn < 0, as in the plain kernel, not at a driver's dn = 0

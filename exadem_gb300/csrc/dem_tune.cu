@@ -239,6 +239,7 @@ extern "C" int dem_autotune(dem_ctx* c, int steps_per_trial, int skin_policy, de
   double best = 1e300, before = 0;
   double best_skin = skin0, best_cell = c->prm.cell_size;
   const int mode0 = c->mul_mode;
+  c->mul_auto = false;  // every trial runs the mode it names
   if ((rc = trial(skin0, c->prm.cell_size, c->tune_block, c->tune_contact_bps, mode0, &before))) return rc;
   best = before;
   for (double sk : skins)

@@ -33,6 +33,7 @@
 
 #include "contact_core.cuh"
 #include "poly_core.cuh"
+#include "step_core.cuh"
 
 namespace dem {
 namespace {
@@ -51,6 +52,8 @@ struct BondArgs {
   const dem_inner_bond_params* ibp;  // ng == 0: ibp[0] for every pair
   int ng;
   double dt;
+  const unsigned long long* flag;  // step in a batch: nothing once a trigger of a step up to it was raised
+  unsigned step;
 };
 
 __host__ __device__ __forceinline__ const dem_inner_bond_params& bond_params(const dem_inner_bond_params* ibp, int ng,
@@ -86,6 +89,7 @@ __device__ __forceinline__ void bond_law(double dn, V3 n, double dn0, double wei
 }
 
 __global__ void __launch_bounds__(BT) k_bond_force(BondArgs a) {
+  if (a.step && *a.flag != 0ull && *a.flag <= a.step) return;
   const uint64_t b = (uint64_t)blockIdx.x * BT + threadIdx.x;
   if (b >= a.nb) return;
   const BondArrays& B = a.B;
@@ -160,9 +164,15 @@ struct CritArgs {
   ParamTable pt;
   unsigned long long* flag;    // rebuild flag
   unsigned long long* broken;  // interfaces broken
+  unsigned step;               // in a batch: nothing once an earlier step raised the flag
 };
 
 __global__ void __launch_bounds__(BT) k_bond_criterion(CritArgs a) {
+  // (a block may see the flag that another block of this step raises: the step's number)
+  if (a.step) {
+    const unsigned long long f = *reinterpret_cast<const volatile unsigned long long*>(a.flag);
+    if (f != 0ull && f < a.step) return;
+  }
   const uint64_t q = (uint64_t)blockIdx.x * BT + threadIdx.x;
   if (q >= a.nif) return;
   const BondArrays& B = a.B;
@@ -199,7 +209,7 @@ __global__ void __launch_bounds__(BT) k_bond_criterion(CritArgs a) {
     B.ft[2][j] = nf.z;
   }
   atomicAdd(a.broken, 1ull);
-  atomicExch(a.flag, 1ull);
+  atomicExch(a.flag, a.step ? (unsigned long long)a.step : 1ull);
 }
 
 // ---- rebuild: compaction, interfaces, new slots, per-slot lists
@@ -793,7 +803,21 @@ int launch_bond_needs(dem_ctx* c, uint32_t* need) {
   return DEM_OK;
 }
 
-int launch_bond_criterion(dem_ctx* c) {
+void bond_integ_args(const dem_ctx* c, IntegArgs& g) {
+  g.nb = c->nb ? 1 : 0;
+  const BondArrays& B = c->B[c->bcur];
+  for (int d = 0; d < 3; d++) {
+    g.bf[d] = B.f[d];
+    g.bti[d] = B.ti[d];
+    g.btj[d] = B.tj[d];
+  }
+  g.b_own_first = c->b_own_first;
+  g.b_own_cnt = c->b_own_cnt;
+  g.b_rev_off = c->b_rev_off;
+  g.b_rev_idx = c->b_rev_idx;
+}
+
+int launch_bond_criterion(dem_ctx* c, unsigned step) {
   if (!c->nif) return DEM_OK;
   ProfScope ps(c, K_BOND, 1);
   CritArgs a;
@@ -805,15 +829,16 @@ int launch_bond_criterion(dem_ctx* c) {
   a.pt = c->ptable();
   a.flag = c->d_scalars;
   a.broken = c->d_scalars + SC_BROKEN;
+  a.step = step;
   k_bond_criterion<<<grid_for(c->nif, BT), BT, 0, c->stream>>>(a);
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;
 }
 
-int launch_bond_force(dem_ctx* c) {
+int launch_bond_force(dem_ctx* c, unsigned step) {
   if (!c->nb) return DEM_OK;
   if (c->ib_ng < 0) return c->fail(DEM_ERR_STATE, "bonds without inner bond parameters");
-  ProfScope ps(c, K_BOND, 2);
+  ProfScope ps(c, K_BOND, step ? 1 : 2);
   BondArgs a;
   a.P = c->P[c->pcur];
   a.B = c->B[c->bcur];
@@ -826,8 +851,10 @@ int launch_bond_force(dem_ctx* c) {
   a.ibp = c->ibp_dev;
   a.ng = c->ib_ng;
   a.dt = c->prm.dt;
+  a.flag = c->d_scalars;
+  a.step = step;
   k_bond_force<<<grid_for(c->nb, BT), BT, 0, c->stream>>>(a);
-  k_bond_gather<<<grid_for(c->n, BT), BT, 0, c->stream>>>(c->P[c->pcur], c->B[c->bcur], c->n, c->b_own_first,
+  if (!step) k_bond_gather<<<grid_for(c->n, BT), BT, 0, c->stream>>>(c->P[c->pcur], c->B[c->bcur], c->n, c->b_own_first,
                                                           c->b_own_cnt, c->b_rev_off, c->b_rev_idx);
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;

@@ -26,6 +26,7 @@
 #include "mesh_core.cuh"
 #include "poly_core.cuh"
 #include "poly_f32.cuh"
+#include "step_core.cuh"
 
 namespace dem {
 namespace {
@@ -131,54 +132,102 @@ __global__ void k_poly_vertices(PolyArgs a, double thr2, unsigned long long* fla
 // prolog (integration) + vertex_displ_over (backup_dem.hpp:65-110) decided in
 // FP32 per vertex (decide_displ); an undecided vertex is recomputed in FP64
 // exactly as the reference does (world vertex minus the stored backup vertex).
-// No vertex is written.
+// No vertex is written.  Returns whether a vertex of particle s moved too far.
 template <int Mode>
-__global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_poly_fused_prolog(PolyArgs a, double delta_t, double half_delta_t, double delta_t2_2,
-                                    double thr2, float thr, unsigned long long* flag) {
-  const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ bool poly_prolog(const PolyArgs& a, const IntegArgs& g, float thr, uint64_t s) {
   bool over = false;
-  if (s < a.n) {
-    prolog_one<Mode, true>(a.P, s, delta_t, half_delta_t, delta_t2_2);
-    const ShapeDev& sh = a.shapes[a.P.type[s]];
-    const double h = a.P.f[HOM][s];
-    const V3 p = mk(a.P.f[RX][s], a.P.f[RY][s], a.P.f[RZ][s]);
-    const Q4 q = {a.P.f[QW][s], a.P.f[QX][s], a.P.f[QY][s], a.P.f[QZ][s]};
-    const F3 dp = f3((float)(p.x - a.P.f[BX][s]), (float)(p.y - a.P.f[BY][s]), (float)(p.z - a.P.f[BZ][s]));
-    const float4 qn = make_float4((float)q.w, (float)q.x, (float)q.y, (float)q.z);
-    const float4 qb = a.qb[s];
-    const float hf = (float)h;
-    const float q2 = fmaxf(fmaxf(qn.x * qn.x + qn.y * qn.y + qn.z * qn.z + qn.w * qn.w,
-                                 qb.x * qb.x + qb.y * qb.y + qb.z * qb.z + qb.w * qb.w),
-                           1.f);
-    bool k_skip_vertices = false;
-    const float pabs = (float)(fabs(p.x) + fabs(p.y) + fabs(p.z));
-    // Rigid-body bound on every vertex displacement: with F(q) = q v q* in the
-    // form v + 2w (u x v) + 2 u x (u x v), |dF/dq| <= 6 |q| |v| |dq|, so
-    // |F(q) v0' - F(q_b) v0'| <= 6 max(|q|, |q_b|) |q - q_b| |v0'|.  The FP32
-    // |q - q_b| carries at most 4u max|q| of rounding (both quaternions rounded
-    // to FP32), the other terms a relative 1e-5; below thr (1 - 1e-4) no vertex
-    // can reach the threshold and the per-vertex test is skipped.
-    {
-      const float qm = sqrtf(q2);
-      const float dqx = qn.x - qb.x, dqy = qn.y - qb.y, dqz = qn.z - qb.z, dqw = qn.w - qb.w;
-      const float dq = sqrtf(dqx * dqx + dqy * dqy + dqz * dqz + dqw * dqw) + 8.f * 5.9604645e-08f * qm;
-      const float bound = (flen(dp) + 6.f * qm * dq * hf * (float)sh.maxv) * 1.00001f + 4.440892e-16f * pabs;
-      if (bound < thr * 0.9999f) over = false, k_skip_vertices = true;
-    }
-    for (int k = 0; k < sh.nv && !over && !k_skip_vertices; k++) {
-      const F3 v0 = f3(sh.vf[3 * k], sh.vf[3 * k + 1], sh.vf[3 * k + 2]) * hf;
-      const int d = decide_displ(dp, qn, qb, v0, q2, pabs, thr);
-      if (d == DEC_UNDECIDED) {
-        const V3 v = world_vertex(sh, k, p, q, h);
-        const uint64_t idx = s * (uint64_t)a.MV + k;
-        const V3 dr = v - mk(a.bx[idx], a.by[idx], a.bz[idx]);
-        over = dot(dr, dr) >= thr2;
-      } else {
-        over = d == DEC_TRUE;
-      }
+  prolog_one<Mode, true>(a.P, s, g.dt, g.hdt, g.dt2_2);
+  const ShapeDev& sh = a.shapes[a.P.type[s]];
+  const double h = a.P.f[HOM][s];
+  const V3 p = mk(a.P.f[RX][s], a.P.f[RY][s], a.P.f[RZ][s]);
+  const Q4 q = {a.P.f[QW][s], a.P.f[QX][s], a.P.f[QY][s], a.P.f[QZ][s]};
+  const F3 dp = f3((float)(p.x - a.P.f[BX][s]), (float)(p.y - a.P.f[BY][s]), (float)(p.z - a.P.f[BZ][s]));
+  const float4 qn = make_float4((float)q.w, (float)q.x, (float)q.y, (float)q.z);
+  const float4 qb = a.qb[s];
+  const float hf = (float)h;
+  const float q2 = fmaxf(fmaxf(qn.x * qn.x + qn.y * qn.y + qn.z * qn.z + qn.w * qn.w,
+                               qb.x * qb.x + qb.y * qb.y + qb.z * qb.z + qb.w * qb.w),
+                         1.f);
+  bool k_skip_vertices = false;
+  const float pabs = (float)(fabs(p.x) + fabs(p.y) + fabs(p.z));
+  // Rigid-body bound on every vertex displacement: with F(q) = q v q* in the
+  // form v + 2w (u x v) + 2 u x (u x v), |dF/dq| <= 6 |q| |v| |dq|, so
+  // |F(q) v0' - F(q_b) v0'| <= 6 max(|q|, |q_b|) |q - q_b| |v0'|.  The FP32
+  // |q - q_b| carries at most 4u max|q| of rounding (both quaternions rounded
+  // to FP32), the other terms a relative 1e-5; below thr (1 - 1e-4) no vertex
+  // can reach the threshold and the per-vertex test is skipped.
+  {
+    const float qm = sqrtf(q2);
+    const float dqx = qn.x - qb.x, dqy = qn.y - qb.y, dqz = qn.z - qb.z, dqw = qn.w - qb.w;
+    const float dq = sqrtf(dqx * dqx + dqy * dqy + dqz * dqz + dqw * dqw) + 8.f * 5.9604645e-08f * qm;
+    const float bound = (flen(dp) + 6.f * qm * dq * hf * (float)sh.maxv) * 1.00001f + 4.440892e-16f * pabs;
+    if (bound < thr * 0.9999f) over = false, k_skip_vertices = true;
+  }
+  for (int k = 0; k < sh.nv && !over && !k_skip_vertices; k++) {
+    const F3 v0 = f3(sh.vf[3 * k], sh.vf[3 * k + 1], sh.vf[3 * k + 2]) * hf;
+    const int d = decide_displ(dp, qn, qb, v0, q2, pabs, thr);
+    if (d == DEC_UNDECIDED) {
+      const V3 v = world_vertex(sh, k, p, q, h);
+      const uint64_t idx = s * (uint64_t)a.MV + k;
+      const V3 dr = v - mk(a.bx[idx], a.by[idx], a.bz[idx]);
+      over = dot(dr, dr) >= g.thr2;
+    } else {
+      over = d == DEC_TRUE;
     }
   }
-  if (__any_sync(0xffffffffu, over) && (threadIdx.x & 31) == 0) atomicOr(flag, 1ull);
+  return over;
+}
+
+// A step's kernels run ahead of the host: once a prolog has raised the trigger flag (with
+// its step's number) the kernels of that step and of the later ones do nothing, until
+// the host has rebuilt the list and goes on from there.
+__device__ __forceinline__ bool halted(const unsigned long long* flag, unsigned step) {
+  const unsigned long long f = *reinterpret_cast<const volatile unsigned long long*>(flag);
+  return f != 0ull && f <= step;
+}
+
+// The polyhedron step's integration: the epilog of step g.step, then the prolog and the
+// trigger of the next (k_integrate's form).  A particle whose epilog rotation is put
+// off has its prolog put off too (k_poly_rotations).
+template <int Mode>
+__global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_poly_integrate(PolyArgs a, IntegArgs g, float thr) {
+  if (g.step && halted(g.scal, g.step)) return;
+  const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  bool late = false, over = false;
+  if (g.epilog) {
+    bool need = false;
+    V3 v, acc, mom = mk(0.0, 0.0, 0.0);
+    if (s < a.n) {
+      need = epilog_translate<Mode>(g, s, v, acc, mom);
+      a.P.f[VX][s] = v.x;
+      a.P.f[VY][s] = v.y;
+      a.P.f[VZ][s] = v.z;
+    }
+    late = __popc(__ballot_sync(0xffffffffu, need)) <= g.dense && need;
+    if (need && !late) epilog_rotation<Mode>(a.P, s, g.hdt, mom);
+  }
+  if (g.prolog && s < a.n && !late) over = poly_prolog<Mode>(a, g, thr, s);
+  if (__any_sync(0xffffffffu, over) && (threadIdx.x & 31) == 0) atomicExch(g.scal, (unsigned long long)g.step + 1ull);
+  if (g.dense) {
+    const uint32_t pos = warp_append(late, g.scal + SC_ROT_CNT);
+    if (late) g.list[pos] = (uint32_t)s;
+  }
+  if (blockIdx.x == 0 && threadIdx.x < PLISTS) g.scal[SC_PLIST + threadIdx.x] = 0ull;  // for the next contact pass
+}
+
+// halted before this step's integration (its prolog part may have raised the flag since)
+template <int Mode>
+__global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_poly_rotations(PolyArgs a, IntegArgs g, float thr) {
+  if (g.step && halted(g.scal, g.step)) return;
+  const uint64_t cnt = g.scal[SC_ROT_CNT];
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  bool over = false;
+  for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < cnt; w += stride) {
+    const uint32_t s = g.list[w];
+    epilog_rotation<Mode>(a.P, s, g.hdt, mk(a.P.f[MX][s], a.P.f[MY][s], a.P.f[MZ][s]));
+    if (g.prolog) over |= poly_prolog<Mode>(a, g, thr, s);
+  }
+  if (over) atomicExch(g.scal, (unsigned long long)g.step + 1ull);
 }
 
 // vertices of the listed particles (those in the interaction list), FP64
@@ -187,7 +236,9 @@ __global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_poly_fused_prolog(PolyA
 // product h v0 skipped for h = 1 (1 * x = x); an operand outside the integer
 // multiply's fast path makes the vertex run world_vertex itself.
 template <int Mode>
-__global__ void k_poly_vertices_listed(PolyArgs a, const uint32_t* __restrict__ list, uint64_t count) {
+__global__ void k_poly_vertices_listed(PolyArgs a, const uint32_t* __restrict__ list, uint64_t count,
+                                       const unsigned long long* flag, unsigned step) {
+  if (step && halted(flag, step)) return;
   const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count * (uint64_t)a.MV) return;
   const uint32_t s = list[t / (uint64_t)a.MV];
@@ -1768,8 +1819,10 @@ struct PCArgs {
   // stamp[s] = pass: particle s has a live record of this pass (nullptr: not kept)
   uint32_t* stamp;
   uint32_t pass;
+  unsigned long long* scal;  // device scalars
+  unsigned step;             // the step in a batch (halted), or 0
 };
-constexpr int PK = 5;
+constexpr int PK = PLISTS;
 
 __device__ __forceinline__ void pwrite(const PCArgs& a, uint64_t k, V3 ft, V3 mo, V3 f, V3 ti, V3 tj) {
   a.I.ft[0][k] = ft.x;
@@ -1823,8 +1876,12 @@ __device__ __forceinline__ VView pview(const PCArgs& a, uint32_t s) {
 // contact pass then runs one kind, where the list's order, pair by pair, put all four
 // into most warps, one after the other.
 __global__ void k_pscreen(PCArgs a) {
+  if (a.step && halted(a.scal, a.step)) return;
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k == 0) *a.n_active = 0ull;
+  if (k == 0) {
+    *a.n_active = 0ull;
+    if (a.step) a.scal[SC_ROT_CNT] = 0ull;  // the rotations of the step before are done
+  }
   int kind = -1;
   if (k < a.ni) {
     const uint32_t type = meta_type(a.I.meta[k]);
@@ -2007,6 +2064,7 @@ __device__ __forceinline__ void pair_law(const PCArgs& a, uint32_t k, const DetD
 // pile of 1452 polyhedra (2685 listed) 27 + 14 us in two kernels by list order.
 template <bool Fast>
 __global__ void __launch_bounds__(64) k_pcontact(PCArgs a) {
+  if (a.step && halted(a.scal, a.step)) return;
   uint64_t first[PK + 1];  // chunks before each list
   uint64_t cnt[PK];
   first[0] = 0;
@@ -2098,17 +2156,22 @@ PolyArgs make_pargs(dem_ctx* c) {
 }
 }  // namespace
 
-int launch_poly_fused_prolog(dem_ctx* c) {
-  DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars, 0, sizeof(unsigned long long), c->stream));
-  ProfScope ps(c, K_PROLOG, c->n ? 1 : 0);
+int launch_poly_integrate(dem_ctx* c, int epilog, int prolog, unsigned step) {
   if (!c->n) return DEM_OK;
   const PolyArgs a = make_pargs(c);
-  const double dt = c->prm.dt;
-  const double md = c->prm.rcut_inc * 0.5;
-  const auto kern = by_mode(c->mul_mode, k_poly_fused_prolog<0>, k_poly_fused_prolog<1>, k_poly_fused_prolog<2>,
-                            k_poly_fused_prolog<3>);
+  IntegArgs g = make_integ_args(c, epilog, prolog);
+  g.step = step;
+  bond_integ_args(c, g);
+  const float thr = (float)(c->prm.rcut_inc * 0.5);
   const unsigned block = spread_block(c, c->n, PT);
-  kern<<<grid_for(c->n, block), block, 0, c->stream>>>(a, dt, dt * 0.5, dt * dt * 0.5, md * md, (float)md, c->d_scalars);
+  ProfScope ps(c, epilog ? K_EPILOG : K_PROLOG, g.dense && epilog ? 2 : 1);
+  const int mode = integ_mode(c);
+  const auto kern = by_mode(mode, k_poly_integrate<0>, k_poly_integrate<1>, k_poly_integrate<2>, k_poly_integrate<3>);
+  kern<<<grid_for(c->n, block), block, 0, c->stream>>>(a, g, thr);
+  if (g.dense && epilog) {
+    const auto krot = by_mode(mode, k_poly_rotations<0>, k_poly_rotations<1>, k_poly_rotations<2>, k_poly_rotations<3>);
+    krot<<<(unsigned)c->num_sms * 3, 256, 0, c->stream>>>(a, g, thr);
+  }
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;
 }
@@ -2131,14 +2194,15 @@ int launch_vertex_list(dem_ctx* c) {
   return DEM_OK;
 }
 
-int launch_poly_vertices_listed(dem_ctx* c) {
+int launch_poly_vertices_listed(dem_ctx* c, unsigned step) {
   ProfScope ps(c, K_PROLOG, c->nvlist ? 1 : 0);
   if (!c->nvlist) return DEM_OK;
   const PolyArgs a = make_pargs(c);
-  const auto kern = by_mode(c->mul_mode, k_poly_vertices_listed<0>, k_poly_vertices_listed<1>,
+  const auto kern = by_mode(integ_mode(c), k_poly_vertices_listed<0>, k_poly_vertices_listed<1>,
                             k_poly_vertices_listed<2>, k_poly_vertices_listed<3>);
   const unsigned block = spread_block(c, c->nvlist * (uint64_t)c->MV, PT);
-  kern<<<grid_for(c->nvlist * (uint64_t)c->MV, block), block, 0, c->stream>>>(a, c->vlist, c->nvlist);
+  kern<<<grid_for(c->nvlist * (uint64_t)c->MV, block), block, 0, c->stream>>>(a, c->vlist, c->nvlist,
+                                                                                       c->d_scalars, step);
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;
 }
@@ -2403,8 +2467,9 @@ int launch_harvest(dem_ctx* c, float* x, uint8_t* y, uint64_t capacity, uint64_t
   return DEM_OK;
 }
 
-int launch_contact_poly(dem_ctx* c) {
-  DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars + SC_PLIST, 0, PK * sizeof(unsigned long long), c->stream));
+int launch_contact_poly(dem_ctx* c, unsigned step) {
+  // (in a batch the integration before this pass zeroes the list counts)
+  if (!step) DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars + SC_PLIST, 0, PK * sizeof(unsigned long long), c->stream));
   ProfScope ps(c, K_CONTACT, 2);
   PCArgs a;
   a.P = c->P[c->pcur];
@@ -2446,6 +2511,8 @@ int launch_contact_poly(dem_ctx* c) {
     c->live_pass = c->pass_count;
   }
   a.pass = c->pass_count;
+  a.scal = c->d_scalars;
+  a.step = step;
   const unsigned block = spread_block(c, c->ni, PT);
   k_pscreen<<<std::max(1u, grid_for(c->ni, block)), block, 0, c->stream>>>(a);
   if (c->ni) {
