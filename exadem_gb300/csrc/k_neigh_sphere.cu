@@ -22,7 +22,7 @@
 // drivers per particle (k_pre_count / k_pre_fill).  In a batched context the particle's system gives the grid, its cell block and
 // its drivers; a system rebuilt without its own trigger kept its slots, and
 // its previous list is copied as is (so its list is the one it has alone).
-#include "dem_ctx.cuh"
+#include "broad_core.cuh"
 #include "mesh_core.cuh"
 
 namespace dem {
@@ -100,25 +100,6 @@ __device__ inline bool driver_filter(const DriverDev& d, double rcut, V3 p) {
   const double dd = vnorm(dir);
   const double dn = d.radius - (dd + rcut);
   return dn <= 0;
-}
-
-// FP32 proof that driver_filter fails: the distance is evaluated in FP32, where the
-// coordinates (a sum of three FP32 terms) and every operation carry at most 2^-21 of
-// the magnitudes that enter, and the margin is 2^-18 of their sum.  Away from the walls it spares the FP64 filter (26 FP64
-// instructions with a square root per particle and driver; a box has six).
-__device__ __forceinline__ bool driver_far(const DriverDev& d, float rc, float px, float py, float pz) {
-  if (d.kind == 0) {
-    const float h = px * d.nf[0] + py * d.nf[1] + pz * d.nf[2];
-    const float ex = h * d.nf[0] - d.cpf[0], ey = h * d.nf[1] - d.cpf[1], ez = h * d.nf[2] - d.cpf[2];
-    const float pp = fabsf(px) + fabsf(py) + fabsf(pz);
-    const float lim = rc + (pp * d.n1 * d.n1 + d.cp1 + rc) * 3.8146973e-06f;
-    return lim > 1e-15f && lim < 1e15f && ex * ex + ey * ey + ez * ez > lim * lim;
-  }
-  const float qx = px * d.af[0], qy = py * d.af[1], qz = pz * d.af[2];
-  const float ex = qx - d.cf[0], ey = qy - d.cf[1], ez = qz - d.cf[2];
-  const float mag = fabsf(qx) + fabsf(qy) + fabsf(qz) + d.c1 + d.rf + rc;
-  const float lim = d.rf - rc - mag * 3.8146973e-06f;
-  return lim > 1e-15f && mag < 1e15f && ex * ex + ey * ey + ez * ez < lim * lim;
 }
 
 // the stationary drivers (surfaces, cylinders) of particle s's system that pass the filter

@@ -21,6 +21,7 @@
 // i is the partner), so the per-particle gather is the one of the sphere path.
 #include <algorithm>
 
+#include "broad_core.cuh"
 #include "contact_core.cuh"
 #include "integrate_core.cuh"
 #include "mesh_core.cuh"
@@ -57,7 +58,7 @@ struct PolyArgs {
 };
 
 // ---------------------------------------------------------------- vertices
-template <bool Displ, bool Backup>
+template <bool Displ>
 __global__ void k_poly_vertices(PolyArgs a, double thr2, unsigned long long* flag) {
   const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   bool over = false;
@@ -79,53 +80,113 @@ __global__ void k_poly_vertices(PolyArgs a, double thr2, unsigned long long* fla
         const V3 dr = v - mk(a.bx[idx], a.by[idx], a.bz[idx]);
         over |= dot(dr, dr) >= thr2;
       }
-      if (Backup) {
-        a.bx[idx] = v.x;
-        a.by[idx] = v.y;
-        a.bz[idx] = v.z;
-        a.fx[idx] = (float)(v.x - p.x);
-        a.fy[idx] = (float)(v.y - p.y);
-        a.fz[idx] = (float)(v.z - p.z);
-      }
-    }
-    if (Backup) {
-      const OBBd o = compute_obb(sh, p, q, h);
-      double* w = a.obb + s * 15;
-      const double vals[15] = {o.c.x, o.c.y, o.c.z, o.e1.x, o.e1.y, o.e1.z, o.e2.x, o.e2.y, o.e2.z,
-                               o.e3.x, o.e3.y, o.e3.z, o.ext.x, o.ext.y, o.ext.z};
-#pragma unroll
-      for (int k = 0; k < 15; k++) w[k] = vals[k];
-      a.qb[s] = make_float4((float)q.w, (float)q.x, (float)q.y, (float)q.z);
-      // FP32 copy of the gate OBB (relative to the centre, enlarged by 0.5 rV twice as
-      // in the feature enumeration) and vertex slabs along its normalised axes
-      float* fb = a.fbox + s * FBOX_STRIDE;
-      OBBd g = o;
-      obb_enlarge(g, 0.5 * a.rV);
-      obb_enlarge(g, 0.5 * a.rV);
-      const OBBf gf = obb_f32(g, p);
-      store_obbf(fb, gf);
-      const uint64_t base = s * (uint64_t)a.MV;
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        F3 d = gf.e[k];
-        const float dl = flen(d);
-        d = dl > 0.f ? d * (1.f / dl) : f3(k == 0, k == 1, k == 2);
-        float lo = 3.4e38f, hi = -3.4e38f;
-        for (int m = 0; m < sh.nv; m++) {
-          const float pr = fdot(f3(a.fx[base + m], a.fy[base + m], a.fz[base + m]), d);
-          lo = fminf(lo, pr);
-          hi = fmaxf(hi, pr);
-        }
-        fb[15 + 3 * k] = d.x;
-        fb[16 + 3 * k] = d.y;
-        fb[17 + 3 * k] = d.z;
-        fb[24 + k] = 0.5f * (lo + hi);
-        fb[27 + k] = 0.5f * (hi - lo);
-      }
     }
   }
   if (Displ) {
     if (__any_sync(0xffffffffu, over) && (threadIdx.x & 31) == 0) atomicOr(flag, 1ull);
+  }
+}
+
+// Round to nearest even, (float)x, on the integer pipe (a conversion is an FP64
+// instruction): the 29 low bits of the significand rounded off the packed exponent
+// and significand.  Outside the normal FP32 range the conversion itself.
+__device__ __forceinline__ float f32_rn(double x) {
+  const uint64_t u = emu_bits(x);
+  const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
+  if (e - (1023u - 126u) >= 253u) return (u << 1) == 0 ? __uint_as_float((uint32_t)(u >> 32)) : (float)x;
+  const uint64_t m = u & 0x7fffffffffffffffull;
+  const uint64_t r = (m + 0x0fffffffull + ((m >> 29) & 1ull)) >> 29;
+  return __uint_as_float((uint32_t)(r - ((uint64_t)(1023 - 127) << 23)) | ((uint32_t)(u >> 32) & 0x80000000u));
+}
+
+// The vertices of a rebuild, with their backups and FP32 forms: a thread per vertex, and
+// h v0 skipped for h = 1 (1 x = x).
+__global__ void k_poly_vertices_backup(PolyArgs a) {
+  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= a.n * (uint64_t)a.MV) return;
+  const uint64_t s = t / (uint64_t)a.MV;
+  const int k = (int)(t - s * (uint64_t)a.MV);
+  const ShapeDev& sh = a.shapes[a.P.type[s]];
+  if (k >= sh.nv) return;
+  const V3 p = mk(a.P.f[RX][s], a.P.f[RY][s], a.P.f[RZ][s]);
+  const Q4 q = {a.P.f[QW][s], a.P.f[QX][s], a.P.f[QY][s], a.P.f[QZ][s]};
+  const double h = a.P.f[HOM][s];
+  const V3 v0 = sh_v(sh, k);
+  MulFP64 mm;
+  const V3 v = p + qrotate_m(mm, q, emu_bits(h) == 0x3ff0000000000000ull ? v0 : h * v0);
+  a.vx[t] = a.bx[t] = v.x;
+  a.vy[t] = a.by[t] = v.y;
+  a.vz[t] = a.bz[t] = v.z;
+  a.wx[t] = f32_rn(v.x);
+  a.wy[t] = f32_rn(v.y);
+  a.wz[t] = f32_rn(v.z);
+  a.fx[t] = f32_rn(v.x - p.x);
+  a.fy[t] = f32_rn(v.y - p.y);
+  a.fz[t] = f32_rn(v.z - p.z);
+}
+
+// World OBB, FP32 gate box and vertex slabs of each particle, after
+// k_poly_vertices_backup.  One thread per particle did this and its vertices one after
+// the other: 221 us for 200 k polyhedra, 31 us for 8 k; the two kernels take 188 and 19,
+// bound by the FP64 pipe.
+__global__ void k_poly_boxes(PolyArgs a) {
+  const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= a.n) return;
+  const ShapeDev& sh = a.shapes[a.P.type[s]];
+  const V3 p = mk(a.P.f[RX][s], a.P.f[RY][s], a.P.f[RZ][s]);
+  const Q4 q = {a.P.f[QW][s], a.P.f[QX][s], a.P.f[QY][s], a.P.f[QZ][s]};
+  const double h = a.P.f[HOM][s];
+  MulFP64 mm;
+  OBBd o;
+  o.e1 = qrotate_m(mm, q, mk(sh.obb[3], sh.obb[4], sh.obb[5]));
+  o.e2 = qrotate_m(mm, q, mk(sh.obb[6], sh.obb[7], sh.obb[8]));
+  o.e3 = qrotate_m(mm, q, mk(sh.obb[9], sh.obb[10], sh.obb[11]));
+  o.c = qrotate_m(mm, q, mk(sh.obb[0], sh.obb[1], sh.obb[2]));
+  o.ext = mk(sh.obb[12], sh.obb[13], sh.obb[14]);
+  if (emu_bits(h) != 0x3ff0000000000000ull) {  // compute_obb (poly_core.cuh)
+    if (h != 1.0) {
+      o.ext = o.ext * h;
+      o.c = o.c * h;
+    }
+  }
+  o.c = o.c + p;
+  double* w = a.obb + s * 15;
+  const double vals[15] = {o.c.x, o.c.y, o.c.z, o.e1.x, o.e1.y, o.e1.z, o.e2.x, o.e2.y, o.e2.z,
+                           o.e3.x, o.e3.y, o.e3.z, o.ext.x, o.ext.y, o.ext.z};
+#pragma unroll
+  for (int k = 0; k < 15; k++) w[k] = vals[k];
+  a.qb[s] = make_float4(f32_rn(q.w), f32_rn(q.x), f32_rn(q.y), f32_rn(q.z));
+  // FP32 copy of the gate OBB (relative to the centre, enlarged by 0.5 rV twice as
+  // in the feature enumeration) and vertex slabs along its normalised axes
+  float* fb = a.fbox + s * FBOX_STRIDE;
+  obb_enlarge(o, 0.5 * a.rV);
+  obb_enlarge(o, 0.5 * a.rV);
+  OBBf gf;
+  gf.c = f3(f32_rn(o.c.x - p.x), f32_rn(o.c.y - p.y), f32_rn(o.c.z - p.z));
+  gf.e[0] = f3(f32_rn(o.e1.x), f32_rn(o.e1.y), f32_rn(o.e1.z));
+  gf.e[1] = f3(f32_rn(o.e2.x), f32_rn(o.e2.y), f32_rn(o.e2.z));
+  gf.e[2] = f3(f32_rn(o.e3.x), f32_rn(o.e3.y), f32_rn(o.e3.z));
+  gf.ext[0] = f32_rn(o.ext.x);
+  gf.ext[1] = f32_rn(o.ext.y);
+  gf.ext[2] = f32_rn(o.ext.z);
+  store_obbf(fb, gf);
+  const uint64_t base = s * (uint64_t)a.MV;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    F3 d = gf.e[k];
+    const float dl = flen(d);
+    d = dl > 0.f ? d * (1.f / dl) : f3(k == 0, k == 1, k == 2);
+    float lo = 3.4e38f, hi = -3.4e38f;
+    for (int m = 0; m < sh.nv; m++) {
+      const float pr = fdot(f3(a.fx[base + m], a.fy[base + m], a.fz[base + m]), d);
+      lo = fminf(lo, pr);
+      hi = fmaxf(hi, pr);
+    }
+    fb[15 + 3 * k] = d.x;
+    fb[16 + 3 * k] = d.y;
+    fb[17 + 3 * k] = d.z;
+    fb[24 + k] = 0.5f * (lo + hi);
+    fb[27 + k] = 0.5f * (hi - lo);
   }
 }
 
@@ -319,10 +380,17 @@ __device__ __forceinline__ bool bonded_to(const UnitArgs& a, uint32_t s, uint64_
   if (!a.b_cnt) return false;
   const uint32_t cn = a.b_cnt[s];
   if (!cn) return false;
-  const uint32_t b0 = a.b_first[s];
-  for (uint32_t k = b0; k < b0 + cn; k++)
-    if (a.b_idj[k] == id) return true;
-  return false;
+  uint32_t lo = a.b_first[s];
+  const uint32_t end = lo + cn;
+  uint32_t hi = end;
+  while (lo < hi) {  // the bonds of an owner are in the order of their partner's id
+    const uint32_t mid = (lo + hi) >> 1;
+    if (a.b_idj[mid] < id)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  return lo < end && a.b_idj[lo] == id;
 }
 
 __device__ __forceinline__ bool driver_reach(const DriverDev& d, double rcut, V3 p) {
@@ -336,6 +404,14 @@ __device__ __forceinline__ bool driver_reach(const DriverDev& d, double rcut, V3
   const V3 dir = proj - mk(d.center[0], d.center[1], d.center[2]);
   const double dd = vnorm(dir);
   return d.radius - (dd + rcut) <= 0;
+}
+
+// the reach sphere meets the mesh's bin grid
+__device__ __forceinline__ bool mesh_meets(const MeshDev& m, V3 ri, double rc) {
+  const double bs = 1.0 / m.inv_bs;
+  return ri.x + rc >= m.lo[0] && ri.x - rc <= m.lo[0] + (m.dims[0] + 1) * bs && ri.y + rc >= m.lo[1] &&
+         ri.y - rc <= m.lo[1] + (m.dims[1] + 1) * bs && ri.z + rc >= m.lo[2] &&
+         ri.z - rc <= m.lo[2] + (m.dims[2] + 1) * bs;
 }
 
 // FP32 decision of the bounding-sphere filter (same bound as the sphere broad phase).
@@ -364,12 +440,7 @@ __device__ inline void for_each_unit(const UnitArgs& a, uint32_t s, Emit&& emit)
       const DriverDev& d = a.drv[k];
       if (bonded_to(a, s, (uint64_t)k)) continue;
       if (d.kind == 2) {  // a mesh unit when the reach sphere meets the mesh's bin grid
-        const MeshDev& m = a.mesh[d.mesh];
-        const double bs = 1.0 / m.inv_bs;
-        const bool meet = ri.x + rc >= m.lo[0] && ri.x - rc <= m.lo[0] + (m.dims[0] + 1) * bs &&
-                          ri.y + rc >= m.lo[1] && ri.y - rc <= m.lo[1] + (m.dims[1] + 1) * bs &&
-                          ri.z + rc >= m.lo[2] && ri.z - rc <= m.lo[2] + (m.dims[2] + 1) * bs;
-        if (meet) emit(1u, (uint32_t)k, (uint64_t)k);
+        if (mesh_meets(a.mesh[d.mesh], ri, rc)) emit(1u, (uint32_t)k, (uint64_t)k);
       } else if (driver_reach(d, rc, ri)) {
         emit(1u, (uint32_t)k, (uint64_t)k);
       }
@@ -437,6 +508,24 @@ __device__ inline void for_each_unit(const UnitArgs& a, uint32_t s, Emit&& emit)
   }
 }
 
+// (partner id, kind): particle features (types 0-3) before driver features (types 4-5)
+__device__ inline void sort_units(uint32_t b, uint32_t e, uint32_t* u_partner, uint64_t* u_pid, uint32_t* u_kind) {
+  for (uint32_t x = b + 1; x < e; x++) {
+    const uint64_t pk = u_pid[x];
+    const uint32_t kk = u_kind[x], qk = u_partner[x];
+    uint32_t y = x;
+    while (y > b && (u_pid[y - 1] > pk || (u_pid[y - 1] == pk && u_kind[y - 1] > kk))) {
+      u_pid[y] = u_pid[y - 1];
+      u_kind[y] = u_kind[y - 1];
+      u_partner[y] = u_partner[y - 1];
+      y--;
+    }
+    u_pid[y] = pk;
+    u_kind[y] = kk;
+    u_partner[y] = qk;
+  }
+}
+
 __global__ void k_unit_count(UnitArgs a, uint32_t* __restrict__ cnt) {
   const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= a.n) return;
@@ -476,38 +565,139 @@ __global__ void k_unit_fill(UnitArgs a, const uint32_t* __restrict__ off, uint32
       w++;
     });
   }
-  // (partner id, kind): particle features (types 0-3) before driver features (types 4-5)
-  for (uint32_t x = b + 1; x < e; x++) {
-    const uint64_t pk = u_pid[x];
-    const uint32_t kk = u_kind[x], qk = u_partner[x];
-    uint32_t y = x;
-    while (y > b && (u_pid[y - 1] > pk || (u_pid[y - 1] == pk && u_kind[y - 1] > kk))) {
-      u_pid[y] = u_pid[y - 1];
-      u_kind[y] = u_kind[y - 1];
-      u_partner[y] = u_partner[y - 1];
-      y--;
-    }
-    u_pid[y] = pk;
-    u_kind[y] = kk;
-    u_partner[y] = qk;
-  }
+  sort_units(b, e, u_partner, u_pid, u_kind);
 }
 
-// separating axis test of the two world OBBs enlarged by skin/2 (nbh_polyhedron.cpp:264-273)
-__global__ void k_unit_sat(uint64_t nu, const uint32_t* __restrict__ u_owner, const uint32_t* __restrict__ u_partner,
-                           const uint32_t* __restrict__ u_kind, const double* __restrict__ obb, double rV,
-                           uint8_t* __restrict__ pass) {
+// FP32 broad phase, unit count: each pair of bounding spheres is met once, from the
+// particle whose cell comes first, and recorded by its owner (the smaller id), as the
+// spheres' k_count_pairs does it, without images; two lanes a particle.
+// Measured (GB300): pile of 1.5 k 33 -> 16 us, 8 k bonded cubes 91 -> 34 us, 200 k falling
+// polyhedra 76 -> 33 us (a thread per owner over its 27 cells, bisecting each by id).
+constexpr int UNIT_BLOCK = 128;
+constexpr int UNIT_LANES = 2;
+constexpr int UNIT_HITS = 16;
+__global__ void __launch_bounds__(UNIT_BLOCK) k_unit_pairs(UnitArgs a, uint32_t* __restrict__ cnt) {
+  __shared__ uint32_t hits[UNIT_HITS][UNIT_BLOCK];  // candidate, bit 31: undecided
+  const uint32_t gl = threadIdx.x % UNIT_LANES;
+  const uint64_t s = ((uint64_t)blockIdx.x * UNIT_BLOCK + threadIdx.x) / UNIT_LANES;
+  if (s >= a.n) return;
+  auto append = [&](uint32_t o, uint32_t unit) {
+    const uint32_t m = atomicAdd(&cnt[o], 1u);
+    if (m < UREC) a.urec[(uint64_t)o * UREC + m] = unit;
+  };
+  const float4 me = a.crel[s];
+  int cx, cy, cz;
+  cell_coords(a.g, a.cell_of[s], cx, cy, cz);
+  if (gl == 0 && a.ndrv) {
+    // a vertex of A can reach a driver only if the centre is within h*(max|v0| + r) + skin (+ rounding margin)
+    const V3 ri = mk(a.P.f[RX][s], a.P.f[RY][s], a.P.f[RZ][s]);
+    const ShapeDev& sh = a.shapes[a.P.type[s]];
+    const double h = a.P.f[HOM][s];
+    const double reach = h * (sh.maxv + sh.r) + a.rV;
+    const double rc = reach + 1e-9 * (1.0 + reach + fabs(ri.x) + fabs(ri.y) + fabs(ri.z));
+    const float rcf = (float)rc;
+    const float px = a.g.lof[0] + (float)cx * a.g.csf[0] + me.x, py = a.g.lof[1] + (float)cy * a.g.csf[1] + me.y,
+                pz = a.g.lof[2] + (float)cz * a.g.csf[2] + me.z;
+    for (int k = 0; k < a.ndrv; k++) {
+      const DriverDev& d = a.drv[k];
+      if (d.kind != 2 && driver_far(d, rcf, px, py, pz)) continue;
+      if (bonded_to(a, (uint32_t)s, (uint64_t)k)) continue;
+      if (d.kind == 2 ? mesh_meets(a.mesh[d.mesh], ri, rc) : driver_reach(d, rc, ri))
+        append((uint32_t)s, 0x80000000u | (uint32_t)k);
+    }
+  }
+  const float csx = a.csz[0], csy = a.csz[1], csz = a.csz[2];
+  const float cmax = fmaxf(csx, fmaxf(csy, csz));
+  const int d0 = a.g.dims[0], d1 = a.g.dims[1], d2n = a.g.dims[2];
+  const float si = fmaxf(fabsf(me.x), fmaxf(fabsf(me.y), fabsf(me.z)));
+  const float reach = me.w + a.skin_f;
+  auto record = [&](uint32_t hit) {
+    const uint32_t p = (uint32_t)s, q = hit & 0x7fffffffu;
+    const uint64_t idp = a.P.id[p], idq = a.P.id[q];
+    if (idp == idq) return;
+    if (hit >> 31) {  // the FP64 filter
+      const double dx = a.P.f[RX][q] - a.P.f[RX][p], dy = a.P.f[RY][q] - a.P.f[RY][p], dz = a.P.f[RZ][q] - a.P.f[RZ][p];
+      const double d2 = dx * dx + dy * dy + dz * dz;
+      const double rmax = a.P.f[RAD][p] + a.P.f[RAD][q] + a.rV;
+      if (!(d2 > 0.0 && d2 < rmax * rmax && d2 < a.rcut2)) return;
+    }
+    const bool mine = idp < idq;
+    const uint32_t o = mine ? p : q;
+    if (!bonded_to(a, o, mine ? idq : idp)) append(o, mine ? q : p);
+  };
+  uint32_t nh = 0;
+#pragma unroll 1
+  for (int r = 0; r < 5; r++) {  // rows (dy, dz): (0, 0), (1, 0), (-1, 1), (0, 1), (1, 1)
+    const int dy = r == 0 || r == 3 ? 0 : (r == 2 ? -1 : 1), dz = r < 2 ? 0 : 1;
+    const int y = cy + dy, z = cz + dz;
+    if (y < 0 || y >= d1 || z >= d2n) continue;
+    const float oy = (float)dy * csy, oz = (float)dz * csz;
+    const uint32_t* const st = a.cell_start + ((uint32_t)d0 * ((uint32_t)y + (uint32_t)d1 * (uint32_t)z) + (uint32_t)cx);
+    const uint32_t u0 = st[0], u1 = st[1];
+    const uint32_t q0 = r == 0 ? (uint32_t)s + 1u : (cx > 0 ? st[-1] : u0);
+    const uint32_t q1 = cx < d0 - 1 ? st[2] : u1;
+    for (uint32_t q = q0 + gl; q < q1; q += UNIT_LANES) {
+      const float4 cq = a.crel[q];
+      const float sj = fmaxf(fabsf(cq.x), fmaxf(fabsf(cq.y), fabsf(cq.z)));
+      const float ox = q < u0 ? -csx : (q < u1 ? 0.f : csx);
+      const int keep = f32_pair((cq.x - me.x) + ox, (cq.y - me.y) + oy, (cq.z - me.z) + oz, si, sj, cmax, reach + cq.w);
+      if (keep) {
+        const uint32_t hit = q | (keep < 0 ? 0x80000000u : 0u);
+        if (nh < UNIT_HITS)
+          hits[nh++][threadIdx.x] = hit;
+        else
+          record(hit);
+      }
+    }
+  }
+#pragma unroll 4
+  for (uint32_t k = 0; k < nh; k++) record(hits[k][threadIdx.x]);
+}
+
+__global__ void k_unit_expand(uint64_t n, const uint32_t* __restrict__ off, uint32_t* __restrict__ u_owner) {
+  const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= n) return;
+  for (uint32_t x = off[s]; x < off[s + 1]; x++) u_owner[x] = (uint32_t)s;
+}
+
+// The unit list in (partner id, kind) order inside an owner, a thread per unit: its rank
+// among the owner's recorded units (k_fill_entries' form).  More than UREC units: the
+// thread of the first one enumerates and sorts them.
+__global__ void k_unit_entries(UnitArgs a, uint64_t nu, const uint32_t* __restrict__ off,
+                               const uint32_t* __restrict__ u_owner, uint32_t* __restrict__ u_partner,
+                               uint64_t* __restrict__ u_pid, uint32_t* __restrict__ u_kind) {
   const uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= nu) return;
-  if (u_kind[u]) {
-    pass[u] = 1;
+  const uint32_t s = u_owner[u];
+  const uint32_t b = off[s], e = off[s + 1], m = e - b, x = (uint32_t)u - b;
+  if (m > UREC) {
+    if (x == 0) {
+      uint32_t w = b;
+      for_each_unit(a, s, [&](uint32_t kind, uint32_t partner, uint64_t pid) {
+        if (w < e) {
+          u_partner[w] = partner;
+          u_pid[w] = pid;
+          u_kind[w] = kind;
+        }
+        w++;
+      });
+      sort_units(b, e, u_partner, u_pid, u_kind);
+    }
     return;
   }
-  OBBd A = load_obb(obb + (uint64_t)u_owner[u] * 15);
-  OBBd B = load_obb(obb + (uint64_t)u_partner[u] * 15);
-  obb_enlarge(A, 0.5 * rV);
-  obb_enlarge(B, 0.5 * rV);
-  pass[u] = obb_intersect(A, B) ? 1 : 0;
+  const uint32_t* const rec = a.urec + (uint64_t)s * UREC;
+  auto pid_of = [&](uint32_t r) { return r >> 31 ? (uint64_t)(r & 0x7fffffffu) : a.P.id[r]; };
+  const uint32_t r = rec[x], kind = r >> 31;
+  const uint64_t pid = pid_of(r);
+  uint32_t rank = 0;
+  for (uint32_t y = 0; y < m; y++) {
+    const uint32_t q = rec[y];
+    const uint64_t pq = pid_of(q);
+    rank += (pq < pid || (pq == pid && (q >> 31) < kind)) ? 1u : 0u;
+  }
+  u_partner[b + rank] = r & 0x7fffffffu;
+  u_pid[b + rank] = pid;
+  u_kind[b + rank] = kind;
 }
 
 // ---------------------------------------------------------------- features
@@ -522,6 +712,7 @@ struct FeatArgs {
   const double* vz;
   const double* obb;
   double rV;
+  float rVf;  // rV in FP32
   uint64_t nu;
   const uint32_t* u_owner;
   const uint32_t* u_partner;
@@ -1270,9 +1461,58 @@ struct UnitRec {
   uint32_t gA, gB, vB, fA, fB;  // gated A vertices, gated B vertices, B vertices near A, A / B faces near the other
   uint32_t eA[2], eB[2];        // A / B edges near the other (64 bits)
   float dRx, dRy, dRz, S, R;
-  uint32_t pad[2];
+  float ra, rb;  // Minkowski radii
 };
 static_assert(sizeof(UnitRec) == 64, "UnitRec is one 64-byte line");
+
+// Separating axis test of the two world OBBs enlarged by skin/2
+// (nbh_polyhedron.cpp:264-273), and the unit's FP32 scalars for k_feat_prep.
+// A thread per unit: the scalars take nine FP64 instructions (conversions are FP64
+// instructions), which k_feat_prep, a warp per unit, ran once a warp (27 k dense
+// polyhedra: 197 -> 183 us).  The test itself is decided in FP32 (decide_obb) where it
+// can be: 48 -> 18 us for 27 k dense polyhedra; the aligned cubes of a bonded block
+// mostly stay with the FP64 test.
+__global__ void k_unit_sat(FeatArgs a, uint8_t* __restrict__ pass, UnitRec* __restrict__ rec) {
+  const uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= a.nu) return;
+  if (a.u_kind[u]) {
+    pass[u] = 1;
+    return;
+  }
+  const uint32_t A = a.u_owner[u], B = a.u_partner[u];
+  int d = DEC_UNDECIDED;
+  if (rec) {
+    const ShapeDev& SA = a.shapes[a.P.type[A]];
+    const ShapeDev& SB = a.shapes[a.P.type[B]];
+    const double ra = SA.r * a.P.f[HOM][A], rb = SB.r * a.P.f[HOM][B];
+    const F3 dR = f3((float)(a.P.f[RX][B] - a.P.f[RX][A]), (float)(a.P.f[RY][B] - a.P.f[RY][A]),
+                     (float)(a.P.f[RZ][B] - a.P.f[RZ][A]));
+    UnitRec& q = rec[u];
+    q.dRx = dR.x;
+    q.dRy = dR.y;
+    q.dRz = dR.z;
+    q.R = (float)(ra + rb + a.rV);
+    q.ra = (float)ra;
+    q.rb = (float)rb;
+    // the stored FP32 boxes are enlarged by the skin, the test's by half of it
+    OBBf fA = load_obbf(a.fbox + (uint64_t)A * FBOX_STRIDE, f3(0.f, 0.f, 0.f));
+    OBBf fB = load_obbf(a.fbox + (uint64_t)B * FBOX_STRIDE, dR);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      fA.ext[k] -= 0.5f * a.rVf;
+      fB.ext[k] -= 0.5f * a.rVf;
+    }
+    d = decide_obb(fA, fB, a.rVf);
+  }
+  if (d == DEC_UNDECIDED) {
+    OBBd oA = load_obb(a.obb + (uint64_t)A * 15);
+    OBBd oB = load_obb(a.obb + (uint64_t)B * 15);
+    obb_enlarge(oA, 0.5 * a.rV);
+    obb_enlarge(oB, 0.5 * a.rV);
+    d = obb_intersect(oA, oB) ? DEC_TRUE : DEC_FALSE;
+  }
+  pass[u] = d == DEC_TRUE ? 1 : 0;
+}
 
 __device__ __forceinline__ uint64_t u64of(uint32_t lo, uint32_t hi) { return (uint64_t)lo | ((uint64_t)hi << 32); }
 __device__ __forceinline__ int nth_bit64(uint64_t m, int r) {
@@ -1299,9 +1539,14 @@ __global__ void __launch_bounds__(PT, 4) k_feat_prep(FeatArgs a, UnitRec* __rest
     const uint32_t A = a.u_owner[u], B = a.u_partner[u];
     const ShapeDev& SA = a.shapes[a.P.type[A]];
     const ShapeDev& SB = a.shapes[a.P.type[B]];
-    const double ra = SA.r * a.P.f[HOM][A], rb = SB.r * a.P.f[HOM][B];
-    const F3 dR = f3((float)(a.P.f[RX][B] - a.P.f[RX][A]), (float)(a.P.f[RY][B] - a.P.f[RY][A]),
-                     (float)(a.P.f[RZ][B] - a.P.f[RZ][A]));
+    UnitRec q{};
+    q.dRx = rec[u].dRx;  // k_unit_sat
+    q.dRy = rec[u].dRy;
+    q.dRz = rec[u].dRz;
+    q.R = rec[u].R;
+    q.ra = rec[u].ra;
+    q.rb = rec[u].rb;
+    const F3 dR = f3(q.dRx, q.dRy, q.dRz);
     const F3 zero = f3(0.f, 0.f, 0.f);
     const uint64_t oA = (uint64_t)A * a.MV, oB = (uint64_t)B * a.MV;
     const FView fa{a.fvx + oA, a.fvy + oA, a.fvz + oA, zero};
@@ -1309,12 +1554,11 @@ __global__ void __launch_bounds__(PT, 4) k_feat_prep(FeatArgs a, UnitRec* __rest
     float sv = fmaxf(lane < SA.nv ? flen(fa[lane]) : 0.f, lane < SB.nv ? flen(fb[lane]) : 0.f);
 #pragma unroll
     for (int o = 16; o; o >>= 1) sv = fmaxf(sv, __shfl_xor_sync(0xffffffffu, sv, o));
-    const float S = sv * 1.001f + (float)(ra + rb + a.rV);
-    const float R = (float)(ra + rb + a.rV);
+    const float R = q.R;
+    const float S = sv * 1.001f + R;
     const float lim = R + S * 6.1035156e-05f;  // R + 2^-14 S
     const float* bA = a.fbox + (uint64_t)A * FBOX_STRIDE;
     const float* bB = a.fbox + (uint64_t)B * FBOX_STRIDE;
-    UnitRec q{};
     for (int k0 = 0; k0 < SA.nv + SB.nv; k0 += 32) {
       const int k = k0 + lane;
       const bool sideA = k < SA.nv, valid = k < SA.nv + SB.nv;
@@ -1323,7 +1567,7 @@ __global__ void __launch_bounds__(PT, 4) k_feat_prep(FeatArgs a, UnitRec* __rest
       bool near = false;
       if (valid) {
         const F3 p = sideA ? fa[vi] : fb[vi];
-        d = decide_gate(load_obbf(sideA ? bB : bA, sideA ? dR : zero), p, (float)(sideA ? ra : rb), S);
+        d = decide_gate(load_obbf(sideA ? bB : bA, sideA ? dR : zero), p, sideA ? q.ra : q.rb, S);
         if (!sideA) near = slab_near_point(load_slabs(bA, zero), p, lim);
       }
       bool g = d == DEC_TRUE;
@@ -1331,7 +1575,8 @@ __global__ void __launch_bounds__(PT, 4) k_feat_prep(FeatArgs a, UnitRec* __rest
         OBBd o = load_obb(a.obb + (uint64_t)(sideA ? B : A) * 15);
         obb_enlarge(o, 0.5 * a.rV);
         obb_enlarge(o, 0.5 * a.rV);
-        g = vertex_gate(o, sideA ? vview(a, A)[vi] : vview(a, B)[vi], sideA ? ra : rb);
+        g = vertex_gate(o, sideA ? vview(a, A)[vi] : vview(a, B)[vi],
+                        sideA ? SA.r * a.P.f[HOM][A] : SB.r * a.P.f[HOM][B]);
       }
       q.gA |= __reduce_or_sync(0xffffffffu, (g && sideA) ? 1u << vi : 0u);
       q.gB |= __reduce_or_sync(0xffffffffu, (g && valid && !sideA) ? 1u << vi : 0u);
@@ -1346,7 +1591,7 @@ __global__ void __launch_bounds__(PT, 4) k_feat_prep(FeatArgs a, UnitRec* __rest
         const FView& fv = sideA ? fa : fb;
         const int* ev = sideA ? SA.e : SB.e;
         near = slab_near_segment(load_slabs(sideA ? bB : bA, sideA ? dR : zero), fv[ev[2 * e]], fv[ev[2 * e + 1]],
-                                 (float)a.rV, lim);
+                                 a.rVf, lim);
       }
       const uint32_t lo = (near && e < 32) ? 1u << e : 0u, hi = (near && e >= 32) ? 1u << (e - 32) : 0u;
       q.eA[0] |= __reduce_or_sync(0xffffffffu, sideA ? lo : 0u);
@@ -1366,11 +1611,7 @@ __global__ void __launch_bounds__(PT, 4) k_feat_prep(FeatArgs a, UnitRec* __rest
       q.fB |= __reduce_or_sync(0xffffffffu, (near && !sideA) ? 1u << f : 0u);
     }
     if (lane == 0) {
-      q.dRx = dR.x;
-      q.dRy = dR.y;
-      q.dRz = dR.z;
       q.S = S;
-      q.R = R;
       rec[u] = q;
     }
     if (lane < 6) {
@@ -1429,9 +1670,9 @@ __global__ void __launch_bounds__(PT, 8) k_feat_test(FeatArgs a, const UnitRec* 
       if (seg == 0) {
         d = decide_vv(fa[i], fb[j], q.R, q.S);
       } else if (seg == 1) {
-        d = decide_ve(fa[i], fb[SB.e[2 * j]], fb[SB.e[2 * j + 1]], q.R, (float)a.rV, q.S);
+        d = decide_ve(fa[i], fb[SB.e[2 * j]], fb[SB.e[2 * j + 1]], q.R, a.rVf, q.S);
       } else if (seg == 2) {
-        d = decide_ve(fb[j], fa[SA.e[2 * i]], fa[SA.e[2 * i + 1]], q.R, (float)a.rV, q.S);
+        d = decide_ve(fb[j], fa[SA.e[2 * i]], fa[SA.e[2 * i + 1]], q.R, a.rVf, q.S);
       } else if (seg == 3) {
         d = decide_vf_nf(fa[i], fb, SB, j, q.R, q.S);
       } else if (seg == 4) {
@@ -2210,22 +2451,26 @@ int launch_poly_vertices_listed(dem_ctx* c, unsigned step) {
 // vertices (+ displacement flag, or + backup and world OBBs at a rebuild)
 int launch_poly_vertices(dem_ctx* c, int mode) {
   if (!c->n) return DEM_OK;
-  ProfScope ps(c, K_PROLOG, 1);
+  ProfScope ps(c, K_PROLOG, mode == 2 ? 2 : 1);
   const PolyArgs a = make_pargs(c);
   const double md = c->prm.rcut_inc * 0.5;
   const unsigned block = spread_block(c, c->n, PT);
   if (mode == 1) {
     DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars, 0, sizeof(unsigned long long), c->stream));
-    k_poly_vertices<true, false><<<grid_for(c->n, block), block, 0, c->stream>>>(a, md * md, c->d_scalars);
+    k_poly_vertices<true><<<grid_for(c->n, block), block, 0, c->stream>>>(a, md * md, c->d_scalars);
   } else if (mode == 2) {
-    k_poly_vertices<false, true><<<grid_for(c->n, block), block, 0, c->stream>>>(a, 0.0, nullptr);
+    const uint64_t nv = c->n * (uint64_t)c->MV;
+    const unsigned vb = spread_block(c, nv, PT);
+    k_poly_vertices_backup<<<grid_for(nv, vb), vb, 0, c->stream>>>(a);
+    k_poly_boxes<<<grid_for(c->n, block), block, 0, c->stream>>>(a);
   } else {
-    k_poly_vertices<false, false><<<grid_for(c->n, block), block, 0, c->stream>>>(a, 0.0, nullptr);
+    k_poly_vertices<false><<<grid_for(c->n, block), block, 0, c->stream>>>(a, 0.0, nullptr);
   }
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;
 }
 
+static FeatArgs make_fargs(dem_ctx* c, uint64_t nu);
 // Units + SAT; returns the number of units in *nu (host sync).
 int launch_poly_units(dem_ctx* c, uint64_t* nu_out, int (*grow_units)(dem_ctx*, uint64_t)) {
   UnitArgs a;
@@ -2241,7 +2486,6 @@ int launch_poly_units(dem_ctx* c, uint64_t* nu_out, int (*grow_units)(dem_ctx*, 
   a.rV = c->prm.rcut_inc;
   const double nd = 2 * c->rad_max + c->prm.rcut_inc;
   a.rcut2 = nd * nd;
-  a.crel = c->crel;
   for (int d = 0; d < 3; d++) a.csz[d] = (float)c->grid.csz[d];
   a.skin_f = (float)c->prm.rcut_inc;
   a.f32 = c->prm.fp32_broad_phase;
@@ -2249,9 +2493,13 @@ int launch_poly_units(dem_ctx* c, uint64_t* nu_out, int (*grow_units)(dem_ctx*, 
   a.b_cnt = c->nb ? c->b_own_cnt : nullptr;
   a.b_idj = c->nb ? c->B[c->bcur].id_j : nullptr;
   a.urec = c->urec;
+  a.crel = c->crel;
   {
     ProfScope ps(c, K_BROAD_COUNT, 1);
-    k_unit_count<<<grid_for(c->n, PT), PT, 0, c->stream>>>(a, c->pcnt);
+    if (a.f32)  // adds to the counts that the reorder zeroed
+      k_unit_pairs<<<grid_for(c->n * UNIT_LANES, UNIT_BLOCK), UNIT_BLOCK, 0, c->stream>>>(a, c->pcnt);
+    else
+      k_unit_count<<<grid_for(c->n, PT), PT, 0, c->stream>>>(a, c->pcnt);
   }
   int rc = scan_exclusive_u32(c, c->pcnt, c->u_off, c->n);
   if (rc) return rc;
@@ -2259,11 +2507,21 @@ int launch_poly_units(dem_ctx* c, uint64_t* nu_out, int (*grow_units)(dem_ctx*, 
   DEM_CUDA_TRY(c, cudaMemcpyAsync(&nu, c->u_off + c->n, 4, cudaMemcpyDeviceToHost, c->stream));
   DEM_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   if ((rc = grow_units(c, nu))) return rc;
-  ProfScope ps(c, K_BROAD_FILL, 2);
-  k_unit_fill<<<grid_for(c->n, PT), PT, 0, c->stream>>>(a, c->u_off, c->u_owner, c->u_partner, c->u_pid, c->u_kind);
-  if (nu)
-    k_unit_sat<<<grid_for(nu, PT), PT, 0, c->stream>>>(nu, c->u_owner, c->u_partner, c->u_kind, c->pobb,
-                                                       c->prm.rcut_inc, c->u_pass);
+  ProfScope ps(c, K_BROAD_FILL, a.f32 ? (nu ? 3 : 0) : (nu ? 2 : 1));
+  if (a.f32) {
+    if (nu) {
+      k_unit_expand<<<grid_for(c->n, PT), PT, 0, c->stream>>>(c->n, c->u_off, c->u_owner);
+      k_unit_entries<<<grid_for(nu, PT), PT, 0, c->stream>>>(a, nu, c->u_off, c->u_owner, c->u_partner, c->u_pid,
+                                                             c->u_kind);
+    }
+  } else {
+    k_unit_fill<<<grid_for(c->n, PT), PT, 0, c->stream>>>(a, c->u_off, c->u_owner, c->u_partner, c->u_pid, c->u_kind);
+  }
+  if (nu) {
+    const unsigned block = spread_block(c, nu, PT);
+    k_unit_sat<<<grid_for(nu, block), block, 0, c->stream>>>(make_fargs(c, nu), c->u_pass,
+                                                             a.f32 ? reinterpret_cast<UnitRec*>(c->u_rec) : nullptr);
+  }
   DEM_CUDA_TRY(c, cudaGetLastError());
   *nu_out = nu;
   return DEM_OK;
@@ -2281,6 +2539,7 @@ static FeatArgs make_fargs(dem_ctx* c, uint64_t nu) {
   a.vz = c->vtx[2];
   a.obb = c->pobb;
   a.rV = c->prm.rcut_inc;
+  a.rVf = (float)c->prm.rcut_inc;
   a.nu = nu;
   a.u_owner = c->u_owner;
   a.u_partner = c->u_partner;

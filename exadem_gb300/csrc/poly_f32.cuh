@@ -252,6 +252,61 @@ __device__ __forceinline__ int decide_gate(const OBBf& o, F3 p, float rv, float 
   return undecided ? DEC_UNDECIDED : DEC_TRUE;
 }
 
+// OBB::intersect of two particles' boxes (both relative to the first one's centre).  The
+// FP64 test returns false at the first of 15 axes with |t_L| > ra_L + rb_L.  With T =
+// |t| + both boxes' extents (+ the skin, whose half was taken off the stored extents):
+// centres, extents and axes are FP32 roundings, so t_k and the entries R carry at most
+// 16 u T and 8 u, every projection and radius sum, of at most six products of magnitude
+// T with factors up to 1 + tol, at most 100 u T < 2^-17 T.  The axes must be unit
+// vectors to 1/16; other boxes are left undecided.
+__device__ __forceinline__ int decide_obb(const OBBf& A, const OBBf& B, float rV) {
+  const float tol = 1.1920929e-07f;
+  const F3 tt = A.c - B.c;
+  const float T = flen(tt) + A.ext[0] + A.ext[1] + A.ext[2] + B.ext[0] + B.ext[1] + B.ext[2] + 2.f * rV;
+  const float e = 7.6293945e-06f * T;  // 2^-17 T
+  float R[3][3], Ab[3][3];
+  bool unit = true;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    unit = unit && fabsf(fdot(A.e[k], A.e[k]) - 1.f) < 0.0625f && fabsf(fdot(B.e[k], B.e[k]) - 1.f) < 0.0625f;
+#pragma unroll
+    for (int l = 0; l < 3; l++) {
+      R[k][l] = fdot(A.e[k], B.e[l]);
+      Ab[k][l] = fabsf(R[k][l]) + tol;
+    }
+  }
+  if (!unit) return DEC_UNDECIDED;
+  const float t[3] = {fdot(tt, A.e[0]), fdot(tt, A.e[1]), fdot(tt, A.e[2])};
+  bool undecided = false;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const int c = cmp_gt(fabsf(t[k]), A.ext[k] + (B.ext[0] * Ab[k][0] + B.ext[1] * Ab[k][1] + B.ext[2] * Ab[k][2]), e);
+    if (c > 0) return DEC_FALSE;
+    undecided |= c == 0;
+  }
+#pragma unroll
+  for (int l = 0; l < 3; l++) {
+    const float ra = A.ext[0] * Ab[0][l] + A.ext[1] * Ab[1][l] + A.ext[2] * Ab[2][l];
+    const int c = cmp_gt(fabsf(t[0] * R[0][l] + t[1] * R[1][l] + t[2] * R[2][l]), ra + B.ext[l], e);
+    if (c > 0) return DEC_FALSE;
+    undecided |= c == 0;
+  }
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const int k1 = (k + 1) % 3, k2 = (k + 2) % 3;
+#pragma unroll
+    for (int l = 0; l < 3; l++) {
+      const int l1 = (l + 1) % 3, l2 = (l + 2) % 3;
+      const float ra = A.ext[k1] * Ab[k2][l] + A.ext[k2] * Ab[k1][l];
+      const float rb = B.ext[l1] * Ab[k][l2] + B.ext[l2] * Ab[k][l1];
+      const int c = cmp_gt(fabsf(t[k2] * R[k1][l] - t[k1] * R[k2][l]), ra + rb, e);
+      if (c > 0) return DEC_FALSE;
+      undecided |= c == 0;
+    }
+  }
+  return undecided ? DEC_UNDECIDED : DEC_TRUE;
+}
+
 // filter_vv: |vi - vj|^2 <= R^2.  |d| carries 2 ETA + 4u|d|.
 __device__ __forceinline__ int decide_vv(F3 vi, F3 vj, float R, float S) {
   const float d = flen(vi - vj);
