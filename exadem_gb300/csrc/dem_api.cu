@@ -795,6 +795,7 @@ int dem_set_particles(dem_ctx* c, const dem_particles* p, int on_device) {
     return c->fail(DEM_ERR_INVALID_ARG, "positions and radius are required");
   DEM_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   c->gen++;
+  c->bond_damp_stale = true;  // masses and groups
   const uint64_t n = p->n;
   int rc = alloc_particles(c, n);
   if (rc) return rc;
@@ -1100,6 +1101,8 @@ int dem_set_shapes(dem_ctx* c, const dem_shape* shapes, int nshapes) {
     for (int i = 0; i < d.nv; i++)
       mx = std::max(mx, std::sqrt(o.v[3 * i] * o.v[3 * i] + o.v[3 * i + 1] * o.v[3 * i + 1] + o.v[3 * i + 2] * o.v[3 * i + 2]));
     o.maxv = mx;
+    o.rf = (float)o.r;
+    o.maxvf = (float)mx;
     for (int i = 0; i < 2 * d.ne; i++) {
       if (d.edges[i] < 0 || d.edges[i] >= d.nv) return c->fail(DEM_ERR_INVALID_ARG, "edge vertex out of range");
       o.e[i] = d.edges[i];

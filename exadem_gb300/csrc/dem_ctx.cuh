@@ -242,6 +242,7 @@ struct dem_ctx {
   uint32_t* b_rev_idx = nullptr;     // bcap
   uint32_t* b_inv = nullptr;         // bpcap: old slot -> new slot at a reorder
   uint64_t bpcap = 0;
+  bool bond_damp_stale = true;       // bonds or inner bond parameters changed since BondArrays::damp was set
   int ib_ng = -1;                    // -1: no inner bond parameters; 0: one set
   dem_inner_bond_params* ibp_dev = nullptr;
   std::vector<dem_inner_bond_params> ibp_host;

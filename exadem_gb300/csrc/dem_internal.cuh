@@ -105,6 +105,7 @@ struct BondArrays {
   double* tj[3];
   double* dn;
   double* fn[3];
+  double* damp;       // damp_rate 2 sqrt(kn meff) of the pair, from the inner bond parameters in use
 };
 
 // Multi-material contact parameters (multimat_parameters.hpp:38-300,

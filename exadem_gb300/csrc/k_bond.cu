@@ -63,10 +63,9 @@ __host__ __device__ __forceinline__ const dem_inner_bond_params& bond_params(con
 
 // force_law_core (forcefield/inner_bond_force.hpp:24-70)
 __device__ __forceinline__ void bond_law(double dn, V3 n, double dn0, double weight, double dt,
-                                         const dem_inner_bond_params& p, double meff, double& En, V3& tds,
+                                         const dem_inner_bond_params& p, double damp, double& En, V3& tds,
                                          double& Et, V3& ft, V3 cp, V3 pos_i, V3 vel_i, V3& f_i, V3 vrot_i,
                                          V3 pos_j, V3 vel_j, V3 vrot_j) {
-  const double damp = p.damp_rate * 2.0 * sqrt(p.kn * meff);
   MulFP64 mm;
   const V3 contribution_i = point_velocity(mm, vel_i, cp, pos_i, vrot_i);
   const V3 contribution_j = point_velocity(mm, vel_j, cp, pos_j, vrot_j);
@@ -84,8 +83,10 @@ __device__ __forceinline__ void bond_law(double dn, V3 n, double dn0, double wei
   tds = tds + ds;
   ft = kt_w * tds;
   f_i = vfn + ft;
-  En = static_cast<double>(fne <= 0) * (0.5 * kn_w * delta * delta);
-  Et = 0.5 * kt_w * dot(tds, tds);
+  // static_cast<double>(fne <= 0) * e: e itself, or a zero of its sign (e finite)
+  const double e = emu_mulhalf(kn_w) * delta * delta;
+  En = emu_le0(fne) ? e : (exp_below(e, 1024) ? emu_double(emu_sign(e) << 63) : 0.0 * e);
+  Et = emu_mulhalf(kt_w) * dot(tds, tds);
 }
 
 __global__ void __launch_bounds__(BT) k_bond_force(BondArgs a) {
@@ -100,11 +101,9 @@ __global__ void __launch_bounds__(BT) k_bond_force(BondArgs a) {
   const double rj = a.shapes[P.type[j]].r * P.f[HOM][j];
   const DetD d = detect_vv(mk(a.vx[vi], a.vy[vi], a.vz[vi]), ri, mk(a.vx[vj], a.vy[vj], a.vz[vj]), rj);
   const V3 pos_i = mk(P.f[RX][i], P.f[RY][i], P.f[RZ][i]), pos_j = mk(P.f[RX][j], P.f[RY][j], P.f[RZ][j]);
-  const double mi = P.f[MASS][i], mj = P.f[MASS][j];
-  const double meff = (mi * mj) / (mi + mj);
   double En = 0.0, Et = 0.0;
   V3 tds = mk(B.tds[0][b], B.tds[1][b], B.tds[2][b]), ft, f;
-  bond_law(d.dn, d.n, B.dn0[b], B.weight[b], a.dt, bond_params(a.ibp, a.ng, P.group[i], P.group[j]), meff, En, tds,
+  bond_law(d.dn, d.n, B.dn0[b], B.weight[b], a.dt, bond_params(a.ibp, a.ng, P.group[i], P.group[j]), B.damp[b], En, tds,
            Et, ft, d.cp, pos_i, mk(P.f[VX][i], P.f[VY][i], P.f[VZ][i]), f, mk(P.f[WX][i], P.f[WY][i], P.f[WZ][i]),
            pos_j, mk(P.f[VX][j], P.f[VY][j], P.f[VZ][j]), mk(P.f[WX][j], P.f[WY][j], P.f[WZ][j]));
   MulFP64 mm;
@@ -124,6 +123,18 @@ __global__ void __launch_bounds__(BT) k_bond_force(BondArgs a) {
   B.fn[0][b] = fnv.x;
   B.fn[1][b] = fnv.y;
   B.fn[2][b] = fnv.z;
+}
+
+// the damping coefficient of every bond, in the law's operations: it depends on the pair
+// and the parameters only, and took 22 of the law's 150 FP64 instructions
+__global__ void __launch_bounds__(BT) k_bond_damp(BondArgs a) {
+  const uint64_t b = (uint64_t)blockIdx.x * BT + threadIdx.x;
+  if (b >= a.nb) return;
+  const uint32_t i = a.B.i[b], j = a.B.j[b];
+  const dem_inner_bond_params& p = bond_params(a.ibp, a.ng, a.P.group[i], a.P.group[j]);
+  const double mi = a.P.f[MASS][i], mj = a.P.f[MASS][j];
+  const double meff = (mi * mj) / (mi + mj);
+  a.B.damp[b] = p.damp_rate * 2.0 * sqrt(p.kn * meff);
 }
 
 __global__ void __launch_bounds__(BT) k_bond_gather(PArrays P, BondArrays B, uint64_t n,
@@ -177,14 +188,15 @@ __global__ void __launch_bounds__(BT) k_bond_criterion(CritArgs a) {
   if (q >= a.nif) return;
   const BondArrays& B = a.B;
   const uint32_t off = a.iface[q], end = a.iface[q + 1];
+  const int mode = B.mode[off];
+  const bool stress = mode == DEM_RUPTURE_STRESS_ENERGY_SEPARATE;  // the only mode that reads S
   double En = 0.0, Et = 0.0, S = 0.0;
   for (uint32_t j = off; j < end; j++) {
     En += B.en[j];
     Et += B.et[j];
-    if (B.dn[j] > 0.0) S += vnorm(mk(B.fn[0][j], B.fn[1][j], B.fn[2][j]));
+    if (stress && B.dn[j] > 0.0) S += vnorm(mk(B.fn[0][j], B.fn[1][j], B.fn[2][j]));
   }
-  S /= (double)(end - off);
-  const int mode = B.mode[off];
+  if (stress) S /= (double)(end - off);
   const double c1 = B.c1[off], c2 = B.c2[off];
   bool brk = false;
   if (mode == DEM_RUPTURE_ENERGY_MIXED) {
@@ -252,6 +264,7 @@ __global__ void k_bond_compact(BondArrays S, BondArrays D, uint64_t nb, const ui
   D.en[w] = S.en[b];
   D.et[w] = S.et[b];
   D.dn[w] = S.dn[b];
+  D.damp[w] = S.damp[b];
   for (int d = 0; d < 3; d++) {
     D.ft[d][w] = S.ft[d][b];
     D.tds[d][w] = S.tds[d][b];
@@ -355,8 +368,8 @@ void carve_bonds(Carver& cv, BondArrays& B, uint64_t cap) {
   B.sub = cv.take<uint32_t>(cap);
   B.mode = cv.take<int32_t>(cap);
   B.unbroken = cv.take<uint8_t>(cap);
-  double** d1[9] = {&B.dn0, &B.weight, &B.c1, &B.c2, &B.en, &B.et, &B.dn, nullptr, nullptr};
-  for (int k = 0; k < 7; k++) *d1[k] = cv.take<double>(cap);
+  double** d1[8] = {&B.dn0, &B.weight, &B.c1, &B.c2, &B.en, &B.et, &B.dn, &B.damp};
+  for (int k = 0; k < 8; k++) *d1[k] = cv.take<double>(cap);
   for (int d = 0; d < 3; d++) {
     B.ft[d] = cv.take<double>(cap);
     B.tds[d] = cv.take<double>(cap);
@@ -403,9 +416,9 @@ int ensure_bond_cap(dem_ctx* c, uint64_t need) {
     DEM_CUDA_TRY(c, cp(D.sub, S.sub, m * 4));
     DEM_CUDA_TRY(c, cp(D.mode, S.mode, m * 4));
     DEM_CUDA_TRY(c, cp(D.unbroken, S.unbroken, m));
-    const double* sd[7] = {S.dn0, S.weight, S.c1, S.c2, S.en, S.et, S.dn};
-    double* dd[7] = {D.dn0, D.weight, D.c1, D.c2, D.en, D.et, D.dn};
-    for (int k = 0; k < 7; k++) DEM_CUDA_TRY(c, cp(dd[k], sd[k], m * 8));
+    const double* sd[8] = {S.dn0, S.weight, S.c1, S.c2, S.en, S.et, S.dn, S.damp};
+    double* dd[8] = {D.dn0, D.weight, D.c1, D.c2, D.en, D.et, D.dn, D.damp};
+    for (int k = 0; k < 8; k++) DEM_CUDA_TRY(c, cp(dd[k], sd[k], m * 8));
     for (int d = 0; d < 3; d++) {
       DEM_CUDA_TRY(c, cp(D.ft[d], S.ft[d], m * 8));
       DEM_CUDA_TRY(c, cp(D.tds[d], S.tds[d], m * 8));
@@ -660,6 +673,7 @@ int upload_bonds(dem_ctx* c, const std::vector<HostBond>& hb, const dem_bond_lis
   c->bcur = 0;
   c->nb = m;
   c->nbh = 0;
+  c->bond_damp_stale = true;
   if (!m) {
     c->nif = 0;
     return DEM_OK;
@@ -853,6 +867,10 @@ int launch_bond_force(dem_ctx* c, unsigned step) {
   a.dt = c->prm.dt;
   a.flag = c->d_scalars;
   a.step = step;
+  if (c->bond_damp_stale) {
+    k_bond_damp<<<grid_for(c->nb, BT), BT, 0, c->stream>>>(a);
+    c->bond_damp_stale = false;
+  }
   k_bond_force<<<grid_for(c->nb, BT), BT, 0, c->stream>>>(a);
   if (!step) k_bond_gather<<<grid_for(c->n, BT), BT, 0, c->stream>>>(c->P[c->pcur], c->B[c->bcur], c->n, c->b_own_first,
                                                           c->b_own_cnt, c->b_rev_off, c->b_rev_idx);
@@ -880,6 +898,7 @@ int dem_set_inner_bond_params(dem_ctx* c, int ngroups, const dem_inner_bond_para
                                   c->stream));
   DEM_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   c->ibp_host.assign(pairs, pairs + cnt);
+  c->bond_damp_stale = true;
   c->ib_ng = ngroups;
   return DEM_OK;
 }

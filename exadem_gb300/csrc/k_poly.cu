@@ -87,18 +87,6 @@ __global__ void k_poly_vertices(PolyArgs a, double thr2, unsigned long long* fla
   }
 }
 
-// Round to nearest even, (float)x, on the integer pipe (a conversion is an FP64
-// instruction): the 29 low bits of the significand rounded off the packed exponent
-// and significand.  Outside the normal FP32 range the conversion itself.
-__device__ __forceinline__ float f32_rn(double x) {
-  const uint64_t u = emu_bits(x);
-  const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
-  if (e - (1023u - 126u) >= 253u) return (u << 1) == 0 ? __uint_as_float((uint32_t)(u >> 32)) : (float)x;
-  const uint64_t m = u & 0x7fffffffffffffffull;
-  const uint64_t r = (m + 0x0fffffffull + ((m >> 29) & 1ull)) >> 29;
-  return __uint_as_float((uint32_t)(r - ((uint64_t)(1023 - 127) << 23)) | ((uint32_t)(u >> 32) & 0x80000000u));
-}
-
 // The vertices of a rebuild, with their backups and FP32 forms: a thread per vertex, and
 // h v0 skipped for h = 1 (1 x = x).
 __global__ void k_poly_vertices_backup(PolyArgs a) {
@@ -202,15 +190,16 @@ __device__ __forceinline__ bool poly_prolog(const PolyArgs& a, const IntegArgs& 
   const double h = a.P.f[HOM][s];
   const V3 p = mk(a.P.f[RX][s], a.P.f[RY][s], a.P.f[RZ][s]);
   const Q4 q = {a.P.f[QW][s], a.P.f[QX][s], a.P.f[QY][s], a.P.f[QZ][s]};
-  const F3 dp = f3((float)(p.x - a.P.f[BX][s]), (float)(p.y - a.P.f[BY][s]), (float)(p.z - a.P.f[BZ][s]));
-  const float4 qn = make_float4((float)q.w, (float)q.x, (float)q.y, (float)q.z);
+  const float4 qn = make_float4(f32_rn(q.w), f32_rn(q.x), f32_rn(q.y), f32_rn(q.z));
   const float4 qb = a.qb[s];
-  const float hf = (float)h;
+  const float hf = f32_rn(h);
   const float q2 = fmaxf(fmaxf(qn.x * qn.x + qn.y * qn.y + qn.z * qn.z + qn.w * qn.w,
                                qb.x * qb.x + qb.y * qb.y + qb.z * qb.z + qb.w * qb.w),
                          1.f);
-  bool k_skip_vertices = false;
-  const float pabs = (float)(fabs(p.x) + fabs(p.y) + fabs(p.z));
+  const float pabs = (fabsf(f32_rn(p.x)) + fabsf(f32_rn(p.y)) + fabsf(f32_rn(p.z))) * 1.000001f;
+  // r - r_b in FP64, rounded on the integer pipe (from the significands alone the bonded
+  // cubes' 16k particles took 1.50 ms instead of 1.45)
+  const F3 dp = f3(f32_rn(p.x - a.P.f[BX][s]), f32_rn(p.y - a.P.f[BY][s]), f32_rn(p.z - a.P.f[BZ][s]));
   // Rigid-body bound on every vertex displacement: with F(q) = q v q* in the
   // form v + 2w (u x v) + 2 u x (u x v), |dF/dq| <= 6 |q| |v| |dq|, so
   // |F(q) v0' - F(q_b) v0'| <= 6 max(|q|, |q_b|) |q - q_b| |v0'|.  The FP32
@@ -218,13 +207,14 @@ __device__ __forceinline__ bool poly_prolog(const PolyArgs& a, const IntegArgs& 
   // to FP32), the other terms a relative 1e-5; below thr (1 - 1e-4) no vertex
   // can reach the threshold and the per-vertex test is skipped.
   {
+    const float dl = flen(dp);
     const float qm = sqrtf(q2);
     const float dqx = qn.x - qb.x, dqy = qn.y - qb.y, dqz = qn.z - qb.z, dqw = qn.w - qb.w;
     const float dq = sqrtf(dqx * dqx + dqy * dqy + dqz * dqz + dqw * dqw) + 8.f * 5.9604645e-08f * qm;
-    const float bound = (flen(dp) + 6.f * qm * dq * hf * (float)sh.maxv) * 1.00001f + 4.440892e-16f * pabs;
-    if (bound < thr * 0.9999f) over = false, k_skip_vertices = true;
+    const float bound = (dl + 6.f * qm * dq * hf * sh.maxvf) * 1.00001f + 4.440892e-16f * pabs;
+    if (bound < thr * 0.9999f) return false;
   }
-  for (int k = 0; k < sh.nv && !over && !k_skip_vertices; k++) {
+  for (int k = 0; k < sh.nv && !over; k++) {
     const F3 v0 = f3(sh.vf[3 * k], sh.vf[3 * k + 1], sh.vf[3 * k + 2]) * hf;
     const int d = decide_displ(dp, qn, qb, v0, q2, pabs, thr);
     if (d == DEC_UNDECIDED) {
@@ -318,9 +308,9 @@ __global__ void k_poly_vertices_listed(PolyArgs a, const uint32_t* __restrict__ 
   a.vx[idx] = v.x;
   a.vy[idx] = v.y;
   a.vz[idx] = v.z;
-  a.wx[idx] = (float)v.x;
-  a.wy[idx] = (float)v.y;
-  a.wz[idx] = (float)v.z;
+  a.wx[idx] = f32_rn(v.x);
+  a.wy[idx] = f32_rn(v.y);
+  a.wz[idx] = f32_rn(v.z);
 }
 
 // marks the particles whose vertices the interaction list uses: both sides of the
@@ -1527,93 +1517,116 @@ __device__ __forceinline__ void seg_masks(const UnitRec& q, int seg, uint64_t& r
   cols = seg == 0 ? (uint64_t)q.vB : (seg == 1 || seg == 5 ? eB : (seg == 3 ? (uint64_t)q.fB : (uint64_t)q.gB));
 }
 
+// the 16 flags h of items [k0, k0 + 16) of A's nA items followed by B's: A's to bit k0 of
+// their mask, B's to theirs
+__device__ __forceinline__ void split16(uint32_t h, int k0, int nA, uint64_t& ma, uint64_t& mb) {
+  const int na = nA <= k0 ? 0 : (nA - k0 < 16 ? nA - k0 : 16);
+  if (na) ma |= (uint64_t)(h & ((1u << na) - 1u)) << k0;
+  if (na < 16) mb |= (uint64_t)(h >> na) << (k0 + na - nA);
+}
+
+// Gates and near features of the pair units, as bit masks: sixteen lanes a unit, which
+// the shapes of up to eight vertices and faces and twelve edges fill (a warp a unit left
+// 19 of its lanes idle and took twice the instructions); the masks come from ballots.
+// Bound by instruction issue and the latency of the gathered vertices.
 __global__ void __launch_bounds__(PT, 4) k_feat_prep(FeatArgs a, UnitRec* __restrict__ rec, uint32_t* __restrict__ tcnt) {
-  const int lane = threadIdx.x & 31;
-  const uint64_t warp = ((uint64_t)blockIdx.x * PT + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * PT) >> 5;
-  for (uint64_t u = warp; u < a.nu; u += nwarps) {
-    if (!a.pass[u] || a.u_kind[u]) {
-      if (lane < 6) tcnt[(uint64_t)lane * a.nu + u] = 0u;
-      continue;
-    }
-    const uint32_t A = a.u_owner[u], B = a.u_partner[u];
-    const ShapeDev& SA = a.shapes[a.P.type[A]];
-    const ShapeDev& SB = a.shapes[a.P.type[B]];
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 15;
+  const int half = threadIdx.x & 16;
+  const uint64_t first = ((uint64_t)blockIdx.x * PT + threadIdx.x) >> 4;
+  const uint64_t stride = ((uint64_t)gridDim.x * PT) >> 4;
+  for (uint64_t u = first; __any_sync(FULL, u < a.nu); u += stride) {
+    const bool act = u < a.nu && a.pass[u] && !a.u_kind[u];
+    if (u < a.nu && !act && lane < 6) tcnt[(uint64_t)lane * a.nu + u] = 0u;
+    if (!__any_sync(FULL, act)) continue;
     UnitRec q{};
-    q.dRx = rec[u].dRx;  // k_unit_sat
-    q.dRy = rec[u].dRy;
-    q.dRz = rec[u].dRz;
-    q.R = rec[u].R;
-    q.ra = rec[u].ra;
-    q.rb = rec[u].rb;
+    uint32_t A = 0, B = 0;
+    if (act) {
+      A = a.u_owner[u];
+      B = a.u_partner[u];
+      q.dRx = rec[u].dRx;  // k_unit_sat
+      q.dRy = rec[u].dRy;
+      q.dRz = rec[u].dRz;
+      q.R = rec[u].R;
+      q.ra = rec[u].ra;
+      q.rb = rec[u].rb;
+    }
+    const ShapeDev& SA = a.shapes[act ? a.P.type[A] : 0u];
+    const ShapeDev& SB = a.shapes[act ? a.P.type[B] : 0u];
     const F3 dR = f3(q.dRx, q.dRy, q.dRz);
     const F3 zero = f3(0.f, 0.f, 0.f);
     const uint64_t oA = (uint64_t)A * a.MV, oB = (uint64_t)B * a.MV;
     const FView fa{a.fvx + oA, a.fvy + oA, a.fvz + oA, zero};
     const FView fb{a.fvx + oB, a.fvy + oB, a.fvz + oB, dR};
-    float sv = fmaxf(lane < SA.nv ? flen(fa[lane]) : 0.f, lane < SB.nv ? flen(fb[lane]) : 0.f);
+    const int nvA = act ? SA.nv : 0, nvB = act ? SB.nv : 0, neA = act ? SA.ne : 0, neB = act ? SB.ne : 0,
+              nfA = act ? SA.nf : 0, nfB = act ? SB.nf : 0;
+    float sv = 0.f;
+    for (int k = lane; k < nvA || k < nvB; k += 16)
+      sv = fmaxf(sv, fmaxf(k < nvA ? flen(fa[k]) : 0.f, k < nvB ? flen(fb[k]) : 0.f));
 #pragma unroll
-    for (int o = 16; o; o >>= 1) sv = fmaxf(sv, __shfl_xor_sync(0xffffffffu, sv, o));
+    for (int o = 8; o; o >>= 1) sv = fmaxf(sv, __shfl_xor_sync(FULL, sv, o));
     const float R = q.R;
     const float S = sv * 1.001f + R;
     const float lim = R + S * 6.1035156e-05f;  // R + 2^-14 S
     const float* bA = a.fbox + (uint64_t)A * FBOX_STRIDE;
     const float* bB = a.fbox + (uint64_t)B * FBOX_STRIDE;
-    for (int k0 = 0; k0 < SA.nv + SB.nv; k0 += 32) {
+    uint64_t gA = 0, gB = 0, vB = 0, none = 0, eA = 0, eB = 0, fA = 0, fB = 0;
+    for (int k0 = 0; __any_sync(FULL, k0 < nvA + nvB); k0 += 16) {
       const int k = k0 + lane;
-      const bool sideA = k < SA.nv, valid = k < SA.nv + SB.nv;
-      const int vi = sideA ? k : k - SA.nv;
-      int d = DEC_FALSE;
-      bool near = false;
+      const bool sideA = k < nvA, valid = k < nvA + nvB;
+      const int vi = sideA ? k : k - nvA;
+      bool g = false, near = false;
       if (valid) {
         const F3 p = sideA ? fa[vi] : fb[vi];
-        d = decide_gate(load_obbf(sideA ? bB : bA, sideA ? dR : zero), p, sideA ? q.ra : q.rb, S);
+        const int d = decide_gate(load_obbf(sideA ? bB : bA, sideA ? dR : zero), p, sideA ? q.ra : q.rb, S);
         if (!sideA) near = slab_near_point(load_slabs(bA, zero), p, lim);
+        g = d == DEC_TRUE;
+        if (d == DEC_UNDECIDED) {
+          OBBd o = load_obb(a.obb + (uint64_t)(sideA ? B : A) * 15);
+          obb_enlarge(o, 0.5 * a.rV);
+          obb_enlarge(o, 0.5 * a.rV);
+          g = vertex_gate(o, sideA ? vview(a, A)[vi] : vview(a, B)[vi],
+                          sideA ? SA.r * a.P.f[HOM][A] : SB.r * a.P.f[HOM][B]);
+        }
       }
-      bool g = d == DEC_TRUE;
-      if (__any_sync(0xffffffffu, d == DEC_UNDECIDED) && d == DEC_UNDECIDED) {
-        OBBd o = load_obb(a.obb + (uint64_t)(sideA ? B : A) * 15);
-        obb_enlarge(o, 0.5 * a.rV);
-        obb_enlarge(o, 0.5 * a.rV);
-        g = vertex_gate(o, sideA ? vview(a, A)[vi] : vview(a, B)[vi],
-                        sideA ? SA.r * a.P.f[HOM][A] : SB.r * a.P.f[HOM][B]);
-      }
-      q.gA |= __reduce_or_sync(0xffffffffu, (g && sideA) ? 1u << vi : 0u);
-      q.gB |= __reduce_or_sync(0xffffffffu, (g && valid && !sideA) ? 1u << vi : 0u);
-      q.vB |= __reduce_or_sync(0xffffffffu, near ? 1u << vi : 0u);
+      split16((__ballot_sync(FULL, g) >> half) & 0xffffu, k0, nvA, gA, gB);
+      split16((__ballot_sync(FULL, near) >> half) & 0xffffu, k0, nvA, none, vB);
     }
-    for (int k0 = 0; k0 < SA.ne + SB.ne; k0 += 32) {
+    for (int k0 = 0; __any_sync(FULL, k0 < neA + neB); k0 += 16) {
       const int k = k0 + lane;
-      const bool sideA = k < SA.ne, valid = k < SA.ne + SB.ne;
-      const int e = sideA ? k : k - SA.ne;
+      const bool sideA = k < neA;
+      const int e = sideA ? k : k - neA;
       bool near = false;
-      if (valid) {
+      if (k < neA + neB) {
         const FView& fv = sideA ? fa : fb;
         const int* ev = sideA ? SA.e : SB.e;
         near = slab_near_segment(load_slabs(sideA ? bB : bA, sideA ? dR : zero), fv[ev[2 * e]], fv[ev[2 * e + 1]],
                                  a.rVf, lim);
       }
-      const uint32_t lo = (near && e < 32) ? 1u << e : 0u, hi = (near && e >= 32) ? 1u << (e - 32) : 0u;
-      q.eA[0] |= __reduce_or_sync(0xffffffffu, sideA ? lo : 0u);
-      q.eA[1] |= __reduce_or_sync(0xffffffffu, sideA ? hi : 0u);
-      q.eB[0] |= __reduce_or_sync(0xffffffffu, sideA ? 0u : lo);
-      q.eB[1] |= __reduce_or_sync(0xffffffffu, sideA ? 0u : hi);
+      split16((__ballot_sync(FULL, near) >> half) & 0xffffu, k0, neA, eA, eB);
     }
-    for (int k0 = 0; k0 < SA.nf + SB.nf; k0 += 32) {
+    for (int k0 = 0; __any_sync(FULL, k0 < nfA + nfB); k0 += 16) {
       const int k = k0 + lane;
-      const bool sideA = k < SA.nf, valid = k < SA.nf + SB.nf;
-      const int f = sideA ? k : k - SA.nf;
+      const bool sideA = k < nfA;
+      const int f = sideA ? k : k - nfA;
       bool near = false;
-      if (valid)
+      if (k < nfA + nfB)
         near = slab_near_face(load_slabs(sideA ? bB : bA, sideA ? dR : zero), sideA ? fa : fb, sideA ? SA : SB, f,
                               lim);
-      q.fA |= __reduce_or_sync(0xffffffffu, (near && sideA) ? 1u << f : 0u);
-      q.fB |= __reduce_or_sync(0xffffffffu, (near && !sideA) ? 1u << f : 0u);
+      split16((__ballot_sync(FULL, near) >> half) & 0xffffu, k0, nfA, fA, fB);
     }
-    if (lane == 0) {
-      q.S = S;
-      rec[u] = q;
-    }
+    if (!act) continue;
+    q.gA = (uint32_t)gA;
+    q.gB = (uint32_t)gB;
+    q.vB = (uint32_t)vB;
+    q.fA = (uint32_t)fA;
+    q.fB = (uint32_t)fB;
+    q.eA[0] = (uint32_t)eA;
+    q.eA[1] = (uint32_t)(eA >> 32);
+    q.eB[0] = (uint32_t)eB;
+    q.eB[1] = (uint32_t)(eB >> 32);
+    q.S = S;
+    if (lane == 0) rec[u] = q;
     if (lane < 6) {
       uint64_t rows, cols;
       seg_masks(q, lane, rows, cols);
@@ -1690,102 +1703,57 @@ __global__ void __launch_bounds__(PT, 8) k_feat_test(FeatArgs a, const UnitRec* 
   }
 }
 
-// Fill = false: counts per unit (fcnt, utypes) and per (segment, unit) group (kc);
-// Fill = true: the driver units' features (the pairs' come from k_feat_fill_flat)
-template <bool Fill>
-__global__ void __launch_bounds__(PT) k_feat_collect(FeatArgs a, const UnitRec* __restrict__ rec,
-                                                     const uint32_t* __restrict__ toff,
+// Kept tests per unit (fcnt, utypes) and per (segment, unit) group (kc), a thread per
+// unit: a group's tests lie in one to three words of kept bits.  Driver units are
+// counted by k_feat_drivers.
+__global__ void __launch_bounds__(PT) k_feat_collect(FeatArgs a, const uint32_t* __restrict__ toff,
                                                      const uint32_t* __restrict__ keep, uint32_t* __restrict__ kc) {
+  const uint64_t u = (uint64_t)blockIdx.x * PT + threadIdx.x;
+  if (u >= a.nu) return;
+  if (!a.pass[u] || a.u_kind[u]) {
+    a.fcnt[u] = 0u;
+    a.utypes[u] = 0u;
+    return;
+  }
+  uint32_t count = 0, ty[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+  for (int seg = 0; seg < 6; seg++) {
+    const uint64_t g = (uint64_t)seg * a.nu + u;
+    const uint32_t b = toff[g], e = toff[g + 1];
+    uint32_t n = 0;
+    for (uint32_t lo = b & ~31u; lo < e; lo += 32) {
+      uint32_t bits = keep[lo >> 5];
+      if (b > lo) bits &= ~0u << (b - lo);
+      if (e - lo < 32u) bits &= (1u << (e - lo)) - 1u;
+      n += __popc(bits);
+    }
+    kc[g] = n;
+    count += n;
+    ty[(seg + 1) >> 1] += n;
+  }
+  a.fcnt[u] = count;
+  auto sat = [](uint32_t v) { return v > 255u ? 255u : v; };
+  a.utypes[u] = sat(ty[0]) | (sat(ty[1]) << 8) | (sat(ty[2]) << 16) | (sat(ty[3]) << 24);
+}
+
+// The driver units' features: counted (Fill = false, after k_feat_collect) or written;
+// a warp per unit
+template <bool Fill>
+__global__ void __launch_bounds__(PT) k_feat_drivers(FeatArgs a) {
   const int lane = threadIdx.x & 31;
   const uint32_t lt = (1u << lane) - 1u;
   const uint64_t warp = ((uint64_t)blockIdx.x * PT + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * PT) >> 5;
-  for (uint64_t u = warp; u < a.nu; u += nwarps) {
-    const uint32_t base = Fill ? a.foff[u] : 0u;
-    if (!a.pass[u]) {
-      if (!Fill && lane == 0) {
-        a.fcnt[u] = 0;
-        a.utypes[u] = 0u;
-      }
-      continue;
-    }
-    const uint32_t A = a.u_owner[u];
-    if (a.u_kind[u]) {
+  for (uint64_t u0 = warp * 32; u0 < a.nu; u0 += nwarps * 32) {
+    // the driver units among the warp's 32
+    const uint64_t mine = u0 + (uint64_t)lane;
+    unsigned todo = __ballot_sync(0xffffffffu, mine < a.nu && a.pass[mine] && a.u_kind[mine]);
+    while (todo) {
+      const uint64_t u = u0 + (uint64_t)(__ffs(todo) - 1);
+      todo &= todo - 1u;
+      const uint32_t A = a.u_owner[u];
       const ShapeDev& SA = a.shapes[a.P.type[A]];
-      driver_unit<Fill>(a, u, A, SA, SA.r * a.P.f[HOM][A], vview(a, A), base, lane, lt);
-      if (!Fill && lane == 0) a.utypes[u] = 0u;
-      continue;
-    }
-    if (Fill) continue;  // pair units: k_feat_fill_flat
-    const UnitRec q = rec[u];
-    const uint32_t B = a.u_partner[u];
-    const uint64_t pid = a.u_pid[u];
-    uint32_t hlo = 0, hhi = 0;  // previous entries of the pair (owner A, partner id pid)
-    if (Fill && a.have_old) {
-      const uint32_t os = a.perm[A];
-      hlo = a.old_off[os];
-      hhi = a.old_off[os + 1];
-      uint32_t lo = hlo, hi = hhi;
-      while (lo < hi) {  // first entry with partner id >= pid
-        const uint32_t mid = (lo + hi) >> 1;
-        if (a.old.pid[mid] < pid)
-          lo = mid + 1;
-        else
-          hi = mid;
-      }
-      hlo = lo;
-      hi = hhi;
-      while (lo < hi) {  // first entry with partner id > pid
-        const uint32_t mid = (lo + hi) >> 1;
-        if (a.old.pid[mid] <= pid)
-          lo = mid + 1;
-        else
-          hi = mid;
-      }
-      hhi = lo;
-    }
-    uint32_t count = 0, ty[4] = {0u, 0u, 0u, 0u};
-    for (int seg = 0; seg < 6; seg++) {
-      const uint64_t g = (uint64_t)seg * a.nu + u;
-      const uint32_t b = toff[g], e = toff[g + 1];
-      uint32_t n = 0;
-      if (Fill) {
-        uint64_t rows, cols;
-        seg_masks(q, seg, rows, cols);
-        const uint32_t nc = (uint32_t)__popcll(cols);
-        for (uint32_t t0 = b; t0 < e; t0 += 32) {
-          const uint32_t t = t0 + (uint32_t)lane;
-          const bool kp = t < e && ((keep[t >> 5] >> (t & 31u)) & 1u);
-          const unsigned m = __ballot_sync(0xffffffffu, kp);
-          if (kp) {
-            const uint32_t loc = t - b, r = loc / nc;
-            write_feature_in(a, base + count + n + __popc(m & lt), A, B, pid, seg_type(seg), seg_swap(seg),
-                             nth_bit64(rows, (int)r), nth_bit64(cols, (int)(loc - r * nc)), hlo, hhi);
-          }
-          n += __popc(m);
-        }
-      } else {
-        uint32_t c = 0;
-        for (uint32_t w0 = (b >> 5); w0 <= ((e - 1u) >> 5) && b < e; w0 += 32) {
-          const uint32_t wd = w0 + (uint32_t)lane;
-          if (wd <= ((e - 1u) >> 5)) {
-            uint32_t bits = keep[wd];
-            const uint32_t lo = wd << 5;  // first test of the word
-            if (b > lo) bits &= ~0u << (b - lo);
-            if (e - lo < 32u) bits &= (1u << (e - lo)) - 1u;
-            c += __popc(bits);
-          }
-        }
-        n = __reduce_add_sync(0xffffffffu, c);
-        if (lane == 0) kc[g] = n;
-      }
-      count += n;
-      ty[(seg + 1) >> 1] += n;
-    }
-    if (!Fill && lane == 0) {
-      a.fcnt[u] = count;
-      auto sat = [](uint32_t v) { return v > 255u ? 255u : v; };
-      a.utypes[u] = sat(ty[0]) | (sat(ty[1]) << 8) | (sat(ty[2]) << 16) | (sat(ty[3]) << 24);
+      driver_unit<Fill>(a, u, A, SA, SA.r * a.P.f[HOM][A], vview(a, A), Fill ? a.foff[u] : 0u, lane, lt);
     }
   }
 }
@@ -2131,11 +2099,11 @@ __global__ void k_pscreen(PCArgs a) {
       const Roles R = roles(a, k);
       const ShapeDev& si = a.shapes[a.P.type[R.ip]];
       const ShapeDev& sj = a.shapes[a.P.type[R.jp]];
-      const double rim = si.r * a.P.f[HOM][R.ip], rjm = sj.r * a.P.f[HOM][R.jp];
       const uint64_t oi = (uint64_t)R.ip * a.MV, oj = (uint64_t)R.jp * a.MV;
       auto wi = [&](int q) { return f3(a.wx[oi + q], a.wy[oi + q], a.wz[oi + q]); };
       auto wj = [&](int q) { return f3(a.wx[oj + q], a.wy[oj + q], a.wz[oj + q]); };
-      const float Rf = (float)(rim + rjm) * 1.000001f;
+      // the sum of the radii h r from above: four roundings of 2^-24
+      const float Rf = (si.rf * f32_rn(a.P.f[HOM][R.ip]) + sj.rf * f32_rn(a.P.f[HOM][R.jp])) * 1.000001f;
       bool apart;
       if (type == DEM_ITYPE_VERTEX_VERTEX) {
         apart = apart_vv(wi(R.sub_i), wj(R.sub_j), Rf);
@@ -2594,12 +2562,13 @@ int launch_poly_feature_count(dem_ctx* c, uint64_t nu, uint32_t* total) {
       DEM_CUDA_TRY(c, cudaMalloc(&c->t_keep, cap * 4));
       c->t_keepcap = cap;
     }
-    ProfScope ps(c, K_BROAD_COUNT, (nt ? 2 : 1) + (mesh ? 1 : 0));
+    ProfScope ps(c, K_BROAD_COUNT, (nt ? 2 : 1) + (c->ndrv ? 1 : 0) + (mesh ? 1 : 0));
     if (nt) {
       const unsigned tb = (unsigned)std::min<uint64_t>((words * 32 + PT - 1) / PT, (uint64_t)c->num_sms * 32);
       k_feat_test<<<tb, PT, 0, c->stream>>>(a, rec, c->t_off, nt, c->t_keep);
     }
-    k_feat_collect<false><<<blocks, PT, 0, c->stream>>>(a, rec, c->t_off, c->t_keep, c->t_cnt);
+    k_feat_collect<<<grid_for(nu, PT), PT, 0, c->stream>>>(a, c->t_off, c->t_keep, c->t_cnt);
+    if (c->ndrv) k_feat_drivers<false><<<grid_for(nu, PT), PT, 0, c->stream>>>(a);
     c->t_ntests = nt;
     if (mesh) k_mesh_units<false, true><<<blocks, PT, 0, c->stream>>>(a);
   } else {
@@ -2637,7 +2606,7 @@ int launch_poly_feature_fill(dem_ctx* c, uint64_t nu) {
   ProfScope ps(c, K_BROAD_FILL, mesh ? 4 : 2);
   if (nu && c->t_flat) {
     const UnitRec* rec = reinterpret_cast<const UnitRec*>(c->u_rec);
-    if (c->ndrv) k_feat_collect<true><<<blocks, PT, 0, c->stream>>>(a, rec, c->t_off, c->t_keep, nullptr);
+    if (c->ndrv) k_feat_drivers<true><<<grid_for(nu, PT), PT, 0, c->stream>>>(a);
     const uint32_t nt = c->t_ntests;
     if (nt) {
       const unsigned tb = (unsigned)std::min<uint64_t>(((uint64_t)nt + PT - 1) / PT, (uint64_t)c->num_sms * 32);

@@ -28,6 +28,7 @@ struct ShapeDev {
   int fo[SH_MAXF + 1];  // face offsets into fv
   int fv[SH_MAXFV];
   float vf[3 * SH_MAXV];  // FP32 copy of v (split-precision displacement test)
+  float rf, maxvf;        // FP32 roundings of r and maxv
 };
 
 struct OBBd {

@@ -1,6 +1,7 @@
 // step_core.cuh -- the integration's arguments and per-particle bodies shared by the
 // sphere step (k_step_fused.cu) and the polyhedron step (k_poly.cu).
 #pragma once
+#include "f32_round.cuh"
 #include "integrate_core.cuh"
 
 namespace dem {
@@ -158,12 +159,13 @@ static int rotation_dense(const dem_ctx* c) { return c->n <= (uint64_t)c->num_sm
 // grid leaves SMs without a block (at 10 k particles 256 threads reach 40 SMs).
 static unsigned particle_block(const dem_ctx* c) { return spread_block(c, c->n, (unsigned)c->tune_block); }
 
-// Placement of the integration's multiplies: the context's mode, except that below two
-// warps an SM, unless the mode was chosen by the caller or the autotuner, every
-// multiply is on the FP64 pipe: the pipe then waits, and a product built on the integer
-// pipe is a chain of some 20 instructions where the pipe's is one.
+// Placement of the integration's multiplies: the context's mode, except that with at
+// most one warp a scheduler, unless the mode was chosen by the caller or the autotuner,
+// every multiply is on the FP64 pipe: the pipe then waits, and a product built on the
+// integer pipe is a chain of some 20 instructions where the pipe's is one (16 k bonded
+// cubes, 20 steps and a rebuild: 1.45 against 1.48 ms; 200 k: 6.64 against 5.92 ms).
 static int integ_mode(const dem_ctx* c) {
-  return c->mul_auto && c->n <= (uint64_t)c->num_sms * 64u ? 0 : c->mul_mode;
+  return c->mul_auto && c->n <= (uint64_t)c->num_sms * 128u ? 0 : c->mul_mode;
 }
 IntegArgs make_integ_args(dem_ctx* c, int epilog, int prolog);  // k_step_fused.cu
 }  // namespace dem
