@@ -85,7 +85,8 @@ int alloc_particles(dem_ctx* c, uint64_t n) {
   DEM_CUDA_TRY(c, cudaMalloc(&c->cell_tmp, cap * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->perm, cap * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->pcnt, (cap + 1) * 4));
-  DEM_CUDA_TRY(c, cudaMalloc(&c->srec, cap * 16 * sizeof(uint4)));
+  c->srec_n = 16;
+  DEM_CUDA_TRY(c, cudaMalloc(&c->srec, cap * c->srec_n * sizeof(uint4)));
   DEM_CUDA_TRY(c, cudaMalloc(&c->rev_off, (cap + 1) * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->rev_cnt, (cap + 1) * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->own_off[0], (cap + 1) * 4));

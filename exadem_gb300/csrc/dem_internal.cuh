@@ -148,6 +148,7 @@ struct MeshDev {
   const double* x;
   const double* y;
   const double* z;
+  const float4* vh;  // 2 nv: each vertex as two FP32 parts, h then l (mesh_core.cuh, Split3)
   const int* e;   // 2 ne
   const int* fo;  // nf + 1
   const int* fv;  // fo[nf]

@@ -9,12 +9,14 @@
 #include "dem_ctx.cuh"
 #include "integrate_core.cuh"
 #include "mesh_bins.hpp"
+#include "mesh_core.cuh"
 
 namespace dem {
 namespace {
 
 // shape::get_vertex(i, center, 1.0, quat) = center + quat * (1.0 * v)
-__global__ void k_mesh_world(const double* __restrict__ v0, uint64_t nv, Q4 q, V3 c, double* __restrict__ out) {
+__global__ void k_mesh_world(const double* __restrict__ v0, uint64_t nv, Q4 q, V3 c, double* __restrict__ out,
+                             float4* __restrict__ vh) {
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nv) return;
   const V3 v = mk(v0[3 * k], v0[3 * k + 1], v0[3 * k + 2]);
@@ -22,6 +24,9 @@ __global__ void k_mesh_world(const double* __restrict__ v0, uint64_t nv, Q4 q, V
   out[k] = w.x;
   out[nv + k] = w.y;
   out[2 * nv + k] = w.z;
+  const Split3 sp = split3(w);
+  vh[2 * k] = make_float4(sp.h.x, sp.h.y, sp.h.z, 0.f);
+  vh[2 * k + 1] = make_float4(sp.l.x, sp.l.y, sp.l.z, 0.f);
 }
 
 // bins of one mesh for particles of radius <= rad and the skin (mesh_bins.hpp), uploaded
@@ -85,6 +90,20 @@ int ensure_mesh_bins(dem_ctx* c) {
     DEM_CUDA_TRY(c, cudaMalloc(&c->mesh_cnt, cap * 4));
     c->mesh_cnt_cap = cap;
     c->gen++;  // captured kernels hold the old buffer
+  }
+  // A sphere where triangles meet has tens of mesh candidates: with a mesh a particle has
+  // 48 records for them, up to 16 GB in all or as the memory allows (without: k_mesh_fill).
+  if (!c->meshes.empty() && !c->poly && !c->capturing && c->srec_n < 64 && c->pcap <= (1ull << 24)) {
+    uint32_t* grown = nullptr;
+    if (cudaMalloc(&grown, c->pcap * 64 * sizeof(uint4)) == cudaSuccess) {
+      DEM_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+      cudaFree(c->srec);
+      c->srec = grown;
+      c->srec_n = 64;
+      c->gen++;
+    } else {
+      cudaGetLastError();
+    }
   }
   if (!c->meshes.empty() && c->poly && c->prm.learned_sizing)
     return c->fail(DEM_ERR_UNSUPPORTED, "learned record sizing does not bound mesh units: learned_sizing = 0");
@@ -167,7 +186,8 @@ extern "C" int dem_register_mesh(dem_ctx* c, const dem_mesh* s) {
     return rc;
   };
   const size_t vb = (size_t)std::max(nv, 1) * 3 * sizeof(double);
-  if (cudaMalloc(&m.vtx, vb) != cudaSuccess || cudaMalloc(&v0, vb) != cudaSuccess ||
+  const size_t vh0 = (vb + 15) & ~(size_t)15;  // the FP32 parts follow the vertices
+  if (cudaMalloc(&m.vtx, vh0 + (size_t)std::max(nv, 1) * 2 * sizeof(float4)) != cudaSuccess || cudaMalloc(&v0, vb) != cudaSuccess ||
       cudaMalloc(&m.e, (size_t)std::max(2 * ne, 1) * 4) != cudaSuccess ||
       cudaMalloc(&m.fo, (size_t)(nf + 1) * 4) != cudaSuccess ||
       cudaMalloc(&m.fv, (size_t)std::max(nfv, 1) * 4) != cudaSuccess)
@@ -181,8 +201,9 @@ extern "C" int dem_register_mesh(dem_ctx* c, const dem_mesh* s) {
   if (ne) ok = ok && cudaMemcpyAsync(m.e, m.he.data(), (size_t)ne * 8, cudaMemcpyHostToDevice, c->stream) == cudaSuccess;
   ok = ok && cudaMemcpyAsync(m.fo, m.hfo.data(), m.hfo.size() * 4, cudaMemcpyHostToDevice, c->stream) == cudaSuccess;
   if (nfv) ok = ok && cudaMemcpyAsync(m.fv, m.hfv.data(), (size_t)nfv * 4, cudaMemcpyHostToDevice, c->stream) == cudaSuccess;
+  float4* const vh = m.vtx ? reinterpret_cast<float4*>(reinterpret_cast<char*>(m.vtx) + vh0) : nullptr;
   if (nv) {
-    k_mesh_world<<<(unsigned)((nv + 255) / 256), 256, 0, c->stream>>>(v0, (uint64_t)nv, q, ctr, m.vtx);
+    k_mesh_world<<<(unsigned)((nv + 255) / 256), 256, 0, c->stream>>>(v0, (uint64_t)nv, q, ctr, m.vtx, vh);
     ok = ok && cudaGetLastError() == cudaSuccess;
   }
   m.hx.resize(nv);
@@ -201,6 +222,7 @@ extern "C" int dem_register_mesh(dem_ctx* c, const dem_mesh* s) {
   m.dev.x = m.vtx;
   m.dev.y = m.vtx + nv;
   m.dev.z = m.vtx + 2 * (size_t)nv;
+  m.dev.vh = vh;
   m.dev.e = m.e;
   m.dev.fo = m.fo;
   m.dev.fv = m.fv;

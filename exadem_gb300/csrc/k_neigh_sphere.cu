@@ -45,9 +45,11 @@ struct BPArgs {
   const float4* crel;
   float skin_f;
   uint64_t cap;  // interaction buffer capacity (graph step): a fill beyond it writes nothing
-  // FP32 path: the count pass's candidates of each particle (SREC per particle:
+  // FP32 path: the count pass's candidates of each particle (SREC per particle,
+  // then nmrec mesh candidates:
   // partner, meta, partner id), read by the fill when they fit
   uint32_t* srec;
+  uint32_t nmrec;
   uint32_t* rev_cnt;  // FP32 path: the fill's count of each particle's partner list
   uint32_t* rev_pos;  // and the place of each entry in it (a scratch of the records' capacity)
   // per-pair damping damp_rate 2 sqrt(kn meff), in the operation order of the
@@ -231,89 +233,188 @@ __device__ inline void for_each_candidate(const BPArgs& a, uint32_t s, Emit&& em
   for_each_particle<F32>(a, s, sys, emit);
 }
 
-// Mesh candidates (detection_sphere_driver, nbh_sphere.hpp:25-86): every mesh
-// vertex, edge and face of the sphere's bin that passes its filter, partner
-// sub = the feature.  A sphere's bin can list hundreds of features (where many
-// triangles meet), so the whole warp serves its spheres one at a time, a lane
-// per bin item; with Fill the passing items go, in bin order, to the start of
-// the sphere's segment [b, e) (the per-sphere sort orders the segment).
-// Returns the lane's own sphere's count.  Every lane of the warp calls it.
-template <bool F32, bool Fill>
-__device__ uint32_t mesh_phase(const BPArgs& a, uint64_t s, bool want, uint32_t b, uint32_t e, IArrays dst) {
-  const int lane = threadIdx.x & 31;
-  uint32_t mine = 0;
-  unsigned todo = __ballot_sync(0xffffffffu, want);
-  while (todo) {
-    const int L = __ffs(todo) - 1;
-    todo &= todo - 1u;
-    const uint32_t sL = (uint32_t)__shfl_sync(0xffffffffu, (unsigned long long)s, L);
-    const uint32_t bL = __shfl_sync(0xffffffffu, b, L), eL = __shfl_sync(0xffffffffu, e, L);
-    const V3 p = mk(a.P.f[RX][sL], a.P.f[RY][sL], a.P.f[RZ][sL]);
-    const double rad = a.P.f[RAD][sL];
-    const int2 dr = a.sv.drange[a.sv.of(sL)];
-    uint32_t n = 0;
-    for (int k = dr.x; k < dr.x + dr.y; k++) {
-      const DriverDev& d = a.drv[k];
-      if (d.kind != 2) continue;
-      const MeshDev& m = a.mesh[d.mesh];
-      uint64_t bb;
-      if (!mesh_bin_of(m, p, bb)) continue;
-      const uint32_t q0 = m.boff[bb], q1 = m.boff[bb + 1];
-      for (uint32_t t0 = q0; t0 < q1; t0 += 32) {
-        const uint32_t t = t0 + lane;
-        bool pass = false;
-        uint32_t kind = 0, j = 0;
-        if (t < q1) {
-          const uint32_t it = m.bitem[t];
-          kind = it >> 30;
-          j = it & 0x3fffffffu;
-          pass = F32 ? mesh_filter_f32(m, kind, j, a.skin, p, rad) : mesh_filter(m, kind, j, a.skin, p, rad);
-        }
-        const unsigned pm = __ballot_sync(0xffffffffu, pass);
-        if (Fill && pass) {
-          const uint32_t w = bL + n + __popc(pm & ((1u << lane) - 1u));
-          if (w < eL) {
-            dst.partner[w] = (uint32_t)k;
-            dst.pid[w] = (uint64_t)k;
-            dst.meta[w] = make_meta(DEM_ITYPE_VERTEX_MESH_VERTEX + kind, 0, 0, 0, false);
-            dst.sub[w] = j << 16;
-          }
-        }
-        n += __popc(pm);
-      }
-    }
-    if (lane == L) mine = n;
-  }
-  __syncwarp();  // the items other lanes wrote are read by the sphere's own lane
-  return mine;
-}
-
-// the mesh candidates of each triggered sphere, one warp per sphere (lane 0
-// asks mesh_phase for its sphere): a sphere whose bin lists hundreds of
-// features gets a warp of its own.  Kept out of k_count / k_fill so the
-// particle-pair passes keep their register budget.
-template <bool F32>
-__global__ void k_mesh_count(BPArgs a, uint32_t* __restrict__ mcnt, uint32_t* __restrict__ cnt) {
-  const uint64_t s = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (s >= a.n) return;  // the whole warp
-  const bool lead = (threadIdx.x & 31) == 0;
-  const bool trig = a.sv.triggered(a.sv.of(s));
-  const uint32_t m = mesh_phase<F32, false>(a, s, lead && trig, 0u, 0u, IArrays{});
-  if (lead) {
-    mcnt[s] = trig ? m : 0u;
-    cnt[s] = trig ? m : 0u;  // the particle candidates are added to it
-  }
-}
-template <bool F32>
-__global__ void k_mesh_fill(BPArgs a, const uint32_t* __restrict__ off, IArrays dst) {
-  const uint64_t s = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (s >= a.n) return;  // the whole warp
-  const uint32_t b = off[s], e = off[s + 1];
-  const bool trig = e <= a.cap && a.sv.triggered(a.sv.of(s));
-  mesh_phase<F32, true>(a, s, (threadIdx.x & 31) == 0 && trig, b, e, dst);
+// InteractionPair order inside the owner: (partner id, type, partner sub); swap
+// and the owner sub are 0 for spheres
+__device__ inline bool key_less(uint64_t pa, uint32_t ta, uint32_t sa, uint64_t pb, uint32_t tb, uint32_t sb) {
+  return pa < pb || (pa == pb && (ta < tb || (ta == tb && sa < sb)));
 }
 
 constexpr uint32_t SREC = 16;
+
+// Mesh candidates (detection_sphere_driver, nbh_sphere.hpp:25-86): every mesh
+// vertex, edge and face of the sphere's bin that passes its filter, partner
+// sub = the feature.  A block serves the spheres s of its first 32 threads (want), which
+// find their spheres' bins; the bins' items are then dealt to all its threads in one
+// sequence: a test is a chain of loads and FP32 operations of some 5 us, and a bin can list
+// hundreds of features (where many triangles meet).  The spheres of a block lie far apart
+// in the cell order (mesh_sphere), so neighbours at such a place fall to different blocks.
+// emit(s, at, k, kind, j) takes the passing items of sphere s, at counting them in no
+// particular order (the fill orders a sphere's entries by their keys).  Returns the
+// thread's own sphere's count.  Every thread of the block calls it.
+constexpr int MESH_BLOCK = 128;
+constexpr int MESH_SPHERES = 32;
+struct MeshWork {
+  uint32_t pre[MESH_SPHERES + 1], s[MESH_SPHERES], q0[MESH_SPHERES], mesh[MESH_SPHERES], cnt[MESH_SPHERES];
+  int k[MESH_SPHERES];
+  float R[MESH_SPHERES], pabs[MESH_SPHERES];
+  Split3 p[MESH_SPHERES];
+  int nk;
+};
+template <bool F32, class Emit>
+__device__ uint32_t mesh_phase(const BPArgs& a, uint64_t s, bool want, MeshWork& w, Emit&& emit) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int t = threadIdx.x;
+  const bool lead = t < MESH_SPHERES;  // one warp
+  V3 p = mk(0.0, 0.0, 0.0);
+  double rad = 0.0;
+  int2 dr = make_int2(0, 0);
+  if (lead) {
+    Split3 sp{};
+    if (want) {
+      p = mk(a.P.f[RX][s], a.P.f[RY][s], a.P.f[RZ][s]);
+      rad = a.P.f[RAD][s];
+      dr = a.sv.drange[a.sv.of(s)];
+      if (F32) sp = split3(p);
+    }
+    w.s[t] = (uint32_t)s;
+    w.cnt[t] = 0u;
+    w.p[t] = sp;
+    w.pabs[t] = fabsf(sp.h.x) + fabsf(sp.h.y) + fabsf(sp.h.z);
+    const int nk = __reduce_max_sync(FULL, dr.y);
+    if (t == 0) w.nk = nk;
+  }
+  __syncthreads();
+  const int nk = w.nk;
+  for (int kk = 0; kk < nk; kk++) {
+    if (lead) {
+      const int k = dr.x + kk;
+      uint32_t len = 0;
+      if (kk < dr.y && a.drv[k].kind == 2) {
+        const uint32_t mesh = (uint32_t)a.drv[k].mesh;
+        const MeshDev& m = a.mesh[mesh];
+        uint64_t bb;
+        if (mesh_bin_of(m, p, bb)) {
+          const uint32_t q0 = m.boff[bb];
+          len = m.boff[bb + 1] - q0;
+          w.q0[t] = q0;
+          w.mesh[t] = mesh;
+          w.k[t] = k;
+          if (F32 && len) w.R[t] = f32_rn(rad + m.r + a.skin);
+        }
+      }
+      uint32_t sum = len;
+#pragma unroll
+      for (int o = 1; o < MESH_SPHERES; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(FULL, sum, o);
+        if (t >= o) sum += v;
+      }
+      w.pre[t] = sum - len;
+      if (t == MESH_SPHERES - 1) w.pre[MESH_SPHERES] = sum;
+    }
+    __syncthreads();
+    const uint32_t total = w.pre[MESH_SPHERES];
+    for (uint32_t i = t; i < total; i += MESH_BLOCK) {
+      int L = 0;  // the last sphere whose items start at or before i
+#pragma unroll
+      for (int o = MESH_SPHERES / 2; o; o >>= 1)
+        if (i >= w.pre[L + o]) L += o;
+      const MeshDev& m = a.mesh[w.mesh[L]];
+      const uint32_t it = m.bitem[w.q0[L] + (i - w.pre[L])], kind = it >> 30, j = it & 0x3fffffffu, o = w.s[L];
+      const bool pass = F32 ? mesh_filter_f32(m, kind, j, a.skin, a.skin_f, w.p[L], w.R[L], w.pabs[L], a.P.f, o)
+                            : mesh_filter(m, kind, j, a.skin, mk(a.P.f[RX][o], a.P.f[RY][o], a.P.f[RZ][o]),
+                                          a.P.f[RAD][o]);
+      if (pass) emit(o, atomicAdd(&w.cnt[L], 1u), (uint32_t)w.k[L], kind, j);
+    }
+    __syncthreads();
+  }
+  return lead ? w.cnt[t] : 0u;
+}
+
+// the sphere of one of a block's first 32 threads
+__device__ __forceinline__ uint64_t mesh_sphere() { return (uint64_t)threadIdx.x * gridDim.x + blockIdx.x; }
+
+// The mesh candidates of each triggered sphere.  Kept out of the count and fill kernels so
+// the particle-pair passes keep their register budget.  With Rec they become the first
+// records of the sphere (k_fill_entries): partner the driver, the feature in the place of
+// the partner id, in any order.
+// Measured, 50 k mixer: MIXER_COUNT
+template <bool F32, bool Rec>
+__global__ void __launch_bounds__(MESH_BLOCK) k_mesh_count(BPArgs a, uint32_t* __restrict__ mcnt,
+                                                           uint32_t* __restrict__ cnt) {
+  __shared__ MeshWork w;
+  const uint64_t s = mesh_sphere();
+  const bool own = threadIdx.x < MESH_SPHERES && s < a.n;
+  const bool trig = own && a.sv.triggered(a.sv.of(s));
+  uint4* const rec = reinterpret_cast<uint4*>(a.srec);
+  const uint32_t m =
+      mesh_phase<F32>(a, s, trig, w, [&](uint32_t o, uint32_t at, uint32_t k, uint32_t kind, uint32_t j) {
+        if (Rec && at < a.nmrec)
+          rec[(uint64_t)o * (SREC + a.nmrec) + SREC + at] =
+              make_uint4(k, make_meta(DEM_ITYPE_VERTEX_MESH_VERTEX + kind, 0, 0, 0, false), j << 16, 0u);
+      });
+  if (own) {
+    mcnt[s] = m;
+    cnt[s] = m;  // the particle candidates are added to it
+  }
+}
+// The mesh items of each triggered sphere at the start of its segment, in key order; with
+// Rec all entries of the spheres whose records overflowed, the others of the list not at
+// all.  The items are first put into the history's arrays, unordered, and then ranked by
+// the block's threads.
+template <bool F32, bool Rec>
+__global__ void __launch_bounds__(MESH_BLOCK) k_mesh_fill(BPArgs a, const uint32_t* __restrict__ off, IArrays dst) {
+  __shared__ MeshWork w;
+  const uint64_t s = mesh_sphere();
+  const bool own = threadIdx.x < MESH_SPHERES && s < a.n;
+  const uint32_t b = own ? off[s] : 0u, e = own ? off[s + 1] : 0u, mm = own ? a.mcnt[s] : 0u;
+  const bool want = own && e <= a.cap && a.sv.triggered(a.sv.of(s)) &&
+                    (Rec ? mm > a.nmrec || e - b - mm > SREC : mm > 0u);
+  if (!__syncthreads_or(want)) return;
+  auto put = [&](uint32_t x, uint32_t partner, uint64_t pid, uint32_t meta, uint32_t sub) {
+    dst.ft[0][x] = emu_double((uint64_t)partner | (uint64_t)sub << 32);
+    dst.ft[1][x] = emu_double(pid);
+    dst.ft[2][x] = emu_double(meta);
+  };
+  mesh_phase<F32>(a, s, want, w, [&](uint32_t o, uint32_t at, uint32_t k, uint32_t kind, uint32_t j) {
+    const uint32_t x = off[o] + at;
+    if (x < off[o + 1]) put(x, k, k, make_meta(DEM_ITYPE_VERTEX_MESH_VERTEX + kind, 0, 0, 0, false), j << 16);
+  });
+  if (Rec && want) {
+    uint32_t x = b + mm;
+    if (e - x <= SREC) {
+      const uint4* const rec = reinterpret_cast<const uint4*>(a.srec) + s * (SREC + a.nmrec);
+      for (uint32_t y = 0; x < e; x++, y++) put(x, rec[y].x, (uint64_t)rec[y].z | (uint64_t)rec[y].w << 32, rec[y].y, 0u);
+    } else {
+      for_each_candidate<true>(a, (uint32_t)s, [&](uint32_t q, uint64_t pid, uint32_t meta, uint32_t sub) {
+        if (x < e) put(x, q, pid, meta, sub);
+        x++;
+      });
+    }
+  }
+  if (threadIdx.x < MESH_SPHERES) {
+    w.cnt[threadIdx.x] = want ? (Rec ? e - b : mm) : 0u;
+    w.q0[threadIdx.x] = b;
+  }
+  __syncthreads();
+  for (int L = 0; L < MESH_SPHERES; L++) {
+    const uint32_t n = w.cnt[L], first = w.q0[L];
+    for (uint32_t x = threadIdx.x; x < n; x += MESH_BLOCK) {
+      const uint64_t word = emu_bits(dst.ft[0][first + x]), pid = emu_bits(dst.ft[1][first + x]);
+      const uint32_t meta = (uint32_t)emu_bits(dst.ft[2][first + x]), sub = (uint32_t)(word >> 32);
+      uint32_t rank = 0;
+      for (uint32_t y = first; y < first + n; y++)
+        rank += key_less(emu_bits(dst.ft[1][y]), meta_type((uint32_t)emu_bits(dst.ft[2][y])),
+                         (uint32_t)(emu_bits(dst.ft[0][y]) >> 32), pid, meta_type(meta), sub)
+                    ? 1u
+                    : 0u;
+      const uint32_t x1 = first + rank;
+      dst.partner[x1] = (uint32_t)word;
+      dst.pid[x1] = pid;
+      dst.meta[x1] = meta;
+      dst.sub[x1] = sub;
+    }
+  }
+}
 
 __global__ void k_count(BPArgs a, uint32_t* __restrict__ cnt, const uint32_t* __restrict__ old_off) {
   const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -370,7 +471,7 @@ __global__ void __launch_bounds__(PAIR_BLOCK) k_count_pairs(BPArgs a, uint32_t* 
   uint4* const rec = reinterpret_cast<uint4*>(a.srec);
   auto store = [&](uint32_t o, uint32_t at, uint32_t q, uint32_t meta, uint64_t pid) {
     const uint32_t m = at - (a.has_mesh ? a.mcnt[o] : 0u);
-    if (m < SREC) rec[(uint64_t)o * SREC + m] = make_uint4(q, meta, (uint32_t)pid, (uint32_t)(pid >> 32));
+    if (m < SREC) rec[(uint64_t)o * (SREC + a.nmrec) + m] = make_uint4(q, meta, (uint32_t)pid, (uint32_t)(pid >> 32));
   };
   auto append = [&](uint32_t o, uint32_t q, uint32_t meta, uint64_t pid) {
     store(o, atomicAdd(&cnt[o], 1u), q, meta, pid);
@@ -488,12 +589,6 @@ __global__ void __launch_bounds__(PAIR_BLOCK) k_count_pairs(BPArgs a, uint32_t* 
       store(mine ? p : q, at[k], mine ? q : p, make_meta(DEM_ITYPE_VERTEX_VERTEX, 0, 0, 0, false), mine ? idq[k] : idp);
     }
   }
-}
-
-// InteractionPair order inside the owner: (partner id, type, partner sub); swap
-// and the owner sub are 0 for spheres
-__device__ inline bool key_less(uint64_t pa, uint32_t ta, uint32_t sa, uint64_t pb, uint32_t tb, uint32_t sb) {
-  return pa < pb || (pa == pb && (ta < tb || (ta == tb && sa < sb)));
 }
 
 // entry y of the previous list as entry x of the new one, owned by slot s
@@ -629,8 +724,9 @@ __global__ void k_expand_owner(BPArgs a, const uint32_t* __restrict__ off, uint3
 // every comparison and move: 57 and 421 us; eight lanes per particle with shuffles:
 // 9 and 538 us, with two of three lanes idle.
 // The partner lists are counted on the way: the atomic's value is the entry's
-// place in its partner's list (rev_pos).  Particles with mesh candidates or more
-// than SREC others are filled and sorted by the thread of their first entry.
+// place in its partner's list (rev_pos).  Particles whose records
+// overflowed are filled and sorted by the thread of their first entry, or with a mesh
+// come ordered from k_mesh_fill.
 __global__ void __launch_bounds__(128) k_fill_entries(BPArgs a, const uint32_t* __restrict__ off,
                                                       IArrays dst, IArrays old, const uint32_t* __restrict__ old_off,
                                                       const uint32_t* __restrict__ perm, int have_old,
@@ -652,49 +748,55 @@ __global__ void __launch_bounds__(128) k_fill_entries(BPArgs a, const uint32_t* 
       continue;
     }
     const uint32_t mm = a.has_mesh ? a.mcnt[s] : 0u;
-    const uint4* const rec = recs + (uint64_t)s * SREC;
-    auto pid_of = [](uint4 v) { return (uint64_t)v.z | (uint64_t)v.w << 32; };
-    if (mm || m > SREC) {
+    const bool over = mm > a.nmrec || m - mm > SREC;
+    if (over && !a.has_mesh) {
       if (x) continue;
       const uint32_t e = b + m;
-      uint32_t w = b + mm;  // mesh items first (k_mesh_fill)
-      if (m - mm <= SREC) {
-        for (uint32_t y = 0; y < m - mm; y++) {
-          const uint4 v = rec[y];
-          dst.partner[w + y] = v.x;
-          dst.pid[w + y] = pid_of(v);
-          dst.meta[w + y] = v.y;
-          dst.sub[w + y] = 0u;
+      uint32_t w = b;
+      for_each_candidate<true>(a, s, [&](uint32_t q, uint64_t pid, uint32_t meta, uint32_t sub) {
+        if (w < e) {
+          dst.partner[w] = q;
+          dst.pid[w] = pid;
+          dst.meta[w] = meta;
+          dst.sub[w] = sub;
         }
-      } else {
-        for_each_candidate<true>(a, s, [&](uint32_t q, uint64_t pid, uint32_t meta, uint32_t sub) {
-          if (w < e) {
-            dst.partner[w] = q;
-            dst.pid[w] = pid;
-            dst.meta[w] = meta;
-            dst.sub[w] = sub;
-          }
-          w++;
-        });
-      }
+        w++;
+      });
       finish_owner(a, s, b, e, dst, old, old_off, perm, have_old, reuse_damp);
       for (uint32_t y = b; y < e; y++) partner_list(y, dst.partner[y], dst.meta[y]);
       continue;
     }
-    const uint4 v = rec[x];
-    const uint64_t pid = pid_of(v);
-    const uint32_t type = meta_type(v.y);
-    uint32_t rank = 0;
-    for (uint32_t y = 0; y < m; y++) {
-      const uint4 u = rec[y];
-      rank += key_less(pid_of(u), meta_type(u.y), 0u, pid, type, 0u) ? 1u : 0u;
+    uint32_t partner, meta, sub, type, rank = x;
+    uint64_t pid;
+    if (over) {  // in place and in order (k_mesh_fill)
+      partner = dst.partner[k];
+      pid = dst.pid[k];
+      meta = dst.meta[k];
+      sub = dst.sub[k];
+      type = meta_type(meta);
+    } else {
+      const uint4* const rec = recs + (uint64_t)s * (SREC + a.nmrec);
+      auto at = [&](uint32_t y) { return rec[y < mm ? SREC + y : y - mm]; };
+      // a mesh item's partner id is its driver, its sub the feature (k_mesh_count)
+      auto pid_of = [&](uint4 v, uint32_t y) { return y < mm ? (uint64_t)v.x : (uint64_t)v.z | (uint64_t)v.w << 32; };
+      const uint4 v = at(x);
+      partner = v.x;
+      meta = v.y;
+      type = meta_type(meta);
+      pid = pid_of(v, x);
+      sub = x < mm ? v.z : 0u;
+      rank = 0;
+      for (uint32_t y = 0; y < m; y++) {
+        const uint4 u = at(y);
+        rank += key_less(pid_of(u, y), meta_type(u.y), y < mm ? u.z : 0u, pid, type, sub) ? 1u : 0u;
+      }
     }
     uint32_t hit = ~0u;
     if (have_old) {
       const uint32_t os = perm[s];
       const uint32_t oe = old_off[os + 1];
       for (uint32_t y = old_off[os]; y < oe; y++)
-        if (old.pid[y] == pid && meta_type(old.meta[y]) == type && old.sub[y] == 0u) hit = y;
+        if (old.pid[y] == pid && meta_type(old.meta[y]) == type && old.sub[y] == sub) hit = y;
     }
     double h[6] = {0, 0, 0, 0, 0, 0};
     double damp = 0.0;
@@ -706,19 +808,19 @@ __global__ void __launch_bounds__(128) k_fill_entries(BPArgs a, const uint32_t* 
       }
       damp = old.damp[hit];
     }
-    if (hit == ~0u || !reuse_damp) damp = pair_damp(a, s, v.x, v.y);
+    if (hit == ~0u || !reuse_damp) damp = pair_damp(a, s, partner, meta);
     const uint64_t w = b + rank;
-    dst.partner[w] = v.x;
+    dst.partner[w] = partner;
     dst.pid[w] = pid;
-    dst.meta[w] = v.y;
-    dst.sub[w] = 0u;
+    dst.meta[w] = meta;
+    dst.sub[w] = sub;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
       dst.ft[d][w] = h[d];
       dst.mo[d][w] = h[3 + d];
     }
     dst.damp[w] = damp;
-    partner_list(w, v.x, v.y);
+    partner_list(w, partner, meta);
   }
 }
 
@@ -1078,6 +1180,7 @@ BPArgs make_args(dem_ctx* c) {
   a.skin_f = (float)c->prm.rcut_inc;
   a.cap = c->capturing ? c->gcap : ~0ull;
   a.srec = c->srec;
+  a.nmrec = c->srec_n - SREC;
   a.rev_cnt = c->rev_cnt;
   a.rev_pos = c->L2;
   a.cp = c->prm.config;
@@ -1109,10 +1212,12 @@ int launch_count_sphere(dem_ctx* c) {
   ProfScope ps(c, K_BROAD_COUNT, c->n ? (mesh ? 2 : 1) : 0);
   if (c->n && mesh) {
     if (!c->mesh_cnt) return c->fail(DEM_ERR_STATE, "mesh count buffer missing");
-    if (c->prm.fp32_broad_phase)
-      k_mesh_count<true><<<grid_for(c->n * 32, 128), 128, 0, c->stream>>>(make_args(c), c->mesh_cnt, c->pcnt);
-    else
-      k_mesh_count<false><<<grid_for(c->n * 32, 128), 128, 0, c->stream>>>(make_args(c), c->mesh_cnt, c->pcnt);
+    // with records (k_count_pairs' path) the fill takes the mesh items from them
+    const auto kern = !c->prm.fp32_broad_phase ? k_mesh_count<false, false>
+                      : c->cell_broad_phase    ? k_mesh_count<true, false>
+                                               : k_mesh_count<true, true>;
+    kern<<<grid_for(c->n, MESH_SPHERES), MESH_BLOCK, 0, c->stream>>>(make_args(c), c->mesh_cnt,
+                                                                                             c->pcnt);
   }
   if (c->n) {
     if (c->prm.fp32_broad_phase && c->cell_broad_phase) {
@@ -1136,10 +1241,11 @@ int launch_fill_sphere(dem_ctx* c, uint32_t* new_off, uint64_t total) {
   const bool cells = c->prm.fp32_broad_phase && c->cell_broad_phase;
   ProfScope ps(c, K_BROAD_FILL, c->n ? (mesh ? 1 : 0) + (cells ? 3 : c->prm.fp32_broad_phase ? 2 : 1) : 0);
   if (c->n && mesh) {
-    if (c->prm.fp32_broad_phase)
-      k_mesh_fill<true><<<grid_for(c->n * 32, 128), 128, 0, c->stream>>>(make_args(c), new_off, c->I[nw]);
-    else
-      k_mesh_fill<false><<<grid_for(c->n * 32, 128), 128, 0, c->stream>>>(make_args(c), new_off, c->I[nw]);
+    const auto kern = !c->prm.fp32_broad_phase ? k_mesh_fill<false, false>
+                      : c->cell_broad_phase    ? k_mesh_fill<true, false>
+                                               : k_mesh_fill<true, true>;
+    kern<<<grid_for(c->n, MESH_SPHERES), MESH_BLOCK, 0, c->stream>>>(make_args(c), new_off,
+                                                                                             c->I[nw]);
   }
   if (c->n) {
     const int have_old = c->hist_valid ? 1 : 0, reuse = (c->hist_valid && !c->damp_stale) ? 1 : 0;

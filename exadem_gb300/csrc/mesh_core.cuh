@@ -8,6 +8,7 @@
 #pragma once
 #include "../../include/dem_hotpath.h"
 #include "poly_core.cuh"
+#include "f32_round.cuh"
 #include "poly_f32.cuh"
 
 namespace dem {
@@ -26,32 +27,44 @@ __device__ inline bool mesh_filter(const MeshDev& m, uint32_t kind, uint32_t j, 
   return vf_core_list(rad + m.r + rV, p, v, m.fv + b, m.fo[j + 1] - b, dist, n);
 }
 
-// mesh_filter decided in FP32 first (poly_f32.cuh): coordinates relative to the
-// sphere centre p, each an FP32 rounding of the FP64 difference (error u S with
-// S a bound of their lengths plus the filter range); a decided test has the
-// FP64 result, an undecided one runs mesh_filter
-__device__ inline bool mesh_filter_f32(const MeshDev& m, uint32_t kind, uint32_t j, double rV, V3 p, double rad) {
-  const VView v = mesh_view(m);
+// A sphere centre or mesh vertex x as two FP32 values h + l (|x - h - l| <= 2^-47 |x|)
+struct Split3 {
+  F3 h, l;
+};
+__device__ __forceinline__ Split3 split3(V3 p) {
+  Split3 r;
+  r.h = f3(f32_rn(p.x), f32_rn(p.y), f32_rn(p.z));
+  r.l = f3(f32_rn(p.x - (double)r.h.x), f32_rn(p.y - (double)r.h.y), f32_rn(p.z - (double)r.h.z));
+  return r;
+}
+
+// mesh_filter decided in FP32 first (poly_f32.cuh), without an FP64 instruction:
+// coordinates relative to the sphere centre p, (v_h - p_h) + (v_l - p_l).  With S a bound
+// of their lengths plus the filter range R their error is at most 2 u S, and 2^-44 of a
+// coordinate, which the 2^-19 |p|_1 in S (pabs) turns into another u S: the 3 u S that the
+// decisions allow.  A decided test has the FP64 result, an undecided one runs mesh_filter.
+__device__ inline bool mesh_filter_f32(const MeshDev& m, uint32_t kind, uint32_t j, double rV, float rVf,
+                                       const Split3& p, float R, float pabs, const double* const* f, uint32_t s) {
   auto rel = [&](int k) {
-    const V3 w = v[k];
-    return f3((float)(w.x - p.x), (float)(w.y - p.y), (float)(w.z - p.z));
+    const float4 h = m.vh[2 * k], l = m.vh[2 * k + 1];
+    return f3((h.x - p.h.x) + (l.x - p.l.x), (h.y - p.h.y) + (l.y - p.l.y), (h.z - p.h.z) + (l.z - p.l.z));
   };
-  const float R = (float)(rad + m.r + rV);
+  const float S0 = R + pabs * 1.9073486e-06f;
   int dec;
   if (kind == 0) {
     const F3 a = rel((int)j);
-    dec = decide_vv(f3(0.f, 0.f, 0.f), a, R, flen(a) * 1.000001f + R);
+    dec = decide_vv(f3(0.f, 0.f, 0.f), a, R, flen(a) * 1.000001f + S0);
   } else if (kind == 1) {
     const F3 a = rel(m.e[2 * j]), b = rel(m.e[2 * j + 1]);
-    dec = decide_ve(f3(0.f, 0.f, 0.f), a, b, R, (float)rV, fmaxf(flen(a), flen(b)) * 1.000001f + R);
+    dec = decide_ve(f3(0.f, 0.f, 0.f), a, b, R, rVf, fmaxf(flen(a), flen(b)) * 1.000001f + S0);
   } else {
     const int b = m.fo[j], nf = m.fo[j + 1] - b;
     float S = 0.f;
     for (int k = 0; k < nf; k++) S = fmaxf(S, flen(rel(m.fv[b + k])));
-    dec = decide_vf_list(f3(0.f, 0.f, 0.f), nf, [&](int k) { return rel(m.fv[b + k]); }, R, S * 1.000001f + R);
+    dec = decide_vf_list(f3(0.f, 0.f, 0.f), nf, [&](int k) { return rel(m.fv[b + k]); }, R, S * 1.000001f + S0);
   }
   if (dec != DEC_UNDECIDED) return dec == DEC_TRUE;
-  return mesh_filter(m, kind, j, rV, p, rad);
+  return mesh_filter(m, kind, j, rV, mk(f[RX][s], f[RY][s], f[RZ][s]), f[RAD][s]);
 }
 
 // detect<type> for a sphere and mesh feature j
