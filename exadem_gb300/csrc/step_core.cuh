@@ -74,20 +74,34 @@ __device__ __forceinline__ bool epilog_translate(const IntegArgs& a, uint64_t s,
   const uint32_t o0 = a.own_off[s], no = a.own_off[s + 1] - o0;
   const uint32_t r0 = a.rev_off[s];
   const uint32_t nt = a.pass && a.stamp[s] != a.pass ? 0u : no + (a.rev_off[s + 1] - r0);
-  for (uint32_t q = 0; q < nt; q++) {
-    const bool own = q < no;
-    const uint32_t k = own ? o0 + q : a.rev_idx[r0 + (q - no)];
-    if (!R.live[k]) continue;
-    const double* t0 = own ? R.ti[0] : R.tj[0];
-    const double* t1 = own ? R.ti[1] : R.tj[1];
-    const double* t2 = own ? R.ti[2] : R.tj[2];
-    const V3 rf = mk(R.f[0][k], R.f[1][k], R.f[2][k]), rt = mk(t0[k], t1[k], t2[k]);
-    if (((emu_bits(rf.x) | emu_bits(rf.y) | emu_bits(rf.z) | emu_bits(rt.x) | emu_bits(rt.y) | emu_bits(rt.z))
-         << 1) != 0) {
-      const uint64_t flip = own ? 0ull : 0x8000000000000000ull;  // -rf for a partner record (exact)
-      f = f + mk(emu_double(emu_bits(rf.x) ^ flip), emu_double(emu_bits(rf.y) ^ flip),
-                 emu_double(emu_bits(rf.z) ^ flip));
-      mom = mom + rt;
+  // Two records at a time, their indexes and flags loaded together: a record is a chain of
+  // three loads (10 k box, 100 steps: 3.40 to 3.31 ms; four or eight are no faster, and
+  // above 100 k particles the FP64 pipe is the bound either way).
+  constexpr int GB = 2;
+  for (uint32_t q = 0; q < nt; q += GB) {
+    uint32_t kk[GB];
+    unsigned live = 0;
+#pragma unroll
+    for (int u = 0; u < GB; u++) kk[u] = q + u < no ? o0 + q + u : (q + u < nt ? a.rev_idx[r0 + (q + u - no)] : 0u);
+#pragma unroll
+    for (int u = 0; u < GB; u++)
+      if (q + u < nt && R.live[kk[u]]) live |= 1u << u;
+#pragma unroll
+    for (int u = 0; u < GB; u++) {
+      if (!(live >> u & 1u)) continue;
+      const bool own = q + u < no;
+      const uint32_t k = kk[u];
+      const double* t0 = own ? R.ti[0] : R.tj[0];
+      const double* t1 = own ? R.ti[1] : R.tj[1];
+      const double* t2 = own ? R.ti[2] : R.tj[2];
+      const V3 rf = mk(R.f[0][k], R.f[1][k], R.f[2][k]), rt = mk(t0[k], t1[k], t2[k]);
+      if (((emu_bits(rf.x) | emu_bits(rf.y) | emu_bits(rf.z) | emu_bits(rt.x) | emu_bits(rt.y) | emu_bits(rt.z))
+           << 1) != 0) {
+        const uint64_t flip = own ? 0ull : 0x8000000000000000ull;  // -rf for a partner record (exact)
+        f = f + mk(emu_double(emu_bits(rf.x) ^ flip), emu_double(emu_bits(rf.y) ^ flip),
+                   emu_double(emu_bits(rf.z) ^ flip));
+        mom = mom + rt;
+      }
     }
   }
   if (a.nb) {  // the inner bonds (k_bond_force): owned, then as j, in bond order
