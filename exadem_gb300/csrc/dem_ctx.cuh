@@ -211,7 +211,7 @@ struct dem_ctx {
   uint32_t* t_cnt = nullptr;          // tests per (segment, unit), segment-major (6 ucap + 1); then kept tests
   uint32_t t_ntests = 0;              // tests of the last flattened count pass
   uint32_t* t_off = nullptr;          // their offsets (6 ucap + 1)
-  uint32_t* t_keep = nullptr;         // kept bit per test (t_keepcap words)
+  uint32_t* t_keep = nullptr;         // kept bit per test (t_keepcap words), then a group per word
   uint64_t t_keepcap = 0;
   bool t_flat = false;                // the last count pass was the flattened one
   uint32_t* f_cnt = nullptr;          // features per unit (ucap+1)
