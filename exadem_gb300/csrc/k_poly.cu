@@ -1528,8 +1528,10 @@ __device__ __forceinline__ void split16(uint32_t h, int k0, int nA, uint64_t& ma
 // Gates and near features of the pair units, as bit masks: sixteen lanes a unit, which
 // the shapes of up to eight vertices and faces and twelve edges fill (a warp a unit left
 // 19 of its lanes idle and took twice the instructions); the masks come from ballots.
-// Bound by instruction issue and the latency of the gathered vertices.
-__global__ void __launch_bounds__(PT, 4) k_feat_prep(FeatArgs a, UnitRec* __restrict__ rec, uint32_t* __restrict__ tcnt) {
+// Bound by instruction issue and the latency of the gathered vertices, which eight blocks
+// an SM hide better than four with their registers unspilled (dense 27 k: a warp a unit
+// 183 us, this with four blocks 118, with eight 99, ten 116; 8 k bonded cubes 109, 64, 53, 65).
+__global__ void __launch_bounds__(PT, 8) k_feat_prep(FeatArgs a, UnitRec* __restrict__ rec, uint32_t* __restrict__ tcnt) {
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 15;
   const int half = threadIdx.x & 16;
