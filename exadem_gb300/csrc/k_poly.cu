@@ -11,12 +11,12 @@
 //           spheres are within the skin (the chunk_neighbors filter), one unit per
 //           driver that can reach A; sorted by (partner id, kind);
 //   SAT     one thread per unit: OBB(A), OBB(B) enlarged by skin/2, separating axis test;
-//   features  one warp per surviving unit: per-vertex OBB gates (one lane per
-//           vertex), then every gated feature test enumerated in InteractionPair
-//           order -- VV, VE, VE(swap), VF, VF(swap), EE -- so the ballot-compacted
-//           output of the fill pass is already sorted; history by full key.
-// Contact: dense detection pass over all feature interactions (types 0-3 and
-// vertex-driver 4/5), overlapping ones appended to a list for the Hooke pass.
+//   features  per-vertex OBB gates and near features as bit masks (half a warp a
+//           unit), then every gated feature test enumerated in InteractionPair
+//           order -- VV, VE, VE(swap), VF, VF(swap), EE -- a thread per test, so the
+//           kept ones are already sorted; history by full key.
+// Contact: an FP32 screen over all feature interactions sorts those that may touch by
+// kind; detection and law run over the lists, a warp one kind.
 // Force records are in the owner frame (for swap = 1 the contact law's particle
 // i is the partner), so the per-particle gather is the one of the sphere path.
 #include <algorithm>

@@ -468,7 +468,7 @@ __device__ inline int decide_ee(F3 vfi, F3 vsi, F3 vfj, F3 vsj, float R, float S
   return cn < 0 ? DEC_TRUE : (cn > 0 ? DEC_FALSE : DEC_UNDECIDED);
 }
 
-// ---- contact screen of the polyhedron contact law (k_pdetect)
+// ---- contact screen of the polyhedron contact law (k_pscreen)
 // Inputs are FP32 roundings of the FP64 world vertices (error u |x| per
 // coordinate).  With W a bound of every |coordinate| involved, a difference of
 // two inputs carries at most 3 u W per coordinate, so its norm at most
