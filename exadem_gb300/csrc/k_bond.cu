@@ -89,6 +89,8 @@ __device__ __forceinline__ void bond_law(double dn, V3 n, double dn0, double wei
   Et = emu_mulhalf(kt_w) * dot(tds, tds);
 }
 
+// Bound by the FP64 pipe (83 % busy).  16 k cubes, 154 k bonds: 52 us with the damping's
+// division and square root and the two energies' conversion here, 45 without.
 __global__ void __launch_bounds__(BT) k_bond_force(BondArgs a) {
   if (a.step && *a.flag != 0ull && *a.flag <= a.step) return;
   const uint64_t b = (uint64_t)blockIdx.x * BT + threadIdx.x;
@@ -178,6 +180,8 @@ struct CritArgs {
   unsigned step;               // in a batch: nothing once an earlier step raised the flag
 };
 
+// One thread per interface; only the stress mode reads the normal forces and takes their
+// norms (16 k cubes: 9 us with them, 4.5 without).
 __global__ void __launch_bounds__(BT) k_bond_criterion(CritArgs a) {
   // (a block may see the flag that another block of this step raises: the step's number)
   if (a.step) {
