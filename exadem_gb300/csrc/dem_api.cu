@@ -93,8 +93,6 @@ int alloc_particles(dem_ctx* c, uint64_t n) {
   DEM_CUDA_TRY(c, cudaMalloc(&c->own_off[1], (cap + 1) * 4));
   cudaFree(c->crel);
   DEM_CUDA_TRY(c, cudaMalloc(&c->crel, cap * sizeof(float4)));
-  cudaFree(c->rot_list);
-  DEM_CUDA_TRY(c, cudaMalloc(&c->rot_list, cap * 4));
   c->pcap = cap;
   return DEM_OK;
 }
@@ -565,7 +563,7 @@ int poly_steps(dem_ctx* c, int nsteps) {
   }
   int rc;
   const unsigned n = (unsigned)nsteps;
-  DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars, 0, (SC_ROT_CNT + 1) * sizeof(unsigned long long), c->stream));
+  DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars, 0, SC_STEP * sizeof(unsigned long long), c->stream));
   if ((rc = launch_poly_integrate(c, 0, 1, 0))) return rc;  // the first step's prolog; zeroes the list counts
   unsigned s = 1;  // the first step that is not finished; its prolog is done
   while (s <= n) {
@@ -740,7 +738,6 @@ int dem_ctx_destroy(dem_ctx* c) {
   cudaFree(c->srec);
   cudaFree(c->pcnt);
   cudaFree(c->crel);
-  cudaFree(c->rot_list);
   cudaFree(c->scan_blk);
   cudaFree(c->d_scalars);
   cudaFree(c->d_red);

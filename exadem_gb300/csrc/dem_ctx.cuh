@@ -24,7 +24,7 @@ struct MlpState;  // k_mlp.cu
 // [3..4] compaction list counts, [8] learned-record overflows, [12] interfaces broken,
 // [16..23] learned bin counters and cursors (14 u32), [24..28] work list counts of the polyhedron contact pass
 constexpr int DEM_NSCALARS = 32;
-constexpr int SC_ROT_CNT = 6, SC_RADMAX = 7, SC_LEARNED_OVF = 8, SC_BROKEN = 12, SC_LEARNED_BINS = 16, SC_PLIST = 24;
+constexpr int SC_STEP = 6 /* scalars of a step: before it */, SC_RADMAX = 7, SC_LEARNED_OVF = 8, SC_BROKEN = 12, SC_LEARNED_BINS = 16, SC_PLIST = 24;
 constexpr int PLISTS = 5;  // work lists of the polyhedron contact pass
 
 // features recorded per polyhedron unit by the count pass of the FP32-decided
@@ -138,7 +138,6 @@ struct dem_ctx {
   // compacted contact passes (rcap each): work lists and detection results
   uint32_t* L1 = nullptr;
   uint32_t* L2 = nullptr;
-  uint32_t* rot_list = nullptr;  // pcap: particles whose rotations run in k_rotations
   bool damp_stale = false;       // contact parameters changed since the list's per-pair damping was set
   // analysis (dem_set_analysis): per-interaction contact state, rcap entries
   bool analysis = false;

@@ -11,7 +11,7 @@
 //   compacted contact law (screen, detection and law)
 // so a step needs no host synchronisation: dem_step replays the graph nsteps
 // times and reads the device counters once at the end.  A step without a rebuild
-// is three kernels (four with a rotation list) and the conditional node, where it
+// is three kernels and the conditional node, where it
 // was seven kernels and five memsets: 23 of the 66 us of a 1 k box's step were the
 // gaps between them.
 //
@@ -81,7 +81,7 @@ __global__ void k_graph_begin(unsigned long long* gs, unsigned long long ni, uns
                               unsigned long long* scal) {
   const int t = threadIdx.x;
   if (t < GS_COUNT) gs[t] = t == GS_NI ? ni : (t == GS_CAP ? cap : 0ull);
-  if (t <= SC_ROT_CNT) scal[t] = 0ull;
+  if (t < SC_STEP) scal[t] = 0ull;
 }
 
 size_t particle_block_bytes(const dem_ctx* c) {

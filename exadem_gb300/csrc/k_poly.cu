@@ -239,12 +239,17 @@ __device__ __forceinline__ bool halted(const unsigned long long* flag, unsigned 
 
 // The polyhedron step's integration: the epilog of step g.step, then the prolog and the
 // trigger of the next (k_integrate's form).  A particle whose epilog rotation is put
-// off has its prolog put off too (k_poly_rotations).  Bound by the FP64 pipe (200 k falling
-// polyhedra 26 us a step), by one particle's FP64 chain below a warp a scheduler (1.5 k: 17).
+// off has its prolog put off too.  Bound by the FP64 pipe (200 k falling
+// polyhedra 26 us a step; 100 steps with a kernel of listed rotations besides 5.98 ms, 5.51 without), by one particle's FP64 chain below a warp a scheduler (1.5 k: 17).
 template <int Mode>
 __global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_poly_integrate(PolyArgs a, IntegArgs g, float thr) {
   if (g.step && halted(g.scal, g.step)) return;
   const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ PutOff off;
+  if (g.dense && g.epilog) {
+    if (threadIdx.x == 0) off.n = 0u;
+    __syncthreads();
+  }
   bool late = false, over = false;
   if (g.epilog) {
     bool need = false;
@@ -259,27 +264,17 @@ __global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_poly_integrate(PolyArgs
     if (need && !late) epilog_rotation<Mode>(a.P, s, g.hdt, mom);
   }
   if (g.prolog && s < a.n && !late) over = poly_prolog<Mode>(a, g, thr, s);
+  if (g.dense && g.epilog) {
+    put_off(off, late, (uint32_t)s);
+    __syncthreads();
+    if (threadIdx.x < off.n) {
+      const uint32_t w = off.s[threadIdx.x];
+      epilog_rotation<Mode>(a.P, w, g.hdt, mk(a.P.f[MX][w], a.P.f[MY][w], a.P.f[MZ][w]));
+      if (g.prolog) over |= poly_prolog<Mode>(a, g, thr, w);
+    }
+  }
   if (__any_sync(0xffffffffu, over) && (threadIdx.x & 31) == 0) atomicExch(g.scal, (unsigned long long)g.step + 1ull);
-  if (g.dense) {
-    const uint32_t pos = warp_append(late, g.scal + SC_ROT_CNT);
-    if (late) g.list[pos] = (uint32_t)s;
-  }
   if (blockIdx.x == 0 && threadIdx.x < PLISTS) g.scal[SC_PLIST + threadIdx.x] = 0ull;  // for the next contact pass
-}
-
-// halted before this step's integration (its prolog part may have raised the flag since)
-template <int Mode>
-__global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_poly_rotations(PolyArgs a, IntegArgs g, float thr) {
-  if (g.step && halted(g.scal, g.step)) return;
-  const uint64_t cnt = g.scal[SC_ROT_CNT];
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  bool over = false;
-  for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < cnt; w += stride) {
-    const uint32_t s = g.list[w];
-    epilog_rotation<Mode>(a.P, s, g.hdt, mk(a.P.f[MX][s], a.P.f[MY][s], a.P.f[MZ][s]));
-    if (g.prolog) over |= poly_prolog<Mode>(a, g, thr, s);
-  }
-  if (over) atomicExch(g.scal, (unsigned long long)g.step + 1ull);
 }
 
 // vertices of the listed particles (those in the interaction list), FP64
@@ -2102,10 +2097,7 @@ __device__ __forceinline__ VView pview(const PCArgs& a, uint32_t s) {
 __global__ void k_pscreen(PCArgs a) {
   if (a.step && halted(a.scal, a.step)) return;
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k == 0) {
-    *a.n_active = 0ull;
-    if (a.step) a.scal[SC_ROT_CNT] = 0ull;  // the rotations of the step before are done
-  }
+  if (k == 0) *a.n_active = 0ull;
   int kind = -1;
   if (k < a.ni) {
     const uint32_t type = meta_type(a.I.meta[k]);
@@ -2388,14 +2380,10 @@ int launch_poly_integrate(dem_ctx* c, int epilog, int prolog, unsigned step) {
   bond_integ_args(c, g);
   const float thr = (float)(c->prm.rcut_inc * 0.5);
   const unsigned block = spread_block(c, c->n, PT);
-  ProfScope ps(c, epilog ? K_EPILOG : K_PROLOG, g.dense && epilog ? 2 : 1);
+  ProfScope ps(c, epilog ? K_EPILOG : K_PROLOG, 1);
   const int mode = integ_mode(c);
   const auto kern = by_mode(mode, k_poly_integrate<0>, k_poly_integrate<1>, k_poly_integrate<2>, k_poly_integrate<3>);
   kern<<<grid_for(c->n, block), block, 0, c->stream>>>(a, g, thr);
-  if (g.dense && epilog) {
-    const auto krot = by_mode(mode, k_poly_rotations<0>, k_poly_rotations<1>, k_poly_rotations<2>, k_poly_rotations<3>);
-    krot<<<(unsigned)c->num_sms * 3, 256, 0, c->stream>>>(a, g, thr);
-  }
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;
 }

@@ -55,7 +55,6 @@ struct CArgs {
   int int_share;            // k_cfused: Hooke tiles out of 8 run with AllInt (the integer pipe)
   unsigned long long* n_active;
   int overlap_only;             // a pair counts as active at dn < 0 only
-  unsigned long long* rot_cnt;  // graph step: the rotation list, run before this pass, is emptied by the screen
 };
 
 // L1 as one list: the particle pairs (front, n1 of them), then the driver pairs
@@ -98,7 +97,6 @@ __device__ __forceinline__ V3 partner_pos(const CArgs& a, uint32_t meta, uint32_
 
 __global__ void __launch_bounds__(128) k_cscreen(CArgs a) {
   const uint64_t ni = a.ni_dev ? *a.ni_dev : a.ni;
-  if (a.rot_cnt && blockIdx.x == 0 && threadIdx.x == 0) *a.rot_cnt = 0ull;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < ni; base += stride) {
   const uint64_t k = base + threadIdx.x;
@@ -487,8 +485,10 @@ __device__ __forceinline__ bool displ_over(V3 r, V3 b, double thr2, float thr2f)
 //
 // The rotational halves are exactly idle or integer logic for many particles
 // (rotation_idle, spin_free_step); the others run them here when more than `dense`
-// lanes of their warp need it, otherwise they are appended to a list for
-// k_rotations, so sparse rotating particles do not hold whole warps on the FP64 pipe.
+// lanes of their warp need it, otherwise the block puts them off and runs them packed
+// at its end, so sparse rotating particles do not hold whole warps on the FP64 pipe (a
+// list for a kernel of its own packs a little better, and cost 6 us a step when empty:
+// 50 k mixer, 20 steps, 3.55 -> 3.31 ms, 125 k bed 5.45 -> 5.28 ms, 2 M bed 15.4 both).
 // The trigger depends on positions only.
 //
 // In the graph the last block to finish does what four memsets and a kernel of one
@@ -504,7 +504,12 @@ __global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_integrate(IntegArgs a) 
   const bool pro = a.prolog != 0;
   const bool mine = s < a.n;
   V3 v = mk(0.0, 0.0, 0.0), acc = v;
-  bool late = false;  // the epilog's rotation is due in k_rotations
+  __shared__ PutOff off;
+  if (a.dense) {
+    if (threadIdx.x == 0) off.n = 0u;
+    __syncthreads();
+  }
+  bool late = false;  // the epilog's rotation is put off
   if (epi) {
     bool need = false;
     V3 mom = mk(0.0, 0.0, 0.0);
@@ -551,8 +556,13 @@ __global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_integrate(IntegArgs a) 
     turn = false;
   }
   if (a.dense) {
-    const uint32_t pos = warp_append(late || turn, a.scal + SC_ROT_CNT);
-    if (late || turn) a.list[pos] = (uint32_t)s | (late ? ROT_EPILOG : 0u);
+    put_off(off, late || turn, (uint32_t)s | (late ? ROT_EPILOG : 0u));
+    __syncthreads();
+    if (threadIdx.x < off.n) {
+      const uint32_t e = off.s[threadIdx.x], w = e & ~ROT_EPILOG;
+      if (e & ROT_EPILOG) epilog_rotation<Mode>(P, w, a.hdt, mk(P.f[MX][w], P.f[MY][w], P.f[MZ][w]));
+      if (pro && !prolog_spin_free<Mode>(P, w, a.dt, a.hdt)) prolog_rotation<Mode>(P, w, a.dt, a.hdt);
+    }
   }
   if (a.gs) {
     __syncthreads();
@@ -566,18 +576,6 @@ __global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_integrate(IntegArgs a) 
         a.gs[GS_STEP] += 1ull;
       }
     }
-  }
-}
-
-// the rotations listed by k_integrate: the epilog's where it is due, and the prolog's
-template <int Mode>
-__global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_rotations(IntegArgs a) {
-  const uint64_t cnt = a.scal[SC_ROT_CNT];
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < cnt; w += stride) {
-    const uint32_t e = a.list[w], s = e & ~ROT_EPILOG;
-    if (e & ROT_EPILOG) epilog_rotation<Mode>(a.P, s, a.hdt, mk(a.P.f[MX][s], a.P.f[MY][s], a.P.f[MZ][s]));
-    if (a.prolog && !prolog_spin_free<Mode>(a.P, s, a.dt, a.hdt)) prolog_rotation<Mode>(a.P, s, a.dt, a.hdt);
   }
 }
 
@@ -607,7 +605,6 @@ CArgs make_cargs(dem_ctx* c) {
   a.l1cap = c->rcap;
   a.int_share = c->tune_int_share;
   a.n_active = c->d_scalars + 1;
-  a.rot_cnt = c->capturing ? c->d_scalars + SC_ROT_CNT : nullptr;
   return a;
 }
 }  // namespace
@@ -630,7 +627,6 @@ IntegArgs make_integ_args(dem_ctx* c, int epilog, int prolog) {
   a.thr2 = max_displ * max_displ;
   a.thr2f = (float)a.thr2;
   a.sv = c->sysview();
-  a.list = c->rot_list;
   a.scal = c->d_scalars;
   a.dense = rotation_dense(c);
   a.epilog = epilog;
@@ -649,17 +645,11 @@ static int launch_integrate(dem_ctx* c, int epilog, int prolog, cudaGraphConditi
   a.gs = c->capturing ? c->d_gs : nullptr;
   a.cond = cond;
   const unsigned block = particle_block(c);
-  ProfScope ps(c, epilog ? K_EPILOG : K_PROLOG, c->n ? (a.dense ? 2 : 1) : 0);
-  if (!c->capturing && a.dense)
-    DEM_CUDA_TRY(c, cudaMemsetAsync(c->d_scalars + SC_ROT_CNT, 0, sizeof(unsigned long long), c->stream));
+  ProfScope ps(c, epilog ? K_EPILOG : K_PROLOG, c->n ? 1 : 0);
   if (c->n) {
     const int mode = integ_mode(c);
     const auto kern = by_mode(mode, k_integrate<0>, k_integrate<1>, k_integrate<2>, k_integrate<3>);
     kern<<<grid_for(c->n, block), block, 0, c->stream>>>(a);
-    if (a.dense) {
-      const auto krot = by_mode(mode, k_rotations<0>, k_rotations<1>, k_rotations<2>, k_rotations<3>);
-      krot<<<(unsigned)c->num_sms * 3, 256, 0, c->stream>>>(a);
-    }
   }
   DEM_CUDA_TRY(c, cudaGetLastError());
   return DEM_OK;

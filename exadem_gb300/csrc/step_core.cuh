@@ -20,8 +20,7 @@ struct IntegArgs {
   double thr2;
   float thr2f;
   SysView sv;
-  uint32_t* list;             // particles whose rotations run in k_rotations
-  unsigned long long* scal;   // device scalars (flag, active contacts, work list and rotation list counts)
+  unsigned long long* scal;   // device scalars (flag, active contacts and work list counts)
   int dense;
   int epilog, prolog;
   unsigned long long* gs;     // graph step: its counters; epilog is then "not the call's first step"
@@ -34,7 +33,24 @@ struct IntegArgs {
   const double *bf[3], *bti[3], *btj[3];
   const uint32_t *b_own_first, *b_own_cnt, *b_rev_off, *b_rev_idx;
 };
-constexpr uint32_t ROT_EPILOG = 0x80000000u;  // list entry whose epilog rotation is due too
+constexpr uint32_t ROT_EPILOG = 0x80000000u;  // put-off rotation whose epilog part is due too
+
+// The rotations that a block's warps put off (few lanes of a warp need one) and its first
+// warps then run together.
+struct PutOff {
+  uint32_t s[256], n;
+};
+
+// The warp's put-off rotations; all 32 lanes must call it.
+__device__ __forceinline__ void put_off(PutOff& q, bool want, uint32_t entry) {
+  const unsigned mask = __ballot_sync(0xffffffffu, want);
+  if (!mask) return;
+  const int lane = threadIdx.x & 31;
+  uint32_t base = 0;
+  if (lane == 0) base = atomicAdd(&q.n, (uint32_t)__popc(mask));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (want) q.s[base + (uint32_t)__popc(mask & ((1u << lane) - 1u))] = entry;
+}
 
 // All 32 lanes must call it.  Returns the slot of this lane when want is set.
 __device__ __forceinline__ uint32_t warp_append(bool want, unsigned long long* counter) {
@@ -164,10 +180,9 @@ __device__ __forceinline__ bool epilog_translate(const IntegArgs& a, uint64_t s,
 
 // Lanes of a warp above which the rotations run in place.  While the particles give
 // every scheduler at most one warp (32 lanes a scheduler, four schedulers an SM) the
-// FP64 pipes wait for that warp alone, so a list only adds a second pass over it:
-// every rotation in place and no list kernel (9 + 5 us of the 10 k box's 90 us
-// step).  With more warps a sparse one keeps its pipe from the next, and more than 24
-// lanes pay for the pass.
+// FP64 pipes wait for that warp alone, so every rotation runs in place.  With more warps a
+// sparse one keeps its pipe from the next, and up to 24 lanes it pays to put its rotations
+// off to the end of the block (PutOff).
 static int rotation_dense(const dem_ctx* c) { return c->n <= (uint64_t)c->num_sms * 128u ? 0 : 24; }
 // Threads per block of the prolog and the epilog: the tuned size, halved while the
 // grid leaves SMs without a block (at 10 k particles 256 threads reach 40 SMs).
