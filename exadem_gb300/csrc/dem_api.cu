@@ -520,9 +520,13 @@ int update_neighbors(dem_ctx* c) {
 
 // The contact law of the operators: with fused_step the compacted kernels of the fused
 // step (same bits; the FP64 law on dense warps: 53 k bed 95 -> 45 us), which a
-// context without it keeps to the plain kernel.
+// context without it keeps to the plain kernel.  They read the damping stored with
+// each pair, so it is brought up to date first where the contact parameters changed
+// since the list was built (the plain kernel computes it on every call).
 int sphere_contacts(dem_ctx* c) {
-  return c->prm.fused_step && c->n && c->ni ? launch_contact_compact(c, true) : launch_contact_sphere(c);
+  if (!c->prm.fused_step || !c->n || !c->ni) return launch_contact_sphere(c);
+  const int rc = refresh_pair_damp(c);
+  return rc ? rc : launch_contact_compact(c, true);
 }
 
 // gravity, contact laws, gather; then the inner bonds (config_fragmentation.msp compute_force)
