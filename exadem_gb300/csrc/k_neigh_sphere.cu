@@ -507,11 +507,10 @@ __global__ void __launch_bounds__(PAIR_BLOCK) k_count_pairs(BPArgs a, uint32_t* 
   };
   if (gl == 0) {
     const int2 dr = a.sv.drange[sys];
-    const float px = g.lof[0] + (float)cx * csx + me.x, py = g.lof[1] + (float)cy * csy + me.y,
-                pz = g.lof[2] + (float)cz * csz + me.z;
+    const PosF at = pos_f32(g, cx, cy, cz, me);
     for (int k = dr.x; k < dr.x + dr.y; k++) {
       const DriverDev& d = a.drv[k];
-      if (d.kind == 2 || driver_far(d, me.w + a.skin_f, px, py, pz)) continue;  // mesh drivers: mesh_phase
+      if (d.kind == 2 || driver_far(d, me.w + a.skin_f, at)) continue;  // mesh drivers: mesh_phase
       if (driver_filter(d, a.P.f[RAD][s] + a.skin, mk(a.P.f[RX][s], a.P.f[RY][s], a.P.f[RZ][s])))
         append((uint32_t)s, (uint32_t)k,
                make_meta(d.kind == 0 ? DEM_ITYPE_VERTEX_SURFACE : DEM_ITYPE_VERTEX_CYLINDER, 0, 0, 0, false),

@@ -582,11 +582,10 @@ __global__ void __launch_bounds__(UNIT_BLOCK) k_unit_pairs(UnitArgs a, uint32_t*
     const double reach = h * (sh.maxv + sh.r) + a.rV;
     const double rc = reach + 1e-9 * (1.0 + reach + fabs(ri.x) + fabs(ri.y) + fabs(ri.z));
     const float rcf = (float)rc;
-    const float px = a.g.lof[0] + (float)cx * a.g.csf[0] + me.x, py = a.g.lof[1] + (float)cy * a.g.csf[1] + me.y,
-                pz = a.g.lof[2] + (float)cz * a.g.csf[2] + me.z;
+    const PosF at = pos_f32(a.g, cx, cy, cz, me);
     for (int k = 0; k < a.ndrv; k++) {
       const DriverDev& d = a.drv[k];
-      if (d.kind != 2 && driver_far(d, rcf, px, py, pz)) continue;
+      if (d.kind != 2 && driver_far(d, rcf, at)) continue;
       if (bonded_to(a, (uint32_t)s, (uint64_t)k)) continue;
       if (d.kind == 2 ? mesh_meets(a.mesh[d.mesh], ri, rc) : driver_reach(d, rc, ri))
         append((uint32_t)s, 0x80000000u | (uint32_t)k);
