@@ -1481,13 +1481,15 @@ __global__ void k_unit_sat(FeatArgs a, uint8_t* __restrict__ pass, UnitRec* __re
     q.rb = (float)rb;
     // the stored FP32 boxes are enlarged by the skin, the test's by half of it
     OBBf fA = load_obbf(a.fbox + (uint64_t)A * FBOX_STRIDE, f3(0.f, 0.f, 0.f));
-    OBBf fB = load_obbf(a.fbox + (uint64_t)B * FBOX_STRIDE, dR);
+    OBBf fB = load_obbf(a.fbox + (uint64_t)B * FBOX_STRIDE, f3(0.f, 0.f, 0.f));
+    const float off = flen(fA.c) + flen(fB.c);
+    fB.c = fB.c + dR;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       fA.ext[k] -= 0.5f * a.rVf;
       fB.ext[k] -= 0.5f * a.rVf;
     }
-    d = decide_obb(fA, fB, a.rVf);
+    d = decide_obb(fA, fB, a.rVf, off);
   }
   if (d == DEC_UNDECIDED) {
     OBBd oA = load_obb(a.obb + (uint64_t)A * 15);

@@ -253,16 +253,19 @@ __device__ __forceinline__ int decide_gate(const OBBf& o, F3 p, float rv, float 
 }
 
 // OBB::intersect of two particles' boxes (both relative to the first one's centre).  The
-// FP64 test returns false at the first of 15 axes with |t_L| > ra_L + rb_L.  With T =
-// |t| + both boxes' extents (+ the skin, whose half was taken off the stored extents):
-// centres, extents and axes are FP32 roundings, so t_k and the entries R carry at most
+// FP64 test returns false at the first of 15 axes with |t_L| > ra_L + rb_L.  off bounds the
+// distances of the two boxes' centres from their own particles' positions, |cA| + |cB|.
+// With T = |t| + both boxes' extents (+ the skin, whose half was taken off the stored
+// extents) + off: centres, their shift by the distance of the positions (at most |t| + off),
+// extents and axes are FP32 roundings, so t_k and the entries R carry at most
 // 16 u T and 8 u, every projection and radius sum, of at most six products of magnitude
 // T with factors up to 1 + tol, at most 100 u T < 2^-17 T.  The axes must be unit
 // vectors to 1/16; other boxes are left undecided.
-__device__ __forceinline__ int decide_obb(const OBBf& A, const OBBf& B, float rV) {
+__device__ __forceinline__ int decide_obb(const OBBf& A, const OBBf& B, float rV, float off) {
   const float tol = 1.1920929e-07f;
   const F3 tt = A.c - B.c;
-  const float T = flen(tt) + A.ext[0] + A.ext[1] + A.ext[2] + B.ext[0] + B.ext[1] + B.ext[2] + 2.f * rV;
+  const float T =
+      flen(tt) + A.ext[0] + A.ext[1] + A.ext[2] + B.ext[0] + B.ext[1] + B.ext[2] + 2.f * rV + off;
   const float e = 7.6293945e-06f * T;  // 2^-17 T
   float R[3][3], Ab[3][3];
   bool unit = true;
