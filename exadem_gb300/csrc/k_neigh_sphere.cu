@@ -239,6 +239,34 @@ __device__ inline bool key_less(uint64_t pa, uint32_t ta, uint32_t sa, uint64_t 
   return pa < pb || (pa == pb && (ta < tb || (ta == tb && sa < sb)));
 }
 
+// Entry (qa, ma) before (qb, mb) among entries of one owner with equal keys: particles that
+// share an id.  They follow the stencil, as for_each_particle meets them: by the cell of
+// the image in z, y and x, then by slot.  Distinct ids never come here.
+__device__ __noinline__ bool image_before(const BPArgs& a, int sys, uint32_t qa, uint32_t ma, uint32_t qb, uint32_t mb) {
+  const GridDev& g = a.sv.g[sys];
+  const uint32_t coff = a.sv.coff[sys];
+  int ca[3], cb[3];
+  cell_coords(g, a.cell_of[qa] - coff, ca[0], ca[1], ca[2]);
+  cell_coords(g, a.cell_of[qb] - coff, cb[0], cb[1], cb[2]);
+  for (int d = 2; d >= 0; d--) {
+    const int ia = ca[d] + meta_shift(ma, d) * g.dims[d], ib = cb[d] + meta_shift(mb, d) * g.dims[d];
+    if (ia != ib) return ia < ib;
+  }
+  return qa < qb;
+}
+// The order of entry a of an owner before its entry b.  first orders two entries that
+// nothing else tells apart, so that the ranks of an owner's entries are always a
+// permutation of their places: two entries on one place leave another one unwritten.
+__device__ __forceinline__ bool entry_before(const BPArgs& a, int sys, uint64_t pa, uint32_t ma, uint32_t sa, uint32_t qa,
+                                             uint64_t pb, uint32_t mb, uint32_t sb, uint32_t qb, bool first) {
+  if (pa != pb) return pa < pb;
+  const uint32_t ta = meta_type(ma), tb = meta_type(mb);
+  if (ta != tb) return ta < tb;
+  if (sa != sb) return sa < sb;
+  if (ta != DEM_ITYPE_VERTEX_VERTEX || (qa == qb && ma == mb)) return first;
+  return image_before(a, sys, qa, ma, qb, mb);
+}
+
 constexpr uint32_t SREC = 16;
 
 // Mesh candidates (detection_sphere_driver, nbh_sphere.hpp:25-86): every mesh
@@ -399,15 +427,18 @@ __global__ void __launch_bounds__(MESH_BLOCK) k_mesh_fill(BPArgs a, const uint32
   __syncthreads();
   for (int L = 0; L < MESH_SPHERES; L++) {
     const uint32_t n = w.cnt[L], first = w.q0[L];
+    const int sys = n ? a.sv.of(w.s[L]) : 0;
     for (uint32_t x = threadIdx.x; x < n; x += MESH_BLOCK) {
       const uint64_t word = emu_bits(dst.ft[0][first + x]), pid = emu_bits(dst.ft[1][first + x]);
       const uint32_t meta = (uint32_t)emu_bits(dst.ft[2][first + x]), sub = (uint32_t)(word >> 32);
       uint32_t rank = 0;
-      for (uint32_t y = first; y < first + n; y++)
-        rank += key_less(emu_bits(dst.ft[1][y]), meta_type((uint32_t)emu_bits(dst.ft[2][y])),
-                         (uint32_t)(emu_bits(dst.ft[0][y]) >> 32), pid, meta_type(meta), sub)
+      for (uint32_t y = 0; y < n; y++) {
+        const uint64_t wy = emu_bits(dst.ft[0][first + y]);
+        rank += entry_before(a, sys, emu_bits(dst.ft[1][first + y]), (uint32_t)emu_bits(dst.ft[2][first + y]),
+                             (uint32_t)(wy >> 32), (uint32_t)wy, pid, meta, sub, (uint32_t)word, y < x)
                     ? 1u
                     : 0u;
+      }
       const uint32_t x1 = first + rank;
       dst.partner[x1] = (uint32_t)word;
       dst.pid[x1] = pid;
@@ -741,7 +772,8 @@ __global__ void __launch_bounds__(128) k_fill_entries(BPArgs a, const uint32_t* 
   for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += stride) {
     const uint32_t s = dst.owner[k];
     const uint32_t b = off[s], m = off[s + 1] - b, x = (uint32_t)k - b;
-    if (!a.sv.triggered(a.sv.of(s))) {  // slot kept, partners of the same system kept: copy
+    const int sys = a.sv.of(s);
+    if (!a.sv.triggered(sys)) {  // slot kept, partners of the same system kept: copy
       const uint32_t y = old_off[s] + x;
       copy_entry(dst, (uint32_t)k, old, y, s);
       partner_list(k, old.partner[y], old.meta[y]);
@@ -788,14 +820,14 @@ __global__ void __launch_bounds__(128) k_fill_entries(BPArgs a, const uint32_t* 
       rank = 0;
       for (uint32_t y = 0; y < m; y++) {
         const uint4 u = at(y);
-        rank += key_less(pid_of(u, y), meta_type(u.y), y < mm ? u.z : 0u, pid, type, sub) ? 1u : 0u;
+        rank += entry_before(a, sys, pid_of(u, y), u.y, y < mm ? u.z : 0u, u.x, pid, meta, sub, partner, y < x) ? 1u : 0u;
       }
     }
     uint32_t hit = ~0u;
     if (have_old) {
       const uint32_t os = perm[s];
-      const uint32_t oe = old_off[os + 1];
-      for (uint32_t y = old_off[os]; y < oe; y++)
+      const uint32_t ob = old_off[os];
+      for (uint32_t y = old_off[os + 1]; y-- > ob;)  // backwards: the first of equal keys
         if (old.pid[y] == pid && meta_type(old.meta[y]) == type && old.sub[y] == sub) hit = y;
     }
     double h[6] = {0, 0, 0, 0, 0, 0};

@@ -678,7 +678,9 @@ __global__ void k_unit_entries(UnitArgs a, uint64_t nu, const uint32_t* __restri
   for (uint32_t y = 0; y < m; y++) {
     const uint32_t q = rec[y];
     const uint64_t pq = pid_of(q);
-    rank += (pq < pid || (pq == pid && (q >> 31) < kind)) ? 1u : 0u;
+    // a record orders by kind, then by slot: partners that share an id keep the order of
+    // their cells, as for_each_unit meets them, and every rank is another one
+    rank += (pq < pid || (pq == pid && q < r)) ? 1u : 0u;
   }
   u_partner[b + rank] = r & 0x7fffffffu;
   u_pid[b + rank] = pid;
