@@ -808,13 +808,14 @@ int dem_set_particles(dem_ctx* c, const dem_particles* p, int on_device) {
                             p->vrotz, p->arotx, p->aroty, p->arotz, p->momx, p->momy, p->momz, p->qw, p->qx,
                             p->qy, p->qz, p->inertiax, p->inertiay, p->inertiaz, p->mass, p->radius, p->homothety,
                             nullptr, nullptr, nullptr, nullptr, p->rx, p->ry, p->rz};
-  // Arrays on the context's device go through one launch, others (host arrays, another
-  // device's, managed memory) through copies of their own.  Defaults for absent fields:
+  // Arrays inside an allocation of the context's device go through one launch, others
+  // (host arrays, another device's, managed memory, arrays too short) through copies of
+  // their own, which refuse what they cannot copy.  Defaults for absent fields:
   // 0, except orientation w, inertia, mass and homothety = 1.
   CopyTab tab;
   auto take = [&](void* dst, const void* from, size_t bytes) -> int {
     if (!n) return DEM_OK;
-    if (on_device && device_memory(c, from)) {
+    if (on_device && device_memory(c->device, from, bytes)) {
       tab.add(dst, from, bytes);
     } else {
       DEM_CUDA_TRY(c, cudaMemcpyAsync(dst, from, bytes, k, c->stream));
@@ -922,7 +923,7 @@ int dem_get_particles(dem_ctx* c, dem_particles* out, int on_device) {
   CopyTab tab;  // as in dem_set_particles: arrays on the context's device in one launch
   auto give = [&](void* to, const void* from, size_t bytes) -> int {
     if (!to || !n) return DEM_OK;
-    if (on_device && device_memory(c, to)) {
+    if (on_device && device_memory(c->device, to, bytes)) {
       tab.add(to, from, bytes);
     } else {
       DEM_CUDA_TRY(c, cudaMemcpyAsync(to, from, bytes, k, c->stream));

@@ -308,7 +308,7 @@ struct CopyTab {
 };
 int launch_copies(dem_ctx* c, const CopyTab& t);
 int launch_radius_max(dem_ctx* c, const double* radius, uint64_t n, double* out);  // max(0, radii); waits
-bool device_memory(const dem_ctx* c, const void* p);  // memory of the ctx's device
+bool device_memory(int device, const void* p, uint64_t bytes);  // inside one allocation of the device
 // k_scan.cu
 int scan_exclusive_u32(dem_ctx* c, const uint32_t* in, uint32_t* out, uint64_t n);
 // k_grid.cu

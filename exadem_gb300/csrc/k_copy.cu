@@ -5,8 +5,11 @@
 // 10,000 particles.  One launch takes a table of them, a row of blocks per entry;
 // large copies run at the memory's rate as before (four 16-byte loads in flight a
 // thread).
+#include <cuda.h>  // types of the driver's range query (no symbol of it is linked)
+
 #include <algorithm>
 
+#include "../../include/dem_selftest.h"
 #include "dem_ctx.cuh"
 
 namespace dem {
@@ -94,12 +97,39 @@ int launch_radius_max(dem_ctx* c, const double* radius, uint64_t n, double* out)
   return DEM_OK;
 }
 
-bool device_memory(const dem_ctx* c, const void* p) {
+// A copy of more bytes than the allocation holds is an error of cudaMemcpyAsync, which
+// looks the range up; a kernel would run past it.  So only what is known to lie inside
+// one allocation of the device goes through k_copies.
+bool device_memory(int device, const void* p, uint64_t bytes) {
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return at.type == cudaMemoryTypeDevice && at.device == c->device;
+  if (at.type != cudaMemoryTypeDevice || at.device != device) return false;
+  using Range = CUresult(CUDAAPI*)(CUdeviceptr*, size_t*, CUdeviceptr);
+  static const Range range = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return reinterpret_cast<Range>(fn);
+  }();
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  const CUdeviceptr first = reinterpret_cast<CUdeviceptr>(p);
+  if (!range || range(&base, &size, first) != CUDA_SUCCESS) return false;
+  return first >= base && bytes <= size && first - base <= size - bytes;
 }
 }  // namespace dem
+
+extern "C" int dem_selftest_copy_range(const void* p, uint64_t bytes, int* inside) {
+  if (!p || !inside) return DEM_ERR_INVALID_ARG;
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return DEM_ERR_CUDA;
+  *inside = dem::device_memory(device, p, bytes) ? 1 : 0;
+  return DEM_OK;
+}

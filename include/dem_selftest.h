@@ -38,6 +38,11 @@ int dem_selftest_emu_mul(uint64_t n, uint64_t seed, uint64_t* mismatches);
  * fast_path_taken counts the cases inside the shortcut's range.            */
 int dem_selftest_rolling_clip(uint64_t n, uint64_t seed, uint64_t* mismatches, uint64_t* fast_path_taken);
 
+/* Whether the bytes at p lie inside one allocation of the current device, so
+ * that dem_set_particles and dem_get_particles (on_device = 1) copy them with
+ * their own kernel; what does not goes through cudaMemcpyAsync.             */
+int dem_selftest_copy_range(const void* p, uint64_t bytes, int* inside);
+
 #ifdef __cplusplus
 }
 #endif
