@@ -822,6 +822,7 @@ int dem_set_particles(dem_ctx* c, const dem_particles* p, int on_device) {
     }
     return DEM_OK;
   };
+  static_assert(NPF + 3 <= CopyTab::MAX, "every field, id, type and group in one table");
   constexpr uint64_t one = 0x3ff0000000000000ull;  // 1.0
   for (int f = 0; f < NPF; f++) {
     if (f >= IMASS && f <= IIZ) continue;  // derived below
@@ -920,7 +921,7 @@ int dem_get_particles(dem_ctx* c, dem_particles* out, int on_device) {
                      out->vrotx, out->vroty, out->vrotz, out->arotx, out->aroty, out->arotz, out->momx,
                      out->momy, out->momz, out->qw, out->qx, out->qy, out->qz, out->inertiax, out->inertiay,
                      out->inertiaz, out->mass, out->radius, out->homothety};
-  CopyTab tab;  // as in dem_set_particles: arrays on the context's device in one launch
+  CopyTab tab;  // as in dem_set_particles (and its bound): arrays on the context's device in one launch
   auto give = [&](void* to, const void* from, size_t bytes) -> int {
     if (!to || !n) return DEM_OK;
     if (on_device && device_memory(c->device, to, bytes)) {

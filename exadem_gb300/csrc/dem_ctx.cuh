@@ -297,7 +297,7 @@ struct CopyTab {
   uint64_t bytes[MAX];
   uint64_t fill[MAX];
   int n = 0;
-  void add(void* d, const void* s, uint64_t b, uint64_t f = 0) {
+  void add(void* d, const void* s, uint64_t b, uint64_t f = 0) {  // the callers' counts are asserted
     if (!d || !b) return;
     src[n] = s;
     dst[n] = d;

@@ -256,6 +256,7 @@ int snapshot(dem_ctx* c, bool save) {
   }
   char* p = static_cast<char*>(c->snap);
   CopyTab tab;  // one launch: 15 copies took 35 us of a call, whatever its size
+  static_assert(14 <= CopyTab::MAX, "particles, offsets and the list's twelve arrays in one table");
   auto mv = [&](void* dev, size_t bytes) {
     if (save)
       tab.add(p, dev, bytes);
