@@ -76,7 +76,7 @@ int alloc_particles(dem_ctx* c, uint64_t n) {
   cudaFree(c->cell_tmp);
   cudaFree(c->perm);
   cudaFree(c->pcnt);
-  cudaFree(c->srec);
+  free_records_f32(c);
   cudaFree(c->rev_off);
   cudaFree(c->rev_cnt);
   cudaFree(c->own_off[0]);
@@ -85,8 +85,6 @@ int alloc_particles(dem_ctx* c, uint64_t n) {
   DEM_CUDA_TRY(c, cudaMalloc(&c->cell_tmp, cap * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->perm, cap * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->pcnt, (cap + 1) * 4));
-  c->srec_n = 16;
-  DEM_CUDA_TRY(c, cudaMalloc(&c->srec, cap * c->srec_n * sizeof(uint4)));
   DEM_CUDA_TRY(c, cudaMalloc(&c->rev_off, (cap + 1) * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->rev_cnt, (cap + 1) * 4));
   DEM_CUDA_TRY(c, cudaMalloc(&c->own_off[0], (cap + 1) * 4));
@@ -494,6 +492,7 @@ int update_neighbors(dem_ctx* c) {
   }
   int rc;
   if (!c->capturing && (rc = ensure_mesh_bins(c))) return rc;
+  if ((rc = ensure_records_f32(c))) return rc;
   if ((rc = launch_bin_particles(c))) return rc;
   if ((rc = launch_reorder_particles(c))) return rc;
   if ((rc = launch_count_sphere(c))) return rc;
@@ -739,7 +738,7 @@ int dem_ctx_destroy(dem_ctx* c) {
   cudaFree(c->cell_of);
   cudaFree(c->cell_tmp);
   cudaFree(c->perm);
-  cudaFree(c->srec);
+  free_records_f32(c);
   cudaFree(c->pcnt);
   cudaFree(c->crel);
   cudaFree(c->scan_blk);
@@ -1186,6 +1185,7 @@ int dem_step(dem_ctx* c, int nsteps) {
     return c->fail(DEM_ERR_STATE, "drivers were registered after dem_set_multimat: set the table again");
   if ((rc = refresh_pair_damp(c))) return rc;  // contact parameters changed since the list was built
   if ((rc = ensure_mesh_bins(c))) return rc;    // before a graph capture of the rebuild
+  if ((rc = ensure_records_f32(c))) return rc;
   // graph replay unless per-kernel timing is on (events cannot be recorded inside a graph)
   if (c->prm.graph_step && c->prm.fused_step && !c->poly && c->n && nsteps > 0 && !c->prof_on)
     return step_graph(c, nsteps);

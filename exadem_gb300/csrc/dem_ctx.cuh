@@ -118,8 +118,13 @@ struct dem_ctx {
   uint32_t* cell_tmp = nullptr;    // n, cell of each particle in the old order
   uint32_t* perm = nullptr;        // n, new slot -> old slot
   uint32_t* pcnt = nullptr;        // n+1 candidate counts (then offsets)
-  uint32_t* srec = nullptr;        // spheres: srec_n (partner, meta, partner id) candidates per particle from the count pass
-  uint32_t srec_n = 16;
+  // spheres, FP32 build: srec_n + srec_m (partner, meta, partner id) candidates per particle
+  // from the count pass, allocated by the first build (ensure_records_f32)
+  uint4* srec = nullptr;
+  uint32_t srec_n = 0, srec_m = 0;
+  uint64_t srec_cap = 0;     // particles they are for
+  bool srec_mesh = false;    // planned with a mesh
+  uint64_t srec_budget = 0;  // bytes they may take; 0: a sixteenth of the free memory
   float4* crel = nullptr;          // n: cell-relative x, y, z and radius in FP32 (broad phase)
 
   // interactions (double-buffered for the history carry-over)
@@ -320,6 +325,9 @@ int refresh_pair_damp(dem_ctx* c);  // k_neigh_sphere.cu
 int mark_records_live(dem_ctx* c);  // dem_api.cu
 int ext_ensure_contact_state(dem_ctx* c);  // dem_api.cu: analysis arrays of the records' capacity
 int launch_fill_sphere(dem_ctx* c, uint32_t* new_off, uint64_t total);
+int ensure_records_f32(dem_ctx* c);  // before a list build of spheres (not inside a capture)
+void free_records_f32(dem_ctx* c);
+int record_plan(uint64_t particles, bool mesh, uint64_t budget);
 int launch_reverse_lists(dem_ctx* c, bool counted = false);
 bool fill_counts_partners(const dem_ctx* c);
 // k_mesh.cu: bins of the mesh drivers for the current radius bound and skin

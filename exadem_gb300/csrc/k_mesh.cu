@@ -91,20 +91,6 @@ int ensure_mesh_bins(dem_ctx* c) {
     c->mesh_cnt_cap = cap;
     c->gen++;  // captured kernels hold the old buffer
   }
-  // A sphere where triangles meet has tens of mesh candidates: with a mesh a particle has
-  // 48 records for them, up to 16 GB in all or as the memory allows (without: k_mesh_fill).
-  if (!c->meshes.empty() && !c->poly && !c->capturing && c->srec_n < 64 && c->pcap <= (1ull << 24)) {
-    uint32_t* grown = nullptr;
-    if (cudaMalloc(&grown, c->pcap * 64 * sizeof(uint4)) == cudaSuccess) {
-      DEM_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-      cudaFree(c->srec);
-      c->srec = grown;
-      c->srec_n = 64;
-      c->gen++;
-    } else {
-      cudaGetLastError();
-    }
-  }
   if (!c->meshes.empty() && c->poly && c->prm.learned_sizing)
     return c->fail(DEM_ERR_UNSUPPORTED, "learned record sizing does not bound mesh units: learned_sizing = 0");
   bool changed = false;

@@ -22,6 +22,7 @@
 // drivers per particle (k_pre_count / k_pre_fill).  In a batched context the particle's system gives the grid, its cell block and
 // its drivers; a system rebuilt without its own trigger kept its slots, and
 // its previous list is copied as is (so its list is the one it has alone).
+#include "../../include/dem_selftest.h"
 #include "broad_core.cuh"
 #include "mesh_core.cuh"
 
@@ -45,11 +46,11 @@ struct BPArgs {
   const float4* crel;
   float skin_f;
   uint64_t cap;  // interaction buffer capacity (graph step): a fill beyond it writes nothing
-  // FP32 path: the count pass's candidates of each particle (SREC per particle,
+  // FP32 path: the count pass's candidates of each particle (nrec per particle,
   // then nmrec mesh candidates:
   // partner, meta, partner id), read by the fill when they fit
-  uint32_t* srec;
-  uint32_t nmrec;
+  uint4* srec;
+  uint32_t nrec, nmrec;
   uint32_t* rev_cnt;  // FP32 path: the fill's count of each particle's partner list
   uint32_t* rev_pos;  // and the place of each entry in it (a scratch of the records' capacity)
   // per-pair damping damp_rate 2 sqrt(kn meff), in the operation order of the
@@ -267,8 +268,6 @@ __device__ __forceinline__ bool entry_before(const BPArgs& a, int sys, uint64_t 
   return image_before(a, sys, qa, ma, qb, mb);
 }
 
-constexpr uint32_t SREC = 16;
-
 // Mesh candidates (detection_sphere_driver, nbh_sphere.hpp:25-86): every mesh
 // vertex, edge and face of the sphere's bin that passes its filter, partner
 // sub = the feature.  A block serves the spheres s of its first 32 threads (want), which
@@ -374,11 +373,11 @@ __global__ void __launch_bounds__(MESH_BLOCK) k_mesh_count(BPArgs a, uint32_t* _
   const uint64_t s = mesh_sphere();
   const bool own = threadIdx.x < MESH_SPHERES && s < a.n;
   const bool trig = own && a.sv.triggered(a.sv.of(s));
-  uint4* const rec = reinterpret_cast<uint4*>(a.srec);
+  uint4* const rec = a.srec;
   const uint32_t m =
       mesh_phase<F32>(a, s, trig, w, [&](uint32_t o, uint32_t at, uint32_t k, uint32_t kind, uint32_t j) {
         if (Rec && at < a.nmrec)
-          rec[(uint64_t)o * (SREC + a.nmrec) + SREC + at] =
+          rec[(uint64_t)o * (a.nrec + a.nmrec) + a.nrec + at] =
               make_uint4(k, make_meta(DEM_ITYPE_VERTEX_MESH_VERTEX + kind, 0, 0, 0, false), j << 16, 0u);
       });
   if (own) {
@@ -397,7 +396,7 @@ __global__ void __launch_bounds__(MESH_BLOCK) k_mesh_fill(BPArgs a, const uint32
   const bool own = threadIdx.x < MESH_SPHERES && s < a.n;
   const uint32_t b = own ? off[s] : 0u, e = own ? off[s + 1] : 0u, mm = own ? a.mcnt[s] : 0u;
   const bool want = own && e <= a.cap && a.sv.triggered(a.sv.of(s)) &&
-                    (Rec ? mm > a.nmrec || e - b - mm > SREC : mm > 0u);
+                    (Rec ? mm > a.nmrec || e - b - mm > a.nrec : mm > 0u);
   if (!__syncthreads_or(want)) return;
   auto put = [&](uint32_t x, uint32_t partner, uint64_t pid, uint32_t meta, uint32_t sub) {
     dst.ft[0][x] = emu_double((uint64_t)partner | (uint64_t)sub << 32);
@@ -410,8 +409,8 @@ __global__ void __launch_bounds__(MESH_BLOCK) k_mesh_fill(BPArgs a, const uint32
   });
   if (Rec && want) {
     uint32_t x = b + mm;
-    if (e - x <= SREC) {
-      const uint4* const rec = reinterpret_cast<const uint4*>(a.srec) + s * (SREC + a.nmrec);
+    if (e - x <= a.nrec) {
+      const uint4* const rec = a.srec + s * (a.nrec + a.nmrec);
       for (uint32_t y = 0; x < e; x++, y++) put(x, rec[y].x, (uint64_t)rec[y].z | (uint64_t)rec[y].w << 32, rec[y].y, 0u);
     } else {
       for_each_candidate<true>(a, (uint32_t)s, [&](uint32_t q, uint64_t pid, uint32_t meta, uint32_t sub) {
@@ -500,10 +499,10 @@ __global__ void __launch_bounds__(PAIR_BLOCK) k_count_pairs(BPArgs a, uint32_t* 
   const float4 me = a.crel[s];
   int cx, cy, cz;
   cell_coords(g, a.cell_of[s] - coff, cx, cy, cz);
-  uint4* const rec = reinterpret_cast<uint4*>(a.srec);
+  uint4* const rec = a.srec;
   auto store = [&](uint32_t o, uint32_t at, uint32_t q, uint32_t meta, uint64_t pid) {
     const uint32_t m = at - (a.has_mesh ? a.mcnt[o] : 0u);
-    if (m < SREC) rec[(uint64_t)o * (SREC + a.nmrec) + m] = make_uint4(q, meta, (uint32_t)pid, (uint32_t)(pid >> 32));
+    if (m < a.nrec) rec[(uint64_t)o * (a.nrec + a.nmrec) + m] = make_uint4(q, meta, (uint32_t)pid, (uint32_t)(pid >> 32));
   };
   auto append = [&](uint32_t o, uint32_t q, uint32_t meta, uint64_t pid) {
     store(o, atomicAdd(&cnt[o], 1u), q, meta, pid);
@@ -767,7 +766,7 @@ __global__ void __launch_bounds__(128) k_fill_entries(BPArgs a, const uint32_t* 
   auto partner_list = [&](uint64_t x, uint32_t q, uint32_t meta) {
     if (meta_type(meta) == DEM_ITYPE_VERTEX_VERTEX && !meta_owner_only(meta)) a.rev_pos[x] = atomicAdd(&a.rev_cnt[q], 1u);
   };
-  const uint4* const recs = reinterpret_cast<const uint4*>(a.srec);
+  const uint4* const recs = a.srec;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += stride) {
     const uint32_t s = dst.owner[k];
@@ -780,7 +779,7 @@ __global__ void __launch_bounds__(128) k_fill_entries(BPArgs a, const uint32_t* 
       continue;
     }
     const uint32_t mm = a.has_mesh ? a.mcnt[s] : 0u;
-    const bool over = mm > a.nmrec || m - mm > SREC;
+    const bool over = mm > a.nmrec || m - mm > a.nrec;
     if (over && !a.has_mesh) {
       if (x) continue;
       const uint32_t e = b + m;
@@ -807,8 +806,8 @@ __global__ void __launch_bounds__(128) k_fill_entries(BPArgs a, const uint32_t* 
       sub = dst.sub[k];
       type = meta_type(meta);
     } else {
-      const uint4* const rec = recs + (uint64_t)s * (SREC + a.nmrec);
-      auto at = [&](uint32_t y) { return rec[y < mm ? SREC + y : y - mm]; };
+      const uint4* const rec = recs + (uint64_t)s * (a.nrec + a.nmrec);
+      auto at = [&](uint32_t y) { return rec[y < mm ? a.nrec + y : y - mm]; };
       // a mesh item's partner id is its driver, its sub the feature (k_mesh_count)
       auto pid_of = [&](uint4 v, uint32_t y) { return y < mm ? (uint64_t)v.x : (uint64_t)v.z | (uint64_t)v.w << 32; };
       const uint4 v = at(x);
@@ -1212,7 +1211,8 @@ BPArgs make_args(dem_ctx* c) {
   a.skin_f = (float)c->prm.rcut_inc;
   a.cap = c->capturing ? c->gcap : ~0ull;
   a.srec = c->srec;
-  a.nmrec = c->srec_n - SREC;
+  a.nrec = c->srec_n;
+  a.nmrec = c->srec_m;
   a.rev_cnt = c->rev_cnt;
   a.rev_pos = c->L2;
   a.cp = c->prm.config;
@@ -1237,6 +1237,55 @@ int refresh_pair_damp(dem_ctx* c) {
 static unsigned cell_grid(const dem_ctx* c) {
   const uint64_t want = (c->ncell + CELL_WARPS - 1) / CELL_WARPS;
   return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)c->num_sms * 16));
+}
+
+// Records of a particle in the FP32 build: 16 hold the candidates of nearly every sphere
+// (more are enumerated again, and sorted one by one), and a sphere where triangles meet
+// has tens of mesh candidates.  They take 256 bytes a particle and 768 with a mesh, which
+// a run whose lists fill the memory may not have: a sixteenth of the free memory at most,
+// else four records, 64 bytes.
+constexpr uint32_t REC_PLANS[3][2] = {{16, 48}, {16, 0}, {4, 0}};
+int record_plan(uint64_t particles, bool mesh, uint64_t budget) {
+  int k = mesh ? 0 : 1;
+  while (k < 2 && particles * (REC_PLANS[k][0] + REC_PLANS[k][1]) * sizeof(uint4) > budget) k++;
+  return k;
+}
+
+void free_records_f32(dem_ctx* c) {
+  cudaFree(c->srec);
+  c->srec = nullptr;
+  c->srec_n = c->srec_m = 0;
+  c->srec_cap = 0;
+}
+
+// the records of the build that uses them, for the particles' capacity
+int ensure_records_f32(dem_ctx* c) {
+  if (c->poly || !c->prm.fp32_broad_phase || c->cell_broad_phase || !c->n) return DEM_OK;
+  const bool mesh = !c->meshes.empty();
+  if (c->srec && c->srec_cap == c->pcap && c->srec_mesh == mesh) return DEM_OK;
+  if (c->capturing) return c->fail(DEM_ERR_STATE, "list records missing inside a graph capture");
+  DEM_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+  free_records_f32(c);
+  c->gen++;  // captured kernels hold the old buffer
+  uint64_t budget = c->srec_budget;
+  if (!budget) {
+    size_t left = 0, total = 0;
+    DEM_CUDA_TRY(c, cudaMemGetInfo(&left, &total));
+    budget = left / 16;
+  }
+  for (int k = record_plan(c->pcap, mesh, budget); k < 3; k++) {
+    const uint32_t n = REC_PLANS[k][0], m = REC_PLANS[k][1];
+    if (cudaMalloc(&c->srec, c->pcap * (n + m) * sizeof(uint4)) == cudaSuccess) {
+      c->srec_n = n;
+      c->srec_m = m;
+      c->srec_cap = c->pcap;
+      c->srec_mesh = mesh;
+      return DEM_OK;
+    }
+    cudaGetLastError();
+    c->srec = nullptr;
+  }
+  return c->fail(DEM_ERR_OOM, "list records: device allocation failed");
 }
 
 int launch_count_sphere(dem_ctx* c) {
@@ -1343,3 +1392,24 @@ int launch_reverse_lists(dem_ctx* c, bool counted) {
 // whether launch_fill_sphere counts the partner lists itself
 bool fill_counts_partners(const dem_ctx* c) { return c->prm.fp32_broad_phase && !c->cell_broad_phase; }
 }  // namespace dem
+
+extern "C" int dem_selftest_record_plan(uint64_t particles, int mesh, uint64_t budget, uint32_t* records) {
+  if (!records) return DEM_ERR_INVALID_ARG;
+  const int k = dem::record_plan(particles, mesh != 0, budget);
+  records[0] = dem::REC_PLANS[k][0];
+  records[1] = dem::REC_PLANS[k][1];
+  return DEM_OK;
+}
+
+extern "C" int dem_selftest_records(dem_ctx* c, uint64_t budget, uint32_t* records) {
+  if (!c || !records) return DEM_ERR_INVALID_ARG;
+  records[0] = c->srec_n;
+  records[1] = c->srec_m;
+  if (budget) {
+    DEM_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    c->srec_budget = budget;
+    dem::free_records_f32(c);
+    c->gen++;
+  }
+  return DEM_OK;
+}

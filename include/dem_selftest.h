@@ -6,6 +6,7 @@
 #ifndef DEM_SELFTEST_H
 #define DEM_SELFTEST_H
 #include <stdint.h>
+#include "dem_hotpath.h"
 #ifdef __cplusplus
 extern "C" {
 #endif
@@ -42,6 +43,14 @@ int dem_selftest_rolling_clip(uint64_t n, uint64_t seed, uint64_t* mismatches, u
  * that dem_set_particles and dem_get_particles (on_device = 1) copy them with
  * their own kernel; what does not goes through cudaMemcpyAsync.             */
 int dem_selftest_copy_range(const void* p, uint64_t bytes, int* inside);
+
+/* The candidate records a particle of the FP32 sphere list build gets where
+ * they may take `budget` bytes in all: records[0] for particles and walls,
+ * records[1] for mesh features.  dem_selftest_records returns those that the
+ * context holds now; budget > 0 drops them and bounds the following builds'
+ * (0: no change; a context starts with a sixteenth of the free memory).     */
+int dem_selftest_record_plan(uint64_t particles, int mesh, uint64_t budget, uint32_t* records);
+int dem_selftest_records(dem_ctx* ctx, uint64_t budget, uint32_t* records);
 
 #ifdef __cplusplus
 }
