@@ -253,6 +253,7 @@ def declare_library(lib) -> None:
     _sig(lib, "dem_selftest_copy_range", [C.c_void_p, C.c_uint64, C.POINTER(C.c_int)])
     _sig(lib, "dem_selftest_record_plan", [C.c_uint64, C.c_int, C.c_uint64, C.POINTER(C.c_uint32)])
     _sig(lib, "dem_selftest_records", [_CTX, C.c_uint64, C.POINTER(C.c_uint32)])
+    _sig(lib, "dem_selftest_integration_mode", [_CTX, C.POINTER(C.c_int)])
 
 
 # Symbols declared in include/dem_hotpath.h, dem_selftest.h and dem_learned.h (the product library).
@@ -265,7 +266,8 @@ EXPORTED = ["dem_ctx_create", "dem_ctx_destroy", "dem_last_error", "dem_ctx_stre
             "dem_rebuild_count", "dem_interaction_count", "dem_get_interactions", "dem_set_interactions", "dem_packing_profile",
             "dem_profile", "dem_kernel_stats", "dem_reset_kernel_stats",
             "dem_simulation_state_noalloc", "dem_selftest_division", "dem_selftest_poly_decisions", "dem_selftest_emu_mul", "dem_selftest_rolling_clip", "dem_selftest_copy_range",
-            "dem_selftest_record_plan", "dem_selftest_records", "dem_set_shapes", "dem_compute_vertices",
+            "dem_selftest_record_plan", "dem_selftest_records",
+            "dem_selftest_integration_mode", "dem_set_shapes", "dem_compute_vertices",
             "dem_contact_polyhedron", "dem_vertex_displ_over", "dem_set_systems", "dem_system_count",
             "dem_simulation_state_systems", "dem_set_graph_capacity", "dem_autotune", "dem_set_mul_mode", "dem_get_mul_mode", "dem_set_multimat", "dem_set_analysis", "dem_get_contact_state", "dem_stress_tensor", "dem_mlp_harvest",
             "dem_mlp_init", "dem_mlp_set_params", "dem_mlp_get_params", "dem_mlp_forward", "dem_mlp_loss_grad",

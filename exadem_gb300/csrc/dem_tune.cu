@@ -21,7 +21,9 @@
 #include <cstring>
 #include <vector>
 
+#include "../../include/dem_selftest.h"
 #include "dem_ctx.cuh"
+#include "step_core.cuh"
 
 namespace dem {
 int ext_update_neighbors(dem_ctx* c);
@@ -162,18 +164,9 @@ struct Timer {
 
 using namespace dem;
 
-extern "C" int dem_autotune(dem_ctx* c, int steps_per_trial, int skin_policy, dem_tune_result* out) {
-  if (!c || !out || steps_per_trial < 1 || skin_policy < 0 || skin_policy > 2) return DEM_ERR_INVALID_ARG;
-  if (c->poly) return c->fail(DEM_ERR_UNSUPPORTED, "the autotuner covers the fused sphere step");
-  if (!c->prm.fused_step) return c->fail(DEM_ERR_STATE, "the autotuner tunes the fused step (fused_step = 1)");
-  if (!c->n) return c->fail(DEM_ERR_STATE, "no particles");
+// the trials, with the profile and the graph step off; a state saved in base is the caller's to free
+static int tune(dem_ctx* c, int steps_per_trial, int skin_policy, dem_tune_result* out, Saved& base) {
   int rc;
-  if (!c->have_list && (rc = ext_update_neighbors(c))) return rc;
-  const bool prof = c->prof_on;
-  c->prof_on = false;
-  const int graph = c->prm.graph_step;
-  c->prm.graph_step = 0;  // trials run the host-launched fused step (same kernels)
-
   // fastest particle: rebuild period of each skin
   unsigned int* d_v = nullptr;
   DEM_CUDA_TRY(c, cudaMalloc(&d_v, sizeof(unsigned int)));
@@ -187,7 +180,6 @@ extern "C" int dem_autotune(dem_ctx* c, int steps_per_trial, int skin_policy, de
   std::memcpy(&vmax, &vbits, sizeof(vmax));
   const double dt = c->prm.dt;
 
-  Saved base;
   if ((rc = save_state(c, base))) return rc;
   const double skin0 = c->prm.rcut_inc;
   const double nd0 = 2 * c->rad_max;
@@ -238,7 +230,9 @@ extern "C" int dem_autotune(dem_ctx* c, int steps_per_trial, int skin_policy, de
 
   double best = 1e300, before = 0;
   double best_skin = skin0, best_cell = c->prm.cell_size;
-  const int mode0 = c->mul_mode;
+  // what the integration runs now, so that the first trial times the context as it is
+  const bool auto0 = c->mul_auto;
+  const int mode0 = integ_mode(c), own_mode = c->mul_mode;
   c->mul_auto = false;  // every trial runs the mode it names
   if ((rc = trial(skin0, c->prm.cell_size, c->tune_block, c->tune_contact_bps, mode0, &before))) return rc;
   best = before;
@@ -298,13 +292,15 @@ extern "C" int dem_autotune(dem_ctx* c, int steps_per_trial, int skin_policy, de
   // tried: on GB300 its emulated additions made the contact kernel slower at every
   // share measured, 2/8 to 8/8)
   const int best_share = c->tune_int_share;
-  cudaFree(base.dev);
 
   // apply: launch shapes and cell size keep the current list (they take effect at the
   // next rebuild); a new skin rebuilds now (no effect on any result without cohesion)
   c->tune_block = best_block;
   c->tune_contact_bps = best_bps;
-  c->mul_mode = best_mode;
+  // where the rule by particle count already gave the fastest mode, the rule stays: other
+  // particles may follow
+  c->mul_auto = auto0 && best_mode == mode0;
+  c->mul_mode = c->mul_auto ? own_mode : best_mode;
   c->fuse_contact = best_fuse;
   c->tune_int_share = best_share;
   const bool skin_changed = best_skin != skin0;
@@ -312,9 +308,6 @@ extern "C" int dem_autotune(dem_ctx* c, int steps_per_trial, int skin_policy, de
   c->prm.rcut_inc = best_skin;
   if ((rc = ext_setup_grid(c))) return rc;
   if (skin_changed && (rc = ext_update_neighbors(c))) return rc;  // the list of the new skin
-  c->prm.graph_step = graph;
-  c->prof_on = prof;
-  c->gen++;
   out->rcut_inc = best_skin;
   out->cell_size = best_cell;
   out->block = best_block;
@@ -326,5 +319,37 @@ extern "C" int dem_autotune(dem_ctx* c, int steps_per_trial, int skin_policy, de
   out->mul_mode = best_mode;
   out->fused_contact = best_fuse ? 1 : 0;
   out->contact_int_share = best_share;
+  return DEM_OK;
+}
+
+extern "C" int dem_autotune(dem_ctx* c, int steps_per_trial, int skin_policy, dem_tune_result* out) {
+  if (!c || !out || steps_per_trial < 1 || skin_policy < 0 || skin_policy > 2) return DEM_ERR_INVALID_ARG;
+  if (c->poly) return c->fail(DEM_ERR_UNSUPPORTED, "the autotuner covers the fused sphere step");
+  if (!c->prm.fused_step) return c->fail(DEM_ERR_STATE, "the autotuner tunes the fused step (fused_step = 1)");
+  if (!c->n) return c->fail(DEM_ERR_STATE, "no particles");
+  int rc;
+  if (!c->have_list && (rc = ext_update_neighbors(c))) return rc;
+  const bool prof = c->prof_on, mul_auto = c->mul_auto;
+  const int graph = c->prm.graph_step;
+  c->prof_on = false;
+  c->prm.graph_step = 0;  // trials run the host-launched fused step (same kernels)
+  Saved base;
+  rc = tune(c, steps_per_trial, skin_policy, out, base);
+  if (rc) {  // a trial failed (a skin too wide for a periodic axis, no memory): as before the call
+    const std::string why = c->last_err;
+    if (base.dev) restore_state(c, base);
+    c->mul_auto = mul_auto;
+    c->last_err = why;
+  }
+  cudaFree(base.dev);
+  c->prm.graph_step = graph;
+  c->prof_on = prof;
+  c->gen++;
+  return rc;
+}
+
+extern "C" int dem_selftest_integration_mode(const dem_ctx* c, int* mode) {
+  if (!c || !mode) return DEM_ERR_INVALID_ARG;
+  *mode = integ_mode(c);
   return DEM_OK;
 }

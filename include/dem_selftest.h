@@ -52,6 +52,10 @@ int dem_selftest_copy_range(const void* p, uint64_t bytes, int* inside);
 int dem_selftest_record_plan(uint64_t particles, int mesh, uint64_t budget, uint32_t* records);
 int dem_selftest_records(dem_ctx* ctx, uint64_t budget, uint32_t* records);
 
+/* The multiply placement that the integration of the present particles runs:
+ * that of dem_set_mul_mode or dem_autotune, else the rule by particle count. */
+int dem_selftest_integration_mode(const dem_ctx* ctx, int* mode);
+
 #ifdef __cplusplus
 }
 #endif
