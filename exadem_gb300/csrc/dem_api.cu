@@ -232,6 +232,7 @@ static int make_grid(dem_ctx* c, const double* lo, const double* hi, const int32
     g.csf[d] = (float)g.csz[d];
     g.icsz[d] = (float)(1.0 / g.csz[d]);
     g.cmaxf = std::max(g.cmaxf, g.csf[d]);
+    g.lo1 += std::fabs(g.lof[d]);
     if (d < 2 && g.dims[d] > 1) {
       uint32_t l = 0;
       while ((1ull << l) < (uint64_t)g.dims[d]) l++;
@@ -956,7 +957,7 @@ static int add_driver(dem_ctx* c, const DriverDev& d) {
       h.cf[k] = (float)d.center[k];
     }
     h.rf = (float)d.radius;
-    h.n1 = sum(d.normal);
+    h.n1 = sum(d.kind == 1 ? d.axis : d.normal);
     h.cp1 = sum(d.center_proj);
     h.c1 = sum(d.center);
   }

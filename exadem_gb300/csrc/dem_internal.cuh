@@ -133,6 +133,7 @@ struct DriverDev {
   double offset, radius;
   double normal[3], center[3], center_proj[3], axis[3], vel[3], vrot[3];
   // FP32 roundings and magnitude sums for the sphere list's first test (driver_far)
+  // (n1: of the normal, for a cylinder of the axis)
   float nf[3], cpf[3], af[3], cf[3], rf, n1, cp1, c1;
 };
 
@@ -169,9 +170,9 @@ struct GridDev {
   double csz[3];
   int periodic[3];
   double L[3];
-  // FP32 roundings of lo, csz, 1 / csz and the largest csz, and the multipliers and
+  // FP32 roundings of lo, csz, 1 / csz, the largest csz and |lo|_1, and the multipliers and
   // shifts that divide a cell index by dims[0] and dims[1] (cell_coords)
-  float lof[3], csf[3], icsz[3], cmaxf;
+  float lof[3], csf[3], icsz[3], cmaxf, lo1;
   uint32_t dmul[2], dshift[2];
 };
 // x, y, z of cell c < 2^31 of the grid: exact quotients by a multiplication
