@@ -55,13 +55,13 @@ PARTICLE_BYTES_PER_STEP = 344
 PREROLL = {"spheres": 3000, "polyhedra": 0, "polyhedra_dense": 0, "drums": 0, "mixer": 300, "polyhedra_mesh": 0,
            "fragments": 0}
 # DRAM bytes (read + write) per launch of k_cfused per listed pair and of
-# the integration (epilog) per particle, from the ncu capture of the pre-rolled 250k-sphere
+# the epilog half of k_integrate per particle, from the ncu capture of the pre-rolled 250k-sphere
 # bed (the same workload at 1/8 of its size); they scale with the listed pairs and
 # the particles.  Both kernels run their FP64 pipe at the fraction recorded here
 # (sm__pipe_fp64_cycles_active of peak sustained).
-TRAFFIC = {"source": "profiles/k_cfused_fp64_lanes_spheres_bed_250k.md",
-           "contact_bytes_per_listed_pair": 212.0, "epilog_bytes_per_particle": 445.0,
-           "contact_fp64_pipe_active": 0.807, "epilog_fp64_pipe_active": 0.820}
+TRAFFIC = {"source": "profiles/counters_cases.md",
+           "contact_bytes_per_listed_pair": 209.0, "epilog_bytes_per_particle": 442.0,
+           "contact_fp64_pipe_active": 0.799, "epilog_fp64_pipe_active": 0.758}
 
 
 def parse():
@@ -96,7 +96,7 @@ def parse():
                     help="eighths of the fused contact tiles whose law runs on the integer pipe (no effect on "
                          "results; default: the autotuner's choice)")
     ap.add_argument("--cell-broad-phase", action="store_true",
-                    help="spheres: the warp-per-cell staged broad phase instead of thread per owner "
+                    help="spheres: the warp-per-cell staged broad phase instead of pairs met once "
                          "(same lists)")
     ap.add_argument("--learned", action="store_true",
                     help="polyhedra: harvest candidate pairs, train the MLP, time with learned sizing "
@@ -667,7 +667,7 @@ def run_native(args, rank, world, local, dist):
                 "algorithmic_bytes_per_unit": CONTACT_BYTES_PER_INTERACTION, "avg_launch_ms": t_law * 1e3,
                 "share_of_step": shares.get("contact", 0.0),
                 "traffic_source": TRAFFIC["source"] if fused_contact else None,
-                "traffic_scaling": ("212 B per listed pair measured at 250k spheres (826k listed pairs), "
+                "traffic_scaling": ("209 B per listed pair measured at 250k spheres (831k listed pairs), "
                                     "times the listed pairs here") if fused_contact else None,
                 "fp64_pipe_active": TRAFFIC["contact_fp64_pipe_active"] if fused_contact else None,
                 "note": "FP64-pipe bound, not HBM bound: the FP64 pipe runs at the fp64_pipe_active fraction of "
@@ -676,7 +676,7 @@ def run_native(args, rank, world, local, dist):
     achieved_i = PARTICLE_BYTES_PER_STEP * w.n / t_integ / 1e9 if t_integ > 0 else 0.0
     t_e = TRAFFIC["epilog_bytes_per_particle"]
     roofline_integration = {
-        "bound": "hbm", "kernel": "integration (k_integrate + k_rotations)",
+        "bound": "hbm", "kernel": "integration (k_integrate, epilog and prolog halves)",
         "achieved": achieved_i, "peak": peak, "unit": "GB/s", "frac": achieved_i / peak, "peak_kind": peak_kind,
         "epilog_traffic": (t_e * w.n if fused_contact else None),
         "algorithmic_bytes_per_launch": PARTICLE_BYTES_PER_STEP * w.n,

@@ -89,7 +89,7 @@ __device__ __forceinline__ void bond_law(double dn, V3 n, double dn0, double wei
   Et = emu_mulhalf(kt_w) * dot(tds, tds);
 }
 
-// Bound by the FP64 pipe (83 % busy).  16 k cubes, 154 k bonds: 52 us with the damping's
+// Bound by the FP64 pipe (81 % busy).  16 k cubes, 154 k bonds: 52 us with the damping's
 // division and square root and the two energies' conversion here, 45 without.
 __global__ void __launch_bounds__(BT) k_bond_force(BondArgs a) {
   if (a.step && *a.flag != 0ull && *a.flag <= a.step) return;

@@ -239,8 +239,10 @@ __device__ __forceinline__ bool halted(const unsigned long long* flag, unsigned 
 
 // The polyhedron step's integration: the epilog of step g.step, then the prolog and the
 // trigger of the next (k_integrate's form).  A particle whose epilog rotation is put
-// off has its prolog put off too.  Bound by the FP64 pipe (200 k falling
-// polyhedra 26 us a step; 100 steps with a kernel of listed rotations besides 5.98 ms, 5.51 without), by one particle's FP64 chain below a warp a scheduler (1.5 k: 17).
+// off has its prolog put off too.  Bound by the FP64 pipe and by the latency of its loads
+// (200 k falling polyhedra 24 us a step, the pipe 41 % busy; 100 steps with a kernel of
+// listed rotations besides 5.98 ms, 5.51 without), by one particle's FP64 chain below a
+// warp a scheduler (1.5 k: 17 us).
 template <int Mode>
 __global__ void __launch_bounds__(256, (Mode ? 3 : 1)) k_poly_integrate(PolyArgs a, IntegArgs g, float thr) {
   if (g.step && halted(g.scal, g.step)) return;
@@ -1431,17 +1433,19 @@ __global__ void __launch_bounds__(PT, 4) k_feat_dec(FeatArgs a) {
 
 // ---- flattened FP32-decided enumeration (count pass without learned sizing)
 // The tests of k_feat_dec, spread over the whole GPU instead of a warp per unit:
-//   k_feat_prep   one warp per unit: the vertex gates and the near-feature
+//   k_feat_prep   half a warp per unit: the vertex gates and the near-feature
 //                 filters of k_feat_dec, kept as bit masks (UnitRec), and the
 //                 test count of each of the six segments;
 //   scan          over the (segment, unit) test counts, segment-major: the test
 //                 index space is (segment, unit, row, column);
+//   k_feat_words  the (segment, unit) group of every 32nd test;
 //   k_feat_test   32 consecutive tests per warp: every lane of a warp runs the
 //                 same decision (one segment) on its own test, so the FP32
 //                 arithmetic is dense and the kernel small; one kept-bit per test;
-//   k_feat_collect one warp per unit: the kept bits of its six segments, in
-//                 segment order, give its count (and its types), or in the fill
-//                 pass its features in the order k_feat writes them.
+//   k_feat_collect a thread per unit: the kept bits of its six segments give its
+//                 count, its types and its groups' counts;
+//   k_feat_fill_flat a thread per kept test, in the order k_feat writes them;
+//   k_feat_drivers the units with a driver, in both passes.
 // The decisions and the FP64 fallback are those of dec_segment, so the list is
 // the same bit for bit.
 struct UnitRec {
@@ -2063,18 +2067,6 @@ __device__ __forceinline__ void pwrite(const PCArgs& a, uint64_t k, V3 ft, V3 mo
   a.R.tj[2][k] = tj.z;
 }
 
-__device__ __forceinline__ uint32_t warp_append2(bool want, unsigned long long* counter) {
-  const unsigned mask = __ballot_sync(0xffffffffu, want);
-  const int lane = threadIdx.x & 31;
-  unsigned long long base = 0;
-  if (mask) {
-    const int leader = __ffs(mask) - 1;
-    if (lane == leader) base = atomicAdd(counter, (unsigned long long)__popc(mask));
-    base = __shfl_sync(0xffffffffu, base, leader);
-  }
-  return (uint32_t)base + (uint32_t)__popc(mask & ((1u << lane) - 1u));
-}
-
 // Roles of an interaction in the contact law: i = pi_, j = pj_ (swap exchanges owner and partner).
 struct Roles {
   uint32_t ip, jp, sub_i, sub_j;
@@ -2138,7 +2130,7 @@ __global__ void k_pscreen(PCArgs a) {
   }
 #pragma unroll
   for (int q = 0; q < PK; q++) {
-    const uint32_t pos = warp_append2(kind == q, a.cnt + q);
+    const uint32_t pos = warp_append(kind == q, a.cnt + q);
     if (kind == q) a.list[q][pos] = (uint32_t)k;
   }
 }

@@ -5,14 +5,15 @@
 // this file, and neither changes a single result bit:
 //  * lanes that need no FP64 work must not share a warp with lanes that do:
 //    a warp instruction with one active lane costs the FP64 pipe as much as a
-//    full one.  The contact law therefore runs in three passes:
+//    full one.  The contact law therefore runs over compacted lists:
 //      k_cscreen  one thread per interaction; an FP32 test proves most pairs
 //                 apart (history reset, zero record, no FP64 at all); the others
 //                 are appended to list L1 with warp-aggregated atomics;
-//      k_cdetect  dense over L1: FP64 detection; no contact -> reset; cohesive
-//                 attraction without overlap (cheap branch) finished here;
-//                 overlapping pairs append (k, dn, n, cp) to list L2;
-//      k_chooke   dense over L2: the full Hooke law with friction and rolling.
+//      k_cfused   dense over L1: FP64 detection; no contact -> reset; the pairs
+//                 that overlap and those that attract wait in two queues in
+//                 shared memory and run their law in full tiles;
+//      or, as the autotuner may choose, k_cdetect over L1 and k_chooke over its
+//      list L2 of the overlapping pairs.
 //  * the divisions by mass and inertia use exact reciprocal-based division
 //    (math_exact.cuh) and reset + gravity + gather + force_to_accel + epilog,
 //    with the next step's prolog + displacement trigger, are one kernel.

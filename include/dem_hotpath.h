@@ -95,7 +95,10 @@ typedef struct dem_params {
    *                   where undecided;
    * fp32_contact_screen: FP32 test that skips the FP64 contact law (spheres)
    *                   or detection (polyhedra, fused step) for pairs that are
-   *                   provably apart.                                      */
+   *                   provably apart.
+   * Decided in FP32 without a switch, each with a margin of its rounding error
+   * inside which FP64 decides: the cell of a particle at a rebuild, and with
+   * fused_step the displacement trigger.                                    */
   int32_t fp32_broad_phase;
   int32_t fp32_contact_screen;
   /* fused_step: dem_step runs the fused kernels (prolog + displacement test,
@@ -386,8 +389,9 @@ int dem_autotune(dem_ctx* ctx, int steps_per_trial, int skin_policy, dem_tune_re
  * rotations and derivative, normalisation, Euler terms) on the integer pipe;
  * bit 1: the other multiplies (Verlet pushes, quotient estimates); bit 2:
  * the sphere contact law's multiplies.  0 = FP64 pipe only.  Results are
- * identical in every mode (0..7).  Default 2; the autotuner picks the fastest
- * for the sphere step.                                                     */
+ * identical in every mode (0..7).  Default 2, and 0 while the particles give a
+ * scheduler at most one warp; the autotuner picks the fastest for the sphere
+ * step.                                                                     */
 int dem_set_mul_mode(dem_ctx* ctx, int mode);
 int dem_get_mul_mode(dem_ctx* ctx, int* mode);
 /* Share (0..8, in eighths) of the fused contact kernel's tiles of overlapping
@@ -401,13 +405,14 @@ int dem_get_mul_mode(dem_ctx* ctx, int* mode);
 int dem_set_contact_int_share(dem_ctx* ctx, int eighths);
 /* Sphere broad phase with fp32_broad_phase (replaces the particle-pair part of
  * nbh_sphere, src/sphere/nbh_sphere.cu:64-309, as the default kernels do):
- * 0 = one thread per owner particle (default); 1 = one warp per cell, the
+ * 0 = each pair met once, from the particle whose cell comes first, two lanes
+ * a particle (default); 1 = one warp per cell, the
  * 27-cell neighbourhood's FP32 coordinates, radii and ids staged in shared
  * memory, candidates compacted with warp ballots, drivers tested per particle.
  * The lists are identical in both modes.  Measured on GB300 (2 M sphere bed,
  * about 35 particles per neighbourhood): mode 1 runs the count and fill passes
- * slower, since a warp per cell leaves lanes idle where a thread per owner keeps
- * all 32 busy and L1 already serves the stencil reuse. */
+ * slower, since a warp per cell leaves lanes idle where a thread per owner (and
+ * the default more so) keeps all 32 busy and L1 already serves the stencil reuse. */
 int dem_set_sphere_cell_broad_phase(dem_ctx* ctx, int on);
 /* Number of neighbour rebuilds done so far (trigger_move_particles count). */
 int dem_rebuild_count(dem_ctx* ctx, uint64_t* out);

@@ -1,7 +1,7 @@
 """Mesh candidates of spheres on the GPU against the oracle's lists: the bins' items
-dealt to the lanes of a warp eight spheres at a time, two mesh drivers, a vertex where
+of 32 spheres dealt to the threads of a block, two mesh drivers, a vertex where
 48 triangles meet (spheres with more candidates than a record holds), numbers of
-spheres that leave lanes and warps partly empty, the mesh far from the origin, both
+spheres that leave threads and blocks partly empty, the mesh far from the origin, both
 list builds of the FP32 broad phase and the FP64 one."""
 import numpy as np
 import pytest
